@@ -30,12 +30,19 @@ extern "C" {
                                 rank, rounded up to 4, 8, 16, 32 or 64, is at most a quarter of E rounded up to
                                 a multiple of 32 (M2D_ERR_SHAPE otherwise; the models use R = E/16) */
 
+/*
+ * M2D_PROJ_PARAMS_F32: WT, WL, bT, bL and the gradients d_WT, d_WL, d_bT, d_bL, d_Wx are FP32 arrays
+ * whatever `dtype` is.  The parameters are rounded to `dtype` before use (what a caller's cast would do)
+ * and the gradients leave the fp32 accumulators unrounded: no cast launches around a bf16 call.
+ */
+#define M2D_PROJ_PARAMS_F32 1
+
 typedef struct m2d_proj_desc {
     uint32_t struct_bytes;     /* = sizeof(m2d_proj_desc) */
-    int32_t dtype;             /* m2d_dtype of every tensor below */
+    int32_t dtype;             /* m2d_dtype of every tensor below (but see flags) */
     int64_t P;                 /* pixels = B*H*W; P * max(E, proj_pitch) must stay below 2^31 - 2^26 (M2D_ERR_TOO_LARGE) */
     int32_t E, R, N;           /* channels, dt rank, state size; K = 2R+3N columns are in use */
-    int32_t reserved0;
+    int32_t flags;             /* 0 or M2D_PROJ_* bits */
     int64_t proj_pitch;        /* row pitch, in elements, of proj and d_proj (>= K) */
     const void *x;             /* (P,E)      scan input                              [wgrad] */
     const void *proj;          /* (P,pitch)  x-projection output                     [fwd, bwd] */

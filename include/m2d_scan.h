@@ -33,7 +33,7 @@
 extern "C" {
 #endif
 
-#define M2D_ABI_VERSION 3
+#define M2D_ABI_VERSION 4
 
 typedef enum m2d_dtype {
     M2D_F32 = 0,   /* float in memory, float arithmetic */
@@ -90,6 +90,18 @@ typedef enum m2d_status {
 #define M2D_SCAN_A_LOG 4u
 
 /*
+ * M2D_SCAN_D_F32: desc->D and desc->d_D are FP32 arrays whatever `dtype` is (D is rounded to `dtype`
+ * before use, as the reference's cast of the parameter does): no cast launches around a bf16 call.
+ */
+#define M2D_SCAN_D_F32 0x10u
+
+/*
+ * M2D_SCAN_BC_ZEROED (backward, FP32): d_BT, d_BL and d_C are zero already.  For callers that hand over
+ * columns of a wider buffer: clearing the whole buffer in one pass is faster than clearing its columns.
+ */
+#define M2D_SCAN_BC_ZEROED 0x20u
+
+/*
  * M2D_SCAN_TEST_WITHHOLD: test hook, rejected with M2D_ERR_FLAGS unless the environment variable
  * M2D_TEST_HOOKS is 1.  In a launch that runs several CTAs per image, the CTA that owns the first
  * band of image 0 never publishes that band's column counter and every wait gives up after a few
@@ -110,7 +122,9 @@ typedef enum m2d_status {
  *                                       H*W*pitch).  The reference produces these as views into
  *                                       one projection output with pitch 2R+3N
  *                                       (wavefront_cuda.py:78-82); a contiguous tensor has pitch N.
- *   d_BT, d_BL, d_C                     (B,H,W,N) contiguous
+ *   d_BT, d_BL, d_C                     (B,H,W,N) with unit stride over N and a pixel pitch in elements,
+ *                                       the same for all three (0: contiguous, i.e. N), so that they can
+ *                                       be columns of the gradient of one projection output
  * All tensors share `dtype`.
  */
 typedef struct m2d_scan_desc {
@@ -126,6 +140,7 @@ typedef struct m2d_scan_desc {
     void *y;                    /* forward output */
     const void *gy;             /* backward input: upstream gradient of y */
     void *d_x, *d_dT, *d_dL, *d_AT, *d_AL, *d_BT, *d_BL, *d_C, *d_D;   /* backward outputs */
+    int64_t d_BC_pitch;         /* pixel pitch of d_BT, d_BL, d_C in elements; 0 = N */
     void *workspace;            /* scratch, 256-byte aligned, see *_workspace() */
     uint64_t workspace_bytes;
 } m2d_scan_desc;
@@ -167,6 +182,14 @@ int64_t m2d_scan_fwd_status_offset(const m2d_scan_desc *desc);
 int64_t m2d_scan_bwd_status_offset(const m2d_scan_desc *desc);   /* same, for m2d_scan_bwd's workspace */
 int m2d_scan_fwd_chain(const m2d_scan_desc *desc);
 int m2d_scan_bwd_chain(const m2d_scan_desc *desc);
+
+/*
+ * 1 if a wait between CTAs has given up in any launch of this process since the last call of this
+ * function, else 0; does not synchronise.  (The kernel that gives up writes to host memory, so a failure
+ * shows here as soon as it has happened; the status word of the launch's own workspace says which one
+ * it was.)  Launches made under M2D_SCAN_TEST_WITHHOLD do not count.
+ */
+int m2d_take_wait_failure(void);
 
 /*
  * The rule every launch applies when it picks, or has to shorten, the number of CTAs per image:

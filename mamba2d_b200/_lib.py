@@ -7,19 +7,23 @@ import ctypes
 import os
 
 HERE = os.path.dirname(os.path.abspath(__file__))
-LIB_PATH = os.environ.get("M2D_SCAN_LIB", os.path.join(HERE, "libm2d_scan.so"))   # override: an alternative build of the same ABI
+DEFAULT_LIB_PATH = os.path.join(HERE, "libm2d_scan.so")
+LIB_PATH = os.environ.get("M2D_SCAN_LIB", DEFAULT_LIB_PATH)   # override: an alternative build of the same ABI
 
 M2D_F32, M2D_BF16 = 0, 1
 M2D_SCAN_REVERSE = 1
 M2D_SCAN_GELU_OUT = 2
 M2D_SCAN_A_LOG = 4
+M2D_SCAN_D_F32 = 0x10
+M2D_SCAN_BC_ZEROED = 0x20
 M2D_SCAN_TEST_WITHHOLD = 0x100
-ABI_VERSION = 3
+M2D_PROJ_PARAMS_F32 = 1
+ABI_VERSION = 4
 NOALLOC_SCRATCH_BYTES = 32 << 20     # M2D_NOALLOC_SCRATCH_BYTES in include/m2d_scan.h
 
 EXPORTS = ("m2d_abi_version", "m2d_strerror", "m2d_scan_fwd_workspace", "m2d_scan_bwd_workspace",
            "m2d_scan_fwd", "m2d_scan_bwd", "m2d_scan_fwd_noalloc", "m2d_scan_fwd_noalloc_need", "m2d_scan_fwd_status_offset",
-           "m2d_scan_bwd_status_offset", "m2d_scan_fwd_chain", "m2d_scan_bwd_chain", "m2d_scan_chain_bound",
+           "m2d_scan_bwd_status_offset", "m2d_scan_fwd_chain", "m2d_scan_bwd_chain", "m2d_scan_chain_bound", "m2d_take_wait_failure",
            "m2d_proj_workspace", "m2d_dtproj_fwd", "m2d_dtproj_bwd", "m2d_xproj_wgrad",
            "m2d_xproj_wgrad_on_tensor_cores")
 PROJ_MAX_E, PROJ_MAX_R = 640, 64     # M2D_PROJ_MAX_E / M2D_PROJ_MAX_R in include/m2d_proj.h
@@ -39,6 +43,7 @@ class ScanDesc(ctypes.Structure):
         ("d_x", ctypes.c_void_p), ("d_dT", ctypes.c_void_p), ("d_dL", ctypes.c_void_p),
         ("d_AT", ctypes.c_void_p), ("d_AL", ctypes.c_void_p),
         ("d_BT", ctypes.c_void_p), ("d_BL", ctypes.c_void_p), ("d_C", ctypes.c_void_p), ("d_D", ctypes.c_void_p),
+        ("d_BC_pitch", ctypes.c_int64),
         ("workspace", ctypes.c_void_p), ("workspace_bytes", ctypes.c_uint64),
     ]
 
@@ -47,7 +52,7 @@ class ProjDesc(ctypes.Structure):
     """Mirror of ``m2d_proj_desc``."""
     _fields_ = [
         ("struct_bytes", ctypes.c_uint32), ("dtype", ctypes.c_int32), ("P", ctypes.c_int64),
-        ("E", ctypes.c_int32), ("R", ctypes.c_int32), ("N", ctypes.c_int32), ("reserved0", ctypes.c_int32),
+        ("E", ctypes.c_int32), ("R", ctypes.c_int32), ("N", ctypes.c_int32), ("flags", ctypes.c_int32),
         ("proj_pitch", ctypes.c_int64),
         ("x", ctypes.c_void_p), ("proj", ctypes.c_void_p), ("WT", ctypes.c_void_p), ("WL", ctypes.c_void_p),
         ("bT", ctypes.c_void_p), ("bL", ctypes.c_void_p), ("dT", ctypes.c_void_p), ("dL", ctypes.c_void_p),
@@ -106,3 +111,20 @@ def strerror(code):
 def check(code, what):
     if code != 0:
         raise RuntimeError(f"{what}: {strerror(code)} (status {code})")
+
+
+_ENTRY = None
+
+
+def entry():
+    """The native eager entry points (csrc/torch_entry.cpp), loaded once; raises if they are not built."""
+    global _ENTRY
+    if _ENTRY is None:
+        lib()                                   # the library first: same checks, same message
+        import importlib
+        try:
+            _ENTRY = importlib.import_module("mamba2d_b200._entry")
+        except ImportError as exc:
+            raise RuntimeError(f"the native entry points are not built or do not load ({exc}); "
+                               "run `python -m mamba2d_b200.build`") from exc
+    return _ENTRY

@@ -14,6 +14,7 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 INCLUDE = os.path.join(os.path.dirname(HERE), "include")
 OUT = os.path.join(HERE, "libm2d_scan.so")
+ENTRY = os.path.join(HERE, "_entry.so")  # native eager entry points (Python extension)
 OBJ = os.path.join(HERE, "_obj")          # per-source objects (git-ignored, not shipped)
 SOURCES = ["m2d_abi.cu", "m2d_scan_fwd.cu", "m2d_scan_bwd.cu", "m2d_scan_fwd_noalloc.cu", "m2d_proj.cu"]
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
@@ -43,7 +44,40 @@ def _compile(nvcc, src, obj):
     return " ".join(cmd) + "\n" + res.stdout, res.returncode
 
 
+def build_entry(force=False):
+    """The native eager entry points (torch_entry.cpp): a Python extension linked against the library."""
+    src = os.path.join(CSRC, "torch_entry.cpp")
+    deps = [src, OUT] + [os.path.join(INCLUDE, f) for f in os.listdir(INCLUDE) if f.endswith(".h")]
+    if not force and os.path.exists(ENTRY) and os.path.getmtime(ENTRY) >= max(os.path.getmtime(d) for d in deps):
+        return ENTRY
+    import sysconfig
+    import torch
+    from torch.utils.cpp_extension import include_paths, library_paths
+    cuda = os.path.dirname(os.path.dirname(os.path.realpath(_nvcc())))
+    cmd = ["/usr/bin/g++" if os.path.exists("/usr/bin/g++") else "g++", "-O2", "-std=c++17", "-fPIC", "-shared",
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", "-DTORCH_API_INCLUDE_EXTENSION_H",
+           "-DTORCH_EXTENSION_NAME=_entry", "-I", INCLUDE, "-isystem", sysconfig.get_paths()["include"]]
+    for d in include_paths() + [os.path.join(cuda, "include")]:
+        cmd += ["-isystem", d]
+    cmd += [src, "-o", ENTRY]
+    for d in library_paths() + [os.path.join(cuda, "lib64")]:
+        cmd += ["-L", d]
+    cmd += ["-L", HERE, "-l:libm2d_scan.so", "-Wl,-rpath,$ORIGIN", "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_cuda", "-ltorch",
+            "-ltorch_python", "-lcudart"]
+    res = subprocess.run(cmd, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
+    if res.returncode != 0:
+        raise RuntimeError("building torch_entry.cpp failed:\n" + res.stdout)
+    return ENTRY
+
+
 def build(force=False, verbose=False):
+    """Everything: the C-ABI library, then the native entry points on top of it."""
+    out = build_library(force, verbose)
+    build_entry(force)
+    return out
+
+
+def build_library(force=False, verbose=False):
     """Compile every source to an object (in parallel, only the stale ones) and link the library."""
     from concurrent.futures import ThreadPoolExecutor
     srcs = [os.path.join(CSRC, s) for s in SOURCES if os.path.exists(os.path.join(CSRC, s))]

@@ -6,6 +6,10 @@
 
 namespace m2d {
 
+// Host-memory word (mapped into every device) that a kernel sets when one of its waits gives up; nullptr
+// if it cannot be had (no device, or first asked for during a stream capture).  Defined in m2d_abi.cu.
+int* wait_failure_flag();
+
 // Everything of the argument block that comes straight from the descriptor and the plan.
 inline void fill_common_args(ScanArgs& a, const m2d_scan_desc* d, const Plan& pl) {
     a = ScanArgs{};
@@ -18,9 +22,11 @@ inline void fill_common_args(ScanArgs& a, const m2d_scan_desc* d, const Plan& pl
     a.chain = pl.chain;
     a.act = (d->flags & M2D_SCAN_GELU_OUT) ? 1 : 0;
     a.a_log = (d->flags & M2D_SCAN_A_LOG) ? 1 : 0;
+    a.d_f32 = (d->flags & M2D_SCAN_D_F32) || d->dtype == M2D_F32 ? 1 : 0;
     const bool hook = (d->flags & M2D_SCAN_TEST_WITHHOLD) != 0;
     a.withhold = hook ? 1 : 0;
     a.wait_limit = hook ? (1 << 9) : kWaitPolls;
+    a.host_flag = pl.chain > 1 && !hook ? wait_failure_flag() : nullptr;
 }
 
 // Launch a sweep kernel on the plan's grid.  CTAs of a chain wait on one another, so every CTA of a
@@ -30,14 +36,10 @@ inline void fill_common_args(ScanArgs& a, const m2d_scan_desc* d, const Plan& pl
 // the same bound as a planned one (bound_chain).
 inline int launch_sweep_kernel(void (*kern)(const ScanArgs), ScanArgs& a, const Plan& pl, int steps_per_row, cudaStream_t st) {
     dim3 block(pl.warps * 32);
-    if (pl.smem > 48 * 1024 &&
-        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pl.smem) != cudaSuccess)
-        return M2D_ERR_LAUNCH;
+    if (!allow_smem(reinterpret_cast<const void*>(kern), pl.smem)) return M2D_ERR_LAUNCH;
     if (a.chain > 1) {
-        cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
-        int per_sm = 0;
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, (int)block.x, pl.smem) != cudaSuccess || per_sm < 1)
-            return M2D_ERR_LAUNCH;
+        const int per_sm = resident_ctas(reinterpret_cast<const void*>(kern), (int)block.x, pl.smem);
+        if (per_sm < 1) return M2D_ERR_LAUNCH;
         const long long fit = (long long)per_sm * sm_count() / ((long long)pl.grid_x * pl.groups);
         if (fit < a.chain) a.chain = bound_chain(fit, pl.nbands, steps_per_row, pl.Rb);
         for (;;) {

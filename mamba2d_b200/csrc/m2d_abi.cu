@@ -1,5 +1,34 @@
-// C-ABI housekeeping: version and status strings.
-#include "m2d_scan.h"
+// C-ABI housekeeping: version, status strings and the process-wide flag of failed waits.
+#include "launch.cuh"
+
+namespace m2d {
+
+int* wait_failure_flag() {
+    static std::mutex m;
+    static int* flag = nullptr;
+    std::lock_guard<std::mutex> lock(m);
+    if (!flag && device_index() >= 0) {
+        // (an allocation is not part of anything that may be under capture on this thread)
+        cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+        cudaThreadExchangeStreamCaptureMode(&mode);
+        void* p = nullptr;
+        if (cudaHostAlloc(&p, sizeof(int), cudaHostAllocPortable | cudaHostAllocMapped) == cudaSuccess) {
+            flag = static_cast<int*>(p);
+            *flag = 0;
+        } else {
+            cudaGetLastError();
+        }
+        cudaThreadExchangeStreamCaptureMode(&mode);
+    }
+    return flag;
+}
+
+}  // namespace m2d
+
+extern "C" int m2d_take_wait_failure(void) {
+    int* f = m2d::wait_failure_flag();
+    return f ? __atomic_exchange_n(f, 0, __ATOMIC_RELAXED) != 0 : 0;
+}
 
 extern "C" int m2d_abi_version(void) { return M2D_ABI_VERSION; }
 

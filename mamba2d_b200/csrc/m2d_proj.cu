@@ -30,6 +30,7 @@ struct ProjPlan {
 struct ProjArgs {
     int P, pitch, ntiles;              // every element index fits 31 bits (checked on the host)
     int E, R, EB, PS, TP;
+    int params_f32;                    // weights and biases are fp32, rounded to io_t when read
     int wide16;                        // bf16 backward: rows and pointers allow 16-byte copies
     const void *proj, *WT, *WL, *bT, *bL;
     void *dT, *dL;
@@ -49,6 +50,7 @@ static int check_proj(const m2d_proj_desc* d) {
     if (!d) return M2D_ERR_NULL;
     if (d->struct_bytes != sizeof(m2d_proj_desc)) return M2D_ERR_ABI;
     if (d->dtype != M2D_F32 && d->dtype != M2D_BF16) return M2D_ERR_DTYPE;
+    if (d->flags & ~M2D_PROJ_PARAMS_F32) return M2D_ERR_FLAGS;
     if (d->P < 1 || d->E < 1 || d->R < 1 || d->N < 1) return M2D_ERR_SHAPE;
     if (d->E > M2D_PROJ_MAX_E || d->R > M2D_PROJ_MAX_R) return M2D_ERR_TOO_LARGE;
     if (d->proj_pitch < 2ll * d->R + 3ll * d->N) return M2D_ERR_PITCH;
@@ -89,6 +91,14 @@ static ProjPlan plan_proj(const m2d_proj_desc* d) {
     return p;
 }
 
+// Element of a weight or bias: of the I/O type, or fp32 rounded to it.
+template <typename io_t>
+__device__ __forceinline__ float load_param(const void* p, int off, int f32) {
+    if (!f32) return load1(static_cast<const io_t*>(p), off);
+    const float v = __ldg(static_cast<const float*>(p) + off);
+    return sizeof(io_t) == 2 ? __bfloat162float(__float2bfloat16_rn(v)) : v;
+}
+
 // softplus with the reference's threshold of 20 (torch.nn.functional.softplus defaults)
 // log1p(t) for t in (0, 1] as 2*atanh(t / (2 + t)): the argument stays below 1/3, where seven terms of
 // the series are exact to fp32 rounding (next term 2 s^15 / 15 < 1e-8 of the result); half the
@@ -125,16 +135,16 @@ __global__ void __launch_bounds__(MAXT) dtproj_fwd_kernel(const ProjArgs a) {
     const int dir = blockIdx.y;
     const int te = threadIdx.x % a.EB, ps = threadIdx.x / a.EB;
     const bool e_ok = te < a.E;
-    const io_t* W = static_cast<const io_t*>(dir ? a.WL : a.WT);
-    const io_t* bias = static_cast<const io_t*>(dir ? a.bL : a.bT);
+    const void* W = dir ? a.WL : a.WT;
+    const void* bias = dir ? a.bL : a.bT;
     const io_t* proj = static_cast<const io_t*>(a.proj);
     io_t* out = static_cast<io_t*>(dir ? a.dL : a.dT);
     const int col0 = dir * a.R;
 
     float w[RB];
 #pragma unroll
-    for (int r = 0; r < RB; ++r) w[r] = (e_ok && r < a.R) ? load1(W, te * a.R + r) : 0.f;
-    const float b = e_ok ? load1(bias, te) : 0.f;
+    for (int r = 0; r < RB; ++r) w[r] = (e_ok && r < a.R) ? load_param<io_t>(W, te * a.R + r, a.params_f32) : 0.f;
+    const float b = e_ok ? load_param<io_t>(bias, te, a.params_f32) : 0.f;
 
     // The rank-R rows of the next tile are fetched into registers while this tile is computed
     // (TP*RB <= 2*blockDim is guaranteed by the host: two values per thread at most).
@@ -206,7 +216,7 @@ __global__ void __launch_bounds__(MAXT) dtproj_bwd_kernel(const ProjArgs a) {
     const int lane = threadIdx.x & 31;
     const int te = threadIdx.x % a.EB, ps = threadIdx.x / a.EB;
     const bool e_ok = te < a.E;
-    const io_t* W = static_cast<const io_t*>(dir ? a.WL : a.WT);
+    const void* W = dir ? a.WL : a.WT;
     const io_t* proj = static_cast<const io_t*>(a.proj);
     const io_t* delta = static_cast<const io_t*>(dir ? a.dL : a.dT);
     const io_t* g = static_cast<const io_t*>(dir ? a.g_dL : a.g_dT);
@@ -226,7 +236,7 @@ __global__ void __launch_bounds__(MAXT) dtproj_bwd_kernel(const ProjArgs a) {
 #pragma unroll
         for (int e = 0; e < 32; ++e) {
             const int r = h * RL + rl, ch = e_slice + e;
-            wreg[h][e] = (ch < a.E && r < a.R) ? load1(W, ch * a.R + r) : 0.f;
+            wreg[h][e] = (ch < a.E && r < a.R) ? load_param<io_t>(W, ch * a.R + r, a.params_f32) : 0.f;
         }
 
     float acc[RB];
@@ -367,9 +377,9 @@ __global__ void __launch_bounds__(MAXT) dtproj_bwd_kernel(const ProjArgs a) {
 
 // d_W[e][r] (r < R) and d_b[e] (r == RB) = sum over CTAs of the partials.  Block (32, 8): 32
 // neighbouring results, the CTAs dealt round-robin to the 8 rows of the block.
-template <typename io_t>
+template <typename g_t>
 __global__ void dtproj_bwd_finalize(const float* __restrict__ partials, int ctas, int RB, int EB, int E, int R,
-                                    io_t* d_WT, io_t* d_WL, io_t* d_bT, io_t* d_bL) {
+                                    g_t* d_WT, g_t* d_WL, g_t* d_bT, g_t* d_bL) {
     __shared__ float red[8][33];
     const int n = 2 * (RB + 1) * EB;
     const int idx = blockIdx.x * 32 + threadIdx.x;
@@ -512,6 +522,7 @@ static ProjArgs proj_args(const m2d_proj_desc* d, const ProjPlan& p) {
     a.proj = d->proj; a.WT = d->WT; a.WL = d->WL; a.bT = d->bT; a.bL = d->bL;
     a.dT = d->dT; a.dL = d->dL; a.g_dT = d->g_dT; a.g_dL = d->g_dL;
     a.d_proj = d->d_proj;
+    a.params_f32 = (d->flags & M2D_PROJ_PARAMS_F32) ? 1 : 0;
     a.partials = static_cast<float*>(d->workspace);
     a.wide16 = d->E % 8 == 0 && aligned(d->g_dT, 16) && aligned(d->g_dL, 16) && aligned(d->dT, 16) && aligned(d->dL, 16);
     return a;
@@ -523,11 +534,8 @@ static ProjArgs proj_args(const m2d_proj_desc* d, const ProjPlan& p) {
 // spent waiting for the fuller ones).  Never more than the plan's gx, which sized the workspace.
 template <typename K>
 static int balanced_gx(K kern, const ProjPlan& p, size_t smem) {
-    int per_sm = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, p.threads, smem) != cudaSuccess || per_sm < 1) {
-        cudaGetLastError();
-        return p.gx;
-    }
+    const int per_sm = resident_ctas(reinterpret_cast<const void*>(kern), p.threads, smem);
+    if (per_sm < 1) return p.gx;
     const int gx = per_sm * sm_count() / 2;
     return gx < 1 ? 1 : (gx < p.gx ? gx : p.gx);
 }
@@ -554,15 +562,18 @@ static int launch_dt_bwd(const m2d_proj_desc* d, const ProjArgs& a, const ProjPl
                 : p.threads <= 384 ? dtproj_bwd_kernel<io_t, RB, 384>
                 : p.threads <= 512 ? dtproj_bwd_kernel<io_t, RB, 512>
                                    : dtproj_bwd_kernel<io_t, RB, M2D_PROJ_MAX_E>;
-    if (smem > 48 * 1024 && cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
-        return M2D_ERR_LAUNCH;
+    if (!allow_smem(reinterpret_cast<const void*>(kern), smem)) return M2D_ERR_LAUNCH;
     const int gx = balanced_gx(kern, p, smem);
     kern<<<dim3(gx, 2), p.threads, smem, st>>>(a);
     if (cudaGetLastError() != cudaSuccess) return M2D_ERR_LAUNCH;
     const int n = 2 * (RB + 1) * p.EB;
-    dtproj_bwd_finalize<io_t><<<(n + 31) / 32, dim3(32, 8), 0, st>>>(a.partials, gx, RB, p.EB, d->E, d->R,
-                                                             static_cast<io_t*>(d->d_WT), static_cast<io_t*>(d->d_WL),
-                                                             static_cast<io_t*>(d->d_bT), static_cast<io_t*>(d->d_bL));
+    auto finalize = [&](auto out) {                // element type of the parameters' gradients
+        typedef decltype(out) g_t;
+        dtproj_bwd_finalize<g_t><<<(n + 31) / 32, dim3(32, 8), 0, st>>>(a.partials, gx, RB, p.EB, d->E, d->R, static_cast<g_t*>(d->d_WT),
+                                                                static_cast<g_t*>(d->d_WL), static_cast<g_t*>(d->d_bT), static_cast<g_t*>(d->d_bL));
+    };
+    if (a.params_f32) finalize(float{});
+    else finalize(io_t{});
     return cudaGetLastError() == cudaSuccess ? M2D_OK : M2D_ERR_LAUNCH;
 }
 
@@ -579,6 +590,14 @@ static int dispatch_dt(const m2d_proj_desc* d, bool bwd, cudaStream_t st) {
     }
 }
 
+template <typename io_t>
+static void launch_wgrad_finalize(const m2d_proj_desc* d, const float* partials, int slabs, long long ke, cudaStream_t st) {
+    const dim3 block(32, 8);
+    const int grid = (int)((ke + 31) / 32);
+    if (d->flags & M2D_PROJ_PARAMS_F32) xproj_wgrad_finalize<float><<<grid, block, 0, st>>>(partials, slabs, ke, static_cast<float*>(d->d_Wx));
+    else xproj_wgrad_finalize<io_t><<<grid, block, 0, st>>>(partials, slabs, ke, static_cast<io_t*>(d->d_Wx));
+}
+
 // bf16 operands: the tensor-core kernel, when the problem meets its alignment rules (otherwise, and for
 // fp32, whose 1e-4 bar rules out tf32 operands, the CUDA-core kernel below).  Returns -1 for "not taken".
 static int launch_wgrad_tc(const m2d_proj_desc* d, const ProjPlan& p, cudaStream_t st) {
@@ -591,11 +610,11 @@ static int launch_wgrad_tc(const m2d_proj_desc* d, const ProjPlan& p, cudaStream
     a.partials = static_cast<float*>(d->workspace);
     a.status = reinterpret_cast<int*>(static_cast<char*>(d->workspace) + p.wg_partials - 256);
     if (cudaMemsetAsync(a.status, 0, sizeof(int), st) != cudaSuccess) return M2D_ERR_LAUNCH;
-    if (cudaFuncSetAttribute(xproj_wgrad_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)t.smem) != cudaSuccess) return M2D_ERR_LAUNCH;
+    if (!allow_smem(reinterpret_cast<const void*>(xproj_wgrad_tc_kernel), t.smem)) return M2D_ERR_LAUNCH;
     xproj_wgrad_tc_kernel<<<dim3(t.grid_x, t.ny), 128, t.smem, st>>>(map_a, map_b, a);
     if (cudaGetLastError() != cudaSuccess) return M2D_ERR_LAUNCH;
     const long long ke = (long long)p.K * d->E;
-    xproj_wgrad_finalize<__nv_bfloat16><<<(int)((ke + 31) / 32), dim3(32, 8), 0, st>>>(a.partials, t.grid_x, ke, static_cast<__nv_bfloat16*>(d->d_Wx));
+    launch_wgrad_finalize<__nv_bfloat16>(d, a.partials, t.grid_x, ke, st);
     return cudaGetLastError() == cudaSuccess ? M2D_OK : M2D_ERR_LAUNCH;
 }
 
@@ -613,7 +632,7 @@ static int launch_wgrad(const m2d_proj_desc* d, cudaStream_t st) {
     xproj_wgrad_kernel<io_t><<<dim3(p.slabs, p.tilesE, p.tilesK), 256, 0, st>>>(a);
     if (cudaGetLastError() != cudaSuccess) return M2D_ERR_LAUNCH;
     const long long ke = (long long)p.K * d->E;
-    xproj_wgrad_finalize<io_t><<<(int)((ke + 31) / 32), dim3(32, 8), 0, st>>>(a.partials, p.slabs, ke, static_cast<io_t*>(d->d_Wx));
+    launch_wgrad_finalize<io_t>(d, a.partials, p.slabs, ke, st);
     return cudaGetLastError() == cudaSuccess ? M2D_OK : M2D_ERR_LAUNCH;
 }
 

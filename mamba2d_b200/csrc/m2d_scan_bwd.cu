@@ -96,7 +96,7 @@ __global__ void __launch_bounds__(M2D_BWD_MAXW * 32, 2) m2d_bwd_chained_kernel(c
     for (int k = threadIdx.x; k < total; k += blockDim.x) handoff[k] = make_float4(0.f, 0.f, 0.f, 0.f);
 
     const int ch_own = g * kGroup + lane;
-    const float D_own = ch_own < a.E ? load1(static_cast<const io_t*>(a.D), ch_own) : 0.f;
+    const float D_own = ch_own < a.E ? load_D<io_t>(a, ch_own) : 0.f;
     float dAT[4][4], dAL[4][4], dD[4];
 #pragma unroll
     for (int c = 0; c < 4; ++c) {
@@ -182,7 +182,7 @@ __global__ void __launch_bounds__(M2D_BWD_MAXW * 32, M2D_BWD_MINB) m2d_bwd_kerne
     for (int k = threadIdx.x; k < total; k += blockDim.x) smem[k] = make_float4(0.f, 0.f, 0.f, 0.f);
 
     const int ch_own = g * kGroup + lane;
-    const float D_own = ch_own < a.E ? load1(static_cast<const io_t*>(a.D), ch_own) : 0.f;
+    const float D_own = ch_own < a.E ? load_D<io_t>(a, ch_own) : 0.f;
     float dAT[4][4], dAL[4][4], dD[4];
 #pragma unroll
     for (int c = 0; c < 4; ++c) {
@@ -253,13 +253,14 @@ __global__ void __launch_bounds__(M2D_BWD_MAXW * 32, M2D_BWD_MINB) m2d_bwd_kerne
 // they are gradients of the fp32 parameter A_log).
 template <typename io_t>
 __global__ void m2d_bwd_finalize(const float* __restrict__ acc, io_t* d_BT, io_t* d_BL, io_t* d_C, void* d_AT, void* d_AL,
-                                 io_t* d_D, long long npn, long long en, int E, int a_log) {
+                                 void* d_D, long long npn, int N, int pitch, long long en, int E, int a_log, int d_f32) {
     const long long tid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     const long long nthreads = (long long)gridDim.x * blockDim.x;
     for (long long k = tid; k < npn; k += nthreads) {
-        store1(d_BT, k, acc[k]);
-        store1(d_BL, k, acc[npn + k]);
-        store1(d_C, k, acc[2 * npn + k]);
+        const long long at = pitch == N ? k : k / N * pitch + k % N;
+        store1(d_BT, at, acc[k]);
+        store1(d_BL, at, acc[npn + k]);
+        store1(d_C, at, acc[2 * npn + k]);
     }
     const float* accA = acc + 3 * npn;
     for (long long k = tid; k < en; k += nthreads) {
@@ -271,7 +272,18 @@ __global__ void m2d_bwd_finalize(const float* __restrict__ acc, io_t* d_BT, io_t
             store1(static_cast<io_t*>(d_AL), k, accA[en + k]);
         }
     }
-    for (long long k = tid; k < E; k += nthreads) store1(d_D, k, accA[2 * en + k]);
+    for (long long k = tid; k < E; k += nthreads) {
+        if (d_f32) static_cast<float*>(d_D)[k] = accA[2 * en + k];
+        else store1(static_cast<io_t*>(d_D), k, accA[2 * en + k]);
+    }
+}
+
+// Zero the columns of a wider buffer that d_BT, d_BL and d_C are: one pass when they are neighbours.
+static bool zero_columns(const ScanArgs& a, const m2d_scan_desc* d, cudaStream_t st) {
+    const size_t rows = (size_t)d->B * d->H * d->W, pitch = (size_t)a.acc_pitch * 4, width = (size_t)d->N * 4;
+    if (a.accBL == a.accBT + d->N && a.accC == a.accBL + d->N) return cudaMemset2DAsync(a.accBT, pitch, 0, 3 * width, rows, st) == cudaSuccess;
+    return cudaMemset2DAsync(a.accBT, pitch, 0, width, rows, st) == cudaSuccess && cudaMemset2DAsync(a.accBL, pitch, 0, width, rows, st) == cudaSuccess &&
+           cudaMemset2DAsync(a.accC, pitch, 0, width, rows, st) == cudaSuccess;
 }
 
 template <typename io_t>
@@ -295,18 +307,20 @@ static int launch_bwd(const m2d_scan_desc* d, const Plan& pl, bool vec, cudaStre
     a.d_x = d->d_x; a.d_dT = d->d_dT; a.d_dL = d->d_dL;
     const size_t npn = (size_t)d->B * d->H * d->W * d->N, en = (size_t)d->E * d->N;
     if (d->dtype == M2D_F32) {
+        a.acc_pitch = d->d_BC_pitch ? (int)d->d_BC_pitch : d->N;
         a.accBT = static_cast<float*>(d->d_BT); a.accBL = static_cast<float*>(d->d_BL); a.accC = static_cast<float*>(d->d_C);
         a.accAT = static_cast<float*>(d->d_AT); a.accAL = static_cast<float*>(d->d_AL); a.accD = static_cast<float*>(d->d_D);
         // the six accumulated outputs start from zero; a caller that carved the three per-pixel ones
         // out of one buffer and the three per-channel ones out of another, in this order, gets two
         // memsets instead of six (they are 3 us each against a 200 us kernel at the smallest stage)
-        const bool big_adjacent = a.accBL == a.accBT + npn && a.accC == a.accBL + npn;
+        const bool pitched = a.acc_pitch != d->N;
+        const bool big_adjacent = !pitched && a.accBL == a.accBT + npn && a.accC == a.accBL + npn;
         const bool small_adjacent = a.accAL == a.accAT + en && a.accD == a.accAL + en;
         bool ok;
-        if (big_adjacent && a.accAT == a.accC + npn && small_adjacent) {
+        if (big_adjacent && !(d->flags & M2D_SCAN_BC_ZEROED) && a.accAT == a.accC + npn && small_adjacent) {
             ok = cudaMemsetAsync(a.accBT, 0, (3 * npn + 2 * en + (size_t)d->E) * 4, st) == cudaSuccess;
         } else {
-            ok = big_adjacent ? cudaMemsetAsync(a.accBT, 0, 3 * npn * 4, st) == cudaSuccess
+            ok = (d->flags & M2D_SCAN_BC_ZEROED) ? true : pitched ? zero_columns(a, d, st) : big_adjacent ? cudaMemsetAsync(a.accBT, 0, 3 * npn * 4, st) == cudaSuccess
                               : (cudaMemsetAsync(a.accBT, 0, npn * 4, st) == cudaSuccess && cudaMemsetAsync(a.accBL, 0, npn * 4, st) == cudaSuccess &&
                                  cudaMemsetAsync(a.accC, 0, npn * 4, st) == cudaSuccess);
             ok = ok && (small_adjacent ? cudaMemsetAsync(a.accAT, 0, (2 * en + (size_t)d->E) * 4, st) == cudaSuccess
@@ -316,6 +330,7 @@ static int launch_bwd(const m2d_scan_desc* d, const Plan& pl, bool vec, cudaStre
         if (!ok) return M2D_ERR_LAUNCH;
     } else {
         float* acc = reinterpret_cast<float*>(ws + L.acc);
+        a.acc_pitch = d->N;
         a.accBT = acc; a.accBL = acc + npn; a.accC = acc + 2 * npn;
         a.accAT = acc + 3 * npn; a.accAL = a.accAT + en; a.accD = a.accAL + en;
         if (cudaMemsetAsync(acc, 0, L.acc_bytes, st) != cudaSuccess) return M2D_ERR_LAUNCH;
@@ -328,8 +343,8 @@ static int launch_bwd(const m2d_scan_desc* d, const Plan& pl, bool vec, cudaStre
     if (d->dtype != M2D_F32) {
         const int fin_blocks = (int)((npn + 255) / 256 < 148 * 8 ? (npn + 255) / 256 : 148 * 8);
         m2d_bwd_finalize<io_t><<<fin_blocks, 256, 0, st>>>(a.accBT, static_cast<io_t*>(d->d_BT), static_cast<io_t*>(d->d_BL),
-                                                          static_cast<io_t*>(d->d_C), d->d_AT, d->d_AL, static_cast<io_t*>(d->d_D),
-                                                          (long long)npn, (long long)en, d->E, a.a_log);
+                                                          static_cast<io_t*>(d->d_C), d->d_AT, d->d_AL, d->d_D,
+                                                          (long long)npn, d->N, d->d_BC_pitch ? (int)d->d_BC_pitch : d->N, (long long)en, d->E, a.a_log, a.d_f32);
         if (cudaGetLastError() != cudaSuccess) return M2D_ERR_LAUNCH;
     }
     return M2D_OK;

@@ -20,7 +20,7 @@ __global__ void __launch_bounds__(256, 2) m2d_fwd_chained_kernel(const FwdArgs a
     for (int k = threadIdx.x; k < total; k += blockDim.x) handoff[k] = make_float4(0.f, 0.f, 0.f, 0.f);
 
     const int ch_own = g * kGroup + lane;
-    const float D_own = ch_own < a.E ? load1(static_cast<const io_t*>(a.D), ch_own) : 0.f;
+    const float D_own = ch_own < a.E ? load_D<io_t>(a, ch_own) : 0.f;
     __syncthreads();
     float4* const params = reinterpret_cast<float4*>(reinterpret_cast<char*>(handoff) + sweep_smem_bytes((blockDim.x >> 5), CB));
     if (threadIdx.x < 32) stage_params<io_t>(params, a.AT, a.AL, a.N, ch0, chv, n0, nv, lane, a.a_log);
@@ -47,7 +47,7 @@ __global__ void __launch_bounds__(256, 2) m2d_fwd_kernel(const FwdArgs a) {
     const int total = (int)(rows_fwd_smem_bytes(nwarps) / sizeof(float4));
     for (int k = threadIdx.x; k < total; k += blockDim.x) smem[k] = make_float4(0.f, 0.f, 0.f, 0.f);
     const int ch_own = g * kGroup + lane;
-    const float D_own = ch_own < a.E ? load1(static_cast<const io_t*>(a.D), ch_own) : 0.f;
+    const float D_own = ch_own < a.E ? load_D<io_t>(a, ch_own) : 0.f;
     __syncthreads();
     float4* const params = reinterpret_cast<float4*>(reinterpret_cast<char*>(smem) + rows_fwd_smem_bytes(nwarps));
     if (threadIdx.x < 32) stage_params<io_t>(params, a.AT, a.AL, a.N, ch0, chv, n0, nv, lane, a.a_log);

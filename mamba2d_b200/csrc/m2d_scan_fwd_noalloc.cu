@@ -33,7 +33,6 @@ namespace m2d {
 // it must go through cudaGetSymbolAddress before a kernel can be given a pointer to it.
 static __device__ __align__(256) unsigned char g_noalloc_ring[M2D_NOALLOC_SCRATCH_BYTES];
 
-constexpr int kMaxDevices = 64;
 static std::mutex g_ring_mutex;
 static float4* g_ring_ptr[kMaxDevices] = {};   // device address of g_noalloc_ring on each device
 
@@ -69,7 +68,7 @@ __global__ void __launch_bounds__(256, 2) m2d_fwd_noalloc_kernel(const ScanArgs 
     const int total = (int)(bytes / sizeof(float4));
     for (int k = threadIdx.x; k < total; k += blockDim.x) smem[k] = make_float4(0.f, 0.f, 0.f, 0.f);
     const int ch_own = g * kGroup + lane;
-    const float D_own = ch_own < a.E ? load1(static_cast<const io_t*>(a.D), ch_own) : 0.f;
+    const float D_own = ch_own < a.E ? load_D<io_t>(a, ch_own) : 0.f;
     __syncthreads();
     float4* const params = reinterpret_cast<float4*>(reinterpret_cast<char*>(smem) + bytes);
     if (threadIdx.x < 32) stage_params<io_t>(params, a.AT, a.AL, a.N, ch0, chv, n0, nv, lane, a.a_log);

@@ -1,18 +1,70 @@
 // Host-side descriptor validation and launch planning (header-only, used by both entry points).
 #pragma once
 
+#include <array>
+#include <atomic>
 #include <cstdlib>
+#include <mutex>
+#include <unordered_map>
 
 #include "common.cuh"
 
 namespace m2d {
 
+constexpr int kMaxDevices = 64;
+
+// Index of the current device for the per-device caches below, or -1 (no device, or one beyond the caches).
+inline int device_index() {
+    int dev = -1;
+    if (cudaGetDevice(&dev) != cudaSuccess) { cudaGetLastError(); return -1; }
+    return dev < kMaxDevices ? dev : -1;
+}
+
+// SMs of the current device, asked for once per device (plans are made several times per call).
 inline int sm_count() {
-    int dev = 0, n = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) {
+    static std::atomic<int> cache[kMaxDevices];
+    const int dev = device_index();
+    int n = dev >= 0 ? cache[dev].load(std::memory_order_relaxed) : 0;
+    if (n > 0) return n;
+    if (dev < 0 || cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) {
         cudaGetLastError();   // clear; planning still works on a machine without a device
-        n = 148;
+        return 148;
     }
+    cache[dev].store(n, std::memory_order_relaxed);
+    return n;
+}
+
+// Per (kernel, device): the dynamic shared memory it has been allowed, and its resident CTAs per SM for the
+// last (block size, shared memory) asked about.  The runtime calls behind both cost a microsecond or more
+// each, as much as a launch; they are made once.
+struct KernelFacts {
+    size_t smem_allowed = 48 * 1024;
+    int block = 0, per_sm = 0;
+    size_t smem = 0;
+};
+inline KernelFacts& kernel_facts(const void* kern, std::unique_lock<std::mutex>& lock) {
+    static std::mutex m;
+    static std::unordered_map<const void*, std::array<KernelFacts, kMaxDevices>> all;
+    lock = std::unique_lock<std::mutex>(m);
+    const int dev = device_index();
+    return all[kern][dev < 0 ? 0 : dev];
+}
+inline bool allow_smem(const void* kern, size_t smem) {
+    std::unique_lock<std::mutex> lock;
+    KernelFacts& f = kernel_facts(kern, lock);
+    if (smem <= f.smem_allowed) return true;
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) { cudaGetLastError(); return false; }
+    f.smem_allowed = smem;
+    return true;
+}
+// Resident CTAs per SM (0: the query failed).
+inline int resident_ctas(const void* kern, int block, size_t smem) {
+    std::unique_lock<std::mutex> lock;
+    KernelFacts& f = kernel_facts(kern, lock);
+    if (f.block == block && f.smem == smem) return f.per_sm;
+    int n = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kern, block, smem) != cudaSuccess) { cudaGetLastError(); return 0; }
+    f.block = block; f.smem = smem; f.per_sm = n;
     return n;
 }
 
@@ -27,8 +79,8 @@ inline int check_desc(const m2d_scan_desc* d, bool bwd, bool need_ptrs) {
     if (d->struct_bytes != sizeof(m2d_scan_desc)) return M2D_ERR_ABI;
     if (d->dtype != M2D_F32 && d->dtype != M2D_BF16) return M2D_ERR_DTYPE;
     {
-        unsigned known = M2D_SCAN_REVERSE | M2D_SCAN_A_LOG;
-        if (!bwd) known |= M2D_SCAN_GELU_OUT;      // an output activation exists in the forward only
+        unsigned known = M2D_SCAN_REVERSE | M2D_SCAN_A_LOG | M2D_SCAN_D_F32;
+        known |= bwd ? M2D_SCAN_BC_ZEROED : M2D_SCAN_GELU_OUT;      // an output activation exists in the forward only, gradients in the backward
         if (test_hooks_enabled()) known |= M2D_SCAN_TEST_WITHHOLD;
         if (d->flags & ~known) return M2D_ERR_FLAGS;
     }
@@ -38,11 +90,13 @@ inline int check_desc(const m2d_scan_desc* d, bool bwd, bool need_ptrs) {
     {
         // the kernels index every tensor with 31-bit element offsets
         long long widest = d->E > 48 ? d->E : 48;
+        if (bwd && d->d_BC_pitch > widest) widest = d->d_BC_pitch;
         if (d->BT_pitch > widest) widest = d->BT_pitch;
         if (d->BL_pitch > widest) widest = d->BL_pitch;
         if (d->C_pitch > widest) widest = d->C_pitch;
         if ((long long)d->B * d->H * d->W * widest >= (1ll << 31)) return M2D_ERR_TOO_LARGE;
     }
+    if (bwd && d->d_BC_pitch != 0 && d->d_BC_pitch < d->N) return M2D_ERR_PITCH;
     if (need_ptrs) {
         if (!d->x || !d->dT || !d->dL || !d->AT || !d->AL || !d->BT || !d->BL || !d->C || !d->D) return M2D_ERR_NULL;
         if (bwd && (!d->gy || !d->d_x || !d->d_dT || !d->d_dL || !d->d_AT || !d->d_AL || !d->d_BT || !d->d_BL || !d->d_C || !d->d_D))

@@ -147,7 +147,7 @@ __device__ __forceinline__ void reverse_sweep(const ScanArgs& a, float4* handoff
         }
         const int j = W - 1 - st.jl;
         if (chain > 1 && st.pull_l && st.seen < st.jl + 1)
-            st.seen = wait_columns(st.pcount, st.jl + 1, a.status, a.wait_limit);
+            st.seen = wait_columns(st.pcount, st.jl + 1, a);
         if (st.row_l) {
             char* stg = stage + par * kStageBytes;
             if (VEC) {
@@ -324,7 +324,7 @@ __device__ __forceinline__ void reverse_sweep(const ScanArgs& a, float4* handoff
                 float v = hi4 ? m1 : m0;
                 v += __shfl_xor_sync(0xffffffffu, hi4 ? m0 : m1, 4);
                 // this lane now owns array (hi16 ? d_BL : d_BT), state n0 + 2*hi8 + hi4
-                if (db_lane) atomicAdd(db_acc + ((long long)st.pixc * a.N + db_n), v);
+                if (db_lane) atomicAdd(db_acc + ((long long)st.pixc * a.acc_pitch + db_n), v);
             }
           };
             if (st.row0_c || j == 0) cell(std::false_type{});

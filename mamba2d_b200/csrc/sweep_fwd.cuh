@@ -43,17 +43,20 @@ struct ScanArgs {
     float4* bnd;              // [image][group][band][W][4][32] float4
     int* progress;            // [image][group][band]: columns of the band's last row published so far
     int* status;              // nonzero if a wait on `progress` gave up (results are then invalid); never null
+    int* host_flag;           // the same news in host memory, where the next call sees it without synchronising; may be null
     int wait_limit;           // polls before such a wait gives up
     int withhold;             // test hook: the first band of image 0 never publishes its column counter
     int act;                  // forward only: 1 = apply GELU (erf form) to y before it is stored
     int a_log;                // AT / AL hold the fp32 parameter A_log (A = -exp(A_log)); d_AT / d_AL are then fp32 d_A_log
+    int d_f32;                // D and d_D are fp32 whatever the I/O type
     // ---- backward only ----
     const void* gy;
     float4* hs;               // full state record: [b][group][H*W] blocks; a block is [4][32] float4 (fp32 I/O)
                               // or [2][32] uint4 holding 16 bf16 states per lane (bf16 I/O)
     // fp32 accumulators of the reduced gradients, zeroed before the kernel.  For fp32 I/O they are
     // the caller's gradient tensors themselves; for bf16 I/O they live in the workspace.
-    float *accBT, *accBL, *accC;   // [B*H*W][N]
+    float *accBT, *accBL, *accC;   // [B*H*W] rows of N values at a pitch of acc_pitch
+    int acc_pitch;
     float *accAT, *accAL;          // [E][N]
     float* accD;                   // [E]
     void *d_x, *d_dT, *d_dL;
@@ -88,6 +91,14 @@ __device__ __forceinline__ float load_A(const void* A, long long idx, int a_log,
     return v;
 }
 
+// D[e] as a float; an fp32 parameter is rounded to the I/O type the way the caller's cast would.
+template <typename io_t>
+__device__ __forceinline__ float load_D(const ScanArgs& a, int e) {
+    if (!a.d_f32) return load1(static_cast<const io_t*>(a.D), e);
+    const float v = __ldg(static_cast<const float*>(a.D) + e);
+    return sizeof(io_t) == 2 ? __bfloat162float(__float2bfloat16_rn(v)) : v;
+}
+
 template <typename io_t>
 __device__ __forceinline__ void stage_params(float4* dst, const void* AT, const void* AL, int N, int ch0, int chv, int n0, int nv, int lane,
                                              int a_log) {
@@ -118,12 +129,14 @@ struct CellIn {
 // returns a huge value (the caller then stops waiting for the rest of the row), so a kernel can
 // never spin forever.
 constexpr int kWaitPolls = 1 << 22;
-__device__ __forceinline__ int wait_columns(const int* counter, int need, int* status, int limit) {
+__device__ __forceinline__ int wait_columns(const int* counter, int need, const ScanArgs& a) {
+    int* const status = a.status;
     int seen = ld_acquire_gpu(counter);
     int polls = 0;
     while (seen < need) {
-        if (++polls > limit || *reinterpret_cast<volatile int*>(status) != 0) {
+        if (++polls > a.wait_limit || *reinterpret_cast<volatile int*>(status) != 0) {
             atomicExch(status, 1);
+            if (a.host_flag) *reinterpret_cast<volatile int*>(a.host_flag) = 1;
             return 0x7fffffff;
         }
         __nanosleep(64);
@@ -231,7 +244,7 @@ __device__ __forceinline__ void forward_sweep(const ScanArgs& a, float4* handoff
         const int col0 = st.jl * CB;
         if (chain > 1 && st.pull_l) {
             const int need = min(col0 + CB, W);
-            if (st.seen < need) st.seen = wait_columns(st.pcount, need, a.status, a.wait_limit);
+            if (st.seen < need) st.seen = wait_columns(st.pcount, need, a);
         }
         if (st.row_l) {
 #pragma unroll
@@ -393,7 +406,7 @@ __device__ __forceinline__ void forward_sweep(const ScanArgs& a, float4* handoff
                         float k = hi8 ? k1 : k0;
                         k += __shfl_xor_sync(0xffffffffu, hi8 ? k0 : k1, 8);
                         k += __shfl_xor_sync(0xffffffffu, k, 4);
-                        if (dc_lane) atomicAdd(a.accC + ((long long)st.pixc * a.N + dc_n), k);
+                        if (dc_lane) atomicAdd(a.accC + ((long long)st.pixc * a.acc_pitch + dc_n), k);
                         st.phs += HsBlock<io_t>::f4;
                     } else {
                         const float ysum = reduce_states(yacc[0], yacc[1], yacc[2], yacc[3], nq);

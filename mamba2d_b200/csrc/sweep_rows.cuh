@@ -271,7 +271,7 @@ __device__ __forceinline__ void forward_rows(const ScanArgs& a, float4* smem, co
             float k = hi8 ? k1 : k0;
             k += __shfl_xor_sync(0xffffffffu, hi8 ? k0 : k1, 8);
             k += __shfl_xor_sync(0xffffffffu, k, 4);
-            if (dc_lane) atomicAdd(a.accC + ((long long)(w.pix0 + dir * col) * a.N + dc_n), k);
+            if (dc_lane) atomicAdd(a.accC + ((long long)(w.pix0 + dir * col) * a.acc_pitch + dc_n), k);
         } else {
             const float ysum = reduce_states(yacc[0], yacc[1], yacc[2], yacc[3], nq);
             float yv = fmaf(sel4(vx, nq), D_own, ysum);
@@ -554,7 +554,7 @@ __device__ __forceinline__ void reverse_rows(const ScanArgs& a, float4* smem, co
           float v = hi4 ? m1 : m0;
           v += __shfl_xor_sync(0xffffffffu, hi4 ? m0 : m1, 4);
           // this lane now owns array (hi16 ? d_BL : d_BT), state n0 + 2*hi8 + hi4
-          if (db_lane) atomicAdd(db_acc + ((long long)pixc * a.N + db_n), v);
+          if (db_lane) atomicAdd(db_acc + ((long long)pixc * a.acc_pitch + db_n), v);
       }
           };
 

@@ -379,6 +379,7 @@ def _xproj_wgrad_fake(d_proj, x, d_state, dt_rank):
 _EAGER.update({scan_fwd_op: lambda *a: scan_fwd(*a[:10], False, *a[10:]),
                scan_bwd_op: lambda *a: list(scan_bwd(*a[:11], True, *a[11:])), dtproj_fwd_op: _dtproj_fwd,
                dtproj_bwd_op: _dtproj_bwd, xproj_wgrad_op: _xproj_wgrad})
+_EAGER_BODIES = dict(_EAGER)
 
 
 def _proj_forward(x, AT_log, AL_log, x_proj_w, dt_projT_w, dt_projT_b, dt_projL_w, dt_projL_b, want_A=True):
@@ -497,10 +498,32 @@ def proj_params(x, AT_log, AL_log, x_proj_w, dt_projT_w, dt_projT_b, dt_projL_w,
 # Autograd Functions
 # -----------------------------------------------------------------------------
 
+def _native(x):
+    """The native entry points (csrc/torch_entry.cpp) if an eager call on ``x`` may take them, else None.
+
+    They run the same kernels as the functions of this file without the Python, the parameter casts and
+    the copies around them.  Not taken: while a compiler traces, when every launch is to be checked
+    (M2D_CHECK_STATUS=1: the check synchronises), with another library in place of the package's own
+    (M2D_SCAN_LIB), and while an operator body in ``_EAGER`` is replaced."""
+    if (not x.is_cuda or torch.compiler.is_compiling() or _CHECK_STATUS == "1" or _lib.LIB_PATH != _lib.DEFAULT_LIB_PATH
+            or _EAGER != _EAGER_BODIES):
+        return None
+    return _lib.entry()
+
+
 class wf_cuda_fn_pr(torch.autograd.Function):
     """Partial recomputation: projections are computed once and saved; the hidden state is
     recomputed inside the backward kernel.  With ``a_log`` the ``AT`` / ``AL`` arguments are the fp32
     parameters A_log and their gradients are gradients with respect to A_log."""
+
+    @classmethod
+    def apply(cls, x, deltaT, deltaL, AT, AL, BT, BL, C, D, reverse=False, a_log=False):
+        native = _native(x)
+        if native is not None:
+            y = native.scan(x, deltaT, deltaL, AT, AL, BT, BL, C, D, bool(reverse), bool(a_log))
+            if y is not None:
+                return y
+        return super().apply(x, deltaT, deltaL, AT, AL, BT, BL, C, D, reverse, a_log)
 
     @staticmethod
     def forward(ctx, x, deltaT, deltaL, AT, AL, BT, BL, C, D, reverse=False, a_log=False):
@@ -572,15 +595,21 @@ def wavefront_scan_cuda(x, AT_log, AL_log, x_proj_w, dt_projT_w, dt_projT_b, dt_
     if H < 2 or W < 2:
         raise ValueError(f"Wavefront scan kernel requires spatial dims > 1. Got H={H}, W={W}.")
 
+    if recomp not in ("partial", "full"):
+        raise ValueError(f"Unknown recomputation mode, got {recomp}...")
+    native = _native(x)
+    if native is not None:
+        y = native.block(x, AT_log, AL_log, x_proj_w, dt_projT_w, dt_projT_b, dt_projL_w, dt_projL_b, D, recomp == "full",
+                         reverse, act_out == "gelu")
+        if y is not None:
+            return y
+
     x_proj_w = x_proj_w.to(x.dtype)
     dt_projT_w = dt_projT_w.to(x.dtype)
     dt_projT_b = dt_projT_b.to(x.dtype)
     dt_projL_w = dt_projL_w.to(x.dtype)
     dt_projL_b = dt_projL_b.to(x.dtype)
     D = D.to(x.dtype)
-
-    if recomp not in ("partial", "full"):
-        raise ValueError(f"Unknown recomputation mode, got {recomp}...")
     params = (x, AT_log, AL_log, x_proj_w, dt_projT_w, dt_projT_b, dt_projL_w, dt_projL_b, D)
     if act_out == "gelu" and not (torch.is_grad_enabled() and any(t.requires_grad for t in params)) \
             and not torch.compiler.is_compiling():
