@@ -222,10 +222,8 @@ int m2d_scan_bwd(const m2d_scan_desc *desc, void *stream);
  *   - The array is M2D_NOALLOC_SCRATCH_BYTES (32 MiB) and every GPU that loads the library keeps
  *     it until the process exits.
  *   - A problem needing more scratch than that returns M2D_ERR_TOO_LARGE before any device work.
- *     m2d_scan_fwd_noalloc_need() reports the need: a status word plus one ring of W slots of 2 KiB
- *     per CTA when the map has more rows than a CTA has row-warps (8), with at most two CTAs per SM.
- *     This entry always runs one CTA per (image, channel group), so its need can differ from what
- *     m2d_scan_fwd_workspace() reports for the same problem.
+ *     m2d_scan_fwd_noalloc_need() reports the need.  A problem that m2d_scan_fwd would split over
+ *     several CTAs per image runs with one where only that fits the array.
  *   - All calls on a device share the array.  The call clears the one word that must start at
  *     zero itself, but calls that overlap in time on one GPU race on the array: keep them on one
  *     stream or order them with events.

@@ -250,6 +250,7 @@ struct Plan {
     int cb;            // cells per step and warp (forward only)
     int chain;         // CTAs per chain (> 1 when there are far fewer images than SMs)
     bool rows;         // batch mode with the nested-loop kernel (its own shared-memory layout)
+    int wave;          // channels per lane of the wave kernel (several CTAs per image), or 0
     size_t smem;       // dynamic shared memory per CTA
     size_t scratch;    // workspace bytes
 };

@@ -10,6 +10,9 @@ namespace m2d {
 // if it cannot be had (no device, or first asked for during a stream capture).  Defined in m2d_abi.cu.
 int* wait_failure_flag();
 
+// Forward launch of a plan with its scratch (d->workspace is not looked at).  Defined in m2d_scan_fwd.cu.
+int launch_forward(const m2d_scan_desc* d, const Plan& pl, char* scratch, cudaStream_t st);
+
 // Everything of the argument block that comes straight from the descriptor and the plan.
 inline void fill_common_args(ScanArgs& a, const m2d_scan_desc* d, const Plan& pl) {
     a = ScanArgs{};

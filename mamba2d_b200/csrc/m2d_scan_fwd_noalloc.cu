@@ -25,7 +25,6 @@
 #include <mutex>
 
 #include "launch.cuh"
-#include "sweep_rows.cuh"
 
 namespace m2d {
 
@@ -53,65 +52,28 @@ static int ring_address(float4** out) {
     return M2D_OK;
 }
 
-// ROWS: the nested-loop sweep; otherwise the flat step loop (maps narrower than three columns).
-template <typename io_t, bool VEC, bool ROWS>
-__global__ void __launch_bounds__(256, 2) m2d_fwd_noalloc_kernel(const ScanArgs a) {
-    extern __shared__ float4 smem[];
-    const int lane = threadIdx.x & 31;
-    const int nwarps = blockDim.x >> 5;
-    const int cq = lane >> 2, nq = lane & 3;
-    const int g = blockIdx.y;
-    const int ch0 = g * kGroup + cq * 4, n0 = nq * 4;
-    const int chv = min(4, max(0, a.E - ch0));
-    const int nv = min(4, max(0, a.N - n0));
-    const size_t bytes = ROWS ? rows_fwd_smem_bytes(nwarps) : sweep_smem_bytes(nwarps);
-    const int total = (int)(bytes / sizeof(float4));
-    for (int k = threadIdx.x; k < total; k += blockDim.x) smem[k] = make_float4(0.f, 0.f, 0.f, 0.f);
-    const int ch_own = g * kGroup + lane;
-    const float D_own = ch_own < a.E ? load_D<io_t>(a, ch_own) : 0.f;
-    __syncthreads();
-    float4* const params = reinterpret_cast<float4*>(reinterpret_cast<char*>(smem) + bytes);
-    if (threadIdx.x < 32) stage_params<io_t>(params, a.AT, a.AL, a.N, ch0, chv, n0, nv, lane, a.a_log);
-    __syncthreads();
-    const int nb = (a.B - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x;
-    if (ROWS) forward_rows<io_t, VEC, false>(a, smem, params, D_own, blockIdx.x, gridDim.x, nb);
-    else forward_sweep<io_t, VEC, false, false, 1>(a, smem, params, D_own, blockIdx.x, gridDim.x, nb);
-}
-
-template <typename io_t>
-static int launch_noalloc(const m2d_scan_desc* d, const Plan& pl, bool vec, float4* scratch, cudaStream_t st) {
-    ScanArgs a;
-    fill_common_args(a, d, pl);
-    a.y = d->y;
-    // same layout as a caller's workspace: [status word][per-CTA rings]
-    char* base = reinterpret_cast<char*>(scratch);
-    a.status = reinterpret_cast<int*>(base);
-    a.ring = reinterpret_cast<float4*>(base + kStatusBytes);
-    a.chain = 1;
-    if (cudaMemsetAsync(base, 0, sizeof(int), st) != cudaSuccess) return M2D_ERR_LAUNCH;
-    void (*kern)(const ScanArgs) = pl.rows ? (vec ? m2d_fwd_noalloc_kernel<io_t, true, true> : m2d_fwd_noalloc_kernel<io_t, false, true>)
-                                           : (vec ? m2d_fwd_noalloc_kernel<io_t, true, false> : m2d_fwd_noalloc_kernel<io_t, false, false>);
-    return launch_sweep_kernel(kern, a, pl, d->W, st);
+// The plan of the regular entry where its scratch fits the array, else one CTA per (image, channel group),
+// which needs the per-CTA rings only.
+static Plan plan_noalloc(const m2d_scan_desc* d) {
+    const Plan p = plan_fwd(d);
+    return p.scratch <= M2D_NOALLOC_SCRATCH_BYTES ? p : plan_fwd(d, false);
 }
 
 }  // namespace m2d
 
 extern "C" uint64_t m2d_scan_fwd_noalloc_need(const m2d_scan_desc* d) {
     if (m2d::check_desc(d, false, false) != M2D_OK) return 0;
-    return m2d::plan_fwd(d, false).scratch;
+    return m2d::plan_noalloc(d).scratch;
 }
 
 extern "C" int m2d_scan_fwd_noalloc(const m2d_scan_desc* d, void* stream) {
     int rc = m2d::check_desc(d, false, true);
     if (rc != M2D_OK) return rc;
     if (!d->y) return M2D_ERR_NULL;
-    const m2d::Plan pl = m2d::plan_fwd(d, false);   // one CTA per image: the fixed array holds per-CTA rings only
+    const m2d::Plan pl = m2d::plan_noalloc(d);
     if (pl.scratch > M2D_NOALLOC_SCRATCH_BYTES) return M2D_ERR_TOO_LARGE;   // decided before any device work
     float4* ring = nullptr;
     rc = m2d::ring_address(&ring);
     if (rc != M2D_OK) return rc;
-    const bool vec = m2d::vector_ok(d, false);
-    cudaStream_t st = static_cast<cudaStream_t>(stream);
-    if (d->dtype == M2D_F32) return m2d::launch_noalloc<float>(d, pl, vec, ring, st);
-    return m2d::launch_noalloc<__nv_bfloat16>(d, pl, vec, ring, st);
+    return m2d::launch_forward(d, pl, reinterpret_cast<char*>(ring), static_cast<cudaStream_t>(stream));
 }

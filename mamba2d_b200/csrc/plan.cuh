@@ -140,6 +140,7 @@ inline Plan plan_common(const m2d_scan_desc* d, int max_warps, int warps_per_sm,
     Plan p;
     p.cb = cb;
     p.rows = false;
+    p.wave = 0;
     p.groups = (d->E + kGroup - 1) / kGroup;
     p.warps = pick_warps(d->H, max_warps);
     p.Rb = p.warps;
@@ -201,26 +202,56 @@ inline int bound_chain(long long want, int nbands, int steps_per_row, int Rb) {
     return want < 1 ? 1 : (int)want;
 }
 
+// Bytes of the boundary rows of a wave launch: one row of W columns per band and C channels.
+inline size_t wave_edge_bytes(const m2d_scan_desc* d, int C) {
+    if (d->H <= 8) return 0;
+    return align256((size_t)d->B * ((d->E + C - 1) / C) * ((d->H + 7) / 8) * d->W * 16 * C * sizeof(float));
+}
+
+// Wave kernel (wave.cuh): bands of eight rows, 8 * C channels per CTA, one CTA per SM, `chain` CTAs per
+// image (at least one).
+inline Plan plan_wave(const m2d_scan_desc* d, int C) {
+    Plan p{};
+    p.wave = C;
+    p.warps = 8;
+    p.Rb = 8;
+    p.nbands = (d->H + 7) / 8;
+    p.groups = (d->E + 8 * C - 1) / (8 * C);
+    p.grid_x = d->B;
+    const long long slots = sm_count(), ctas = (long long)p.grid_x * p.groups;
+    p.chain = ctas <= slots ? bound_chain(slots / ctas, p.nbands, d->W, p.Rb) : 1;
+    return p;
+}
+
+// Steps a wave launch takes: bands walked one after the other by the busiest CTA, and the start-up of the
+// chain (a band can start when the one above it is about 15 columns in: the eight rows of its wave, the chunk
+// of columns being published, the trip through L2).
+inline double wave_steps(const m2d_scan_desc* d, const Plan& p) {
+    const long long slots = sm_count(), ctas = (long long)p.grid_x * p.groups * p.chain;
+    const long long rounds = (ctas + slots - 1) / slots * ((p.nbands + p.chain - 1) / p.chain);
+    return (double)rounds * ((d->W + 12) / 4 * 4) + (p.chain - 1) * 15.0;
+}
+
 inline Plan plan_fwd(const m2d_scan_desc* d, bool allow_chain = true) {
-    Plan p = plan_best(d, 8, 16, 1);
-    // Few images on a large map: give every image a chain of CTAs, each owning every chain-th band,
-    // so that the bands of one image run as a pipeline across SMs.  All CTAs must be resident.
-    const long long slots = (long long)(16 / p.warps > 0 ? 16 / p.warps : 1) * sm_count();
-    const long long ctas = (long long)p.grid_x * p.groups;
-    if (allow_chain && p.nbands > 1 && ctas * 2 <= slots)
-        p.chain = bound_chain(slots / ctas, p.nbands, (d->W + p.cb - 1) / p.cb, p.Rb);
-    if (p.chain == 1 && d->W >= 3) {
-        // batch mode: the nested-loop kernel (maps narrower than three columns keep the flat one)
-        p = plan_best(d, 8, 16, 1, 2);
-        p.rows = true;
-        p.smem = rows_fwd_smem_bytes(p.warps) + kParamF4 * sizeof(float4);
-    }
+    // batch mode: the nested-loop kernel (maps narrower than three columns take the flat one)
+    Plan p = d->W >= 3 ? plan_best(d, 8, 16, 1, 2) : plan_best(d, 8, 16, 1);
+    p.rows = d->W >= 3;
+    if (p.rows) p.smem = rows_fwd_smem_bytes(p.warps) + kParamF4 * sizeof(float4);
     p.scratch = kStatusBytes;
-    if (p.chain > 1) {
-        const size_t nband = (size_t)d->B * p.groups * p.nbands;
-        p.scratch += align256(nband * sizeof(int)) + align256(nband * d->W * kSlotF4 * sizeof(float4));
-    } else if (p.nbands > 1) {
-        p.scratch += align256((size_t)p.grid_x * p.groups * d->W * kSlotF4 * sizeof(float4));
+    if (p.nbands > 1) p.scratch += align256((size_t)p.grid_x * p.groups * d->W * kSlotF4 * sizeof(float4));
+    if (allow_chain) {
+        // The batch kernel runs one CTA per (image, 32 channels) and is at its best when those fill the GPU;
+        // the wave kernel splits an image over CTAs as well.  Measured times per step: 0.9 us (batch), 0.62 us
+        // (wave, four channels per lane) and 0.42 us (two channels, twice the CTAs); they put the lines
+        // where the measured times cross within 10 % (56x56x64: wave up to batch 64, 290 against 381 us
+        // there; 14x14x320: up to batch 8).
+        const long long per = ((long long)d->B + p.grid_x - 1) / p.grid_x;
+        double best = 0.9 * ((double)per * p.nbands * d->W + p.Rb);
+        for (const int C : {4, 2}) {
+            const Plan w = plan_wave(d, C);
+            const double t = (C == 4 ? 0.62 : 0.42) * wave_steps(d, w);
+            if (t < best) { best = t; p = w; p.scratch = kStatusBytes + wave_edge_bytes(d, C); }
+        }
     }
     return p;
 }

@@ -57,9 +57,9 @@ def test_scan_equals_the_op_by_op_path(dt, tol, monkeypatch):
 
 
 def test_what_the_native_path_does_not_take_goes_op_by_op():
-    w = inputs.make_module_params(36, 16, seed=5)                          # 36 channels: dt rank 16 is beyond the kernels' range
-    w["dt_projT_w"], w["dt_projL_w"] = torch.randn(36, 16) * 0.2, torch.randn(36, 16) * 0.2
-    w["x_proj_w"] = torch.randn(2 * 16 + 48, 36) * 0.1
+    w = inputs.make_module_params(36, 16, seed=5)                          # 36 channels: dt rank 20 is beyond the kernels' range
+    w["dt_projT_w"], w["dt_projL_w"] = torch.randn(36, 20) * 0.2, torch.randn(36, 20) * 0.2
+    w["x_proj_w"] = torch.randn(2 * 20 + 48, 36) * 0.1
     ws = [w[k].cuda() for k in NAMES]
     x = torch.randn(1, 4, 5, 36).cuda()
     assert _lib.entry().block(x, *ws, False, False, False) is None
