@@ -27,16 +27,6 @@ __device__ __forceinline__ float ex2(float v) {
 
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
-// Release / acquire accesses to a progress counter in global memory shared by CTAs of one launch.
-__device__ __forceinline__ int ld_acquire_gpu(const int* p) {
-    int v;
-    asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-    return v;
-}
-__device__ __forceinline__ void st_release_gpu(int* p, int v) {
-    asm volatile("st.release.gpu.global.s32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
-}
-
 // Predicated forms (no branch, no reconvergence point): the copy / store happens iff `on`.
 __device__ __forceinline__ void cp_async16_if(bool on, unsigned smem_addr, const void* gmem) {
     asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %2, 0;\n\t@p cp.async.cg.shared.global [%0], [%1], 16;\n\t}"
@@ -247,9 +237,7 @@ struct Plan {
     int Rb;            // rows per band (<= warps)
     int nbands;        // ceil(H / Rb)
     int grid_x;        // image chains per channel group; chain k walks images k, k + grid_x, ...
-    int cb;            // cells per step and warp (forward only)
     int chain;         // CTAs per chain (> 1 when there are far fewer images than SMs)
-    bool rows;         // batch mode with the nested-loop kernel (its own shared-memory layout)
     int wave;          // channels per lane of the wave kernel (several CTAs per image), or 0
     size_t smem;       // dynamic shared memory per CTA
     size_t scratch;    // workspace bytes

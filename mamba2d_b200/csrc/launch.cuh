@@ -2,7 +2,7 @@
 #pragma once
 
 #include "plan.cuh"
-#include "sweep_fwd.cuh"
+#include "scan_args.cuh"
 
 namespace m2d {
 
@@ -37,14 +37,14 @@ inline void fill_common_args(ScanArgs& a, const m2d_scan_desc* d, const Plan& pl
 // cleanly, and the chain is shortened until the device accepts it (the workspace layout depends on
 // the planned chain only through "is there one", not on its length).  A shortened chain goes through
 // the same bound as a planned one (bound_chain).
-inline int launch_sweep_kernel(void (*kern)(const ScanArgs), ScanArgs& a, const Plan& pl, int steps_per_row, cudaStream_t st) {
+inline int launch_sweep_kernel(void (*kern)(const ScanArgs), ScanArgs& a, const Plan& pl, cudaStream_t st) {
     dim3 block(pl.warps * 32);
     if (!allow_smem(reinterpret_cast<const void*>(kern), pl.smem)) return M2D_ERR_LAUNCH;
     if (a.chain > 1) {
         const int per_sm = resident_ctas(reinterpret_cast<const void*>(kern), (int)block.x, pl.smem);
         if (per_sm < 1) return M2D_ERR_LAUNCH;
         const long long fit = (long long)per_sm * sm_count() / ((long long)pl.grid_x * pl.groups);
-        if (fit < a.chain) a.chain = bound_chain(fit, pl.nbands, steps_per_row, pl.Rb);
+        if (fit < a.chain) a.chain = bound_chain(fit, pl.nbands, a.W, pl.Rb);
         for (;;) {
             dim3 grid(pl.grid_x * a.chain, pl.groups);
             void* args[] = {&a};
@@ -52,7 +52,7 @@ inline int launch_sweep_kernel(void (*kern)(const ScanArgs), ScanArgs& a, const 
             if (e == cudaSuccess) return M2D_OK;
             cudaGetLastError();
             if (e != cudaErrorCooperativeLaunchTooLarge || a.chain == 1) return M2D_ERR_LAUNCH;
-            a.chain = bound_chain(a.chain > 2 ? a.chain - a.chain / 4 - 1 : 1, pl.nbands, steps_per_row, pl.Rb);
+            a.chain = bound_chain(a.chain > 2 ? a.chain - a.chain / 4 - 1 : 1, pl.nbands, a.W, pl.Rb);
         }
     }
     dim3 grid(pl.grid_x, pl.groups);

@@ -3,8 +3,8 @@
 #include <cstdlib>
 
 #include "launch.cuh"
-#include "sweep_bwd.cuh"
 #include "sweep_rows.cuh"
+#include "wave_bwd.cuh"
 
 // Row-warps per CTA of the backward kernel (two CTAs per SM): the register budget per thread follows
 // from it (6 warps: 168 registers).
@@ -19,33 +19,26 @@ namespace m2d {
 
 // Workspace layout of the backward pass (all regions 256-byte aligned):
 //   status   one word, nonzero if a wait between CTAs gave up
-//   counters chained CTAs only: two column counters per band (recompute sweep, adjoint sweep)
-//   ring     per-CTA band-boundary ring, ctas*W*2 KiB (only if nbands > 1); with chained CTAs one
-//            boundary row per band instead (h downwards in the recompute sweep, pT upwards in the
-//            adjoint sweep)
-//   hs       state record written by the recompute sweep     B*groups*H*W*2 KiB (1 KiB with bf16 I/O)
+//   edge     batch: per-CTA band-boundary ring, ctas*W*2 KiB (only if nbands > 1); wave: the boundary rows
+//            of the recompute sweep (h, downwards) and of the adjoint sweep (pT, upwards)
+//   hs       state record written by the recompute sweep: batch B*groups*H*W*2 KiB (1 KiB with bf16 I/O), wave
+//            512*C bytes per (list, warp, band, step)
 //   acc      bf16 I/O only: fp32 accumulators 3 x [B*H*W][N] | 2 x [E][N] | [E], zeroed before the
 //            main kernel and cast by a second kernel.  With fp32 I/O the kernel accumulates straight
 //            into the caller's (zeroed) gradient tensors and this region is empty.
 struct BwdLayout {
-    size_t counters, ring, hs, acc, acc_bytes, total;
+    size_t edge, hs, acc, acc_bytes, total;
 };
 
 inline BwdLayout bwd_layout(const m2d_scan_desc* d, const Plan& p) {
     BwdLayout L;
     size_t off = kStatusBytes;
-    L.counters = off;
-    L.ring = off;
-    if (p.chain > 1) {
-        const size_t nband = (size_t)d->B * p.groups * p.nbands;
-        off += align256(2 * nband * sizeof(int));
-        L.ring = off;
-        off += align256(nband * d->W * kSlotF4 * sizeof(float4));
-    } else if (p.nbands > 1) {
-        off += align256((size_t)p.grid_x * p.groups * d->W * kSlotF4 * sizeof(float4));
-    }
+    L.edge = off;
+    if (p.wave) off += 2 * wave_edge_bytes(d, p, true);
+    else if (p.nbands > 1) off += align256((size_t)p.grid_x * p.groups * d->W * kSlotF4 * sizeof(float4));
     L.hs = off;
-    off += align256((size_t)d->B * p.groups * d->H * d->W * (d->dtype == M2D_F32 ? 128 : 64) * sizeof(float4));
+    if (p.wave) off += align256((size_t)p.grid_x * p.groups * p.warps * p.nbands * (d->W + 7) * p.wave * 512);
+    else off += align256((size_t)d->B * p.groups * d->H * d->W * (d->dtype == M2D_F32 ? 128 : 64) * sizeof(float4));
     L.acc = off;
     L.acc_bytes = 0;
     if (d->dtype != M2D_F32) {
@@ -58,112 +51,30 @@ inline BwdLayout bwd_layout(const m2d_scan_desc* d, const Plan& p) {
 }
 
 inline Plan plan_bwd(const m2d_scan_desc* d) {
-    // tuning knob: M2D_BWD_WARPS=<1..max> overrides the row-warps per CTA of the backward kernel
-    int maxw = M2D_BWD_MAXW;
-    if (const char* e = getenv("M2D_BWD_WARPS")) { const int v = atoi(e); if (v >= 1 && v <= M2D_BWD_MAXW) maxw = v; }
-    Plan p = plan_best(d, maxw, 2 * M2D_BWD_MAXW);
-    p.smem = bwd_smem_bytes(p.warps) + kParamF4 * sizeof(float4);
-    // few images on a large map: chain CTAs along the bands of an image, as the forward does
-    {
-        const long long slots = (long long)(2 * M2D_BWD_MAXW / p.warps > 0 ? 2 * M2D_BWD_MAXW / p.warps : 1) * sm_count();
-        const long long ctas = (long long)p.grid_x * p.groups;
-        if (p.nbands > 1 && ctas * 2 <= slots) p.chain = bound_chain(slots / ctas, p.nbands, d->W, p.Rb);
-    }
-    if (p.chain == 1 && d->W >= 3) {
-        // batch mode: the nested-loop kernel (maps narrower than three columns keep the flat one)
-        p = plan_best(d, maxw, 2 * M2D_BWD_MAXW, 1, 2);
-        p.rows = true;
+    // Batch or wave, as in plan_fwd.  Measured times per step of both sweeps together: 2.45 us in batch mode
+    // with two CTAs per SM, 1.95 us with one, 1.2 us in the wave kernel with two channels per lane (four
+    // spill and are slower at every size measured).  56x56x64: wave up to batch 32, 581 against 738 us.
+    Plan p{};
+    double best = 1e30;
+    if (d->W >= 3) {
+        // tuning knob: M2D_BWD_WARPS=<1..max> overrides the row-warps per CTA of the batch kernel
+        int maxw = M2D_BWD_MAXW;
+        if (const char* e = getenv("M2D_BWD_WARPS")) { const int v = atoi(e); if (v >= 1 && v <= M2D_BWD_MAXW) maxw = v; }
+        p = plan_best(d, maxw, 2 * M2D_BWD_MAXW);
         p.smem = rows_bwd_smem_bytes(p.warps) + kParamF4 * sizeof(float4);
+        best = ((long long)p.grid_x * p.groups > sm_count() ? 2.45 : 1.95) * batch_steps(d, p);
     }
+    const Plan w = plan_wave(d, 2);
+    if (1.2 * wave_steps(d, w) + 10.0 < best) p = w;
     p.scratch = bwd_layout(d, p).total;
     return p;
 }
 
-// Several CTAs per image (large maps, few images): the flat step loops with the cross-CTA hand-off.
+// Few images: several CTAs per image.
 template <typename io_t, bool VEC>
-__global__ void __launch_bounds__(M2D_BWD_MAXW * 32, 2) m2d_bwd_chained_kernel(const ScanArgs a) {
-    constexpr bool CHAINED = true;
-    extern __shared__ float4 handoff[];
-    const int lane = threadIdx.x & 31, r = threadIdx.x >> 5;
-    const int nwarps = blockDim.x >> 5;
-    const int cq = lane >> 2, nq = lane & 3;
-    const int g = blockIdx.y;
-    const int ch0 = g * kGroup + cq * 4, n0 = nq * 4;
-    const int chv = min(4, max(0, a.E - ch0));
-    const int nv = min(4, max(0, a.N - n0));
-
-    const int total = (int)(bwd_smem_bytes(nwarps) / sizeof(float4));
-    for (int k = threadIdx.x; k < total; k += blockDim.x) handoff[k] = make_float4(0.f, 0.f, 0.f, 0.f);
-
-    const int ch_own = g * kGroup + lane;
-    const float D_own = ch_own < a.E ? load_D<io_t>(a, ch_own) : 0.f;
-    float dAT[4][4], dAL[4][4], dD[4];
-#pragma unroll
-    for (int c = 0; c < 4; ++c) {
-        dD[c] = 0.f;
-#pragma unroll
-        for (int n = 0; n < 4; ++n) dAT[c][n] = dAL[c][n] = 0.f;
-    }
-    __syncthreads();
-    float4* const params = reinterpret_cast<float4*>(reinterpret_cast<char*>(handoff) + bwd_smem_bytes(nwarps));
-    if (threadIdx.x < 32) stage_params<io_t>(params, a.AT, a.AL, a.N, ch0, chv, n0, nv, lane, a.a_log);
-    __syncthreads();
-
-    // gridDim.x = chains x a.chain: CTA (chain_id, cpos) walks images chain_id, chain_id + chains, ...
-    const int chains = (int)gridDim.x / a.chain;
-    const int chain_id = (int)blockIdx.x / a.chain, cpos = (int)blockIdx.x % a.chain;
-    for (int b = chain_id; b < a.B; b += chains) {
-        forward_sweep<io_t, VEC, true, CHAINED, 1>(a, handoff, params, D_own, b, 0, 1, cpos, a.chain);
-        reverse_sweep<io_t, VEC, CHAINED>(a, handoff, params, D_own, dAT, dAL, dD, b, cpos, a.chain);
-    }
-
-    // ---- per-(channel,state) sums: fold the CTA's row-warps through shared memory, then one
-    //      atomic per value from warp 0 ----------------------------------------------------------
-    float* red = reinterpret_cast<float*>(handoff);     // reuse: needs 36 floats per thread
-    const int slot = 2 * (nwarps + 1) * kSlotF4 * 4;     // floats available
-    const bool fits = (int)blockDim.x * 36 <= slot;
-    if (fits && nwarps > 1) {
-        float* mine = red + (size_t)threadIdx.x * 36;
-#pragma unroll
-        for (int c = 0; c < 4; ++c) {
-#pragma unroll
-            for (int n = 0; n < 4; ++n) { mine[c * 4 + n] = dAT[c][n]; mine[16 + c * 4 + n] = dAL[c][n]; }
-            mine[32 + c] = dD[c];
-        }
-        __syncthreads();
-        if (r == 0) {
-            for (int w = 1; w < nwarps; ++w) {
-                const float* o = red + (size_t)(w * 32 + lane) * 36;
-#pragma unroll
-                for (int c = 0; c < 4; ++c) {
-#pragma unroll
-                    for (int n = 0; n < 4; ++n) { dAT[c][n] += o[c * 4 + n]; dAL[c][n] += o[16 + c * 4 + n]; }
-                    dD[c] += o[32 + c];
-                }
-            }
-        }
-    }
-    if (r == 0 || !(fits && nwarps > 1)) {
-#pragma unroll
-        for (int c = 0; c < 4; ++c) {
-            if (c < chv) {
-#pragma unroll
-                for (int n = 0; n < 4; ++n) {
-                    if (n < nv) {
-                        const long long idx = (long long)(ch0 + c) * a.N + n0 + n;
-                        // with A given as A_log the gradient asked for is d_A_log = d_A * A (A = -exp(A_log),
-                        // models/kernels/wavefront_cuda.py:72-73); the product is linear, so every CTA
-                        // scales its own partial sum
-                        const float sT = a.a_log ? load_A<io_t>(a.AT, idx, 1, true) : 1.f;
-                        const float sL = a.a_log ? load_A<io_t>(a.AL, idx, 1, true) : 1.f;
-                        atomicAdd(a.accAT + idx, dAT[c][n] * sT);
-                        atomicAdd(a.accAL + idx, dAL[c][n] * sL);
-                    }
-                }
-                if (nq == 0) atomicAdd(a.accD + ch0 + c, dD[c]);
-            }
-        }
-    }
+__global__ void __launch_bounds__(256, 1) m2d_bwd_wave_kernel(const ScanArgs a) {
+    extern __shared__ float4 smem[];
+    wave_backward<io_t, 2, VEC>(a, reinterpret_cast<char*>(smem));
 }
 
 // Batch mode (one CTA per image and channel group): both sweeps written as nested loops.
@@ -293,13 +204,14 @@ static int launch_bwd(const m2d_scan_desc* d, const Plan& pl, bool vec, cudaStre
     ScanArgs a;
     fill_common_args(a, d, pl);
     a.status = reinterpret_cast<int*>(ws);
-    a.ring = reinterpret_cast<float4*>(ws + L.ring);
+    a.ring = reinterpret_cast<float4*>(ws + L.edge);
     size_t zero_bytes = sizeof(int);
-    if (pl.chain > 1) {
-        const size_t nband = (size_t)d->B * pl.groups * pl.nbands;
-        a.bnd = reinterpret_cast<float4*>(ws + L.ring);
-        a.progress = reinterpret_cast<int*>(ws + L.counters);
-        zero_bytes = kStatusBytes + 2 * nband * sizeof(int);
+    if (pl.wave) {
+        const size_t edge = wave_edge_bytes(d, pl, true);
+        a.bnd = reinterpret_cast<float4*>(ws + L.edge);
+        a.bnd_up = reinterpret_cast<float4*>(ws + L.edge + edge);
+        a.bnd_rows = wave_rows(pl, true);
+        if (pl.chain > 1) zero_bytes = kStatusBytes + 2 * edge;
     }
     if (cudaMemsetAsync(ws, 0, zero_bytes, st) != cudaSuccess) return M2D_ERR_LAUNCH;
     a.gy = d->gy;
@@ -335,10 +247,13 @@ static int launch_bwd(const m2d_scan_desc* d, const Plan& pl, bool vec, cudaStre
         a.accAT = acc + 3 * npn; a.accAL = a.accAT + en; a.accD = a.accAL + en;
         if (cudaMemsetAsync(acc, 0, L.acc_bytes, st) != cudaSuccess) return M2D_ERR_LAUNCH;
     }
-    // (the flat kernel with a chain of one CTA is the fallback for maps the nested-loop kernel does not take)
-    void (*kern)(const ScanArgs) = pl.rows ? (vec ? m2d_bwd_kernel<io_t, true> : m2d_bwd_kernel<io_t, false>)
-                                           : (vec ? m2d_bwd_chained_kernel<io_t, true> : m2d_bwd_chained_kernel<io_t, false>);
-    const int rc = launch_sweep_kernel(kern, a, pl, d->W, st);
+    Plan p = pl;
+    if (pl.wave) {
+        a.acc_vec = d->N % 4 == 0 && a.acc_pitch % 4 == 0 && aligned(a.accBT, 16) && aligned(a.accBL, 16) && aligned(a.accC, 16);
+        p.smem = WaveSmem<io_t, 2, true>::kBytes;
+    }
+    const int rc = launch_sweep_kernel(pl.wave ? (vec ? m2d_bwd_wave_kernel<io_t, true> : m2d_bwd_wave_kernel<io_t, false>)
+                                               : (vec ? m2d_bwd_kernel<io_t, true> : m2d_bwd_kernel<io_t, false>), a, p, st);
     if (rc != M2D_OK) return rc;
     if (d->dtype != M2D_F32) {
         const int fin_blocks = (int)((npn + 255) / 256 < 148 * 8 ? (npn + 255) / 256 : 148 * 8);

@@ -5,38 +5,16 @@
 
 namespace m2d {
 
-// Several CTAs per image (large maps, few images).
+// Few images: several CTAs per image.
 template <typename io_t, int C, bool VEC, bool ACT>
-__global__ void __launch_bounds__(256, C == 4 ? 1 : 2) m2d_fwd_wave_kernel(const ScanArgs a) {
+__global__ void __launch_bounds__(256, 1) m2d_fwd_wave_kernel(const ScanArgs a) {
     extern __shared__ float4 smem[];
-    wave_forward<io_t, C, VEC, ACT>(a, reinterpret_cast<char*>(smem));
-}
-
-// Maps of two columns: the flat step loop.
-template <typename io_t, bool VEC>
-__global__ void __launch_bounds__(256, 2) m2d_fwd_flat_kernel(const FwdArgs a) {
-    extern __shared__ float4 handoff[];
-    const int lane = threadIdx.x & 31;
-    const int cq = lane >> 2, nq = lane & 3;
-    const int g = blockIdx.y;
-    const int ch0 = g * kGroup + cq * 4, n0 = nq * 4;
-    const int chv = min(4, max(0, a.E - ch0));
-    const int nv = min(4, max(0, a.N - n0));
-    const int total = (int)(sweep_smem_bytes(blockDim.x >> 5) / sizeof(float4));
-    for (int k = threadIdx.x; k < total; k += blockDim.x) handoff[k] = make_float4(0.f, 0.f, 0.f, 0.f);
-    const int ch_own = g * kGroup + lane;
-    const float D_own = ch_own < a.E ? load_D<io_t>(a, ch_own) : 0.f;
-    __syncthreads();
-    float4* const params = reinterpret_cast<float4*>(reinterpret_cast<char*>(handoff) + sweep_smem_bytes(blockDim.x >> 5));
-    if (threadIdx.x < 32) stage_params<io_t>(params, a.AT, a.AL, a.N, ch0, chv, n0, nv, lane, a.a_log);
-    __syncthreads();
-    const int nb = (a.B - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x;
-    forward_sweep<io_t, VEC, false, false, 1>(a, handoff, params, D_own, blockIdx.x, gridDim.x, nb);
+    wave_forward<io_t, C, VEC, ACT ? kReadoutGelu : kReadout>(a, reinterpret_cast<char*>(smem));
 }
 
 // Batch mode (one CTA per image and channel group): the sweep written as nested loops.
 template <typename io_t, bool VEC>
-__global__ void __launch_bounds__(256, 2) m2d_fwd_kernel(const FwdArgs a) {
+__global__ void __launch_bounds__(256, 2) m2d_fwd_kernel(const ScanArgs a) {
     extern __shared__ float4 smem[];
     const int lane = threadIdx.x & 31;
     const int nwarps = blockDim.x >> 5;
@@ -59,29 +37,25 @@ __global__ void __launch_bounds__(256, 2) m2d_fwd_kernel(const FwdArgs a) {
 
 template <typename io_t>
 static int launch_fwd(const m2d_scan_desc* d, const Plan& pl, bool vec, char* ws, cudaStream_t st) {
-    FwdArgs a;
+    ScanArgs a;
     fill_common_args(a, d, pl);
     a.y = d->y;
     a.status = reinterpret_cast<int*>(ws);
     a.ring = reinterpret_cast<float4*>(ws + kStatusBytes);
-    // the status word and, in a wave launch, the boundary rows of every band behind it
-    const size_t zero = pl.wave ? kStatusBytes + wave_edge_bytes(d, pl.wave) : sizeof(int);
+    // the status word and, where CTAs of a wave launch read each other's, the boundary rows behind it
+    const size_t zero = pl.wave && pl.chain > 1 ? kStatusBytes + wave_edge_bytes(d, pl, false) : sizeof(int);
     if (cudaMemsetAsync(ws, 0, zero, st) != cudaSuccess) return M2D_ERR_LAUNCH;
-    if (pl.wave) {
-        a.bnd = reinterpret_cast<float4*>(ws + kStatusBytes);
-        Plan p = pl;
-        p.smem = pl.wave == 4 ? wave_fwd_smem<io_t, 4>() : wave_fwd_smem<io_t, 2>();
-        auto pick = [&](auto act) {
-            constexpr bool ACT = decltype(act)::value;
-            return pl.wave == 4 ? (vec ? m2d_fwd_wave_kernel<io_t, 4, true, ACT> : m2d_fwd_wave_kernel<io_t, 4, false, ACT>)
-                                : (vec ? m2d_fwd_wave_kernel<io_t, 2, true, ACT> : m2d_fwd_wave_kernel<io_t, 2, false, ACT>);
-        };
-        void (*kern)(const ScanArgs) = a.act ? pick(std::true_type{}) : pick(std::false_type{});
-        return launch_sweep_kernel(kern, a, p, d->W, st);
-    }
-    void (*kern)(const FwdArgs) = pl.rows ? (vec ? m2d_fwd_kernel<io_t, true> : m2d_fwd_kernel<io_t, false>)
-                                          : (vec ? m2d_fwd_flat_kernel<io_t, true> : m2d_fwd_flat_kernel<io_t, false>);
-    return launch_sweep_kernel(kern, a, pl, d->W, st);
+    if (!pl.wave) return launch_sweep_kernel(vec ? m2d_fwd_kernel<io_t, true> : m2d_fwd_kernel<io_t, false>, a, pl, st);
+    a.bnd = reinterpret_cast<float4*>(ws + kStatusBytes);
+    a.bnd_rows = wave_rows(pl, false);
+    Plan p = pl;
+    p.smem = pl.wave == 4 ? WaveSmem<io_t, 4, false>::kBytes : WaveSmem<io_t, 2, false>::kBytes;
+    auto pick = [&](auto act) {
+        constexpr bool ACT = decltype(act)::value;
+        return pl.wave == 4 ? (vec ? m2d_fwd_wave_kernel<io_t, 4, true, ACT> : m2d_fwd_wave_kernel<io_t, 4, false, ACT>)
+                            : (vec ? m2d_fwd_wave_kernel<io_t, 2, true, ACT> : m2d_fwd_wave_kernel<io_t, 2, false, ACT>);
+    };
+    return launch_sweep_kernel(a.act ? pick(std::true_type{}) : pick(std::false_type{}), a, p, st);
 }
 
 int launch_forward(const m2d_scan_desc* d, const Plan& pl, char* scratch, cudaStream_t st) {

@@ -134,21 +134,16 @@ inline int pick_warps(int H, int max_warps) {
     return best;
 }
 
-// `lead`: how many steps before the band below reads a boundary block it must have been written (1 for
-// the flat step loops, 2 for the nested-loop sweeps, which request everything two steps ahead).
-inline Plan plan_common(const m2d_scan_desc* d, int max_warps, int warps_per_sm, int cb = 1, int lead = 1) {
-    Plan p;
-    p.cb = cb;
-    p.rows = false;
-    p.wave = 0;
+// Batch mode: one CTA per (image, 32-channel group), images chained per CTA.
+inline Plan plan_common(const m2d_scan_desc* d, int max_warps, int warps_per_sm) {
+    Plan p{};
     p.groups = (d->E + kGroup - 1) / kGroup;
     p.warps = pick_warps(d->H, max_warps);
     p.Rb = p.warps;
     p.nbands = (d->H + p.Rb - 1) / p.Rb;
-    const int nch = (d->W + cb - 1) / cb;    // steps per row
-    if (p.nbands > 1 && p.Rb > nch - lead) {
-        // a band boundary must be written at least `lead` steps before the next band reads it
-        p.Rb = nch - lead > 1 ? nch - lead : 1;
+    if (p.nbands > 1 && p.Rb > d->W - 2) {
+        // a band boundary must be written two steps before the band below reads it
+        p.Rb = d->W - 2 > 1 ? d->W - 2 : 1;
         p.warps = p.Rb;
         p.nbands = (d->H + p.Rb - 1) / p.Rb;
     }
@@ -159,20 +154,18 @@ inline Plan plan_common(const m2d_scan_desc* d, int max_warps, int warps_per_sm,
     if (per_group < 1) per_group = 1;
     const long long per = (d->B + per_group - 1) / per_group;    // images per CTA
     p.grid_x = (int)((d->B + per - 1) / per);
-    p.smem = ((size_t)2 * cb * (p.warps + 1) * kSlotF4 + (size_t)p.warps * 2 * cb * kStageSlots + 256) * sizeof(float4);   // + parameters
-    p.scratch = 0;
     p.chain = 1;
     return p;
 }
 
 // Try every cap on the row-warps per CTA and keep the plan that keeps the most warps resident,
 // discounted by the rows lost to padding; ties go to the larger CTA.
-inline Plan plan_best(const m2d_scan_desc* d, int max_warps, int warps_per_sm, int cb = 1, int lead = 1) {
-    Plan best = plan_common(d, max_warps, warps_per_sm, cb, lead);
+inline Plan plan_best(const m2d_scan_desc* d, int max_warps, int warps_per_sm) {
+    Plan best = plan_common(d, max_warps, warps_per_sm);
     double best_score = -1.0;
     const double cap = (double)warps_per_sm * sm_count();
     for (int w = max_warps; w >= 2; --w) {
-        const Plan p = plan_common(d, w, warps_per_sm, cb, lead);
+        const Plan p = plan_common(d, w, warps_per_sm);
         double resident = (double)p.grid_x * p.groups * p.warps;
         if (resident > cap) resident = cap;
         const double eff = (double)d->H / ((double)p.nbands * p.Rb);
@@ -182,17 +175,22 @@ inline Plan plan_best(const m2d_scan_desc* d, int max_warps, int warps_per_sm, i
     return best;
 }
 
+// Steps the busiest CTA of a batch launch takes.
+inline double batch_steps(const m2d_scan_desc* d, const Plan& p) {
+    const long long per = ((long long)d->B + p.grid_x - 1) / p.grid_x;
+    return (double)per * p.nbands * d->W + p.Rb;
+}
+
 inline size_t align256(size_t v) { return (v + 255) & ~(size_t)255; }
 
 // Scratch layout shared by every entry point: [status word, 256 bytes][the rest].
 constexpr size_t kStatusBytes = 256;
 
-// CTAs per image that a launch may use.  When a CTA owns more than one band the chain closes into a
-// ring: its first warp enters the second band while (through the per-step block barrier) the warps
-// behind it are still up to Rb-1 steps back in the first, and so on around the ring.  The ring must
-// be shorter than one row of steps, or the head would wait on data that waits on the head.  `want`
-// is the chain the resident CTA slots allow; `steps_per_row` the steps a warp needs for one row.
-// Every place that picks or shortens a chain goes through this rule.
+// CTAs per image that a wave launch may use: at most one per band, and, when CTAs own more than one band
+// each (the chain closes into a ring), fewer than one row of steps divided by the rows of a band, so that a
+// CTA finds the band above its next one well ahead of it.  `want` is the chain the resident CTA slots allow;
+// `steps_per_row` the steps a warp needs for one row.  Every place that picks or shortens a chain goes
+// through this rule.
 inline int bound_chain(long long want, int nbands, int steps_per_row, int Rb) {
     if (want > nbands) want = nbands;
     if (want < nbands) {
@@ -202,14 +200,9 @@ inline int bound_chain(long long want, int nbands, int steps_per_row, int Rb) {
     return want < 1 ? 1 : (int)want;
 }
 
-// Bytes of the boundary rows of a wave launch: one row of W columns per band and C channels.
-inline size_t wave_edge_bytes(const m2d_scan_desc* d, int C) {
-    if (d->H <= 8) return 0;
-    return align256((size_t)d->B * ((d->E + C - 1) / C) * ((d->H + 7) / 8) * d->W * 16 * C * sizeof(float));
-}
-
-// Wave kernel (wave.cuh): bands of eight rows, 8 * C channels per CTA, one CTA per SM, `chain` CTAs per
-// image (at least one).
+// Wave kernels (wave.cuh): bands of eight rows, 8 * C channels per CTA, one CTA per SM.  Where images and
+// channel groups alone do not fill the GPU every image gets a chain of CTAs; otherwise a CTA walks a list of
+// images.
 inline Plan plan_wave(const m2d_scan_desc* d, int C) {
     Plan p{};
     p.wave = C;
@@ -217,10 +210,18 @@ inline Plan plan_wave(const m2d_scan_desc* d, int C) {
     p.Rb = 8;
     p.nbands = (d->H + 7) / 8;
     p.groups = (d->E + 8 * C - 1) / (8 * C);
-    p.grid_x = d->B;
-    const long long slots = sm_count(), ctas = (long long)p.grid_x * p.groups;
+    const long long slots = sm_count(), ctas = (long long)d->B * p.groups;
     p.chain = ctas <= slots ? bound_chain(slots / ctas, p.nbands, d->W, p.Rb) : 1;
+    const long long lists = slots / p.groups > 0 ? slots / p.groups : 1, per = (d->B + lists - 1) / lists;
+    p.grid_x = p.chain > 1 ? d->B : (int)((d->B + per - 1) / per);
     return p;
+}
+
+// Boundary rows a wave launch keeps per (list, channel group): one per band where another CTA reads them or
+// the backward's second sweep comes back to them, else two in turn.
+inline int wave_rows(const Plan& p, bool bwd) { return p.nbands == 1 ? 0 : (p.chain == 1 && !bwd ? 2 : p.nbands); }
+inline size_t wave_edge_bytes(const m2d_scan_desc* d, const Plan& p, bool bwd) {
+    return align256((size_t)p.grid_x * ((d->E + p.wave - 1) / p.wave) * wave_rows(p, bwd) * d->W * 16 * p.wave * sizeof(float));
 }
 
 // Steps a wave launch takes: bands walked one after the other by the busiest CTA, and the start-up of the
@@ -228,30 +229,32 @@ inline Plan plan_wave(const m2d_scan_desc* d, int C) {
 // of columns being published, the trip through L2).
 inline double wave_steps(const m2d_scan_desc* d, const Plan& p) {
     const long long slots = sm_count(), ctas = (long long)p.grid_x * p.groups * p.chain;
-    const long long rounds = (ctas + slots - 1) / slots * ((p.nbands + p.chain - 1) / p.chain);
-    return (double)rounds * ((d->W + 12) / 4 * 4) + (p.chain - 1) * 15.0;
+    const long long images = p.chain > 1 ? 1 : ((long long)d->B + p.grid_x - 1) / p.grid_x;
+    const long long bands = (ctas + slots - 1) / slots * images * ((p.nbands + p.chain - 1) / p.chain);
+    return (double)bands * ((d->W + 12) / 4 * 4) + (p.chain - 1) * 15.0;
 }
 
 inline Plan plan_fwd(const m2d_scan_desc* d, bool allow_chain = true) {
-    // batch mode: the nested-loop kernel (maps narrower than three columns take the flat one)
-    Plan p = d->W >= 3 ? plan_best(d, 8, 16, 1, 2) : plan_best(d, 8, 16, 1);
-    p.rows = d->W >= 3;
-    if (p.rows) p.smem = rows_fwd_smem_bytes(p.warps) + kParamF4 * sizeof(float4);
-    p.scratch = kStatusBytes;
-    if (p.nbands > 1) p.scratch += align256((size_t)p.grid_x * p.groups * d->W * kSlotF4 * sizeof(float4));
-    if (allow_chain) {
-        // The batch kernel runs one CTA per (image, 32 channels) and is at its best when those fill the GPU;
-        // the wave kernel splits an image over CTAs as well.  Measured times per step: 0.9 us (batch), 0.62 us
-        // (wave, four channels per lane) and 0.42 us (two channels, twice the CTAs); they put the lines
-        // where the measured times cross within 10 % (56x56x64: wave up to batch 64, 290 against 381 us
-        // there; 14x14x320: up to batch 8).
-        const long long per = ((long long)d->B + p.grid_x - 1) / p.grid_x;
-        double best = 0.9 * ((double)per * p.nbands * d->W + p.Rb);
-        for (const int C : {4, 2}) {
-            const Plan w = plan_wave(d, C);
-            const double t = (C == 4 ? 0.62 : 0.42) * wave_steps(d, w);
-            if (t < best) { best = t; p = w; p.scratch = kStatusBytes + wave_edge_bytes(d, C); }
-        }
+    // The batch kernel runs one CTA per (image, 32 channels) and is at its best when those fill the GPU; the
+    // wave kernels split an image over CTAs as well.  Measured times per step: 0.9 us (batch), 0.62 us (wave,
+    // four channels per lane) and 0.42 us (two channels, twice the CTAs); they put the lines where the
+    // measured times cross within 10 % (56x56x64: wave up to batch 64, 290 against 381 us there; 14x14x320:
+    // up to batch 8).  The batch kernel needs three columns.
+    Plan p{};
+    double best = 1e30;
+    if (d->W >= 3) {
+        p = plan_best(d, 8, 16);
+        p.smem = rows_fwd_smem_bytes(p.warps) + kParamF4 * sizeof(float4);
+        p.scratch = kStatusBytes;
+        if (p.nbands > 1) p.scratch += align256((size_t)p.grid_x * p.groups * d->W * kSlotF4 * sizeof(float4));
+        best = 0.9 * batch_steps(d, p);
+    }
+    for (const int C : {4, 2}) {
+        if (!allow_chain && d->W >= 3) break;
+        Plan w = plan_wave(d, C);
+        if (!allow_chain) w.chain = 1;
+        const double t = (C == 4 ? 0.62 : 0.42) * wave_steps(d, w);
+        if (t < best) { best = t; p = w; p.scratch = kStatusBytes + wave_edge_bytes(d, w, false); }
     }
     return p;
 }

@@ -1,9 +1,16 @@
 // Wavefront sweeps of the batch mode (one CTA per image and channel group), written as nested loops.
 //
-// Same algorithm and data layout as forward_sweep / reverse_sweep in sweep_fwd.cuh / sweep_bwd.cuh --
-// warp r owns row q*Rb + r of band q and lags r steps behind warp 0; one __syncthreads per step -- but
-// every warp walks its own sequence "for each (image, band): for each column" instead of decoding a
-// flat step counter: all per-row decisions (row 0, pull from the ring, push to the ring, output
+// A CTA owns one 32-channel group and walks `nb` images; each image is cut into `nbands` bands of `Rb`
+// rows; warp r owns row q*Rb + r of band q and walks its W columns, one per step, lagging r steps behind
+// warp 0, so that the row above is always one step ahead (the anti-diagonal wavefront).  Warp r hands its
+// fresh state to warp r+1 through a double-buffered shared-memory slot; one __syncthreads per step keeps
+// the warps in lock step.  The last row of a band reaches the first row of the next band through a per-CTA
+// ring in global memory.  The recompute sweep of the backward also accumulates d_C = sum_e gy*h, while h
+// is in registers; the adjoint sweep mirrors the forward one (bands last to first, the bottom row leads,
+// columns right to left), and the block h[i][j-1] that a warp stages for itself is the h[i-1][j] of the warp
+// of the row below in the same step, so each block crosses L2 -> SM once.
+//
+// Every warp walks its own sequence "for each (image, band): for each column": all per-row decisions (row 0, pull from the ring, push to the ring, output
 // offsets) are taken once per row, and the loop over the columns carries only running indices.  Every
 // warp executes the same number of barriers (idle steps where it has no cell).
 //
@@ -17,7 +24,7 @@
 // written at least two steps before the band below reads it: the plan keeps Rb <= W - 2.
 #pragma once
 
-#include "sweep_bwd.cuh"
+#include "scan_args.cuh"
 
 namespace m2d {
 
@@ -319,8 +326,7 @@ __device__ __forceinline__ void forward_rows(const ScanArgs& a, float4* smem, co
     cp_async_wait_all();                                      // (only empty groups can be pending here)
 }
 
-// Adjoint sweep of one CTA over image b, batch mode, written as nested loops: same algorithm and
-// data layout as reverse_sweep in sweep_bwd.cuh.  Bands are visited last to first, the bottom row of
+// Adjoint sweep of one CTA over image b.  Bands are visited last to first, the bottom row of
 // a band leads (rank rr = Rb-1-r), columns run right to left.  Every warp executes the same number
 // of barriers: rr + 2 steps before its first cell (the last three of them request, in this order, the
 // right-most state block of its first row for the warp below, cell W-1 and cell W-2), W steps per
