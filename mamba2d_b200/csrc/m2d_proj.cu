@@ -13,6 +13,7 @@
 
 #include "common.cuh"
 #include "plan.cuh"
+#include "proj_mma.cuh"
 #include "wgrad_tc.cuh"
 
 namespace m2d {
@@ -89,14 +90,6 @@ static ProjPlan plan_proj(const m2d_proj_desc* d) {
     p.slabs = (int)((d->P + p.rows_per_slab - 1) / p.rows_per_slab);
     p.wg_partials = align256((size_t)p.slabs * p.K * d->E * sizeof(float)) + 256;   // + the status word of the tensor-core kernel
     return p;
-}
-
-// Element of a weight or bias: of the I/O type, or fp32 rounded to it.
-template <typename io_t>
-__device__ __forceinline__ float load_param(const void* p, int off, int f32) {
-    if (!f32) return load1(static_cast<const io_t*>(p), off);
-    const float v = __ldg(static_cast<const float*>(p) + off);
-    return sizeof(io_t) == 2 ? __bfloat162float(__float2bfloat16_rn(v)) : v;
 }
 
 // softplus with the reference's threshold of 20 (torch.nn.functional.softplus defaults)
@@ -551,6 +544,20 @@ static int launch_dt_fwd(const ProjArgs& a, const ProjPlan& p, cudaStream_t st) 
     return cudaGetLastError() == cudaSuccess ? M2D_OK : M2D_ERR_LAUNCH;
 }
 
+// Sums of the parameters' gradients over the CTAs of the backward kernels.
+template <typename io_t>
+static int launch_dt_finalize(const m2d_proj_desc* d, const ProjPlan& p, const float* partials, int ctas, cudaStream_t st) {
+    const int n = 2 * (p.RB + 1) * p.EB;
+    auto finalize = [&](auto out) {                // element type of the parameters' gradients
+        typedef decltype(out) g_t;
+        dtproj_bwd_finalize<g_t><<<(n + 31) / 32, dim3(32, 8), 0, st>>>(partials, ctas, p.RB, p.EB, d->E, d->R, static_cast<g_t*>(d->d_WT),
+                                                                static_cast<g_t*>(d->d_WL), static_cast<g_t*>(d->d_bT), static_cast<g_t*>(d->d_bL));
+    };
+    if (d->flags & M2D_PROJ_PARAMS_F32) finalize(float{});
+    else finalize(io_t{});
+    return cudaGetLastError() == cudaSuccess ? M2D_OK : M2D_ERR_LAUNCH;
+}
+
 template <typename io_t, int RB>
 static int launch_dt_bwd(const m2d_proj_desc* d, const ProjArgs& a, const ProjPlan& p, cudaStream_t st) {
     const size_t loop_bytes = (2 * (size_t)p.TP * RB + (size_t)(p.threads / 32) * kProjIters * kSlabStride) * sizeof(float) +
@@ -566,20 +573,80 @@ static int launch_dt_bwd(const m2d_proj_desc* d, const ProjArgs& a, const ProjPl
     const int gx = balanced_gx(kern, p, smem);
     kern<<<dim3(gx, 2), p.threads, smem, st>>>(a);
     if (cudaGetLastError() != cudaSuccess) return M2D_ERR_LAUNCH;
-    const int n = 2 * (RB + 1) * p.EB;
-    auto finalize = [&](auto out) {                // element type of the parameters' gradients
-        typedef decltype(out) g_t;
-        dtproj_bwd_finalize<g_t><<<(n + 31) / 32, dim3(32, 8), 0, st>>>(a.partials, gx, RB, p.EB, d->E, d->R, static_cast<g_t*>(d->d_WT),
-                                                                static_cast<g_t*>(d->d_WL), static_cast<g_t*>(d->d_bT), static_cast<g_t*>(d->d_bL));
-    };
-    if (a.params_f32) finalize(float{});
-    else finalize(io_t{});
+    return launch_dt_finalize<io_t>(d, p, a.partials, gx, st);
+}
+
+// Which kernels a call gets.  The tensor-core ones read and write rows of 16-byte pieces (E a multiple of 8,
+// aligned tensors), and the backward's sums fit its registers up to 39 ranks.  Measured, CUDA cores against
+// tensor cores: bf16 forward 90 / 55 us (P = 401408, E = 64), 59 / 36 (25088, 320), 8 / 6 (784, 384); bf16
+// backward 88 / 52 (100352, 128), 176 / 62 (25088, 320), but 21 / 25 at P = 784, where its tiles are fewer
+// than the SMs.  With fp32 tensors a product is six: the forward gains from about 3 M elements on (85 / 67,
+// 43 / 38 at P = 6272, E = 512; 6.2 / 8.9 at P = 9805, E = 96), the backward loses everywhere (131 / 149).
+static bool mma_fwd_ok(const m2d_proj_desc* d) {
+    return d->E % 8 == 0 && aligned(d->dT, 16) && aligned(d->dL, 16) && (d->dtype == M2D_BF16 || d->P * d->E >= 3000000);
+}
+static bool mma_bwd_ok(const m2d_proj_desc* d) {
+    return d->dtype == M2D_BF16 && d->E % 8 == 0 && d->R < 40 && d->P >= 4736 && aligned(d->dT, 16) && aligned(d->dL, 16) &&
+           aligned(d->g_dT, 16) && aligned(d->g_dL, 16);
+}
+
+template <typename io_t>
+static int launch_mma_fwd(const m2d_proj_desc* d, cudaStream_t st) {
+    MmaFwdArgs a;
+    a.P = (int)d->P; a.pitch = (int)d->proj_pitch; a.E = d->E; a.R = d->R; a.nk = mma_k<io_t>(d->R);
+    a.params_f32 = (d->flags & M2D_PROJ_PARAMS_F32) ? 1 : 0;
+    a.proj = d->proj; a.WT = d->WT; a.WL = d->WL; a.bT = d->bT; a.bL = d->bL; a.dT = d->dT; a.dL = d->dL;
+    // up to 256 channels per CTA (the tile of r is split and read once per chunk of channels); fewer while the
+    // pixels alone do not give every SM a CTA
+    const long long tiles = (d->P + 127) / 128;
+    int chunk = d->E < 256 ? (d->E + 31) / 32 * 32 : 256;
+    while (chunk > 32 && tiles * 2 * ((d->E + chunk - 1) / chunk) < sm_count()) chunk = (chunk / 2 + 31) / 32 * 32;
+    a.chunk = chunk;
+    const size_t smem = mma_fwd_smem(chunk, a.nk);
+    auto kern = dtproj_fwd_mma_kernel<io_t>;
+    if (!allow_smem(reinterpret_cast<const void*>(kern), smem)) return M2D_ERR_LAUNCH;
+    const int chunks = (d->E + chunk - 1) / chunk, per_sm = resident_ctas(reinterpret_cast<const void*>(kern), 256, smem);
+    long long gx = (long long)(per_sm > 0 ? per_sm : 1) * sm_count() / (2 * chunks);
+    if (gx > tiles) gx = tiles;
+    kern<<<dim3((unsigned)(gx < 1 ? 1 : gx), 2, chunks), 256, smem, st>>>(a);
     return cudaGetLastError() == cudaSuccess ? M2D_OK : M2D_ERR_LAUNCH;
+}
+
+template <int CH, int NCH, int NT>
+static int launch_mma_bwd(const m2d_proj_desc* d, const ProjPlan& p, cudaStream_t st) {
+    MmaBwdArgs a;
+    a.P = (int)d->P; a.pitch = (int)d->proj_pitch; a.E = d->E; a.R = d->R; a.RB = p.RB; a.EB = p.EB;
+    a.params_f32 = (d->flags & M2D_PROJ_PARAMS_F32) ? 1 : 0;
+    a.proj = d->proj; a.WT = d->WT; a.WL = d->WL; a.dT = d->dT; a.dL = d->dL; a.g_dT = d->g_dT; a.g_dL = d->g_dL;
+    a.d_proj = d->d_proj;
+    a.partials = static_cast<float*>(d->workspace);
+    const size_t smem = mma_bwd_smem<CH>(NCH, NT);
+    auto kern = dtproj_bwd_mma_kernel<CH, NCH, NT>;
+    if (!allow_smem(reinterpret_cast<const void*>(kern), smem)) return M2D_ERR_LAUNCH;
+    const int per_sm = resident_ctas(reinterpret_cast<const void*>(kern), 256, smem);
+    long long gx = (long long)(per_sm > 0 ? per_sm : 1) * sm_count() / 2;
+    const long long tiles = (d->P + MmaTile<CH>::kPix - 1) / MmaTile<CH>::kPix;
+    if (gx > tiles) gx = tiles;
+    if (gx > p.gx) gx = p.gx;                      // the workspace holds that many partial results
+    kern<<<dim3((unsigned)(gx < 1 ? 1 : gx), 2), 256, smem, st>>>(a);
+    if (cudaGetLastError() != cudaSuccess) return M2D_ERR_LAUNCH;
+    return launch_dt_finalize<__nv_bfloat16>(d, p, a.partials, gx < 1 ? 1 : (int)gx, st);
 }
 
 template <typename io_t>
 static int dispatch_dt(const m2d_proj_desc* d, bool bwd, cudaStream_t st) {
     const ProjPlan p = plan_proj(d);
+    if (!bwd && mma_fwd_ok(d)) return launch_mma_fwd<io_t>(d, st);
+    if constexpr (sizeof(io_t) == 2) if (bwd && mma_bwd_ok(d)) {
+        // register blocks (chunks of channels, rank tiles) that cover the shipped widths (R = E / 16) closely and
+        // everything else with some padding
+        const int nch = (d->E + 127) / 128, nt = (d->R + 8) / 8;
+        if (d->E <= 64 && nt <= 1) return launch_mma_bwd<64, 1, 1>(d, p, st);
+        if (d->E <= 192 && nt <= 2) return launch_mma_bwd<64, 3, 2>(d, p, st);
+        if (nch <= 3 && nt <= 3) return launch_mma_bwd<128, 3, 3>(d, p, st);
+        if (nch <= 3) return launch_mma_bwd<128, 3, 5>(d, p, st);
+        return launch_mma_bwd<128, 5, 5>(d, p, st);
+    }
     const ProjArgs a = proj_args(d, p);
     switch (p.RB) {
         case 4: return bwd ? launch_dt_bwd<io_t, 4>(d, a, p, st) : launch_dt_fwd<io_t, 4>(a, p, st);

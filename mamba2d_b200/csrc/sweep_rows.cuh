@@ -282,7 +282,7 @@ __device__ __forceinline__ void forward_rows(const ScanArgs& a, float4* smem, co
         } else {
             const float ysum = reduce_states(yacc[0], yacc[1], yacc[2], yacc[3], nq);
             float yv = fmaf(sel4(vx, nq), D_own, ysum);
-            if (a.act) yv = 0.5f * yv * (1.f + erff(yv * 0.70710678118654752f));
+            if (a.act) yv = gelu_erf(yv);
             if (y_lane) store1(static_cast<io_t*>(a.y), (w.pix0 + dir * col) * E + g * kGroup + lane, yv);
         }
     };

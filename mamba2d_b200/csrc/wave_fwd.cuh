@@ -156,7 +156,7 @@ __device__ __forceinline__ void wave_forward_band(const ScanArgs& a, char* smem,
             if (KIND != kRecord) read_staged<io_t, 4>(ln.lane_b + so + 32 * sizeof(io_t), cN);
             if (KIND != kRecord) {
                 float yv = wave_reduce(yr, nq);
-                if (KIND == kReadoutGelu) yv = 0.5f * yv * (1.f + erff(yv * 0.70710678118654752f));
+                if (KIND == kReadoutGelu) yv = gelu_erf(yv);
                 yp += ystep;
                 store_if(yr_on, yp, yv);
             }
