@@ -63,7 +63,7 @@ def build_entry(force=False):
     for d in library_paths() + [os.path.join(cuda, "lib64")]:
         cmd += ["-L", d]
     cmd += ["-L", HERE, "-l:libm2d_scan.so", "-Wl,-rpath,$ORIGIN", "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_cuda", "-ltorch",
-            "-ltorch_python", "-lcudart"]
+            "-ltorch_python", "-lcudart", "-lcublas"]
     res = subprocess.run(cmd, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
     if res.returncode != 0:
         raise RuntimeError("building torch_entry.cpp failed:\n" + res.stdout)

@@ -12,6 +12,7 @@
 #include "m2d_proj.h"
 
 #include "common.cuh"
+#include "launch.cuh"
 #include "plan.cuh"
 #include "proj_mma.cuh"
 #include "wgrad_tc.cuh"
@@ -88,7 +89,7 @@ static ProjPlan plan_proj(const m2d_proj_desc* d) {
     if (slabs < 1) slabs = 1;
     p.rows_per_slab = (int)(((d->P + slabs - 1) / slabs + 31) / 32 * 32);
     p.slabs = (int)((d->P + p.rows_per_slab - 1) / p.rows_per_slab);
-    p.wg_partials = align256((size_t)p.slabs * p.K * d->E * sizeof(float)) + 256;   // + the status word of the tensor-core kernel
+    p.wg_partials = align256((size_t)p.slabs * p.K * d->E * sizeof(float));
     return p;
 }
 
@@ -675,8 +676,7 @@ static int launch_wgrad_tc(const m2d_proj_desc* d, const ProjPlan& p, cudaStream
     TcArgs a;
     a.K = p.K; a.E = d->E; a.nbk = t.nbk; a.stages = t.stages; a.total_blocks = t.total_blocks; a.blocks_per_cta = t.blocks_per_cta;
     a.partials = static_cast<float*>(d->workspace);
-    a.status = reinterpret_cast<int*>(static_cast<char*>(d->workspace) + p.wg_partials - 256);
-    if (cudaMemsetAsync(a.status, 0, sizeof(int), st) != cudaSuccess) return M2D_ERR_LAUNCH;
+    a.status = wait_failure_flag();      // host memory: a wait that gives up shows in m2d_take_wait_failure()
     if (!allow_smem(reinterpret_cast<const void*>(xproj_wgrad_tc_kernel), t.smem)) return M2D_ERR_LAUNCH;
     xproj_wgrad_tc_kernel<<<dim3(t.grid_x, t.ny), 128, t.smem, st>>>(map_a, map_b, a);
     if (cudaGetLastError() != cudaSuccess) return M2D_ERR_LAUNCH;

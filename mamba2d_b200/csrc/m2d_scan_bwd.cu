@@ -19,13 +19,13 @@ namespace m2d {
 
 // Workspace layout of the backward pass (all regions 256-byte aligned):
 //   status   one word, nonzero if a wait between CTAs gave up
+//   acc      bf16 I/O only: fp32 accumulators 3 x [B*H*W][N] | 2 x [E][N] | [E], zeroed before the
+//            main kernel (with the status word, in one memset) and cast by a second kernel.  With fp32 I/O
+//            the kernel accumulates straight into the caller's (zeroed) gradient tensors and this region is empty.
 //   edge     batch: per-CTA band-boundary ring, ctas*W*2 KiB (only if nbands > 1); wave: the boundary rows
 //            of the recompute sweep (h, downwards) and of the adjoint sweep (pT, upwards)
 //   hs       state record written by the recompute sweep: batch B*groups*H*W*2 KiB (1 KiB with bf16 I/O), wave
 //            512*C bytes per (list, warp, band, step)
-//   acc      bf16 I/O only: fp32 accumulators 3 x [B*H*W][N] | 2 x [E][N] | [E], zeroed before the
-//            main kernel and cast by a second kernel.  With fp32 I/O the kernel accumulates straight
-//            into the caller's (zeroed) gradient tensors and this region is empty.
 struct BwdLayout {
     size_t edge, hs, acc, acc_bytes, total;
 };
@@ -33,12 +33,6 @@ struct BwdLayout {
 inline BwdLayout bwd_layout(const m2d_scan_desc* d, const Plan& p) {
     BwdLayout L;
     size_t off = kStatusBytes;
-    L.edge = off;
-    if (p.wave) off += 2 * wave_edge_bytes(d, p, true);
-    else if (p.nbands > 1) off += align256((size_t)p.grid_x * p.groups * d->W * kSlotF4 * sizeof(float4));
-    L.hs = off;
-    if (p.wave) off += align256((size_t)p.grid_x * p.groups * p.warps * p.nbands * (d->W + 7) * p.wave * 512);
-    else off += align256((size_t)d->B * p.groups * d->H * d->W * (d->dtype == M2D_F32 ? 128 : 64) * sizeof(float4));
     L.acc = off;
     L.acc_bytes = 0;
     if (d->dtype != M2D_F32) {
@@ -46,6 +40,12 @@ inline BwdLayout bwd_layout(const m2d_scan_desc* d, const Plan& p) {
         L.acc_bytes = align256((3 * npn + 2 * en + d->E) * sizeof(float));
     }
     off += L.acc_bytes;
+    L.edge = off;
+    if (p.wave) off += 2 * wave_edge_bytes(d, p, true);
+    else if (p.nbands > 1) off += align256((size_t)p.grid_x * p.groups * d->W * kSlotF4 * sizeof(float4));
+    L.hs = off;
+    if (p.wave) off += align256((size_t)p.grid_x * p.groups * p.warps * p.nbands * (d->W + 7) * p.wave * 512);
+    else off += align256((size_t)d->B * p.groups * d->H * d->W * (d->dtype == M2D_F32 ? 128 : 64) * sizeof(float4));
     L.total = off;
     return L;
 }
@@ -205,13 +205,13 @@ static int launch_bwd(const m2d_scan_desc* d, const Plan& pl, bool vec, cudaStre
     fill_common_args(a, d, pl);
     a.status = reinterpret_cast<int*>(ws);
     a.ring = reinterpret_cast<float4*>(ws + L.edge);
-    size_t zero_bytes = sizeof(int);
+    size_t zero_bytes = L.acc_bytes ? kStatusBytes + L.acc_bytes : sizeof(int);
     if (pl.wave) {
         const size_t edge = wave_edge_bytes(d, pl, true);
         a.bnd = reinterpret_cast<float4*>(ws + L.edge);
         a.bnd_up = reinterpret_cast<float4*>(ws + L.edge + edge);
         a.bnd_rows = wave_rows(pl, true);
-        if (pl.chain > 1) zero_bytes = kStatusBytes + 2 * edge;
+        if (pl.chain > 1) zero_bytes = L.edge + 2 * edge;
     }
     if (cudaMemsetAsync(ws, 0, zero_bytes, st) != cudaSuccess) return M2D_ERR_LAUNCH;
     a.gy = d->gy;
@@ -245,7 +245,6 @@ static int launch_bwd(const m2d_scan_desc* d, const Plan& pl, bool vec, cudaStre
         a.acc_pitch = d->N;
         a.accBT = acc; a.accBL = acc + npn; a.accC = acc + 2 * npn;
         a.accAT = acc + 3 * npn; a.accAL = a.accAT + en; a.accD = a.accAL + en;
-        if (cudaMemsetAsync(acc, 0, L.acc_bytes, st) != cudaSuccess) return M2D_ERR_LAUNCH;
     }
     Plan p = pl;
     if (pl.wave) {

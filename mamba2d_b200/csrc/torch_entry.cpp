@@ -13,6 +13,7 @@
 #include <ATen/autocast_mode.h>
 #include <ATen/cuda/CUDAContext.h>
 #include <c10/cuda/CUDAGuard.h>
+#include <cublas_v2.h>
 #include <torch/extension.h>
 
 #include "m2d_proj.h"
@@ -40,71 +41,48 @@ struct Dims {
     int64_t B, H, W, E, N, R, K;
 };
 
-struct ScanIn {      // what the scan reads; BT, BL, C with their pixel pitch
-    Tensor x, dT, dL, AT, AL, BT, BL, C, D;
+// What the scan reads, as addresses in tensors that the caller holds; BT, BL, C with their pixel pitch.
+struct ScanIn {
+    const void *x, *dT, *dL, *AT, *AL, *BT, *BL, *C, *D;
     int64_t pBT, pBL, pC;
 };
+struct ScanGrads {
+    void *x, *dT, *dL, *AT, *AL, *BT, *BL, *C, *D;
+    int64_t pBC;         // pixel pitch of the gradients of B and C (0: N)
+};
 
-m2d_scan_desc scan_desc(const Dims& s, const ScanIn& in, unsigned flags) {
+m2d_scan_desc scan_desc(const Dims& s, int dtype, const ScanIn& in, unsigned flags) {
     m2d_scan_desc d{};
     d.struct_bytes = sizeof(d);
-    d.dtype = dtype_of(in.x);
+    d.dtype = dtype;
     d.B = (int)s.B; d.H = (int)s.H; d.W = (int)s.W; d.E = (int)s.E; d.N = (int)s.N;
     d.flags = flags;
-    d.x = in.x.data_ptr(); d.dT = in.dT.data_ptr(); d.dL = in.dL.data_ptr();
-    d.AT = in.AT.data_ptr(); d.AL = in.AL.data_ptr();
-    d.BT = in.BT.data_ptr(); d.BL = in.BL.data_ptr(); d.C = in.C.data_ptr();
+    d.x = in.x; d.dT = in.dT; d.dL = in.dL;
+    d.AT = in.AT; d.AL = in.AL;
+    d.BT = in.BT; d.BL = in.BL; d.C = in.C;
     d.BT_pitch = in.pBT; d.BL_pitch = in.pBL; d.C_pitch = in.pC;
-    d.D = in.D.data_ptr();
+    d.D = in.D;
     return d;
 }
 
-Tensor scan_forward(const Dims& s, const ScanIn& in, unsigned flags) {
-    m2d_scan_desc d = scan_desc(s, in, flags);
-    Tensor y = at::empty({s.B, s.H, s.W, s.E}, in.x.options());
-    d.y = y.data_ptr();
-    d.workspace_bytes = m2d_scan_fwd_workspace(&d);
-    const Tensor ws = scratch(d.workspace_bytes, in.x);
-    d.workspace = ws.data_ptr();
-    check(m2d_scan_fwd(&d, stream_of(in.x)), "m2d_scan_fwd");
-    return y;
+void set_grads(m2d_scan_desc& d, const void* gy, const ScanGrads& g) {
+    d.gy = gy;
+    d.d_x = g.x; d.d_dT = g.dT; d.d_dL = g.dL;
+    d.d_AT = g.AT; d.d_AL = g.AL; d.d_D = g.D;
+    d.d_BT = g.BT; d.d_BL = g.BL; d.d_C = g.C;
+    d.d_BC_pitch = g.pBC;
 }
 
-struct ScanGrads {
-    Tensor x, dT, dL, AT, AL, D;
-};
-
-// `bt`, `bl`, `c`: where the gradients of B and C go, at `pitch` elements per pixel.
-ScanGrads scan_backward(const Dims& s, const ScanIn& in, const Tensor& gy, void* bt, void* bl, void* c, int64_t pitch, unsigned flags) {
-    m2d_scan_desc d = scan_desc(s, in, flags);
-    const auto fp32 = in.x.options().dtype(at::kFloat);
-    ScanGrads g;
-    // the per-channel gradients are neighbours in the order the library zeroes them, where they share a type
-    const auto aopt = (flags & M2D_SCAN_A_LOG) ? fp32 : in.x.options(), dopt = (flags & M2D_SCAN_D_F32) ? fp32 : in.x.options();
-    if (aopt.dtype() == dopt.dtype()) {
-        const Tensor small = at::empty({2 * s.E * s.N + s.E}, aopt);
-        g.AT = small.narrow(0, 0, s.E * s.N).view({s.E, s.N});
-        g.AL = small.narrow(0, s.E * s.N, s.E * s.N).view({s.E, s.N});
-        g.D = small.narrow(0, 2 * s.E * s.N, s.E);
-    } else {
-        g.AT = at::empty({s.E, s.N}, aopt);
-        g.AL = at::empty({s.E, s.N}, aopt);
-        g.D = at::empty({s.E}, dopt);
+// Several arrays in one allocation (an allocation or a view of a tensor costs the host about 2 us, a third of a
+// launch): byte offsets, 256-byte aligned.
+struct Carve {
+    int64_t bytes = 0;
+    int64_t take(int64_t n) {
+        const int64_t at = bytes;
+        bytes += (n + 255) / 256 * 256;
+        return at;
     }
-    g.x = at::empty({s.B, s.H, s.W, s.E}, in.x.options());
-    g.dT = at::empty({s.B, s.H, s.W, s.E}, in.x.options());
-    g.dL = at::empty({s.B, s.H, s.W, s.E}, in.x.options());
-    d.gy = gy.data_ptr();
-    d.d_x = g.x.data_ptr(); d.d_dT = g.dT.data_ptr(); d.d_dL = g.dL.data_ptr();
-    d.d_AT = g.AT.data_ptr(); d.d_AL = g.AL.data_ptr(); d.d_D = g.D.data_ptr();
-    d.d_BT = bt; d.d_BL = bl; d.d_C = c;
-    d.d_BC_pitch = pitch;
-    d.workspace_bytes = m2d_scan_bwd_workspace(&d);
-    const Tensor ws = scratch(d.workspace_bytes, in.x);
-    d.workspace = ws.data_ptr();
-    check(m2d_scan_bwd(&d, stream_of(in.x)), "m2d_scan_bwd");
-    return g;
-}
+};
 
 // ---- the block call: projections + scan ---------------------------------------------------------
 
@@ -126,36 +104,57 @@ m2d_proj_desc proj_desc(const Dims& s, const Tensor& x, const BlockParams& p) {
     return d;
 }
 
+// proj (P, K), dT and dL (P, E) in one buffer.
 struct Projected {
-    Tensor proj, dT, dL;
+    int64_t dT, dL, bytes;       // offsets behind proj
+    Projected(const Dims& s, int64_t es) {
+        Carve c;
+        c.take(s.B * s.H * s.W * s.K * es);
+        dT = c.take(s.B * s.H * s.W * s.E * es);
+        dL = c.take(s.B * s.H * s.W * s.E * es);
+        bytes = c.bytes;
+    }
 };
 
-Projected project(const Dims& s, const Tensor& x, const BlockParams& p) {
-    const int64_t P = s.B * s.H * s.W;
-    Projected o;
-    o.proj = at::empty({P, s.K}, x.options());
-    at::mm_out(o.proj, x.view({P, s.E}), p.Wx.t());
-    o.dT = at::empty({s.B, s.H, s.W, s.E}, x.options());
-    o.dL = at::empty({s.B, s.H, s.W, s.E}, x.options());
-    m2d_proj_desc d = proj_desc(s, x, p);
-    d.proj = o.proj.data_ptr();
-    d.dT = o.dT.data_ptr(); d.dL = o.dL.data_ptr();
-    check(m2d_dtproj_fwd(&d, stream_of(x)), "m2d_dtproj_fwd");
-    return o;
+// out (rows, n) = a (rows, k) @ w, or += ; `w` is (n, k) if transposed, else (k, n).  Row-major operands are what
+// the library calls transposed ones.
+void gemm(const Tensor& like, int64_t rows, int64_t n, int64_t k, const void* a, const void* w, bool transposed, bool accumulate, void* out) {
+    const cudaDataType_t type = like.scalar_type() == at::kFloat ? CUDA_R_32F : CUDA_R_16BF;
+    const float alpha = 1.f, beta = accumulate ? 1.f : 0.f;
+    // (torch's handle: its stream, its workspace, its TF32 setting)
+    const cublasStatus_t rc = cublasGemmEx(at::cuda::getCurrentCUDABlasHandle(), transposed ? CUBLAS_OP_T : CUBLAS_OP_N, CUBLAS_OP_N, (int)n, (int)rows, (int)k, &alpha,
+                                           w, type, (int)(transposed ? k : n), a, type, (int)k, &beta, out, type, (int)n, CUBLAS_COMPUTE_32F, CUBLAS_GEMM_DEFAULT);
+    TORCH_CHECK(rc == CUBLAS_STATUS_SUCCESS, "cublasGemmEx failed: status ", (int)rc);
 }
 
-ScanIn block_scan_in(const Dims& s, const Tensor& x, const BlockParams& p, const Projected& o) {
+void project(const Dims& s, const Tensor& x, const BlockParams& p, const Projected& o, char* buf) {
+    gemm(x, s.B * s.H * s.W, s.K, s.E, x.data_ptr(), p.Wx.data_ptr(), true, false, buf);
+    m2d_proj_desc d = proj_desc(s, x, p);
+    d.proj = buf;
+    d.dT = buf + o.dT; d.dL = buf + o.dL;
+    check(m2d_dtproj_fwd(&d, stream_of(x)), "m2d_dtproj_fwd");
+}
+
+ScanIn block_scan_in(const Dims& s, const Tensor& x, const BlockParams& p, const Projected& o, const char* buf) {
+    const int64_t es = x.element_size();
     ScanIn in;
-    in.x = x; in.dT = o.dT; in.dL = o.dL;
-    in.AT = p.AT_log; in.AL = p.AL_log; in.D = p.D;
-    in.BT = o.proj.narrow(1, 2 * s.R, s.N);
-    in.BL = o.proj.narrow(1, 2 * s.R + s.N, s.N);
-    in.C = o.proj.narrow(1, 2 * s.R + 2 * s.N, s.N);
+    in.x = x.data_ptr(); in.dT = buf + o.dT; in.dL = buf + o.dL;
+    in.AT = p.AT_log.data_ptr(); in.AL = p.AL_log.data_ptr(); in.D = p.D.data_ptr();
+    in.BT = buf + 2 * s.R * es;
+    in.BL = buf + (2 * s.R + s.N) * es;
+    in.C = buf + (2 * s.R + 2 * s.N) * es;
     in.pBT = in.pBL = in.pC = s.K;
     return in;
 }
 
 unsigned block_flags(const BlockParams& p, bool reverse) { return M2D_SCAN_A_LOG | (p.f32 ? M2D_SCAN_D_F32 : 0u) | (reverse ? M2D_SCAN_REVERSE : 0u); }
+
+// y, given the projections in `buf`; the scan's scratch goes to `ws`.
+void block_scan(const Dims& s, const Tensor& x, m2d_scan_desc& d, char* ws, const Tensor& y) {
+    d.y = y.data_ptr();
+    d.workspace = ws;
+    check(m2d_scan_fwd(&d, stream_of(x)), "m2d_scan_fwd");
+}
 
 Dims block_dims(const Tensor& x, const Tensor& A_log, const Tensor& WT) {
     Dims s;
@@ -183,11 +182,18 @@ public:
         const Tensor x = x_.contiguous();
         const Dims s = block_dims(x, AT_log, WT);
         const BlockParams p = block_params(x, AT_log, AL_log, Wx, WT, bT, WL, bL, D);
-        const Projected o = project(s, x, p);
-        Tensor y = scan_forward(s, block_scan_in(s, x, p, o), block_flags(p, reverse));
+        const Projected o(s, x.element_size());
+        const Tensor buf = scratch(o.bytes, x);
+        char* const bp = static_cast<char*>(buf.data_ptr());
+        project(s, x, p, o, bp);
+        m2d_scan_desc d = scan_desc(s, dtype_of(x), block_scan_in(s, x, p, o, bp), block_flags(p, reverse));
+        d.workspace_bytes = m2d_scan_fwd_workspace(&d);
+        const Tensor ws = scratch(d.workspace_bytes, x);
+        Tensor y = at::empty({s.B, s.H, s.W, s.E}, x.options());
+        block_scan(s, x, d, static_cast<char*>(ws.data_ptr()), y);
         // "full" recomputation keeps x and the parameters only
         if (full) ctx->save_for_backward({x, AT_log, AL_log, Wx, WT, bT, WL, bL, D});
-        else ctx->save_for_backward({x, AT_log, AL_log, Wx, WT, bT, WL, bL, D, o.proj, o.dT, o.dL});
+        else ctx->save_for_backward({x, AT_log, AL_log, Wx, WT, bT, WL, bL, D, buf, p.Wx});
         ctx->saved_data["reverse"] = reverse;
         return y;
     }
@@ -199,41 +205,72 @@ public:
         const c10::cuda::CUDAGuard guard(x.device());
         const bool reverse = ctx->saved_data["reverse"].toBool();
         const Dims s = block_dims(x, v[1], v[4]);
-        const BlockParams p = block_params(x, v[1], v[2], v[3], v[4], v[5], v[6], v[7], v[8]);
-        const int64_t P = s.B * s.H * s.W;
-        Projected o;
-        if (v.size() > 9) { o.proj = v[9]; o.dT = v[10]; o.dL = v[11]; }
-        else o = project(s, x, p);
+        const bool saved = v.size() > 9;
+        const BlockParams p = block_params(x, v[1], v[2], saved ? v[10] : v[3], v[4], v[5], v[6], v[7], v[8]);
+        const int64_t P = s.B * s.H * s.W, es = x.element_size();
+        const Projected o(s, es);
+        const bool f32 = x.scalar_type() == at::kFloat;      // the fp32 scan accumulates dB and dC in place, the bf16 one in its workspace
         const Tensor gy = grads[0].to(x.scalar_type()).contiguous();
 
-        const bool f32 = x.scalar_type() == at::kFloat;      // the fp32 scan accumulates in place, the bf16 one in its workspace
-        const Tensor d_proj = f32 ? at::zeros({P, s.K}, x.options()) : at::empty({P, s.K}, x.options());
-        char* dp = static_cast<char*>(d_proj.data_ptr());
-        const int64_t es = d_proj.element_size();
-        const ScanGrads g = scan_backward(s, block_scan_in(s, x, p, o), gy, dp + 2 * s.R * es, dp + (2 * s.R + s.N) * es,
-                                          dp + (2 * s.R + 2 * s.N) * es, s.K, block_flags(p, reverse) | (f32 ? M2D_SCAN_BC_ZEROED : 0u));
+        // scratch: gradients of the projections' outputs, then what the two library workspaces share
+        Carve c;
+        const int64_t at_dT = c.take(P * s.E * es), at_dL = c.take(P * s.E * es), at_proj = c.take(P * s.K * es), at_buf = saved ? 0 : c.take(o.bytes);
+        m2d_scan_desc sd = scan_desc(s, dtype_of(x), ScanIn{}, block_flags(p, reverse) | (f32 ? M2D_SCAN_BC_ZEROED : 0u));
+        sd.BT_pitch = sd.BL_pitch = sd.C_pitch = sd.d_BC_pitch = s.K;
+        m2d_proj_desc pd = proj_desc(s, x, p);
+        sd.workspace_bytes = m2d_scan_bwd_workspace(&sd);
+        pd.workspace_bytes = m2d_proj_workspace(&pd);
+        const int64_t at_ws = c.take((int64_t)std::max(sd.workspace_bytes, pd.workspace_bytes));
+        const Tensor tmp = scratch(c.bytes, x);
+        char* const t = static_cast<char*>(tmp.data_ptr());
+        char* const d_proj = t + at_proj;
+        if (f32) C10_CUDA_CHECK(cudaMemsetAsync(d_proj, 0, P * s.K * es, at::cuda::getCurrentCUDAStream(x.get_device())));
+        const char* buf = saved ? static_cast<const char*>(v[9].data_ptr()) : t + at_buf;
+        if (!saved) project(s, x, p, o, t + at_buf);
 
-        const auto popt = p.f32 ? x.options().dtype(at::kFloat) : x.options();
-        Tensor dWT = at::empty({s.E, s.R}, popt), dWL = at::empty({s.E, s.R}, popt), dbT = at::empty({s.E}, popt), dbL = at::empty({s.E}, popt);
-        Tensor dWx = at::empty({s.K, s.E}, popt);
-        m2d_proj_desc d = proj_desc(s, x, p);
-        d.x = x.data_ptr(); d.proj = o.proj.data_ptr();
-        d.dT = o.dT.data_ptr(); d.dL = o.dL.data_ptr();
-        d.g_dT = g.dT.data_ptr(); d.g_dL = g.dL.data_ptr();
-        d.d_proj = d_proj.data_ptr();
-        d.d_WT = dWT.data_ptr(); d.d_WL = dWL.data_ptr(); d.d_bT = dbT.data_ptr(); d.d_bL = dbL.data_ptr();
-        d.d_Wx = dWx.data_ptr();
-        d.workspace_bytes = m2d_proj_workspace(&d);
-        const Tensor ws = scratch(d.workspace_bytes, x);
-        d.workspace = ws.data_ptr();
-        check(m2d_dtproj_bwd(&d, stream_of(x)), "m2d_dtproj_bwd");
-        check(m2d_xproj_wgrad(&d, stream_of(x)), "m2d_xproj_wgrad");
-        // d_x = (scan's part) + d_proj @ Wx
-        Tensor dx2 = g.x.view({P, s.E});
-        at::addmm_out(dx2, dx2, d_proj, p.Wx);
+        // the parameters' gradients: A_log's in fp32, the others in the parameters' type; neighbours in one buffer
+        // where that is the same
+        const bool one = f32 || p.f32;
+        const auto fp32 = x.options().dtype(at::kFloat);
+        const int64_t en = s.E * s.N, er = s.E * s.R, rest = 2 * er + 2 * s.E + s.K * s.E;
+        const Tensor a = at::empty({2 * en + (one ? s.E + rest : 0)}, fp32);
+        const Tensor w = one ? a : at::empty({s.E + rest}, x.options());
+        int64_t at = 0;
+        auto view = [&](const Tensor& from, at::IntArrayRef size) {
+            const int64_t cols = size.size() == 2 ? size[1] : 1, off = at;
+            at += size[0] * cols;
+            return size.size() == 2 ? at::as_strided(from, size, {cols, 1}, off) : at::as_strided(from, size, {1}, off);
+        };
+        Tensor dAT = view(a, {s.E, s.N}), dAL = view(a, {s.E, s.N});
+        if (!one) at = 0;
+        Tensor dD = view(w, {s.E}), dWT = view(w, {s.E, s.R}), dWL = view(w, {s.E, s.R}), dbT = view(w, {s.E}), dbL = view(w, {s.E}), dWx = view(w, {s.K, s.E});
+        Tensor dx = at::empty({s.B, s.H, s.W, s.E}, x.options());
+
+        ScanGrads g;
+        g.x = dx.data_ptr(); g.dT = t + at_dT; g.dL = t + at_dL;
+        g.AT = dAT.data_ptr(); g.AL = dAL.data_ptr(); g.D = dD.data_ptr();
+        g.BT = d_proj + 2 * s.R * es; g.BL = d_proj + (2 * s.R + s.N) * es; g.C = d_proj + (2 * s.R + 2 * s.N) * es;
+        g.pBC = s.K;
+        const uint64_t ws_bytes = sd.workspace_bytes;
+        sd = scan_desc(s, dtype_of(x), block_scan_in(s, x, p, o, buf), sd.flags);
+        set_grads(sd, gy.data_ptr(), g);
+        sd.workspace = t + at_ws;
+        sd.workspace_bytes = ws_bytes;
+        check(m2d_scan_bwd(&sd, stream_of(x)), "m2d_scan_bwd");
+
+        pd.x = x.data_ptr(); pd.proj = buf;
+        pd.dT = const_cast<char*>(buf) + o.dT; pd.dL = const_cast<char*>(buf) + o.dL;
+        pd.g_dT = g.dT; pd.g_dL = g.dL;
+        pd.d_proj = d_proj;
+        pd.d_WT = dWT.data_ptr(); pd.d_WL = dWL.data_ptr(); pd.d_bT = dbT.data_ptr(); pd.d_bL = dbL.data_ptr();
+        pd.d_Wx = dWx.data_ptr();
+        pd.workspace = t + at_ws;
+        check(m2d_dtproj_bwd(&pd, stream_of(x)), "m2d_dtproj_bwd");
+        check(m2d_xproj_wgrad(&pd, stream_of(x)), "m2d_xproj_wgrad");
+        gemm(x, P, s.E, s.K, d_proj, p.Wx.data_ptr(), false, true, g.x);      // d_x = (scan's part) + d_proj @ Wx
 
         auto as = [](const Tensor& t, const Tensor& like) { return t.to(like.scalar_type()); };
-        return {g.x, as(g.AT, v[1]), as(g.AL, v[2]), as(dWx, v[3]), dWT, dbT, dWL, dbL, g.D, Tensor(), Tensor()};
+        return {dx, as(dAT, v[1]), as(dAL, v[2]), as(dWx, v[3]), dWT, dbT, dWL, dbL, dD, Tensor(), Tensor()};
     }
 };
 
@@ -275,7 +312,18 @@ c10::optional<Tensor> block(const Tensor& x, const Tensor& AT_log, const Tensor&
     const Tensor xc = x.contiguous();
     const Dims s = block_dims(xc, AT_log, WT);
     const BlockParams p = block_params(xc, AT_log, AL_log, Wx, WT, bT, WL, bL, D);
-    return scan_forward(s, block_scan_in(s, xc, p, project(s, xc, p)), block_flags(p, reverse) | (gelu ? M2D_SCAN_GELU_OUT : 0u));
+    const Projected o(s, xc.element_size());
+    m2d_scan_desc d = scan_desc(s, dtype_of(xc), ScanIn{}, block_flags(p, reverse) | (gelu ? M2D_SCAN_GELU_OUT : 0u));
+    d.BT_pitch = d.BL_pitch = d.C_pitch = s.K;
+    const uint64_t ws_bytes = m2d_scan_fwd_workspace(&d);
+    const Tensor buf = scratch(o.bytes + ws_bytes, xc);
+    char* const bp = static_cast<char*>(buf.data_ptr());
+    project(s, xc, p, o, bp);
+    d = scan_desc(s, dtype_of(xc), block_scan_in(s, xc, p, o, bp), d.flags);
+    d.workspace_bytes = ws_bytes;
+    Tensor y = at::empty({s.B, s.H, s.W, s.E}, xc.options());
+    block_scan(s, xc, d, bp + o.bytes, y);
+    return y;
 }
 
 // ---- the scan alone -----------------------------------------------------------------------------
@@ -291,12 +339,17 @@ Tensor pixel_rows(const Tensor& t, const Dims& s, int64_t* pitch) {
     return t.contiguous();
 }
 
-ScanIn scan_in(const Dims& s, const Tensor& x, const Tensor& dT, const Tensor& dL, const Tensor& AT, const Tensor& AL, const Tensor& BT, const Tensor& BL,
-               const Tensor& C, const Tensor& D) {
+// The scan's inputs, contiguous where they have to be (`keep` holds the copies).
+ScanIn scan_in(const Dims& s, const variable_list& v, variable_list& keep) {
+    keep.reserve(9);
+    for (size_t k = 0; k < 5; ++k) keep.push_back(v[k].contiguous());
     ScanIn in;
-    in.x = x.contiguous(); in.dT = dT.contiguous(); in.dL = dL.contiguous();
-    in.AT = AT.contiguous(); in.AL = AL.contiguous(); in.D = D.contiguous();
-    in.BT = pixel_rows(BT, s, &in.pBT); in.BL = pixel_rows(BL, s, &in.pBL); in.C = pixel_rows(C, s, &in.pC);
+    keep.push_back(pixel_rows(v[5], s, &in.pBT));
+    keep.push_back(pixel_rows(v[6], s, &in.pBL));
+    keep.push_back(pixel_rows(v[7], s, &in.pC));
+    keep.push_back(v[8].contiguous());
+    const void** dst[] = {&in.x, &in.dT, &in.dL, &in.AT, &in.AL, &in.BT, &in.BL, &in.C, &in.D};
+    for (size_t k = 0; k < 9; ++k) *dst[k] = keep[k].data_ptr();
     return in;
 }
 
@@ -312,7 +365,12 @@ public:
                           const Tensor& BT, const Tensor& BL, const Tensor& C, const Tensor& D, int64_t flags) {
         const c10::cuda::CUDAGuard guard(x.device());
         const Dims s = scan_dims(x, AT);
-        Tensor y = scan_forward(s, scan_in(s, x, dT, dL, AT, AL, BT, BL, C, D), (unsigned)flags);
+        variable_list keep;
+        m2d_scan_desc d = scan_desc(s, dtype_of(x), scan_in(s, {x, dT, dL, AT, AL, BT, BL, C, D}, keep), (unsigned)flags);
+        d.workspace_bytes = m2d_scan_fwd_workspace(&d);
+        const Tensor ws = scratch(d.workspace_bytes, x);
+        Tensor y = at::empty({s.B, s.H, s.W, s.E}, x.options());
+        block_scan(s, x, d, static_cast<char*>(ws.data_ptr()), y);
         ctx->save_for_backward({x, dT, dL, AT, AL, BT, BL, C, D});
         ctx->saved_data["flags"] = flags;
         return y;
@@ -321,17 +379,30 @@ public:
     static variable_list backward(AutogradContext* ctx, variable_list grads) {
         const at::NoGradGuard no_grad;
         const variable_list v = ctx->get_saved_variables();
-        const c10::cuda::CUDAGuard guard(v[0].device());
-        const Dims s = scan_dims(v[0], v[3]);
-        const Tensor gy = grads[0].to(v[0].scalar_type()).contiguous();
-        // one buffer for the three per-pixel gradients of B and C: one memset
-        const int64_t n = s.B * s.H * s.W * s.N;
-        const Tensor big = at::empty({3, s.B, s.H, s.W, s.N}, v[0].options());
-        char* bp = static_cast<char*>(big.data_ptr());
+        const Tensor& x = v[0];
+        const c10::cuda::CUDAGuard guard(x.device());
+        const Dims s = scan_dims(x, v[3]);
+        const unsigned flags = (unsigned)ctx->saved_data["flags"].toInt();
+        const Tensor gy = grads[0].to(x.scalar_type()).contiguous();
+        variable_list keep;
+        m2d_scan_desc d = scan_desc(s, dtype_of(x), scan_in(s, v, keep), flags);
+        // one buffer for the three per-pixel gradients of B and C, and one for the per-channel gradients where they
+        // share a type: the library then clears each with one memset
+        const int64_t n = s.B * s.H * s.W * s.N, en = s.E * s.N;
+        const Tensor big = at::empty({3, s.B, s.H, s.W, s.N}, x.options());
+        const bool one = !(flags & M2D_SCAN_A_LOG) || x.scalar_type() == at::kFloat;
+        const Tensor small = at::empty({2 * en + (one ? s.E : 0)}, one ? x.options() : x.options().dtype(at::kFloat));
+        Tensor dAT = at::as_strided(small, {s.E, s.N}, {s.N, 1}, 0), dAL = at::as_strided(small, {s.E, s.N}, {s.N, 1}, en);
+        Tensor dD = one ? at::as_strided(small, {s.E}, {1}, 2 * en) : at::empty({s.E}, x.options());
+        Tensor dx = at::empty(x.sizes(), x.options()), ddT = at::empty(x.sizes(), x.options()), ddL = at::empty(x.sizes(), x.options());
+        char* const bp = static_cast<char*>(big.data_ptr());
         const int64_t es = big.element_size();
-        const ScanGrads g = scan_backward(s, scan_in(s, v[0], v[1], v[2], v[3], v[4], v[5], v[6], v[7], v[8]), gy, bp, bp + n * es, bp + 2 * n * es, 0,
-                                          (unsigned)ctx->saved_data["flags"].toInt());
-        return {g.x, g.dT, g.dL, g.AT, g.AL, big.select(0, 0), big.select(0, 1), big.select(0, 2), g.D, Tensor()};
+        set_grads(d, gy.data_ptr(), {dx.data_ptr(), ddT.data_ptr(), ddL.data_ptr(), dAT.data_ptr(), dAL.data_ptr(), bp, bp + n * es, bp + 2 * n * es, dD.data_ptr(), 0});
+        d.workspace_bytes = m2d_scan_bwd_workspace(&d);
+        const Tensor ws = scratch(d.workspace_bytes, x);
+        d.workspace = ws.data_ptr();
+        check(m2d_scan_bwd(&d, stream_of(x)), "m2d_scan_bwd");
+        return {dx, ddT, ddL, dAT, dAL, big.select(0, 0), big.select(0, 1), big.select(0, 2), dD, Tensor()};
     }
 };
 

@@ -217,7 +217,7 @@ __global__ void __launch_bounds__(128, 1) xproj_wgrad_tc_kernel(const __grid_con
             }
         }
     }
-    if (!have && threadIdx.x == 0) atomicExch(a.status, 1);
+    if (!have && threadIdx.x == 0 && a.status) *reinterpret_cast<volatile int*>(a.status) = 1;
     tc_fence_before();
     __syncthreads();
     if (warp == 0) tmem_dealloc(tmem_d, tmem_cols);
