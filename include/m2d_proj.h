@@ -5,8 +5,8 @@
  * (proj_params, models/kernels/wavefront_cuda.py:63-95):
  *     proj           = x @ Wx^T                           (P, 2R+3N)  = [rT | rL | BT | BL | C]
  *     deltaT, deltaL = softplus(rT @ WT^T + bT), softplus(rL @ WL^T + bL)          (P, E)
- * and differentiates them with autograd.  On B200 the x projection is a well-shaped GEMM and
- * stays on the GEMM library; the rest is not:
+ * and differentiates them with autograd.  On B200 the x projection in bf16 is a well-shaped GEMM and
+ * stays on the GEMM library (in fp32 see m2d_rows_gemm_f32); the rest is not:
  *   - the two dt projections have an inner dimension of R = E/16 (4..36) and are followed by an
  *     element-wise softplus: three passes over (P,E) per direction;
  *   - their weight gradients, and the x projection's, are reductions over all P = B*H*W pixels
@@ -92,6 +92,16 @@ int m2d_xproj_wgrad(const m2d_proj_desc *desc, void *stream);
  * columns, or M2D_WGRAD_TC=0 in the environment).  Needs x and d_proj set; launches nothing.
  */
 int m2d_xproj_wgrad_on_tensor_cores(const m2d_proj_desc *desc);
+
+/*
+ * out (rows, n) = a (rows, k) @ w, or out += where `accumulate` is set; fp32, row-major and dense; `w` is (k, n), or
+ * (n, k) where `transposed` is set.  The x projection of fp32 pixels, x @ Wx^T, and its contribution to d_x,
+ * d_x += d_proj @ Wx, to the precision of fp32 products (split operands on the tensor cores).  n and k
+ * multiples of 4 and 16-byte aligned pointers (M2D_ERR_PITCH otherwise), at most 4 * M2D_PROJ_MAX_E
+ * columns or terms (M2D_ERR_TOO_LARGE).  No workspace.
+ */
+int m2d_rows_gemm_f32(int64_t rows, int32_t n, int32_t k, const float *a, const float *w, int32_t transposed,
+                      int32_t accumulate, float *out, void *stream);
 
 #ifdef __cplusplus
 }

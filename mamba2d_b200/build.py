@@ -16,7 +16,7 @@ INCLUDE = os.path.join(os.path.dirname(HERE), "include")
 OUT = os.path.join(HERE, "libm2d_scan.so")
 ENTRY = os.path.join(HERE, "_entry.so")  # native eager entry points (Python extension)
 OBJ = os.path.join(HERE, "_obj")          # per-source objects (git-ignored, not shipped)
-SOURCES = ["m2d_abi.cu", "m2d_scan_fwd.cu", "m2d_scan_bwd.cu", "m2d_scan_fwd_noalloc.cu", "m2d_proj.cu"]
+SOURCES = ["m2d_abi.cu", "m2d_scan_fwd.cu", "m2d_scan_bwd.cu", "m2d_scan_fwd_noalloc.cu", "m2d_proj.cu", "m2d_gemm.cu"]
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 
 

@@ -190,10 +190,13 @@ __global__ void __launch_bounds__(MAXT) dtproj_fwd_kernel(const ProjArgs a) {
 // per-warp [8 pixels][32 channels] slab of shared memory.  The warp then re-reads the slab with the
 // roles turned round -- a lane owns rank r (and a subset of the 8 pixels), holds W[e][r] of the
 // warp's 32 channels in registers and sums over them -- which yields the warp's share of
-// d_r = s @ W without any shuffle; the shares of the CTA's warps meet in shared memory.
-// Shared memory: rs[TP][RB], drs[TP][RB], slab[warps][8][36] and two buffers of the tile's g and
+// d_r = s @ W without any shuffle; the shares of the CTA's warps meet in shared memory: by adds, or from 32
+// ranks on, where 12 to 20 warps would meet in each, as a copy per warp (P = 784, E = 384: 20.7 -> 17.4 us,
+// P = 6272, E = 512: 57 -> 54; but 131 -> 150 at P = 401408, E = 64, where two warps meet).
+// Shared memory: rs[TP][RB], drs[1 or EB/32][TP][RB], slab[warps][8][36] and two buffers of the tile's g and
 // delta rows; the end-of-kernel reduction accS[RB+1][EB] reuses the same bytes.
 // ------------------------------------------------------------------------------------------------
+template <int RB> constexpr bool kShares = RB >= 32;
 constexpr int kSlabStride = 36;        // 32 channels + 4: rows of a slab start in different banks
 __device__ __forceinline__ float smem_value(const float* p) { return *p; }
 __device__ __forceinline__ float smem_value(const __nv_bfloat16* p) { return bf16_bits_to_float(*reinterpret_cast<const unsigned short*>(p)); }
@@ -203,9 +206,10 @@ __global__ void __launch_bounds__(MAXT) dtproj_bwd_kernel(const ProjArgs a) {
     extern __shared__ float sm[];
     float* accS = sm;                              // used after the tile loop only: overlays everything else
     float* rs = sm;
+    const int slices = kShares<RB> ? a.EB >> 5 : 1;          // copies of drs
     float* drs = rs + a.TP * RB;
-    float* slab = drs + a.TP * RB + (threadIdx.x >> 5) * (kProjIters * kSlabStride);
-    io_t* tiles = reinterpret_cast<io_t*>(drs + a.TP * RB + (blockDim.x >> 5) * (kProjIters * kSlabStride));   // [2 buffers][g | delta][TP*E]
+    float* slab = drs + slices * a.TP * RB + (threadIdx.x >> 5) * (kProjIters * kSlabStride);
+    io_t* tiles = reinterpret_cast<io_t*>(drs + slices * a.TP * RB + (blockDim.x >> 5) * (kProjIters * kSlabStride));   // [2 buffers][g | delta][TP*E]
     const int dir = blockIdx.y;
     const int lane = threadIdx.x & 31;
     const int te = threadIdx.x % a.EB, ps = threadIdx.x / a.EB;
@@ -290,7 +294,7 @@ __global__ void __launch_bounds__(MAXT) dtproj_bwd_kernel(const ProjArgs a) {
             const int idx = threadIdx.x + h * blockDim.x;
             if (idx < tile_elems) {
                 rs[idx] = nxt[h];
-                drs[idx] = 0.f;
+                if (!kShares<RB>) drs[idx] = 0.f;
             }
         }
         cp_async_wait_all();
@@ -344,28 +348,44 @@ __global__ void __launch_bounds__(MAXT) dtproj_bwd_kernel(const ProjArgs a) {
                 }
             }
 #pragma unroll
-            for (int h = 0; h < NH; ++h) atomicAdd(&drs[(k * a.PS + ps) * RB + h * RL + rl], sum[h]);
+            for (int h = 0; h < NH; ++h) {
+                const int at = (k * a.PS + ps) * RB + h * RL + rl;
+                if (kShares<RB>) drs[(e_slice >> 5) * tile_elems + at] = sum[h];
+                else atomicAdd(&drs[at], sum[h]);
+            }
         }
         __syncthreads();
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
             const int idx = threadIdx.x + h * blockDim.x;
             const int pp = idx / RB, r = idx % RB;
-            if (idx < tile_elems && r < a.R && p0 + pp < a.P) store1(d_proj, (p0 + pp) * a.pitch + col0 + r, drs[idx]);
+            if (idx < tile_elems && r < a.R && p0 + pp < a.P) {
+                float sum = 0.f;
+                for (int k = 0; k < slices; ++k) sum += drs[k * tile_elems + idx];
+                store1(d_proj, (p0 + pp) * a.pitch + col0 + r, sum);
+            }
         }
         __syncthreads();
     }
 
-    // CTA-level sum over the PS pixel rows of the block, then one partial per CTA
-    cp_async_wait_all();
-    __syncthreads();
-    for (int idx = threadIdx.x; idx < (RB + 1) * a.EB; idx += blockDim.x) accS[idx] = 0.f;
-    __syncthreads();
-#pragma unroll
-    for (int r = 0; r < RB; ++r) atomicAdd(&accS[r * a.EB + te], acc[r]);
-    atomicAdd(&accS[RB * a.EB + te], accb);
-    __syncthreads();
+    // one partial per CTA: the sum over the PS pixel rows of the block, a row at a time
     float* part = a.partials + ((size_t)dir * gridDim.x + blockIdx.x) * (RB + 1) * a.EB;
+    if (a.PS == 1) {
+#pragma unroll
+        for (int r = 0; r < RB; ++r) part[r * a.EB + te] = acc[r];
+        part[RB * a.EB + te] = accb;
+        return;
+    }
+    cp_async_wait_all();
+    for (int row = 0; row < a.PS; ++row) {
+        __syncthreads();
+        if (ps == row) {
+#pragma unroll
+            for (int r = 0; r < RB; ++r) accS[r * a.EB + te] = row ? accS[r * a.EB + te] + acc[r] : acc[r];
+            accS[RB * a.EB + te] = row ? accS[RB * a.EB + te] + accb : accb;
+        }
+    }
+    __syncthreads();
     for (int idx = threadIdx.x; idx < (RB + 1) * a.EB; idx += blockDim.x) part[idx] = accS[idx];
 }
 
@@ -561,7 +581,7 @@ static int launch_dt_finalize(const m2d_proj_desc* d, const ProjPlan& p, const f
 
 template <typename io_t, int RB>
 static int launch_dt_bwd(const m2d_proj_desc* d, const ProjArgs& a, const ProjPlan& p, cudaStream_t st) {
-    const size_t loop_bytes = (2 * (size_t)p.TP * RB + (size_t)(p.threads / 32) * kProjIters * kSlabStride) * sizeof(float) +
+    const size_t loop_bytes = ((size_t)(1 + (kShares<RB> ? p.EB / 32 : 1)) * p.TP * RB + (size_t)(p.threads / 32) * kProjIters * kSlabStride) * sizeof(float) +
                               (size_t)4 * p.TP * d->E * sizeof(io_t);
     const size_t tail_bytes = (size_t)(RB + 1) * p.EB * sizeof(float);
     const size_t smem = loop_bytes > tail_bytes ? loop_bytes : tail_bytes;

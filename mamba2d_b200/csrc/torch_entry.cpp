@@ -119,6 +119,17 @@ struct Projected {
 // out (rows, n) = a (rows, k) @ w, or += ; `w` is (n, k) if transposed, else (k, n).  Row-major operands are what
 // the library calls transposed ones.
 void gemm(const Tensor& like, int64_t rows, int64_t n, int64_t k, const void* a, const void* w, bool transposed, bool accumulate, void* out) {
+    // fp32: the library's tiles are 64 or 128 columns wide and its time for a few rows is several launches' worth.
+    // Against it, library / own: 110 / 60 us at 401408 x 64 -> 56, 52 / 45 at 100352 x 128 -> 64, 137 / 115 at
+    // 401408 x 56 -> 64, but 14 / 16 at 9805 x 60 -> 96 and 31 / 39 at 6272 x 512 -> 112; with few rows 14 / 8 at
+    // 196 x 320 -> 88 and 16 / 10 at 784 x 384 -> 96.
+    if (like.scalar_type() == at::kFloat && (n <= 64 || rows <= 2048)) {
+        const int rc = m2d_rows_gemm_f32(rows, (int)n, (int)k, static_cast<const float*>(a), static_cast<const float*>(w), transposed, accumulate,
+                                         static_cast<float*>(out), stream_of(like));
+        if (rc == M2D_OK) return;
+        // (an x that is not 16-byte aligned, or a contraction too long for the kernel's shared memory)
+        TORCH_CHECK(rc == M2D_ERR_PITCH || rc == M2D_ERR_TOO_LARGE, "m2d_rows_gemm_f32 failed: ", m2d_strerror(rc));
+    }
     const cudaDataType_t type = like.scalar_type() == at::kFloat ? CUDA_R_32F : CUDA_R_16BF;
     const float alpha = 1.f, beta = accumulate ? 1.f : 0.f;
     // (torch's handle: its stream, its workspace, its TF32 setting)

@@ -1,0 +1,28 @@
+"""fp32 products of pixel rows with a small matrix (csrc/m2d_gemm.cu) against fp64: both kernels, row tiles, column
+chunks and steps of the contraction that are not full, with and without accumulation."""
+import ctypes
+
+import pytest
+import torch
+
+from mamba2d_b200 import _lib
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("transposed,accumulate", [(1, 0), (0, 1)])
+@pytest.mark.parametrize("rows,n,k", [(1, 4, 4), (15, 60, 96), (196, 88, 320), (2047, 132, 640), (2500, 8, 12), (4801, 56, 64), (9805, 60, 96),
+                                      (19073, 16, 36), (20001, 64, 128), (30011, 36, 68), (40037, 44, 100), (9000, 148, 600)])
+def test_rows_gemm(rows, n, k, transposed, accumulate):
+    g = torch.Generator(device="cuda").manual_seed(rows + n + k)
+    a = torch.randn(rows, k, generator=g, device="cuda")
+    w = torch.randn(*((n, k) if transposed else (k, n)), generator=g, device="cuda")
+    out = torch.randn(rows, n, generator=g, device="cuda")
+    want = a.double() @ (w.t() if transposed else w).double() + (out.double() if accumulate else 0.0)
+    ptr = lambda t: ctypes.c_void_p(t.data_ptr())
+    rc = _lib.lib().m2d_rows_gemm_f32(ctypes.c_int64(rows), n, k, ptr(a), ptr(w), transposed, accumulate, ptr(out),
+                                      ctypes.c_void_p(torch.cuda.current_stream().cuda_stream))
+    assert rc == 0
+    scale = (k + 1) ** 0.5                           # of one result
+    assert float((out.double() - want).abs().max()) < 2e-6 * scale
+    assert float((out.double() - want).norm() / want.norm()) < 3e-7
