@@ -54,17 +54,20 @@ typedef struct m2d_proj_desc {
     void *d_WT, *d_WL;         /* (E,R)                                              [bwd] */
     void *d_bT, *d_bL;         /* (E)                                                [bwd] */
     void *d_Wx;                /* (K,E)      gradient of the x-projection weight     [wgrad] */
+    void *clear;               /* memory to zero on the side, or NULL                [fwd] */
+    uint64_t clear_bytes;      /* a multiple of 16; `clear` is 16-byte aligned (M2D_ERR_PITCH otherwise) */
     void *workspace;           /* scratch, 256-byte aligned, see m2d_proj_workspace() */
     uint64_t workspace_bytes;
 } m2d_proj_desc;
 
-/* Bytes of scratch the three calls below need for this problem (the maximum over the three). */
+/* Bytes of scratch that serve each of the calls below for this problem. */
 uint64_t m2d_proj_workspace(const m2d_proj_desc *desc);
 
 /*
  * dT = softplus(proj[:, 0:R] @ WT^T + bT), dL = softplus(proj[:, R:2R] @ WL^T + bL), softplus with
  * the reference's threshold (values above 20 pass through).  Replaces the two F.linear + F.softplus
- * pairs of proj_params (wavefront_cuda.py:84-85).  No workspace.
+ * pairs of proj_params (wavefront_cuda.py:84-85).  No workspace.  `clear`, if set, is zeroed by the same
+ * kernel: memory that a later launch on the stream wants zero (m2d_scan_fwd's boundary rows).
  */
 int m2d_dtproj_fwd(const m2d_proj_desc *desc, void *stream);
 
@@ -84,6 +87,12 @@ int m2d_dtproj_bwd(const m2d_proj_desc *desc, void *stream);
  * d_proj (M2D_ERR_PITCH otherwise).
  */
 int m2d_xproj_wgrad(const m2d_proj_desc *desc, void *stream);
+
+/*
+ * m2d_dtproj_bwd and m2d_xproj_wgrad after one another, with the two sums over partial results in one launch.  Columns
+ * [2R, K) of d_proj are the caller's, as for m2d_xproj_wgrad.
+ */
+int m2d_proj_bwd(const m2d_proj_desc *desc, void *stream);
 
 /*
  * 1 if m2d_xproj_wgrad would run this problem on the tensor cores (bf16 operands staged by TMA,

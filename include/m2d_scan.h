@@ -102,6 +102,13 @@ typedef enum m2d_status {
 #define M2D_SCAN_BC_ZEROED 0x20u
 
 /*
+ * M2D_SCAN_WS_CLEARED (m2d_scan_fwd): the first m2d_scan_fwd_cleared() bytes of the workspace are zero already.
+ * For callers that had an earlier kernel of theirs clear them (m2d_dtproj_fwd can): the boundary rows of a large
+ * map are half a gigabyte.
+ */
+#define M2D_SCAN_WS_CLEARED 0x40u
+
+/*
  * M2D_SCAN_TEST_WITHHOLD: test hook, rejected with M2D_ERR_FLAGS unless the environment variable
  * M2D_TEST_HOOKS is 1.  In a launch that runs several CTAs per image, the CTA that owns the first
  * band of image 0 never publishes that band's column counter and every wait gives up after a few
@@ -158,6 +165,10 @@ const char *m2d_strerror(int status);
  */
 uint64_t m2d_scan_fwd_workspace(const m2d_scan_desc *desc);
 uint64_t m2d_scan_bwd_workspace(const m2d_scan_desc *desc);
+
+/* Bytes at the start of its workspace that m2d_scan_fwd clears first, unless M2D_SCAN_WS_CLEARED is set (a
+ * multiple of 256; 0 for an invalid descriptor). */
+uint64_t m2d_scan_fwd_cleared(const m2d_scan_desc *desc);
 
 /*
  * Forward: y = sum_n h*C + x*D with h the two-neighbour recurrence.

@@ -25,7 +25,8 @@ EXPORTS = ("m2d_abi_version", "m2d_strerror", "m2d_scan_fwd_workspace", "m2d_sca
            "m2d_scan_fwd", "m2d_scan_bwd", "m2d_scan_fwd_noalloc", "m2d_scan_fwd_noalloc_need", "m2d_scan_fwd_status_offset",
            "m2d_scan_bwd_status_offset", "m2d_scan_fwd_chain", "m2d_scan_bwd_chain", "m2d_scan_chain_bound", "m2d_take_wait_failure",
            "m2d_proj_workspace", "m2d_dtproj_fwd", "m2d_dtproj_bwd", "m2d_xproj_wgrad",
-           "m2d_xproj_wgrad_on_tensor_cores")
+           "m2d_xproj_wgrad_on_tensor_cores", "m2d_proj_bwd", "m2d_rows_gemm_f32",
+           "m2d_scan_fwd_cleared")
 PROJ_MAX_E, PROJ_MAX_R = 640, 64     # M2D_PROJ_MAX_E / M2D_PROJ_MAX_R in include/m2d_proj.h
 
 
@@ -58,7 +59,7 @@ class ProjDesc(ctypes.Structure):
         ("bT", ctypes.c_void_p), ("bL", ctypes.c_void_p), ("dT", ctypes.c_void_p), ("dL", ctypes.c_void_p),
         ("g_dT", ctypes.c_void_p), ("g_dL", ctypes.c_void_p), ("d_proj", ctypes.c_void_p),
         ("d_WT", ctypes.c_void_p), ("d_WL", ctypes.c_void_p), ("d_bT", ctypes.c_void_p), ("d_bL", ctypes.c_void_p),
-        ("d_Wx", ctypes.c_void_p), ("workspace", ctypes.c_void_p), ("workspace_bytes", ctypes.c_uint64),
+        ("d_Wx", ctypes.c_void_p), ("clear", ctypes.c_void_p), ("clear_bytes", ctypes.c_uint64), ("workspace", ctypes.c_void_p), ("workspace_bytes", ctypes.c_uint64),
     ]
 
 
@@ -93,9 +94,14 @@ def lib():
             getattr(L, name).argtypes = [ctypes.POINTER(ScanDesc), ctypes.c_void_p]
         L.m2d_proj_workspace.restype = ctypes.c_uint64
         L.m2d_proj_workspace.argtypes = [ctypes.POINTER(ProjDesc)]
-        for name in ("m2d_dtproj_fwd", "m2d_dtproj_bwd", "m2d_xproj_wgrad"):
+        for name in ("m2d_dtproj_fwd", "m2d_dtproj_bwd", "m2d_xproj_wgrad", "m2d_proj_bwd"):
             getattr(L, name).restype = ctypes.c_int
             getattr(L, name).argtypes = [ctypes.POINTER(ProjDesc), ctypes.c_void_p]
+        L.m2d_rows_gemm_f32.restype = ctypes.c_int
+        L.m2d_rows_gemm_f32.argtypes = [ctypes.c_int64, ctypes.c_int32, ctypes.c_int32, ctypes.c_void_p, ctypes.c_void_p, ctypes.c_int32,
+                                        ctypes.c_int32, ctypes.c_void_p, ctypes.c_void_p]
+        L.m2d_scan_fwd_cleared.restype = ctypes.c_uint64
+        L.m2d_scan_fwd_cleared.argtypes = [ctypes.POINTER(ScanDesc)]
         L.m2d_xproj_wgrad_on_tensor_cores.restype = ctypes.c_int
         L.m2d_xproj_wgrad_on_tensor_cores.argtypes = [ctypes.POINTER(ProjDesc)]
         if L.m2d_abi_version() != ABI_VERSION:

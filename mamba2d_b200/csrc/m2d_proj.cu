@@ -30,6 +30,7 @@ struct ProjPlan {
 };
 
 struct ProjArgs {
+    Clear clear;
     int P, pitch, ntiles;              // every element index fits 31 bits (checked on the host)
     int E, R, EB, PS, TP;
     int params_f32;                    // weights and biases are fp32, rounded to io_t when read
@@ -78,7 +79,7 @@ static ProjPlan plan_proj(const m2d_proj_desc* d) {
     p.RB = d->R <= 4 ? 4 : d->R <= 8 ? 8 : d->R <= 16 ? 16 : d->R <= 32 ? 32 : 64;
     p.ntiles = (int)((d->P + p.TP - 1) / p.TP);
     p.gx = p.ntiles < 2 * sms ? p.ntiles : 2 * sms;
-    p.dt_partials = (size_t)2 * p.gx * (p.RB + 1) * p.EB * sizeof(float);
+    p.dt_partials = align256((size_t)2 * p.gx * (p.RB + 1) * p.EB * sizeof(float));
     p.K = 2 * d->R + 3 * d->N;
     p.tilesK = (p.K + 63) / 64;
     p.tilesE = (d->E + 63) / 64;
@@ -134,6 +135,7 @@ __global__ void __launch_bounds__(MAXT) dtproj_fwd_kernel(const ProjArgs a) {
     const io_t* proj = static_cast<const io_t*>(a.proj);
     io_t* out = static_cast<io_t*>(dir ? a.dL : a.dT);
     const int col0 = dir * a.R;
+    a.clear.run();
 
     float w[RB];
 #pragma unroll
@@ -389,37 +391,6 @@ __global__ void __launch_bounds__(MAXT) dtproj_bwd_kernel(const ProjArgs a) {
     for (int idx = threadIdx.x; idx < (RB + 1) * a.EB; idx += blockDim.x) part[idx] = accS[idx];
 }
 
-// d_W[e][r] (r < R) and d_b[e] (r == RB) = sum over CTAs of the partials.  Block (32, 8): 32
-// neighbouring results, the CTAs dealt round-robin to the 8 rows of the block.
-template <typename g_t>
-__global__ void dtproj_bwd_finalize(const float* __restrict__ partials, int ctas, int RB, int EB, int E, int R,
-                                    g_t* d_WT, g_t* d_WL, g_t* d_bT, g_t* d_bL) {
-    __shared__ float red[8][33];
-    const int n = 2 * (RB + 1) * EB;
-    const int idx = blockIdx.x * 32 + threadIdx.x;
-    const size_t step = (size_t)(RB + 1) * EB;
-    int dir = 0, r = 0, e = 0;
-    float s = 0.f;
-    if (idx < n) {
-        dir = idx / (int)step;
-        const int rem = idx % (int)step;
-        r = rem / EB;
-        e = rem % EB;
-        const float* src = partials + (size_t)dir * ctas * step + rem;
-#pragma unroll 4
-        for (int c = threadIdx.y; c < ctas; c += 8) s += src[(size_t)c * step];
-    }
-    red[threadIdx.y][threadIdx.x] = s;
-    __syncthreads();
-    if (threadIdx.y == 0 && idx < n && e < E && (r < R || r == RB)) {
-        float t = 0.f;
-#pragma unroll
-        for (int y = 0; y < 8; ++y) t += red[y][threadIdx.x];
-        if (r == RB) store1(dir ? d_bL : d_bT, e, t);
-        else store1(dir ? d_WL : d_WT, (long long)e * R + r, t);
-    }
-}
-
 // ------------------------------------------------------------------------------------------------
 // d_Wx[k][e] = sum_p d_proj[p][k] * x[p][e].  grid (slabs, tilesE, tilesK); a CTA of 256 threads
 // computes a 64x64 tile of the result over its slab of pixels, 32 pixels per shared-memory stage,
@@ -507,28 +478,60 @@ __global__ void __launch_bounds__(256) xproj_wgrad_kernel(const WgArgs a) {
     }
 }
 
-template <typename io_t>
-__global__ void xproj_wgrad_finalize(const float* __restrict__ partials, int slabs, long long ke, io_t* out) {   // block (32, 8)
+// ------------------------------------------------------------------------------------------------
+// The parameters' gradients from the partial results, d_W[e][r] (r < R), d_b[e] (r == RB) and d_Wx: block (32, 8), 32
+// neighbouring results, the partial results dealt round-robin to the 8 rows of the block.  One launch for the
+// sums of both kernels (a launch costs a small call as much as the sums).
+// ------------------------------------------------------------------------------------------------
+struct DtSums {
+    const float* partials;             // [dir][cta][RB+1][EB]
+    int ctas, RB, EB, E, R;
+    void *d_WT, *d_WL, *d_bT, *d_bL;
+    __host__ __device__ int blocks() const { return partials ? (2 * (RB + 1) * EB + 31) / 32 : 0; }
+};
+struct WgSums {
+    const float* partials;             // [slab][K*E]
+    int slabs;
+    long long ke;
+    void* d_Wx;
+    __host__ __device__ int blocks() const { return partials ? (int)((ke + 31) / 32) : 0; }
+};
+
+template <typename g_t>                // type of the parameters' gradients
+__global__ void proj_bwd_finalize(const DtSums dt, const WgSums wg) {
     __shared__ float red[8][33];
-    const long long idx = (long long)blockIdx.x * 32 + threadIdx.x;
+    const bool is_dt = (int)blockIdx.x < dt.blocks();
+    const long long idx = (long long)(is_dt ? blockIdx.x : blockIdx.x - dt.blocks()) * 32 + threadIdx.x;
+    const long long step = is_dt ? (dt.RB + 1) * dt.EB : wg.ke, n = is_dt ? 2 * step : wg.ke;
+    const int count = is_dt ? dt.ctas : wg.slabs;
+    const int dir = is_dt && idx >= step ? 1 : 0, rem = (int)(idx - dir * step);
     float s = 0.f;
-    if (idx < ke) {
+    if (idx < n) {
+        const float* src = (is_dt ? dt.partials + dir * count * step : wg.partials) + rem;
 #pragma unroll 4
-        for (int c = threadIdx.y; c < slabs; c += 8) s += partials[(size_t)c * ke + idx];
+        for (int c = threadIdx.y; c < count; c += 8) s += src[c * step];
     }
     red[threadIdx.y][threadIdx.x] = s;
     __syncthreads();
-    if (threadIdx.y == 0 && idx < ke) {
-        float t = 0.f;
+    if (threadIdx.y != 0 || idx >= n) return;
+    float t = 0.f;
 #pragma unroll
-        for (int y = 0; y < 8; ++y) t += red[y][threadIdx.x];
-        store1(out, idx, t);
+    for (int y = 0; y < 8; ++y) t += red[y][threadIdx.x];
+    if (!is_dt) {
+        store1(static_cast<g_t*>(wg.d_Wx), idx, t);
+        return;
     }
+    const int r = rem / dt.EB, e = rem % dt.EB;
+    if (e >= dt.E) return;
+    if (r == dt.RB) store1(static_cast<g_t*>(dir ? dt.d_bL : dt.d_bT), e, t);
+    else if (r < dt.R) store1(static_cast<g_t*>(dir ? dt.d_WL : dt.d_WT), (long long)e * dt.R + r, t);
 }
 
 // ------------------------------------------------------------------------------------------------
 // launchers
 // ------------------------------------------------------------------------------------------------
+static Clear clear_of(const m2d_proj_desc* d) { return Clear{static_cast<uint4*>(d->clear), d->clear ? (long long)(d->clear_bytes / 16) : 0}; }
+
 static ProjArgs proj_args(const m2d_proj_desc* d, const ProjPlan& p) {
     ProjArgs a;
     a.P = (int)d->P; a.pitch = (int)d->proj_pitch; a.ntiles = p.ntiles;
@@ -537,6 +540,7 @@ static ProjArgs proj_args(const m2d_proj_desc* d, const ProjPlan& p) {
     a.dT = d->dT; a.dL = d->dL; a.g_dT = d->g_dT; a.g_dL = d->g_dL;
     a.d_proj = d->d_proj;
     a.params_f32 = (d->flags & M2D_PROJ_PARAMS_F32) ? 1 : 0;
+    a.clear = clear_of(d);
     a.partials = static_cast<float*>(d->workspace);
     a.wide16 = d->E % 8 == 0 && aligned(d->g_dT, 16) && aligned(d->g_dL, 16) && aligned(d->dT, 16) && aligned(d->dL, 16);
     return a;
@@ -565,22 +569,19 @@ static int launch_dt_fwd(const ProjArgs& a, const ProjPlan& p, cudaStream_t st) 
     return cudaGetLastError() == cudaSuccess ? M2D_OK : M2D_ERR_LAUNCH;
 }
 
-// Sums of the parameters' gradients over the CTAs of the backward kernels.
 template <typename io_t>
-static int launch_dt_finalize(const m2d_proj_desc* d, const ProjPlan& p, const float* partials, int ctas, cudaStream_t st) {
-    const int n = 2 * (p.RB + 1) * p.EB;
-    auto finalize = [&](auto out) {                // element type of the parameters' gradients
-        typedef decltype(out) g_t;
-        dtproj_bwd_finalize<g_t><<<(n + 31) / 32, dim3(32, 8), 0, st>>>(partials, ctas, p.RB, p.EB, d->E, d->R, static_cast<g_t*>(d->d_WT),
-                                                                static_cast<g_t*>(d->d_WL), static_cast<g_t*>(d->d_bT), static_cast<g_t*>(d->d_bL));
-    };
-    if (d->flags & M2D_PROJ_PARAMS_F32) finalize(float{});
-    else finalize(io_t{});
+static int launch_sums(const m2d_proj_desc* d, const DtSums& dt, const WgSums& wg, cudaStream_t st) {
+    const int blocks = dt.blocks() + wg.blocks();
+    if (d->flags & M2D_PROJ_PARAMS_F32) proj_bwd_finalize<float><<<blocks, dim3(32, 8), 0, st>>>(dt, wg);
+    else proj_bwd_finalize<io_t><<<blocks, dim3(32, 8), 0, st>>>(dt, wg);
     return cudaGetLastError() == cudaSuccess ? M2D_OK : M2D_ERR_LAUNCH;
+}
+static DtSums dt_sums(const m2d_proj_desc* d, const ProjPlan& p, int ctas) {
+    return DtSums{static_cast<const float*>(d->workspace), ctas, p.RB, p.EB, d->E, d->R, d->d_WT, d->d_WL, d->d_bT, d->d_bL};
 }
 
 template <typename io_t, int RB>
-static int launch_dt_bwd(const m2d_proj_desc* d, const ProjArgs& a, const ProjPlan& p, cudaStream_t st) {
+static int launch_dt_bwd(const m2d_proj_desc* d, const ProjArgs& a, const ProjPlan& p, DtSums* sums, cudaStream_t st) {
     const size_t loop_bytes = ((size_t)(1 + (kShares<RB> ? p.EB / 32 : 1)) * p.TP * RB + (size_t)(p.threads / 32) * kProjIters * kSlabStride) * sizeof(float) +
                               (size_t)4 * p.TP * d->E * sizeof(io_t);
     const size_t tail_bytes = (size_t)(RB + 1) * p.EB * sizeof(float);
@@ -594,7 +595,8 @@ static int launch_dt_bwd(const m2d_proj_desc* d, const ProjArgs& a, const ProjPl
     const int gx = balanced_gx(kern, p, smem);
     kern<<<dim3(gx, 2), p.threads, smem, st>>>(a);
     if (cudaGetLastError() != cudaSuccess) return M2D_ERR_LAUNCH;
-    return launch_dt_finalize<io_t>(d, p, a.partials, gx, st);
+    *sums = dt_sums(d, p, gx);
+    return M2D_OK;
 }
 
 // Which kernels a call gets.  The tensor-core ones read and write rows of 16-byte pieces (E a multiple of 8,
@@ -626,6 +628,7 @@ static int launch_mma_fwd(const m2d_proj_desc* d, cudaStream_t st) {
     const size_t smem = mma_fwd_smem(chunk, a.nk);
     auto kern = dtproj_fwd_mma_kernel<io_t>;
     if (!allow_smem(reinterpret_cast<const void*>(kern), smem)) return M2D_ERR_LAUNCH;
+    a.clear = clear_of(d);
     const int chunks = (d->E + chunk - 1) / chunk, per_sm = resident_ctas(reinterpret_cast<const void*>(kern), 256, smem);
     long long gx = (long long)(per_sm > 0 ? per_sm : 1) * sm_count() / (2 * chunks);
     if (gx > tiles) gx = tiles;
@@ -634,7 +637,7 @@ static int launch_mma_fwd(const m2d_proj_desc* d, cudaStream_t st) {
 }
 
 template <int CH, int NCH, int NT>
-static int launch_mma_bwd(const m2d_proj_desc* d, const ProjPlan& p, cudaStream_t st) {
+static int launch_mma_bwd(const m2d_proj_desc* d, const ProjPlan& p, DtSums* sums, cudaStream_t st) {
     MmaBwdArgs a;
     a.P = (int)d->P; a.pitch = (int)d->proj_pitch; a.E = d->E; a.R = d->R; a.RB = p.RB; a.EB = p.EB;
     a.params_f32 = (d->flags & M2D_PROJ_PARAMS_F32) ? 1 : 0;
@@ -649,78 +652,92 @@ static int launch_mma_bwd(const m2d_proj_desc* d, const ProjPlan& p, cudaStream_
     const long long tiles = (d->P + MmaTile<CH>::kPix - 1) / MmaTile<CH>::kPix;
     if (gx > tiles) gx = tiles;
     if (gx > p.gx) gx = p.gx;                      // the workspace holds that many partial results
-    kern<<<dim3((unsigned)(gx < 1 ? 1 : gx), 2), 256, smem, st>>>(a);
+    if (gx < 1) gx = 1;
+    kern<<<dim3((unsigned)gx, 2), 256, smem, st>>>(a);
     if (cudaGetLastError() != cudaSuccess) return M2D_ERR_LAUNCH;
-    return launch_dt_finalize<__nv_bfloat16>(d, p, a.partials, gx < 1 ? 1 : (int)gx, st);
+    *sums = dt_sums(d, p, (int)gx);
+    return M2D_OK;
 }
 
 template <typename io_t>
-static int dispatch_dt(const m2d_proj_desc* d, bool bwd, cudaStream_t st) {
+static int dispatch_dt_fwd(const m2d_proj_desc* d, cudaStream_t st) {
+    if (mma_fwd_ok(d)) return launch_mma_fwd<io_t>(d, st);
     const ProjPlan p = plan_proj(d);
-    if (!bwd && mma_fwd_ok(d)) return launch_mma_fwd<io_t>(d, st);
-    if constexpr (sizeof(io_t) == 2) if (bwd && mma_bwd_ok(d)) {
+    const ProjArgs a = proj_args(d, p);
+    switch (p.RB) {
+        case 4: return launch_dt_fwd<io_t, 4>(a, p, st);
+        case 8: return launch_dt_fwd<io_t, 8>(a, p, st);
+        case 16: return launch_dt_fwd<io_t, 16>(a, p, st);
+        case 32: return launch_dt_fwd<io_t, 32>(a, p, st);
+        default: return launch_dt_fwd<io_t, 64>(a, p, st);
+    }
+}
+
+template <typename io_t>
+static int dispatch_dt_bwd(const m2d_proj_desc* d, const ProjPlan& p, DtSums* sums, cudaStream_t st) {
+    if constexpr (sizeof(io_t) == 2) if (mma_bwd_ok(d)) {
         // register blocks (chunks of channels, rank tiles) that cover the shipped widths (R = E / 16) closely and
         // everything else with some padding
         const int nch = (d->E + 127) / 128, nt = (d->R + 8) / 8;
-        if (d->E <= 64 && nt <= 1) return launch_mma_bwd<64, 1, 1>(d, p, st);
-        if (d->E <= 192 && nt <= 2) return launch_mma_bwd<64, 3, 2>(d, p, st);
-        if (nch <= 3 && nt <= 3) return launch_mma_bwd<128, 3, 3>(d, p, st);
-        if (nch <= 3) return launch_mma_bwd<128, 3, 5>(d, p, st);
-        return launch_mma_bwd<128, 5, 5>(d, p, st);
+        if (d->E <= 64 && nt <= 1) return launch_mma_bwd<64, 1, 1>(d, p, sums, st);
+        if (d->E <= 192 && nt <= 2) return launch_mma_bwd<64, 3, 2>(d, p, sums, st);
+        if (nch <= 3 && nt <= 3) return launch_mma_bwd<128, 3, 3>(d, p, sums, st);
+        if (nch <= 3) return launch_mma_bwd<128, 3, 5>(d, p, sums, st);
+        return launch_mma_bwd<128, 5, 5>(d, p, sums, st);
     }
     const ProjArgs a = proj_args(d, p);
     switch (p.RB) {
-        case 4: return bwd ? launch_dt_bwd<io_t, 4>(d, a, p, st) : launch_dt_fwd<io_t, 4>(a, p, st);
-        case 8: return bwd ? launch_dt_bwd<io_t, 8>(d, a, p, st) : launch_dt_fwd<io_t, 8>(a, p, st);
-        case 16: return bwd ? launch_dt_bwd<io_t, 16>(d, a, p, st) : launch_dt_fwd<io_t, 16>(a, p, st);
-        case 32: return bwd ? launch_dt_bwd<io_t, 32>(d, a, p, st) : launch_dt_fwd<io_t, 32>(a, p, st);
-        default: return bwd ? launch_dt_bwd<io_t, 64>(d, a, p, st) : launch_dt_fwd<io_t, 64>(a, p, st);
+        case 4: return launch_dt_bwd<io_t, 4>(d, a, p, sums, st);
+        case 8: return launch_dt_bwd<io_t, 8>(d, a, p, sums, st);
+        case 16: return launch_dt_bwd<io_t, 16>(d, a, p, sums, st);
+        case 32: return launch_dt_bwd<io_t, 32>(d, a, p, sums, st);
+        default: return launch_dt_bwd<io_t, 64>(d, a, p, sums, st);
     }
-}
-
-template <typename io_t>
-static void launch_wgrad_finalize(const m2d_proj_desc* d, const float* partials, int slabs, long long ke, cudaStream_t st) {
-    const dim3 block(32, 8);
-    const int grid = (int)((ke + 31) / 32);
-    if (d->flags & M2D_PROJ_PARAMS_F32) xproj_wgrad_finalize<float><<<grid, block, 0, st>>>(partials, slabs, ke, static_cast<float*>(d->d_Wx));
-    else xproj_wgrad_finalize<io_t><<<grid, block, 0, st>>>(partials, slabs, ke, static_cast<io_t*>(d->d_Wx));
 }
 
 // bf16 operands: the tensor-core kernel, when the problem meets its alignment rules (otherwise, and for
 // fp32, whose 1e-4 bar rules out tf32 operands, the CUDA-core kernel below).  Returns -1 for "not taken".
-static int launch_wgrad_tc(const m2d_proj_desc* d, const ProjPlan& p, cudaStream_t st) {
+static int launch_wgrad_tc(const m2d_proj_desc* d, const ProjPlan& p, float* partials, WgSums* sums, cudaStream_t st) {
     const TcPlan t = tc_plan(d->P, d->E, p.K, d->proj_pitch, d->x, d->d_proj, p.slabs);
     if (!t.ok) return -1;
     CUtensorMap map_a, map_b;
     if (!tc_make_map(&map_a, d->d_proj, d->P, p.K, d->proj_pitch) || !tc_make_map(&map_b, d->x, d->P, d->E, d->E)) return -1;
     TcArgs a;
     a.K = p.K; a.E = d->E; a.nbk = t.nbk; a.stages = t.stages; a.total_blocks = t.total_blocks; a.blocks_per_cta = t.blocks_per_cta;
-    a.partials = static_cast<float*>(d->workspace);
+    a.partials = partials;
     a.status = wait_failure_flag();      // host memory: a wait that gives up shows in m2d_take_wait_failure()
     if (!allow_smem(reinterpret_cast<const void*>(xproj_wgrad_tc_kernel), t.smem)) return M2D_ERR_LAUNCH;
     xproj_wgrad_tc_kernel<<<dim3(t.grid_x, t.ny), 128, t.smem, st>>>(map_a, map_b, a);
     if (cudaGetLastError() != cudaSuccess) return M2D_ERR_LAUNCH;
-    const long long ke = (long long)p.K * d->E;
-    launch_wgrad_finalize<__nv_bfloat16>(d, a.partials, t.grid_x, ke, st);
-    return cudaGetLastError() == cudaSuccess ? M2D_OK : M2D_ERR_LAUNCH;
+    *sums = WgSums{partials, t.grid_x, (long long)p.K * d->E, d->d_Wx};
+    return M2D_OK;
 }
 
 template <typename io_t>
-static int launch_wgrad(const m2d_proj_desc* d, cudaStream_t st) {
-    const ProjPlan p = plan_proj(d);
+static int launch_wgrad(const m2d_proj_desc* d, const ProjPlan& p, float* partials, WgSums* sums, cudaStream_t st) {
     if (sizeof(io_t) == 2) {
-        const int rc = launch_wgrad_tc(d, p, st);
+        const int rc = launch_wgrad_tc(d, p, partials, sums, st);
         if (rc >= 0) return rc;
     }
     WgArgs a;
     a.P = (int)d->P; a.pitch = (int)d->proj_pitch; a.E = d->E; a.K = p.K; a.rows_per_slab = p.rows_per_slab;
     a.x = d->x; a.d_proj = d->d_proj;
-    a.partials = static_cast<float*>(d->workspace);
+    a.partials = partials;
     xproj_wgrad_kernel<io_t><<<dim3(p.slabs, p.tilesE, p.tilesK), 256, 0, st>>>(a);
     if (cudaGetLastError() != cudaSuccess) return M2D_ERR_LAUNCH;
-    const long long ke = (long long)p.K * d->E;
-    launch_wgrad_finalize<io_t>(d, a.partials, p.slabs, ke, st);
-    return cudaGetLastError() == cudaSuccess ? M2D_OK : M2D_ERR_LAUNCH;
+    *sums = WgSums{partials, p.slabs, (long long)p.K * d->E, d->d_Wx};
+    return M2D_OK;
+}
+
+// Either half of the backward, or both with their sums in one launch; the partial results of the second lie behind
+// those of the first.
+template <typename io_t>
+static int launch_bwd(const m2d_proj_desc* d, const ProjPlan& p, bool dt, bool wgrad, cudaStream_t st) {
+    DtSums ds{};
+    WgSums ws{};
+    int rc = dt ? dispatch_dt_bwd<io_t>(d, p, &ds, st) : M2D_OK;
+    if (rc == M2D_OK && wgrad) rc = launch_wgrad<io_t>(d, p, reinterpret_cast<float*>(static_cast<char*>(d->workspace) + (dt ? p.dt_partials : 0)), &ws, st);
+    return rc == M2D_OK ? launch_sums<io_t>(d, ds, ws, st) : rc;
 }
 
 static bool workspace_ok(const m2d_proj_desc* d, size_t need) {
@@ -734,32 +751,47 @@ using namespace m2d;
 extern "C" uint64_t m2d_proj_workspace(const m2d_proj_desc* d) {
     if (check_proj(d) != M2D_OK) return 0;
     const ProjPlan p = plan_proj(d);
-    return align256(p.dt_partials > p.wg_partials ? p.dt_partials : p.wg_partials);
+    return p.dt_partials + p.wg_partials;
 }
 
 extern "C" int m2d_dtproj_fwd(const m2d_proj_desc* d, void* stream) {
     const int rc = check_proj(d);
     if (rc != M2D_OK) return rc;
     if (!d->proj || !d->WT || !d->WL || !d->bT || !d->bL || !d->dT || !d->dL) return M2D_ERR_NULL;
+    if (d->clear && (!aligned(d->clear, 16) || d->clear_bytes % 16)) return M2D_ERR_PITCH;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    return d->dtype == M2D_F32 ? dispatch_dt<float>(d, false, st) : dispatch_dt<__nv_bfloat16>(d, false, st);
+    return d->dtype == M2D_F32 ? dispatch_dt_fwd<float>(d, st) : dispatch_dt_fwd<__nv_bfloat16>(d, st);
 }
 
-extern "C" int m2d_dtproj_bwd(const m2d_proj_desc* d, void* stream) {
-    const int rc = check_proj(d);
-    if (rc != M2D_OK) return rc;
+static int check_dt_bwd(const m2d_proj_desc* d) {
     if (!d->proj || !d->WT || !d->WL || !d->dT || !d->dL || !d->g_dT || !d->g_dL || !d->d_proj || !d->d_WT || !d->d_WL ||
         !d->d_bT || !d->d_bL)
         return M2D_ERR_NULL;
-    {
-        // the g / delta rows are copied in 4-element pieces
-        const size_t al = d->dtype == M2D_F32 ? 16 : 8;
-        if (d->E % 4 != 0 || !aligned(d->g_dT, al) || !aligned(d->g_dL, al) || !aligned(d->dT, al) || !aligned(d->dL, al)) return M2D_ERR_PITCH;
-    }
-    if (!workspace_ok(d, plan_proj(d).dt_partials)) return M2D_ERR_WORKSPACE;
-    cudaStream_t st = static_cast<cudaStream_t>(stream);
-    return d->dtype == M2D_F32 ? dispatch_dt<float>(d, true, st) : dispatch_dt<__nv_bfloat16>(d, true, st);
+    // the g / delta rows are copied in 4-element pieces
+    const size_t al = d->dtype == M2D_F32 ? 16 : 8;
+    if (d->E % 4 != 0 || !aligned(d->g_dT, al) || !aligned(d->g_dL, al) || !aligned(d->dT, al) || !aligned(d->dL, al)) return M2D_ERR_PITCH;
+    return M2D_OK;
 }
+static int check_wgrad(const m2d_proj_desc* d) {
+    if (!d->x || !d->d_proj || !d->d_Wx) return M2D_ERR_NULL;
+    const size_t al = d->dtype == M2D_F32 ? 16 : 8;
+    if (d->E % 4 != 0 || d->proj_pitch % 4 != 0 || !aligned(d->x, al) || !aligned(d->d_proj, al)) return M2D_ERR_PITCH;
+    return M2D_OK;
+}
+static int proj_bwd(const m2d_proj_desc* d, bool dt, bool wgrad, void* stream) {
+    int rc = check_proj(d);
+    if (rc == M2D_OK && dt) rc = check_dt_bwd(d);
+    if (rc == M2D_OK && wgrad) rc = check_wgrad(d);
+    if (rc != M2D_OK) return rc;
+    const ProjPlan p = plan_proj(d);
+    if (!workspace_ok(d, (dt ? p.dt_partials : 0) + (wgrad ? p.wg_partials : 0))) return M2D_ERR_WORKSPACE;
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    return d->dtype == M2D_F32 ? launch_bwd<float>(d, p, dt, wgrad, st) : launch_bwd<__nv_bfloat16>(d, p, dt, wgrad, st);
+}
+
+extern "C" int m2d_dtproj_bwd(const m2d_proj_desc* d, void* stream) { return proj_bwd(d, true, false, stream); }
+extern "C" int m2d_xproj_wgrad(const m2d_proj_desc* d, void* stream) { return proj_bwd(d, false, true, stream); }
+extern "C" int m2d_proj_bwd(const m2d_proj_desc* d, void* stream) { return proj_bwd(d, true, true, stream); }
 
 extern "C" int m2d_xproj_wgrad_on_tensor_cores(const m2d_proj_desc* d) {
     if (check_proj(d) != M2D_OK || d->dtype != M2D_BF16 || !d->x || !d->d_proj) return 0;
@@ -768,15 +800,4 @@ extern "C" int m2d_xproj_wgrad_on_tensor_cores(const m2d_proj_desc* d) {
     if (!t.ok) return 0;
     CUtensorMap map_a, map_b;
     return tc_make_map(&map_a, d->d_proj, d->P, p.K, d->proj_pitch) && tc_make_map(&map_b, d->x, d->P, d->E, d->E) ? 1 : 0;
-}
-
-extern "C" int m2d_xproj_wgrad(const m2d_proj_desc* d, void* stream) {
-    const int rc = check_proj(d);
-    if (rc != M2D_OK) return rc;
-    if (!d->x || !d->d_proj || !d->d_Wx) return M2D_ERR_NULL;
-    const size_t al = d->dtype == M2D_F32 ? 16 : 8;
-    if (d->E % 4 != 0 || d->proj_pitch % 4 != 0 || !aligned(d->x, al) || !aligned(d->d_proj, al)) return M2D_ERR_PITCH;
-    if (!workspace_ok(d, plan_proj(d).wg_partials)) return M2D_ERR_WORKSPACE;
-    cudaStream_t st = static_cast<cudaStream_t>(stream);
-    return d->dtype == M2D_F32 ? launch_wgrad<float>(d, st) : launch_wgrad<__nv_bfloat16>(d, st);
 }

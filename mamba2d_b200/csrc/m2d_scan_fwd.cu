@@ -35,6 +35,11 @@ __global__ void __launch_bounds__(256, 2) m2d_fwd_kernel(const ScanArgs a) {
     forward_rows<io_t, VEC, false>(a, smem, params, D_own, blockIdx.x, gridDim.x, nb);
 }
 
+// The status word and, where CTAs of a wave launch read each other's, the boundary rows behind it.
+static size_t cleared_bytes(const m2d_scan_desc* d, const Plan& pl) {
+    return kStatusBytes + (pl.wave && pl.chain > 1 ? wave_edge_bytes(d, pl, false) : 0);
+}
+
 template <typename io_t>
 static int launch_fwd(const m2d_scan_desc* d, const Plan& pl, bool vec, char* ws, cudaStream_t st) {
     ScanArgs a;
@@ -42,9 +47,8 @@ static int launch_fwd(const m2d_scan_desc* d, const Plan& pl, bool vec, char* ws
     a.y = d->y;
     a.status = reinterpret_cast<int*>(ws);
     a.ring = reinterpret_cast<float4*>(ws + kStatusBytes);
-    // the status word and, where CTAs of a wave launch read each other's, the boundary rows behind it
-    const size_t zero = pl.wave && pl.chain > 1 ? kStatusBytes + wave_edge_bytes(d, pl, false) : sizeof(int);
-    if (cudaMemsetAsync(ws, 0, zero, st) != cudaSuccess) return M2D_ERR_LAUNCH;
+    const size_t zero = pl.wave && pl.chain > 1 ? cleared_bytes(d, pl) : sizeof(int);
+    if (!(d->flags & M2D_SCAN_WS_CLEARED) && cudaMemsetAsync(ws, 0, zero, st) != cudaSuccess) return M2D_ERR_LAUNCH;
     if (!pl.wave) return launch_sweep_kernel(vec ? m2d_fwd_kernel<io_t, true> : m2d_fwd_kernel<io_t, false>, a, pl, st);
     a.bnd = reinterpret_cast<float4*>(ws + kStatusBytes);
     a.bnd_rows = wave_rows(pl, false);
@@ -68,6 +72,11 @@ int launch_forward(const m2d_scan_desc* d, const Plan& pl, char* scratch, cudaSt
 extern "C" uint64_t m2d_scan_fwd_workspace(const m2d_scan_desc* d) {
     if (m2d::check_desc(d, false, false) != M2D_OK) return 0;
     return m2d::plan_fwd(d).scratch;
+}
+
+extern "C" uint64_t m2d_scan_fwd_cleared(const m2d_scan_desc* d) {
+    if (m2d::check_desc(d, false, false) != M2D_OK) return 0;
+    return m2d::cleared_bytes(d, m2d::plan_fwd(d));
 }
 
 extern "C" int64_t m2d_scan_fwd_status_offset(const m2d_scan_desc* d) {

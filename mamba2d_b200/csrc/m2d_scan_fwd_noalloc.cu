@@ -70,6 +70,7 @@ extern "C" int m2d_scan_fwd_noalloc(const m2d_scan_desc* d, void* stream) {
     int rc = m2d::check_desc(d, false, true);
     if (rc != M2D_OK) return rc;
     if (!d->y) return M2D_ERR_NULL;
+    if (d->flags & M2D_SCAN_WS_CLEARED) return M2D_ERR_FLAGS;      // the scratch is not the caller's
     const m2d::Plan pl = m2d::plan_noalloc(d);
     if (pl.scratch > M2D_NOALLOC_SCRATCH_BYTES) return M2D_ERR_TOO_LARGE;   // decided before any device work
     float4* ring = nullptr;

@@ -80,7 +80,7 @@ inline int check_desc(const m2d_scan_desc* d, bool bwd, bool need_ptrs) {
     if (d->dtype != M2D_F32 && d->dtype != M2D_BF16) return M2D_ERR_DTYPE;
     {
         unsigned known = M2D_SCAN_REVERSE | M2D_SCAN_A_LOG | M2D_SCAN_D_F32;
-        known |= bwd ? M2D_SCAN_BC_ZEROED : M2D_SCAN_GELU_OUT;      // an output activation exists in the forward only, gradients in the backward
+        known |= bwd ? M2D_SCAN_BC_ZEROED : M2D_SCAN_GELU_OUT | M2D_SCAN_WS_CLEARED;      // an output activation exists in the forward only, gradients in the backward
         if (test_hooks_enabled()) known |= M2D_SCAN_TEST_WITHHOLD;
         if (d->flags & ~known) return M2D_ERR_FLAGS;
     }

@@ -97,7 +97,20 @@ __device__ __forceinline__ float2 softplus_grad2(float2 d) {
 // W are dealt to the fragments so that a lane's results over four n-tiles are 8 neighbouring channels:
 // 16-byte stores.
 // ------------------------------------------------------------------------------------------------
+// Memory that a kernel zeroes before anything else, so that the stores drain while its weights and first rows
+// arrive: a memset of its own is a launch.  Worth it for small pieces; the 537 MB of boundary rows of a 1024x1024
+// map cost 95 us here, as a burst or next to each tile, against a memset's 87.
+struct Clear {
+    uint4* p;
+    long long n;
+    __device__ __forceinline__ void run() const {
+        const long long cta = ((long long)blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x, ctas = (long long)gridDim.x * gridDim.y * gridDim.z;
+        for (long long i = cta * blockDim.x + threadIdx.x; i < n; i += ctas * blockDim.x) p[i] = make_uint4(0u, 0u, 0u, 0u);
+    }
+};
+
 struct MmaFwdArgs {
+    Clear clear;
     int P, pitch, E, R, nk, chunk, params_f32;     // chunk: channels per CTA, a multiple of 32
     const void *proj, *WT, *WL, *bT, *bL;
     void *dT, *dL;
@@ -122,6 +135,7 @@ __global__ void __launch_bounds__(256) dtproj_fwd_mma_kernel(const MmaFwdArgs a)
     const void* W = dir ? a.WL : a.WT;
     const void* bp = dir ? a.bL : a.bT;
     constexpr bool F32 = sizeof(io_t) == 4;
+    a.clear.run();
 
     // W into B fragments: every element is read once, in order, and its parts go where the fragments want them
     for (int idx = threadIdx.x; idx < nt * nk * 32; idx += blockDim.x) Bf[idx] = make_uint2(0, 0);

@@ -138,11 +138,22 @@ void gemm(const Tensor& like, int64_t rows, int64_t n, int64_t k, const void* a,
     TORCH_CHECK(rc == CUBLAS_STATUS_SUCCESS, "cublasGemmEx failed: status ", (int)rc);
 }
 
-void project(const Dims& s, const Tensor& x, const BlockParams& p, const Projected& o, char* buf) {
+// What the forward scan wants cleared, if the projection kernel should do it: up to 64 MB, which saves the launch of
+// a memset (from there on the memset's higher rate is worth more).
+uint64_t clear_in_projection(m2d_scan_desc& d) {
+    const uint64_t n = m2d_scan_fwd_cleared(&d);
+    if (n > (64u << 20)) return 0;
+    d.flags |= M2D_SCAN_WS_CLEARED;
+    return n;
+}
+
+// `clear_bytes` at `clear` are zeroed by the way.
+void project(const Dims& s, const Tensor& x, const BlockParams& p, const Projected& o, char* buf, void* clear = nullptr, uint64_t clear_bytes = 0) {
     gemm(x, s.B * s.H * s.W, s.K, s.E, x.data_ptr(), p.Wx.data_ptr(), true, false, buf);
     m2d_proj_desc d = proj_desc(s, x, p);
     d.proj = buf;
     d.dT = buf + o.dT; d.dL = buf + o.dL;
+    d.clear = clear; d.clear_bytes = clear_bytes;
     check(m2d_dtproj_fwd(&d, stream_of(x)), "m2d_dtproj_fwd");
 }
 
@@ -196,10 +207,10 @@ public:
         const Projected o(s, x.element_size());
         const Tensor buf = scratch(o.bytes, x);
         char* const bp = static_cast<char*>(buf.data_ptr());
-        project(s, x, p, o, bp);
         m2d_scan_desc d = scan_desc(s, dtype_of(x), block_scan_in(s, x, p, o, bp), block_flags(p, reverse));
         d.workspace_bytes = m2d_scan_fwd_workspace(&d);
         const Tensor ws = scratch(d.workspace_bytes, x);
+        project(s, x, p, o, bp, ws.data_ptr(), clear_in_projection(d));
         Tensor y = at::empty({s.B, s.H, s.W, s.E}, x.options());
         block_scan(s, x, d, static_cast<char*>(ws.data_ptr()), y);
         // "full" recomputation keeps x and the parameters only
@@ -276,8 +287,7 @@ public:
         pd.d_WT = dWT.data_ptr(); pd.d_WL = dWL.data_ptr(); pd.d_bT = dbT.data_ptr(); pd.d_bL = dbL.data_ptr();
         pd.d_Wx = dWx.data_ptr();
         pd.workspace = t + at_ws;
-        check(m2d_dtproj_bwd(&pd, stream_of(x)), "m2d_dtproj_bwd");
-        check(m2d_xproj_wgrad(&pd, stream_of(x)), "m2d_xproj_wgrad");
+        check(m2d_proj_bwd(&pd, stream_of(x)), "m2d_proj_bwd");
         gemm(x, P, s.E, s.K, d_proj, p.Wx.data_ptr(), false, true, g.x);      // d_x = (scan's part) + d_proj @ Wx
 
         auto as = [](const Tensor& t, const Tensor& like) { return t.to(like.scalar_type()); };
@@ -329,7 +339,7 @@ c10::optional<Tensor> block(const Tensor& x, const Tensor& AT_log, const Tensor&
     const uint64_t ws_bytes = m2d_scan_fwd_workspace(&d);
     const Tensor buf = scratch(o.bytes + ws_bytes, xc);
     char* const bp = static_cast<char*>(buf.data_ptr());
-    project(s, xc, p, o, bp);
+    project(s, xc, p, o, bp, bp + o.bytes, clear_in_projection(d));
     d = scan_desc(s, dtype_of(xc), block_scan_in(s, xc, p, o, bp), d.flags);
     d.workspace_bytes = ws_bytes;
     Tensor y = at::empty({s.B, s.H, s.W, s.E}, xc.options());
