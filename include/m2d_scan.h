@@ -111,7 +111,7 @@ typedef enum m2d_status {
 /*
  * M2D_SCAN_TEST_WITHHOLD: test hook, rejected with M2D_ERR_FLAGS unless the environment variable
  * M2D_TEST_HOOKS is 1.  In a launch that runs several CTAs per image, the CTA that owns the first
- * band of image 0 never publishes that band's column counter and every wait gives up after a few
+ * band of image 0 never publishes that band's boundary row and every wait gives up after a few
  * hundred tries instead of a million: the CTA below runs out of patience, the kernel returns
  * normally and the status word is nonzero.  Nothing faults or hangs; the outputs are void.  It
  * exists so that the give-up path of the bounded waits can be exercised by a test.
