@@ -6,8 +6,8 @@
 // stream in 30 and 46 us (78 us), and 8 us for the 196 rows of one 14x14 image.
 //
 // Here a float is split into three bf16 parts, exact to 24 bits, and a product of floats is the six products of
-// parts that reach above 2^-24 of it, on the tensor cores (mma.sync m16n8k16; see proj_mma.cuh for why not
-// tcgen05: the split would have to go through shared memory, which is what bounds it).  The six are summed
+// parts that reach above 2^-24 of it, on the tensor cores (mma.sync m16n8k16: fragments are split in registers, where
+// tcgen05 would want the parts of every row staged in shared memory).  The six are summed
 // smallest first in a fresh accumulator per 16 terms and that sum is added to the running one by an ordinary
 // fp32 add: the tensor cores' own accumulation truncates, and over E / 16 steps that would show.
 #include <algorithm>
