@@ -605,8 +605,14 @@ static int launch_dt_bwd(const m2d_proj_desc* d, const ProjArgs& a, const ProjPl
 // backward 88 / 52 (100352, 128), 176 / 62 (25088, 320), but 21 / 25 at P = 784, where its tiles are fewer
 // than the SMs.  With fp32 tensors a product is six: the forward gains from about 3 M elements on (85 / 67,
 // 43 / 38 at P = 6272, E = 512; 6.2 / 8.9 at P = 9805, E = 96), the backward loses everywhere (131 / 149).
+// The six products of an fp32 call need six times the rank in shared memory: from 49 ranks on 256 channels a CTA do
+// not fit (R = 64: 298 KB), and the CUDA cores keep those calls.  (128 channels would fit, at E = 256, 640 and R = 64,
+// P = 25088, in 99, 193 us against 91, 201.)
+static int mma_fwd_chunk(int E) { return E < 256 ? (E + 31) / 32 * 32 : 256; }     // channels per CTA at most
+template <typename io_t> static bool mma_fwd_fits(const m2d_proj_desc* d) { return mma_fwd_smem(mma_fwd_chunk(d->E), mma_k<io_t>(d->R)) <= kMaxSmem; }
 static bool mma_fwd_ok(const m2d_proj_desc* d) {
-    return d->E % 8 == 0 && aligned(d->dT, 16) && aligned(d->dL, 16) && (d->dtype == M2D_BF16 || d->P * d->E >= 3000000);
+    if (d->E % 8 != 0 || !aligned(d->dT, 16) || !aligned(d->dL, 16)) return false;
+    return d->dtype == M2D_BF16 ? mma_fwd_fits<__nv_bfloat16>(d) : d->P * d->E >= 3000000 && mma_fwd_fits<float>(d);
 }
 static bool mma_bwd_ok(const m2d_proj_desc* d) {
     return d->dtype == M2D_BF16 && d->E % 8 == 0 && d->R < 40 && d->P >= 4736 && aligned(d->dT, 16) && aligned(d->dL, 16) &&
@@ -622,7 +628,7 @@ static int launch_mma_fwd(const m2d_proj_desc* d, cudaStream_t st) {
     // up to 256 channels per CTA (the tile of r is split and read once per chunk of channels); fewer while the
     // pixels alone do not give every SM a CTA
     const long long tiles = (d->P + 127) / 128;
-    int chunk = d->E < 256 ? (d->E + 31) / 32 * 32 : 256;
+    int chunk = mma_fwd_chunk(d->E);
     while (chunk > 32 && tiles * 2 * ((d->E + chunk - 1) / chunk) < sm_count()) chunk = (chunk / 2 + 31) / 32 * 32;
     a.chunk = chunk;
     const size_t smem = mma_fwd_smem(chunk, a.nk);

@@ -12,6 +12,7 @@
 namespace m2d {
 
 constexpr int kMaxDevices = 64;
+constexpr size_t kMaxSmem = 227 * 1024;     // shared memory a CTA can have
 
 // Index of the current device for the per-device caches below, or -1 (no device, or one beyond the caches).
 inline int device_index() {
