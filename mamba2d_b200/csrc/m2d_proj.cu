@@ -600,22 +600,40 @@ static int launch_dt_bwd(const m2d_proj_desc* d, const ProjArgs& a, const ProjPl
 }
 
 // Which kernels a call gets.  The tensor-core ones read and write rows of 16-byte pieces (E a multiple of 8,
-// aligned tensors), and the backward's sums fit its registers up to 39 ranks.  Measured, CUDA cores against
-// tensor cores: bf16 forward 90 / 55 us (P = 401408, E = 64), 59 / 36 (25088, 320), 8 / 6 (784, 384); bf16
-// backward 88 / 52 (100352, 128), 176 / 62 (25088, 320), but 21 / 25 at P = 784, where its tiles are fewer
-// than the SMs.  With fp32 tensors a product is six: the forward gains from about 3 M elements on (85 / 67,
-// 43 / 38 at P = 6272, E = 512; 6.2 / 8.9 at P = 9805, E = 96), the backward loses everywhere (131 / 149).
+// aligned tensors), and the backward's sums fit its registers up to 39 ranks.  Measured, CUDA cores / tensor cores in
+// us (R = E / 16, cold L2):
+//   forward, bf16: 90 / 55 (P = 401408, E = 64), 68 / 37 (25088, 320), 12 / 10 (784, 384): tensor cores always.
+//   forward, fp32 (a product is six), by elements P * E:
+//                E = 64      128       192       320       384       512       576
+//       2 M     14 / 16   16 / 16   18 / 23   25 / 26   25 / 33   40 / 29   35 / 43
+//       3.25 M  18 / 18   21 / 20   23 / 24   32 / 35   33 / 33   47 / 47   49 / 43
+//       4 M     21 / 21   24 / 25   27 / 31   37 / 35   37 / 45   51 / 47   57 / 54
+//       7 M     31 / 27   35 / 29   41 / 41   57 / 49   57 / 45   70 / 57   93 / 66
+//     The line is at 3 M.  (The tensor-core times are steps: its CTAs take whole tiles of 128 pixels.)
+//   backward, bf16:
+//       P       E = 64      128       320       384       512
+//       784     16 / 15   20 / 21   30 / 35   32 / 46   34 / 53
+//       3136    19 / 15   26 / 22   44 / 38   47 / 48   50 / 54
+//       4736    22 / 16   28 / 22   53 / 41   55 / 52   58 / 58
+//       6272    23 / 17   29 / 24   62 / 44   66 / 69   70 / 74
+//       12544   26 / 18   34 / 28  104 / 65  107 / 89  113 / 90
+//     The line is where its tiles of 64 pixels, in two directions, give every SM one (P = 4736 on 148 SMs); below
+//     it the wider stages lose.
+//   backward, fp32: the tensor cores lose everywhere (131 / 149 at P = 401408, E = 64).
 // The six products of an fp32 call need six times the rank in shared memory: from 49 ranks on 256 channels a CTA do
-// not fit (R = 64: 298 KB), and the CUDA cores keep those calls.  (128 channels would fit, at E = 256, 640 and R = 64,
-// P = 25088, in 99, 193 us against 91, 201.)
-static int mma_fwd_chunk(int E) { return E < 256 ? (E + 31) / 32 * 32 : 256; }     // channels per CTA at most
+// not fit (R = 64: 298 KB), and the CUDA cores keep those calls.  (128 channels would fit; at P = 25088, R = 64 they
+// take 99 us against 91 with E = 256, 193 against 201 with E = 640.)
+static int mma_fwd_chunk(int E) {      // channels per CTA at most: up to 256, the chunks of a wider call alike
+    const int n = (E + 255) / 256;
+    return ((E + n - 1) / n + 31) / 32 * 32;
+}
 template <typename io_t> static bool mma_fwd_fits(const m2d_proj_desc* d) { return mma_fwd_smem(mma_fwd_chunk(d->E), mma_k<io_t>(d->R)) <= kMaxSmem; }
 static bool mma_fwd_ok(const m2d_proj_desc* d) {
     if (d->E % 8 != 0 || !aligned(d->dT, 16) || !aligned(d->dL, 16)) return false;
     return d->dtype == M2D_BF16 ? mma_fwd_fits<__nv_bfloat16>(d) : d->P * d->E >= 3000000 && mma_fwd_fits<float>(d);
 }
 static bool mma_bwd_ok(const m2d_proj_desc* d) {
-    return d->dtype == M2D_BF16 && d->E % 8 == 0 && d->R < 40 && d->P >= 4736 && aligned(d->dT, 16) && aligned(d->dL, 16) &&
+    return d->dtype == M2D_BF16 && d->E % 8 == 0 && d->R < 40 && d->P >= 32 * sm_count() && aligned(d->dT, 16) && aligned(d->dL, 16) &&
            aligned(d->g_dT, 16) && aligned(d->g_dL, 16);
 }
 
@@ -626,7 +644,9 @@ static int launch_mma_fwd(const m2d_proj_desc* d, cudaStream_t st) {
     a.params_f32 = (d->flags & M2D_PROJ_PARAMS_F32) ? 1 : 0;
     a.proj = d->proj; a.WT = d->WT; a.WL = d->WL; a.bT = d->bT; a.bL = d->bL; a.dT = d->dT; a.dL = d->dL;
     // up to 256 channels per CTA (the tile of r is split and read once per chunk of channels); fewer while the
-    // pixels alone do not give every SM a CTA
+    // pixels alone do not give every SM a CTA.  Chunks of one size: with 256 + 64 channels at E = 320 half the CTAs had
+    // a quarter of the work (fp32, us, before / now: P = 9375, 36 / 27; 21875, 57 / 49; 50000, 100 / 77; E = 384, P = 41666,
+    // 94 / 82; E = 576, P = 6944, 65 / 54; bf16 E = 320, P = 12544, 25 / 22)
     const long long tiles = (d->P + 127) / 128;
     int chunk = mma_fwd_chunk(d->E);
     while (chunk > 32 && tiles * 2 * ((d->E + chunk - 1) / chunk) < sm_count()) chunk = (chunk / 2 + 31) / 32 * 32;
