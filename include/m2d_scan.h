@@ -114,9 +114,15 @@ typedef enum m2d_status {
  * band of image 0 never publishes that band's boundary row and every wait gives up after a few
  * hundred tries instead of a million: the CTA below runs out of patience, the kernel returns
  * normally and the status word is nonzero.  Nothing faults or hangs; the outputs are void.  It
- * exists so that the give-up path of the bounded waits can be exercised by a test.
+ * exists so that the give-up path of the bounded waits can be exercised by a test.  In m2d_scan_bwd it acts
+ * on the recompute sweep.
+ * M2D_SCAN_TEST_WITHHOLD_UP (m2d_scan_bwd only): the same in the adjoint sweep, where the last band of every image
+ * hands nothing up.
+ * M2D_SCAN_TEST_REPORT: with one of the two, the failure also counts for m2d_take_wait_failure().
  */
 #define M2D_SCAN_TEST_WITHHOLD 0x100u
+#define M2D_SCAN_TEST_WITHHOLD_UP 0x200u
+#define M2D_SCAN_TEST_REPORT 0x400u
 
 /*
  * Problem descriptor.  Tensor layouts are the ones the reference op receives:
@@ -198,9 +204,17 @@ int m2d_scan_bwd_chain(const m2d_scan_desc *desc);
  * 1 if a wait between CTAs has given up in any launch of this process since the last call of this
  * function, else 0; does not synchronise.  (The kernel that gives up writes to host memory, so a failure
  * shows here as soon as it has happened; the status word of the launch's own workspace says which one
- * it was.)  Launches made under M2D_SCAN_TEST_WITHHOLD do not count.
+ * it was.)  Launches made under M2D_SCAN_TEST_WITHHOLD or ..._UP count with M2D_SCAN_TEST_REPORT only.
  */
 int m2d_take_wait_failure(void);
+
+/*
+ * A number, the same as at an earlier call unless a failure that counts for m2d_take_wait_failure() has shown in
+ * between; takes nothing and does not synchronise.  A caller that has waited for its launch and finds the number it
+ * had before the launch need not read the status word.  -1: failures do not show here (no host word could be had);
+ * read the status word.
+ */
+int64_t m2d_wait_failure_mark(void);
 
 /*
  * The rule every launch applies when it picks, or has to shorten, the number of CTAs per image:

@@ -17,6 +17,8 @@ M2D_SCAN_A_LOG = 4
 M2D_SCAN_D_F32 = 0x10
 M2D_SCAN_BC_ZEROED = 0x20
 M2D_SCAN_TEST_WITHHOLD = 0x100
+M2D_SCAN_TEST_WITHHOLD_UP = 0x200
+M2D_SCAN_TEST_REPORT = 0x400
 M2D_PROJ_PARAMS_F32 = 1
 ABI_VERSION = 4
 NOALLOC_SCRATCH_BYTES = 32 << 20     # M2D_NOALLOC_SCRATCH_BYTES in include/m2d_scan.h
@@ -24,6 +26,7 @@ NOALLOC_SCRATCH_BYTES = 32 << 20     # M2D_NOALLOC_SCRATCH_BYTES in include/m2d_
 EXPORTS = ("m2d_abi_version", "m2d_strerror", "m2d_scan_fwd_workspace", "m2d_scan_bwd_workspace",
            "m2d_scan_fwd", "m2d_scan_bwd", "m2d_scan_fwd_noalloc", "m2d_scan_fwd_noalloc_need", "m2d_scan_fwd_status_offset",
            "m2d_scan_bwd_status_offset", "m2d_scan_fwd_chain", "m2d_scan_bwd_chain", "m2d_scan_chain_bound", "m2d_take_wait_failure",
+           "m2d_wait_failure_mark",
            "m2d_proj_workspace", "m2d_dtproj_fwd", "m2d_dtproj_bwd", "m2d_xproj_wgrad",
            "m2d_xproj_wgrad_on_tensor_cores", "m2d_proj_bwd", "m2d_rows_gemm_f32",
            "m2d_scan_fwd_cleared")
@@ -92,6 +95,7 @@ def lib():
         for name in ("m2d_scan_fwd", "m2d_scan_bwd", "m2d_scan_fwd_noalloc"):
             getattr(L, name).restype = ctypes.c_int
             getattr(L, name).argtypes = [ctypes.POINTER(ScanDesc), ctypes.c_void_p]
+        L.m2d_wait_failure_mark.restype = ctypes.c_int64
         L.m2d_proj_workspace.restype = ctypes.c_uint64
         L.m2d_proj_workspace.argtypes = [ctypes.POINTER(ProjDesc)]
         for name in ("m2d_dtproj_fwd", "m2d_dtproj_bwd", "m2d_xproj_wgrad", "m2d_proj_bwd"):
@@ -117,6 +121,11 @@ def strerror(code):
 def check(code, what):
     if code != 0:
         raise RuntimeError(f"{what}: {strerror(code)} (status {code})")
+
+
+def take_wait_failure():
+    """m2d_take_wait_failure() of the loaded library; False where none is loaded."""
+    return _LIB is not None and _LIB.m2d_take_wait_failure() != 0
 
 
 _ENTRY = None

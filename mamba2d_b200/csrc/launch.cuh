@@ -26,10 +26,11 @@ inline void fill_common_args(ScanArgs& a, const m2d_scan_desc* d, const Plan& pl
     a.act = (d->flags & M2D_SCAN_GELU_OUT) ? 1 : 0;
     a.a_log = (d->flags & M2D_SCAN_A_LOG) ? 1 : 0;
     a.d_f32 = (d->flags & M2D_SCAN_D_F32) || d->dtype == M2D_F32 ? 1 : 0;
-    const bool hook = (d->flags & M2D_SCAN_TEST_WITHHOLD) != 0;
-    a.withhold = hook ? 1 : 0;
+    const bool hook = (d->flags & (M2D_SCAN_TEST_WITHHOLD | M2D_SCAN_TEST_WITHHOLD_UP)) != 0;
+    a.withhold = (d->flags & M2D_SCAN_TEST_WITHHOLD) ? 1 : 0;
+    a.mute_up = (d->flags & M2D_SCAN_TEST_WITHHOLD_UP) ? pl.nbands - 1 : 0;
     a.wait_limit = hook ? (1 << 9) : kWaitPolls;
-    a.host_flag = pl.chain > 1 && !hook ? wait_failure_flag() : nullptr;
+    a.host_flag = pl.chain > 1 && (!hook || (d->flags & M2D_SCAN_TEST_REPORT)) ? wait_failure_flag() : nullptr;
 }
 
 // Launch a sweep kernel on the plan's grid.  CTAs of a chain wait on one another, so every CTA of a

@@ -23,11 +23,33 @@ int* wait_failure_flag() {
     return flag;
 }
 
+// What the host has seen of that word: failures so far, and whether one has not been taken yet.
+static std::mutex g_seen_mutex;
+static int64_t g_seen = 0;
+static bool g_pending = false;
+
+static bool look_at_flag() {        // false: there is no word
+    int* f = wait_failure_flag();
+    if (f && __atomic_exchange_n(f, 0, __ATOMIC_ACQ_REL) != 0) {
+        ++g_seen;
+        g_pending = true;
+    }
+    return f != nullptr;
+}
+
 }  // namespace m2d
 
 extern "C" int m2d_take_wait_failure(void) {
-    int* f = m2d::wait_failure_flag();
-    return f ? __atomic_exchange_n(f, 0, __ATOMIC_RELAXED) != 0 : 0;
+    std::lock_guard<std::mutex> lock(m2d::g_seen_mutex);
+    m2d::look_at_flag();
+    const bool was = m2d::g_pending;
+    m2d::g_pending = false;
+    return was ? 1 : 0;
+}
+
+extern "C" int64_t m2d_wait_failure_mark(void) {
+    std::lock_guard<std::mutex> lock(m2d::g_seen_mutex);
+    return m2d::look_at_flag() ? m2d::g_seen : -1;
 }
 
 extern "C" int m2d_abi_version(void) { return M2D_ABI_VERSION; }

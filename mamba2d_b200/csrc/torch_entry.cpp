@@ -12,6 +12,9 @@
 // autocast to another type); the caller then takes the op-by-op path.
 #include <ATen/autocast_mode.h>
 #include <ATen/cuda/CUDAContext.h>
+#include <ATen/cuda/CUDAEvent.h>
+#include <ATen/cuda/CachingHostAllocator.h>
+#include <ATen/cuda/CUDAGraphsUtils.cuh>
 #include <c10/cuda/CUDAGuard.h>
 #include <cublas_v2.h>
 #include <torch/extension.h>
@@ -31,10 +34,50 @@ int dtype_of(const Tensor& t) { return t.scalar_type() == at::kFloat ? M2D_F32 :
 bool supported(const Tensor& t) { return t.scalar_type() == at::kFloat || t.scalar_type() == at::kBFloat16; }
 Tensor scratch(uint64_t bytes, const Tensor& like) { return at::empty({(int64_t)bytes}, like.options().dtype(at::kByte)); }
 
-// A failed wait of an earlier launch (see m2d_take_wait_failure) surfaces here, like any other
-// asynchronous error.
+// What a call is to do besides its arithmetic; as one number, which a node keeps between its passes.
+struct Options {
+    unsigned flags = 0;      // of the scan
+    bool check = true;       // raise where a launch went wrong, see below
+    bool defer = false;      // ... a forward's in the node's backward
+    unsigned fwd_hooks = 0, bwd_hooks = 0;      // M2D_SCAN_TEST_... bits
+    int64_t packed() const { return (int64_t)flags | (int64_t)check << 16 | (int64_t)defer << 17 | (int64_t)fwd_hooks << 20 | (int64_t)bwd_hooks << 40; }
+    static Options of(int64_t v) { return {(unsigned)(v & 0xffff), (v >> 16 & 1) != 0, (v >> 17 & 1) != 0, (unsigned)(v >> 20 & 0xfffff), (unsigned)(v >> 40)}; }
+};
+
+// CTAs of one image wait on one another, and a wait that gives up makes the launch's outputs void.  The call that made
+// the launch raises then, and no gradient that such a launch is part of is handed out: a pass without gradients and a
+// backward pass wait for their scan before they return (not for the kernels behind it), a forward pass with gradients
+// is looked at by its backward, so that a training step waits once.  Not where no CTA waits on another, not during a
+// stream capture, where nothing can be waited for, and not where the caller does without (M2D_CHECK_STATUS=0).  What
+// the waiting costs is the host's lead over the GPU; us a call, without / with: 1x14x14x320 30.7 / 45, 5x37x53x96
+// 71.7 / 87, 1x1024x1024x64 2115 / 2135, training 6x45x31x192 346 / 388, 2x200x336x64 bf16 1467 / 1500.
+bool looked_at(const Options& opt, int chain) {
+    return opt.check && chain > 1 && at::cuda::currentStreamCaptureStatusMayInitCtx() == at::cuda::CaptureStatus::None;
+}
+[[noreturn]] void raise_void(const char* what) {
+    m2d_take_wait_failure();       // told here, not once more by the next call
+    TORCH_CHECK(false, what, ": a wait between CTAs timed out; the results of this call are invalid");
+}
+// A launch's status word is worth reading only where some launch of the process has failed since `mark`.
+void check_status(int64_t mark, const void* status, const char* what) {
+    if (mark >= 0 && m2d_wait_failure_mark() == mark) return;
+    int word = 0;
+    C10_CUDA_CHECK(cudaMemcpy(&word, status, sizeof(word), cudaMemcpyDeviceToHost));
+    if (word != 0) raise_void(what);
+}
+
+// A failed wait of a launch that no call has looked at (one replayed from a graph, one made without the check, or
+// the weight gradient's kernel, whose result is then NaN) surfaces here, like any other asynchronous error.
 void check_waits() {
     TORCH_CHECK(!m2d_take_wait_failure(), "wavefront scan: a wait between CTAs of an earlier launch timed out; the results of that launch are invalid");
+}
+
+// Whether a call on these makes a node.
+bool wants_grad(std::initializer_list<const Tensor*> inputs) {
+    bool grad = false;
+    if (at::GradMode::is_enabled())
+        for (const Tensor* t : inputs) grad = grad || t->requires_grad();
+    return grad;
 }
 
 struct Dims {
@@ -169,14 +212,55 @@ ScanIn block_scan_in(const Dims& s, const Tensor& x, const BlockParams& p, const
     return in;
 }
 
-unsigned block_flags(const BlockParams& p, bool reverse) { return M2D_SCAN_A_LOG | (p.f32 ? M2D_SCAN_D_F32 : 0u) | (reverse ? M2D_SCAN_REVERSE : 0u); }
+unsigned block_flags(const BlockParams& p, const Options& opt) { return M2D_SCAN_A_LOG | (p.f32 ? M2D_SCAN_D_F32 : 0u) | opt.flags; }
 
-// y, given the projections in `buf`; the scan's scratch goes to `ws`.
-void block_scan(const Dims& s, const Tensor& x, m2d_scan_desc& d, char* ws, const Tensor& y) {
+// y, given the projections in `buf`; the scan's scratch goes to `ws`.  Where the launch is looked at later: its status
+// word, on its way to host memory (the scratch does not live that long).
+Tensor forward_scan(const Tensor& x, m2d_scan_desc& d, char* ws, const Tensor& y, const Options& opt) {
     d.y = y.data_ptr();
     d.workspace = ws;
+    d.flags |= opt.fwd_hooks;
+    const bool look = looked_at(opt, m2d_scan_fwd_chain(&d));
+    const int64_t mark = m2d_wait_failure_mark();
     check(m2d_scan_fwd(&d, stream_of(x)), "m2d_scan_fwd");
+    if (!look) return Tensor();
+    const auto stream = at::cuda::getCurrentCUDAStream(x.get_device());
+    const void* const status = ws + m2d_scan_fwd_status_offset(&d);
+    if (opt.defer) {
+        const Tensor word = at::empty({1}, at::TensorOptions().dtype(at::kInt).pinned_memory(true));
+        C10_CUDA_CHECK(cudaMemcpyAsync(word.data_ptr(), status, sizeof(int), cudaMemcpyDeviceToHost, stream));
+        // (a graph may be dropped, and the word with it, before the copy has landed)
+        at::cuda::CachingHostAllocator_recordEvent(word.data_ptr(), word.storage().data_ptr().get_context(), stream);
+        return word;
+    }
+    C10_CUDA_CHECK(cudaStreamSynchronize(stream));
+    check_status(mark, status, "m2d_scan_fwd");
+    return Tensor();
 }
+
+// The backward's scan, and the look at both passes once it is through; its status word has to last until then.
+class BackwardScan {
+public:
+    BackwardScan(const m2d_scan_desc& d, const Tensor& x, const Options& opt, const Tensor& forward_word)
+        : forward_(forward_word), own_(looked_at(opt, m2d_scan_bwd_chain(&d))), mark_(m2d_wait_failure_mark()),
+          status_(static_cast<const char*>(d.workspace) + m2d_scan_bwd_status_offset(&d)) {
+        check(m2d_scan_bwd(&d, stream_of(x)), "m2d_scan_bwd");
+        if (own_ || forward_.defined()) done_.record(at::cuda::getCurrentCUDAStream(x.get_device()));
+    }
+    void finish() {
+        if (!own_ && !forward_.defined()) return;
+        done_.synchronize();       // (the forward's word was copied on this stream, before)
+        if (forward_.defined() && *static_cast<const volatile int*>(forward_.data_ptr()) != 0) raise_void("m2d_scan_fwd");
+        if (own_) check_status(mark_, status_, "m2d_scan_bwd");
+    }
+
+private:
+    Tensor forward_;
+    bool own_;
+    int64_t mark_;
+    const void* status_;
+    at::cuda::CUDAEvent done_;
+};
 
 Dims block_dims(const Tensor& x, const Tensor& A_log, const Tensor& WT) {
     Dims s;
@@ -199,7 +283,8 @@ BlockParams block_params(const Tensor& x, const Tensor& AT_log, const Tensor& AL
 class BlockFn : public torch::autograd::Function<BlockFn> {
 public:
     static Tensor forward(AutogradContext* ctx, const Tensor& x_, const Tensor& AT_log, const Tensor& AL_log, const Tensor& Wx, const Tensor& WT,
-                          const Tensor& bT, const Tensor& WL, const Tensor& bL, const Tensor& D, bool full, bool reverse) {
+                          const Tensor& bT, const Tensor& WL, const Tensor& bL, const Tensor& D, bool full, int64_t options) {
+        const Options opt = Options::of(options);
         const c10::cuda::CUDAGuard guard(x_.device());
         const Tensor x = x_.contiguous();
         const Dims s = block_dims(x, AT_log, WT);
@@ -207,16 +292,16 @@ public:
         const Projected o(s, x.element_size());
         const Tensor buf = scratch(o.bytes, x);
         char* const bp = static_cast<char*>(buf.data_ptr());
-        m2d_scan_desc d = scan_desc(s, dtype_of(x), block_scan_in(s, x, p, o, bp), block_flags(p, reverse));
+        m2d_scan_desc d = scan_desc(s, dtype_of(x), block_scan_in(s, x, p, o, bp), block_flags(p, opt));
         d.workspace_bytes = m2d_scan_fwd_workspace(&d);
         const Tensor ws = scratch(d.workspace_bytes, x);
         project(s, x, p, o, bp, ws.data_ptr(), clear_in_projection(d));
         Tensor y = at::empty({s.B, s.H, s.W, s.E}, x.options());
-        block_scan(s, x, d, static_cast<char*>(ws.data_ptr()), y);
+        ctx->saved_data["word"] = forward_scan(x, d, static_cast<char*>(ws.data_ptr()), y, opt);
         // "full" recomputation keeps x and the parameters only
         if (full) ctx->save_for_backward({x, AT_log, AL_log, Wx, WT, bT, WL, bL, D});
         else ctx->save_for_backward({x, AT_log, AL_log, Wx, WT, bT, WL, bL, D, buf, p.Wx});
-        ctx->saved_data["reverse"] = reverse;
+        ctx->saved_data["options"] = options;
         return y;
     }
 
@@ -225,7 +310,8 @@ public:
         const variable_list v = ctx->get_saved_variables();
         const Tensor& x = v[0];
         const c10::cuda::CUDAGuard guard(x.device());
-        const bool reverse = ctx->saved_data["reverse"].toBool();
+        const Options opt = Options::of(ctx->saved_data["options"].toInt());
+        check_waits();
         const Dims s = block_dims(x, v[1], v[4]);
         const bool saved = v.size() > 9;
         const BlockParams p = block_params(x, v[1], v[2], saved ? v[10] : v[3], v[4], v[5], v[6], v[7], v[8]);
@@ -237,12 +323,13 @@ public:
         // scratch: gradients of the projections' outputs, then what the two library workspaces share
         Carve c;
         const int64_t at_dT = c.take(P * s.E * es), at_dL = c.take(P * s.E * es), at_proj = c.take(P * s.K * es), at_buf = saved ? 0 : c.take(o.bytes);
-        m2d_scan_desc sd = scan_desc(s, dtype_of(x), ScanIn{}, block_flags(p, reverse) | (f32 ? M2D_SCAN_BC_ZEROED : 0u));
+        m2d_scan_desc sd = scan_desc(s, dtype_of(x), ScanIn{}, block_flags(p, opt) | opt.bwd_hooks | (f32 ? M2D_SCAN_BC_ZEROED : 0u));
         sd.BT_pitch = sd.BL_pitch = sd.C_pitch = sd.d_BC_pitch = s.K;
         m2d_proj_desc pd = proj_desc(s, x, p);
         sd.workspace_bytes = m2d_scan_bwd_workspace(&sd);
         pd.workspace_bytes = m2d_proj_workspace(&pd);
-        const int64_t at_ws = c.take((int64_t)std::max(sd.workspace_bytes, pd.workspace_bytes));
+        constexpr int64_t kStatus = 256;       // the scan's status word stays as it is while the projections' scratch takes the place of the rest
+        const int64_t at_ws = c.take((int64_t)std::max(sd.workspace_bytes, pd.workspace_bytes + kStatus));
         const Tensor tmp = scratch(c.bytes, x);
         char* const t = static_cast<char*>(tmp.data_ptr());
         char* const d_proj = t + at_proj;
@@ -278,7 +365,7 @@ public:
         set_grads(sd, gy.data_ptr(), g);
         sd.workspace = t + at_ws;
         sd.workspace_bytes = ws_bytes;
-        check(m2d_scan_bwd(&sd, stream_of(x)), "m2d_scan_bwd");
+        BackwardScan scan(sd, x, opt, ctx->saved_data["word"].toTensor());
 
         pd.x = x.data_ptr(); pd.proj = buf;
         pd.dT = const_cast<char*>(buf) + o.dT; pd.dL = const_cast<char*>(buf) + o.dL;
@@ -286,10 +373,11 @@ public:
         pd.d_proj = d_proj;
         pd.d_WT = dWT.data_ptr(); pd.d_WL = dWL.data_ptr(); pd.d_bT = dbT.data_ptr(); pd.d_bL = dbL.data_ptr();
         pd.d_Wx = dWx.data_ptr();
-        pd.workspace = t + at_ws;
+        pd.workspace = t + at_ws + kStatus;
         check(m2d_proj_bwd(&pd, stream_of(x)), "m2d_proj_bwd");
         gemm(x, P, s.E, s.K, d_proj, p.Wx.data_ptr(), false, true, g.x);      // d_x = (scan's part) + d_proj @ Wx
 
+        scan.finish();
         auto as = [](const Tensor& t, const Tensor& like) { return t.to(like.scalar_type()); };
         return {dx, as(dAT, v[1]), as(dAL, v[2]), as(dWx, v[3]), dWT, dbT, dWL, dbL, dD, Tensor(), Tensor()};
     }
@@ -318,14 +406,14 @@ bool block_applies(const Tensor& x, const Tensor& AT_log, const Tensor& AL_log, 
 }
 
 c10::optional<Tensor> block(const Tensor& x, const Tensor& AT_log, const Tensor& AL_log, const Tensor& Wx, const Tensor& WT, const Tensor& bT,
-                            const Tensor& WL, const Tensor& bL, const Tensor& D, bool full, bool reverse, bool gelu) {
+                            const Tensor& WL, const Tensor& bL, const Tensor& D, bool full, bool reverse, bool gelu, bool check_status,
+                            unsigned fwd_hooks, unsigned bwd_hooks) {
     if (!block_applies(x, AT_log, AL_log, Wx, WT, bT, WL, bL, D)) return c10::nullopt;
     check_waits();
-    bool grad = false;
-    if (at::GradMode::is_enabled())
-        for (const Tensor* t : {&x, &AT_log, &AL_log, &Wx, &WT, &bT, &WL, &bL, &D}) grad = grad || t->requires_grad();
+    const bool grad = wants_grad({&x, &AT_log, &AL_log, &Wx, &WT, &bT, &WL, &bL, &D});
+    const Options opt{reverse ? M2D_SCAN_REVERSE : 0u, check_status, grad, fwd_hooks, bwd_hooks};
     if (grad) {
-        Tensor y = BlockFn::apply(x, AT_log, AL_log, Wx, WT, bT, WL, bL, D, full, reverse);
+        Tensor y = BlockFn::apply(x, AT_log, AL_log, Wx, WT, bT, WL, bL, D, full, opt.packed());
         return gelu ? at::gelu(y) : y;
     }
     const at::AutoDispatchBelowADInplaceOrView below;
@@ -334,7 +422,7 @@ c10::optional<Tensor> block(const Tensor& x, const Tensor& AT_log, const Tensor&
     const Dims s = block_dims(xc, AT_log, WT);
     const BlockParams p = block_params(xc, AT_log, AL_log, Wx, WT, bT, WL, bL, D);
     const Projected o(s, xc.element_size());
-    m2d_scan_desc d = scan_desc(s, dtype_of(xc), ScanIn{}, block_flags(p, reverse) | (gelu ? M2D_SCAN_GELU_OUT : 0u));
+    m2d_scan_desc d = scan_desc(s, dtype_of(xc), ScanIn{}, block_flags(p, opt) | (gelu ? M2D_SCAN_GELU_OUT : 0u));
     d.BT_pitch = d.BL_pitch = d.C_pitch = s.K;
     const uint64_t ws_bytes = m2d_scan_fwd_workspace(&d);
     const Tensor buf = scratch(o.bytes + ws_bytes, xc);
@@ -343,7 +431,7 @@ c10::optional<Tensor> block(const Tensor& x, const Tensor& AT_log, const Tensor&
     d = scan_desc(s, dtype_of(xc), block_scan_in(s, xc, p, o, bp), d.flags);
     d.workspace_bytes = ws_bytes;
     Tensor y = at::empty({s.B, s.H, s.W, s.E}, xc.options());
-    block_scan(s, xc, d, bp + o.bytes, y);
+    forward_scan(xc, d, bp + o.bytes, y, opt);
     return y;
 }
 
@@ -383,17 +471,18 @@ Dims scan_dims(const Tensor& x, const Tensor& AT) {
 class ScanFn : public torch::autograd::Function<ScanFn> {
 public:
     static Tensor forward(AutogradContext* ctx, const Tensor& x, const Tensor& dT, const Tensor& dL, const Tensor& AT, const Tensor& AL,
-                          const Tensor& BT, const Tensor& BL, const Tensor& C, const Tensor& D, int64_t flags) {
+                          const Tensor& BT, const Tensor& BL, const Tensor& C, const Tensor& D, int64_t options) {
+        const Options opt = Options::of(options);
         const c10::cuda::CUDAGuard guard(x.device());
         const Dims s = scan_dims(x, AT);
         variable_list keep;
-        m2d_scan_desc d = scan_desc(s, dtype_of(x), scan_in(s, {x, dT, dL, AT, AL, BT, BL, C, D}, keep), (unsigned)flags);
+        m2d_scan_desc d = scan_desc(s, dtype_of(x), scan_in(s, {x, dT, dL, AT, AL, BT, BL, C, D}, keep), opt.flags);
         d.workspace_bytes = m2d_scan_fwd_workspace(&d);
         const Tensor ws = scratch(d.workspace_bytes, x);
         Tensor y = at::empty({s.B, s.H, s.W, s.E}, x.options());
-        block_scan(s, x, d, static_cast<char*>(ws.data_ptr()), y);
+        ctx->saved_data["word"] = forward_scan(x, d, static_cast<char*>(ws.data_ptr()), y, opt);
         ctx->save_for_backward({x, dT, dL, AT, AL, BT, BL, C, D});
-        ctx->saved_data["flags"] = flags;
+        ctx->saved_data["options"] = options;
         return y;
     }
 
@@ -403,15 +492,16 @@ public:
         const Tensor& x = v[0];
         const c10::cuda::CUDAGuard guard(x.device());
         const Dims s = scan_dims(x, v[3]);
-        const unsigned flags = (unsigned)ctx->saved_data["flags"].toInt();
+        const Options opt = Options::of(ctx->saved_data["options"].toInt());
+        check_waits();
         const Tensor gy = grads[0].to(x.scalar_type()).contiguous();
         variable_list keep;
-        m2d_scan_desc d = scan_desc(s, dtype_of(x), scan_in(s, v, keep), flags);
+        m2d_scan_desc d = scan_desc(s, dtype_of(x), scan_in(s, v, keep), opt.flags | opt.bwd_hooks);
         // one buffer for the three per-pixel gradients of B and C, and one for the per-channel gradients where they
         // share a type: the library then clears each with one memset
         const int64_t n = s.B * s.H * s.W * s.N, en = s.E * s.N;
         const Tensor big = at::empty({3, s.B, s.H, s.W, s.N}, x.options());
-        const bool one = !(flags & M2D_SCAN_A_LOG) || x.scalar_type() == at::kFloat;
+        const bool one = !(opt.flags & M2D_SCAN_A_LOG) || x.scalar_type() == at::kFloat;
         const Tensor small = at::empty({2 * en + (one ? s.E : 0)}, one ? x.options() : x.options().dtype(at::kFloat));
         Tensor dAT = at::as_strided(small, {s.E, s.N}, {s.N, 1}, 0), dAL = at::as_strided(small, {s.E, s.N}, {s.N, 1}, en);
         Tensor dD = one ? at::as_strided(small, {s.E}, {1}, 2 * en) : at::empty({s.E}, x.options());
@@ -422,13 +512,13 @@ public:
         d.workspace_bytes = m2d_scan_bwd_workspace(&d);
         const Tensor ws = scratch(d.workspace_bytes, x);
         d.workspace = ws.data_ptr();
-        check(m2d_scan_bwd(&d, stream_of(x)), "m2d_scan_bwd");
+        BackwardScan(d, x, opt, ctx->saved_data["word"].toTensor()).finish();
         return {dx, ddT, ddL, dAT, dAL, big.select(0, 0), big.select(0, 1), big.select(0, 2), dD, Tensor()};
     }
 };
 
 c10::optional<Tensor> scan(const Tensor& x, const Tensor& dT, const Tensor& dL, const Tensor& AT, const Tensor& AL, const Tensor& BT, const Tensor& BL,
-                           const Tensor& C, const Tensor& D, bool reverse, bool a_log) {
+                           const Tensor& C, const Tensor& D, bool reverse, bool a_log, bool check_status, unsigned fwd_hooks, unsigned bwd_hooks) {
     // (whatever does not fit goes to the op-by-op path, which names the reason)
     if (!x.is_cuda() || !supported(x) || x.dim() != 4 || AT.dim() != 2 || AT.size(0) != x.size(3)) return c10::nullopt;
     const Dims s = scan_dims(x, AT);
@@ -443,12 +533,20 @@ c10::optional<Tensor> scan(const Tensor& x, const Tensor& dT, const Tensor& dL, 
     for (const Tensor* t : {&AT, &AL})
         if (t->scalar_type() != (a_log ? at::kFloat : x.scalar_type()) || t->device() != x.device()) return c10::nullopt;
     check_waits();
-    return ScanFn::apply(x, dT, dL, AT, AL, BT, BL, C, D, (int64_t)((reverse ? M2D_SCAN_REVERSE : 0u) | (a_log ? M2D_SCAN_A_LOG : 0u)));
+    return ScanFn::apply(x, dT, dL, AT, AL, BT, BL, C, D,
+                         Options{(reverse ? M2D_SCAN_REVERSE : 0u) | (a_log ? M2D_SCAN_A_LOG : 0u), check_status,
+                                 wants_grad({&x, &dT, &dL, &AT, &AL, &BT, &BL, &C, &D}), fwd_hooks, bwd_hooks}.packed());
 }
 
 }  // namespace
 
 PYBIND11_MODULE(_entry, m) {
-    m.def("block", &block, "wavefront_scan_cuda as one autograd node; None where it does not apply");
-    m.def("scan", &scan, "wf_cuda_fn_pr as a native autograd node; None where it does not apply");
+    // check_status: raise where a launch whose CTAs wait on one another went wrong (looked_at); the hooks are test hooks of include/m2d_scan.h
+    using pybind11::arg;
+    m.def("block", &block, "wavefront_scan_cuda as one autograd node; None where it does not apply", arg("x"), arg("AT_log"), arg("AL_log"),
+          arg("x_proj_w"), arg("dt_projT_w"), arg("dt_projT_b"), arg("dt_projL_w"), arg("dt_projL_b"), arg("D"), arg("full"), arg("reverse"),
+          arg("gelu"), arg("check_status") = true, arg("fwd_hooks") = 0u, arg("bwd_hooks") = 0u);
+    m.def("scan", &scan, "wf_cuda_fn_pr as a native autograd node; None where it does not apply", arg("x"), arg("dT"), arg("dL"), arg("AT"),
+          arg("AL"), arg("BT"), arg("BL"), arg("C"), arg("D"), arg("reverse"), arg("a_log"), arg("check_status") = true, arg("fwd_hooks") = 0u,
+          arg("bwd_hooks") = 0u);
 }

@@ -48,7 +48,7 @@ __device__ __forceinline__ void wave_adjoint_band(const ScanArgs& a, char* smem,
     const int q0 = band * kWaveRows;
     const size_t id = ((size_t)slot * ln.cgroups + ln.cg) * a.nbands + band;
     float* pull = band + 1 < a.nbands && chv > 0 ? reinterpret_cast<float*>(a.bnd_up) + id * W * EF : nullptr;
-    float* push = band > 0 && chv > 0 ? reinterpret_cast<float*>(a.bnd_up) + (id - 1) * W * EF : nullptr;
+    float* push = band > 0 && band != a.mute_up && chv > 0 ? reinterpret_cast<float*>(a.bnd_up) + (id - 1) * W * EF : nullptr;
     const float* top_row = band > 0 && chv > 0 ? reinterpret_cast<const float*>(a.bnd) + (id - 1) * W * EF : nullptr;   // as the recompute sweep left it
     const bool lrow = q0 + w < H, crow = q0 + r < H, row0 = q0 + r == 0;
     const int lpix = lrow ? scan_pixel(a, b, q0 + w, W - 1) : 0, cpix = crow ? scan_pixel(a, b, q0 + r, W - 1) : 0;

@@ -49,6 +49,7 @@ def _check_status(kind, d, ws):
     off = getattr(L, f"m2d_scan_{kind}_status_offset")(ctypes.byref(d))
     if off >= 0 and _status_word(ws, off) != 0:
         what = "output is" if kind == "fwd" else "gradients are"
+        _lib.take_wait_failure()             # told here, not once more by the next call of a native entry point
         raise RuntimeError(f"m2d_scan_{kind}: a wait between row-warps or CTAs timed out; the {what} invalid")
 
 
@@ -502,8 +503,10 @@ def _native(x):
     """The native entry points (csrc/torch_entry.cpp) if an eager call on ``x`` may take them, else None.
 
     They run the same kernels as the functions of this file without the Python, the parameter casts and
-    the copies around them.  Not taken: while a compiler traces, when every launch is to be checked
-    (M2D_CHECK_STATUS=1: the check synchronises), with another library in place of the package's own
+    the copies around them, and check the same launches by default (those that run several CTAs per image): a
+    call without gradients waits for its scan, a backward for its own (not for the kernels behind it) and raises
+    for either pass.  Not taken: while a
+    compiler traces, when every launch is to be checked (M2D_CHECK_STATUS=1), with another library in place of the package's own
     (M2D_SCAN_LIB), and while an operator body in ``_EAGER`` is replaced."""
     if (not x.is_cuda or torch.compiler.is_compiling() or _CHECK_STATUS == "1" or _lib.LIB_PATH != _lib.DEFAULT_LIB_PATH
             or _EAGER != _EAGER_BODIES):
@@ -520,7 +523,7 @@ class wf_cuda_fn_pr(torch.autograd.Function):
     def apply(cls, x, deltaT, deltaL, AT, AL, BT, BL, C, D, reverse=False, a_log=False):
         native = _native(x)
         if native is not None:
-            y = native.scan(x, deltaT, deltaL, AT, AL, BT, BL, C, D, bool(reverse), bool(a_log))
+            y = native.scan(x, deltaT, deltaL, AT, AL, BT, BL, C, D, bool(reverse), bool(a_log), _CHECK_STATUS != "0")
             if y is not None:
                 return y
         return super().apply(x, deltaT, deltaL, AT, AL, BT, BL, C, D, reverse, a_log)
@@ -600,7 +603,7 @@ def wavefront_scan_cuda(x, AT_log, AL_log, x_proj_w, dt_projT_w, dt_projT_b, dt_
     native = _native(x)
     if native is not None:
         y = native.block(x, AT_log, AL_log, x_proj_w, dt_projT_w, dt_projT_b, dt_projL_w, dt_projL_b, D, recomp == "full",
-                         reverse, act_out == "gelu")
+                         reverse, act_out == "gelu", _CHECK_STATUS != "0")
         if y is not None:
             return y
 

@@ -5,7 +5,11 @@ Every such wait has a limit; when one runs out the kernel still returns normally
 nonzero status word in its workspace.  A test hook (descriptor flag M2D_SCAN_TEST_WITHHOLD, honoured
 only under M2D_TEST_HOOKS=1) makes exactly that happen: one producer never publishes its progress and
 the limits are a few hundred tries.  Nothing here faults or hangs the GPU: a wait runs out and the
-kernel ends."""
+kernel ends.
+
+The native entry points (csrc/torch_entry.cpp) read the word before they return: of a pass without gradients, or of
+both passes in the backward, so that no gradient of a launch that went wrong is handed out.  A launch they were told
+not to look at is reported by the next call."""
 import ctypes
 
 import pytest
@@ -55,6 +59,122 @@ def test_a_withheld_counter_makes_the_wait_give_up(monkeypatch):
     torch.cuda.synchronize()
     assert wc._status_word(ws, off) == 0
     assert rel_err(y.cpu().numpy(), cpu.forward(inp, "f64")) < 1e-4
+
+
+def _large_map():
+    inp = inputs.make_inputs(1, 96, 64, 64, 16, seed=3)
+    return inp, {k: v.cuda() for k, v in inp.items()}
+
+
+def _grads(y, leaves, gy):
+    return torch.autograd.grad(y, leaves, gy)
+
+
+def _scan(dev, grad, check=True, fwd=0, bwd=0):
+    leaves = [dev[k].detach().requires_grad_(grad) for k in ORDER]
+    return _lib.entry().scan(*leaves, False, False, check, fwd, bwd), leaves
+
+
+def _block(dev, grad, check=True, fwd=0, bwd=0):
+    w = inputs.make_module_params(64, 16, seed=5)
+    names = ("AT_log", "AL_log", "x_proj_w", "dt_projT_w", "dt_projT_b", "dt_projL_w", "dt_projL_b", "D")
+    leaves = [t.detach().requires_grad_(grad) for t in (dev["x"], *(w[k].cuda() for k in names))]
+    return _lib.entry().block(*leaves, False, False, False, check, fwd, bwd), leaves
+
+
+DOWN, UP, REPORT = _lib.M2D_SCAN_TEST_WITHHOLD, _lib.M2D_SCAN_TEST_WITHHOLD_UP, _lib.M2D_SCAN_TEST_REPORT
+
+
+@pytest.mark.parametrize("call", [_scan, _block])
+def test_a_native_forward_raises_in_the_call_that_went_wrong(call, monkeypatch):
+    monkeypatch.setenv("M2D_TEST_HOOKS", "1")
+    inp, dev = _large_map()
+    want, _ = call(dev, False)
+    with pytest.raises(RuntimeError, match="m2d_scan_fwd: a wait between CTAs timed out"):
+        call(dev, False, fwd=DOWN | REPORT)
+    with torch.no_grad(), pytest.raises(RuntimeError, match="m2d_scan_fwd: a wait between CTAs timed out"):
+        call(dev, True, fwd=DOWN | REPORT)
+    y, _ = call(dev, False)                                  # told once: the next call knows nothing of it
+    assert torch.equal(y, want)
+    assert _lib.lib().m2d_take_wait_failure() == 0
+
+
+@pytest.mark.parametrize("call", [_scan, _block])
+def test_no_gradient_of_a_forward_that_went_wrong_is_handed_out(call, monkeypatch):
+    monkeypatch.setenv("M2D_TEST_HOOKS", "1")
+    inp, dev = _large_map()
+    y, leaves = call(dev, True, fwd=DOWN | REPORT)
+    assert torch.isnan(y).any()                              # a row that never came reads as NaN
+    assert _lib.lib().m2d_take_wait_failure() == 1           # (or the next call would tell, before the backward does)
+    with pytest.raises(RuntimeError, match="m2d_scan_fwd: a wait between CTAs timed out"):
+        _grads(y, leaves, dev["gy"])
+    y, leaves = call(dev, True)
+    assert all(torch.isfinite(g).all() for g in _grads(y, leaves, dev["gy"]))
+    y, leaves = call(dev, True)
+    del y, leaves                                            # a graph that is dropped with its word on the way
+    assert _lib.lib().m2d_take_wait_failure() == 0
+
+
+@pytest.mark.parametrize("call", [_scan, _block])
+@pytest.mark.parametrize("hook", [DOWN, UP])                 # the recompute sweep, the adjoint sweep
+def test_a_native_backward_raises_before_its_gradients_are_used(call, hook, monkeypatch):
+    monkeypatch.setenv("M2D_TEST_HOOKS", "1")
+    inp, dev = _large_map()
+    y, leaves = call(dev, True, bwd=hook | REPORT)
+    with pytest.raises(RuntimeError, match="m2d_scan_bwd: a wait between CTAs timed out"):
+        _grads(y, leaves, dev["gy"])
+    y, leaves = call(dev, True)
+    assert all(torch.isfinite(g).all() for g in _grads(y, leaves, dev["gy"]))
+    assert _lib.lib().m2d_take_wait_failure() == 0
+
+
+@pytest.mark.parametrize("call", [_scan, _block])
+def test_an_unchecked_failure_is_reported_by_the_next_call(call, monkeypatch):
+    monkeypatch.setenv("M2D_TEST_HOOKS", "1")
+    inp, dev = _large_map()
+    y, leaves = call(dev, True, check=False, bwd=UP | REPORT)
+    torch.cuda.synchronize()
+    y_bad, _ = call(dev, False, check=False, fwd=DOWN | REPORT)
+    torch.cuda.synchronize()
+    assert torch.isnan(y_bad).any()                          # a row that never came reads as NaN
+    with pytest.raises(RuntimeError, match="earlier launch timed out"):
+        _grads(y, leaves, dev["gy"])                         # the backward looks, too
+    y, leaves = call(dev, True, check=False, bwd=UP | REPORT)
+    _grads(y, leaves, dev["gy"])
+    torch.cuda.synchronize()
+    with pytest.raises(RuntimeError, match="earlier launch timed out"):
+        call(dev, False)
+    assert torch.isfinite(call(dev, False)[0]).all()
+    assert _lib.lib().m2d_take_wait_failure() == 0
+
+
+@pytest.mark.parametrize("hook", [DOWN, UP])
+def test_the_backwards_waits_give_up(hook, monkeypatch):
+    """Through the C interface: the status word, and what the sweep before the withheld row had finished."""
+    monkeypatch.setenv("M2D_TEST_HOOKS", "1")
+    inp, dev = _large_map()
+    L = _lib.lib()
+    want = wc.scan_bwd(*[dev[k] for k in ORDER], dev["gy"])
+    d, keep = wc._make_desc(*[dev[k] for k in ORDER])
+    d.flags = hook
+    assert L.m2d_scan_bwd_chain(ctypes.byref(d)) > 1
+    d.gy = dev["gy"].data_ptr()
+    outs = [torch.zeros_like(t) for t in want]
+    for name, t in zip(("d_x", "d_dT", "d_dL", "d_AT", "d_AL", "d_BT", "d_BL", "d_C", "d_D"), outs):
+        setattr(d, name, t.data_ptr())
+    wc._workspace(d, L.m2d_scan_bwd_workspace(ctypes.byref(d)), dev["x"].device, keep)
+    assert L.m2d_scan_bwd(ctypes.byref(d), ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)) == 0
+    torch.cuda.synchronize()
+    off = L.m2d_scan_bwd_status_offset(ctypes.byref(d))
+    assert wc._status_word(keep[-1], off) != 0
+    with pytest.raises(RuntimeError, match="gradients are invalid"):
+        wc._check_status("bwd", d, keep[-1])
+    assert torch.isnan(outs[1]).any()                        # (d_deltaT, which needs the states and their adjoints)
+    last = outs[1][:, 88:]                                   # the last band: complete where only the way up was cut
+    if hook == UP:
+        assert float((last - want[1][:, 88:]).abs().max()) <= 1e-6 * float(want[1].abs().max())
+    else:
+        assert torch.isnan(last).any()
 
 
 def test_the_hook_is_refused_without_the_environment_variable(monkeypatch):
