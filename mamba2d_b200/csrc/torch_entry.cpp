@@ -233,7 +233,10 @@ Tensor forward_scan(const Tensor& x, m2d_scan_desc& d, char* ws, const Tensor& y
         at::cuda::CachingHostAllocator_recordEvent(word.data_ptr(), word.storage().data_ptr().get_context(), stream);
         return word;
     }
-    C10_CUDA_CHECK(cudaStreamSynchronize(stream));
+    {
+        const pybind11::gil_scoped_release others_run;       // (forward passes come from Python)
+        C10_CUDA_CHECK(cudaStreamSynchronize(stream));
+    }
     check_status(mark, status, "m2d_scan_fwd");
     return Tensor();
 }

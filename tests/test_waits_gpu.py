@@ -208,3 +208,29 @@ def test_a_diverged_image_leaves_the_others_alone(shape):
     for idx in (0, 1, 2, 5, 6, 7):       # the per-pixel gradients (the batch sums d_AT, d_AL, d_D include image 1)
         assert torch.isfinite(g1[idx][keep]).all()
         assert float((g0[idx][keep] - g1[idx][keep]).abs().max()) <= 1e-6 * float(g0[idx].abs().max())
+
+
+def test_a_waiting_call_lets_other_threads_run():
+    """The wait for the scan holds no interpreter lock: a thread gets on with its work meanwhile."""
+    import threading
+    import time
+    x = torch.randn(1, 2048, 1024, 64, device="cuda")
+    w = inputs.make_module_params(64, 16, seed=5)
+    ws = [w[k].cuda() for k in ("AT_log", "AL_log", "x_proj_w", "dt_projT_w", "dt_projT_b", "dt_projL_w", "dt_projL_b", "D")]
+    wc.wavefront_scan_cuda(x, *ws)
+    torch.cuda.synchronize()
+    marks, stop = [], threading.Event()
+
+    def other():
+        while not stop.is_set():
+            marks.append(time.perf_counter())
+    t = threading.Thread(target=other)
+    t.start()
+    spans = []
+    for _ in range(5):
+        a = time.perf_counter()
+        wc.wavefront_scan_cuda(x, *ws)                       # milliseconds, nearly all of it waiting
+        spans.append((a, time.perf_counter()))
+    stop.set()
+    t.join()
+    assert sum(any(a + 0.2 * (b - a) < m < b - 0.2 * (b - a) for m in marks) for a, b in spans) >= 3
