@@ -72,11 +72,11 @@ void check_waits() {
     TORCH_CHECK(!m2d_take_wait_failure(), "wavefront scan: a wait between CTAs of an earlier launch timed out; the results of that launch are invalid");
 }
 
-// Whether a call on these makes a node.
+// Whether a call on these makes a node.  An input with a forward-mode tangent goes there too, although there is no
+// formula for it: the node refuses it, where a pass without one would drop the tangent and say nothing.
 bool wants_grad(std::initializer_list<const Tensor*> inputs) {
     bool grad = false;
-    if (at::GradMode::is_enabled())
-        for (const Tensor* t : inputs) grad = grad || t->requires_grad();
+    for (const Tensor* t : inputs) grad = grad || (at::GradMode::is_enabled() && t->requires_grad()) || t->_fw_grad(0).defined();
     return grad;
 }
 

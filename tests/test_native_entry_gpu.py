@@ -65,3 +65,22 @@ def test_what_the_native_path_does_not_take_goes_op_by_op():
     assert _lib.entry().block(x, *ws, False, False, False) is None
     assert wc.wavefront_scan_cuda(x, *ws).shape == x.shape
     assert _lib.lib().m2d_take_wait_failure() == 0
+
+
+@pytest.mark.parametrize("grad", [False, True])
+@pytest.mark.parametrize("act", [None, "gelu"])
+def test_forward_mode_tangents_are_refused(grad, act):
+    """There is no forward-mode formula: a call says so and does not return an output without a tangent."""
+    import torch.autograd.forward_ad as fw
+    w = inputs.make_module_params(64, 16, seed=5)
+    ws = [w[k].cuda() for k in NAMES]
+    x = torch.randn(2, 7, 5, 64, device="cuda").requires_grad_(grad)
+    with fw.dual_level():
+        dual = fw.make_dual(x, torch.ones_like(x))
+        with pytest.raises(RuntimeError, match="jvp"):
+            wc.wavefront_scan_cuda(dual, *ws, act_out=act)
+        with torch.no_grad(), pytest.raises(RuntimeError, match="jvp"):
+            wc.wavefront_scan_cuda(dual, *ws, act_out=act)
+        tangent = fw.make_dual(ws[7], torch.ones_like(ws[7]))                # of a parameter (D)
+        with pytest.raises(RuntimeError, match="jvp"):
+            wc.wavefront_scan_cuda(x.detach(), *ws[:7], tangent, act_out=act)
