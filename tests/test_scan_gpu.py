@@ -198,3 +198,48 @@ def test_a_log_inside_the_kernels(kind):
             assert u.dtype == torch.float32
             v = v.float() * (AT32 if name == "d_AT" else AL32)
         assert rel_err(u.float().cpu().numpy(), v.float().cpu().numpy()) < tol, name
+
+
+@pytest.mark.parametrize("shape", [(2, 9, 13, 40, 12), (300, 6, 5, 32, 16)])          # wave kernel; batch kernel
+@pytest.mark.parametrize("columns", ["neighbours", "apart", "flag"])
+@pytest.mark.parametrize("kind", ["f32", "bf16"])
+def test_gradients_of_b_and_c_as_columns_of_a_wider_buffer(shape, columns, kind):
+    """d_BT, d_BL, d_C at a pixel pitch: cleared by the call (or by the caller, who says so), the columns between them untouched."""
+    import ctypes
+    from mamba2d_b200 import _lib, scan_bwd
+    from mamba2d_b200 import wavefront_cuda as wc
+    B, H, W, E, N = shape
+    if kind == "bf16" and columns == "flag":
+        pytest.skip("the flag is for fp32, where the kernel accumulates in place")
+    dev = to_dev(inputs.make_inputs(*shape, seed=7), TDT[kind])
+    args = [dev[k] for k in ORDER]
+    want = scan_bwd(*args, dev["gy"])
+    gap = 8 if columns == "apart" else 0
+    pitch = 4 + 3 * (N + gap) + 4
+    at = [4 + k * (N + gap) for k in range(3)]
+    wide = torch.full((B, H, W, pitch), 7.0, device="cuda", dtype=TDT[kind])
+    d, keep = wc._make_desc(*args)
+    if columns == "flag":
+        for a in at:
+            wide[..., a:a + N] = 0
+        d.flags = _lib.M2D_SCAN_BC_ZEROED
+    outs = [torch.full_like(t, float("nan")) for t in want]
+    names = ("d_x", "d_dT", "d_dL", "d_AT", "d_AL", "d_BT", "d_BL", "d_C", "d_D")
+    for name, t in zip(names, outs):
+        setattr(d, name, t.data_ptr())
+    d.d_BT, d.d_BL, d.d_C = (wide.data_ptr() + a * wide.element_size() for a in at)
+    d.d_BC_pitch = pitch
+    d.gy = dev["gy"].data_ptr()
+    L = _lib.lib()
+    wc._workspace(d, L.m2d_scan_bwd_workspace(ctypes.byref(d)), wide.device, keep)
+    assert L.m2d_scan_bwd(ctypes.byref(d), ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)) == 0
+    torch.cuda.synchronize()
+    got = dict(zip(names, outs))
+    got.update(d_BT=wide[..., at[0]:at[0] + N], d_BL=wide[..., at[1]:at[1] + N], d_C=wide[..., at[2]:at[2] + N])
+    tol = 1e-5 if kind == "f32" else 8e-3                     # the order of the sums over channels and CTAs; one rounding
+    for name, ref in zip(names, want):
+        assert rel_err(got[name].float().cpu().numpy(), ref.float().cpu().numpy()) < tol, name
+    used = torch.zeros(pitch, dtype=torch.bool)
+    for a in at:
+        used[a:a + N] = True
+    assert (wide[..., ~used.cuda()] == 7.0).all()
