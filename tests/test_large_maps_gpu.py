@@ -1,6 +1,6 @@
 """Large maps with few images (the resolution sweep of the baseline description: B=1, D=64, fp32,
 H=W from 128 to 2048): here every image is shared by a chain of CTAs, each owning every chain-th
-band, and the chain closes into a ring when there are more bands than resident CTAs.  The forward is
+band (several each from 512 on).  The forward is
 checked against the reference project's own CUDA kernels on the same GPU up to 1024x1024 (their
 state tensor would take 17 GB at 2048x2048) and against the fp64 CPU oracle at 2048x2048; the
 backward against the reference's kernels at 256x256 and at a detection-style shape."""

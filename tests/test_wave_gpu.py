@@ -20,7 +20,9 @@ SHAPES = [
     (1, 16, 3, 6, 4),        # scalar loads, ragged channel group
     (1, 33, 4, 34, 16),      # one chunk of columns
     (3, 24, 13, 18, 5),      # states that are not a multiple of four
-    (1, 200, 9, 64, 16),     # more bands than the chain may have CTAs
+    (1, 200, 9, 64, 16),     # 25 bands, a CTA each
+    (3, 57, 33, 192, 16),    # 8 bands for 3 CTAs: a CTA comes back for a second and third band while others wait on it
+    (2, 140, 26, 128, 12),   # 18 bands for 2 CTAs, ragged states
     (2, 41, 64, 96, 16),
     (60, 17, 7, 64, 16),     # more (image, group) pairs than SMs
     (400, 9, 2, 16, 16),     # lists of several images per CTA
@@ -44,6 +46,17 @@ def test_wave_kernels_against_the_oracle(shape, dt, tol, reverse):
     want = cpu.backward(ref, mode="f64")
     for name, t in zip(cpu.GRAD_NAMES, grads):
         assert rel_err(t.float().cpu().numpy(), back(want[name])) < tol, name
+
+
+@pytest.mark.parametrize("shape,chains", [((1, 200, 9, 64, 16), (25, 25)), ((3, 57, 33, 192, 16), (3, 3)), ((2, 140, 26, 128, 12), (2, 2)),
+                                          ((400, 9, 2, 16, 16), (1, 1))])
+def test_the_shapes_above_get_the_chains_they_are_there_for(shape, chains):
+    d = _lib.ScanDesc()
+    d.struct_bytes = ctypes.sizeof(d)
+    d.B, d.H, d.W, d.E, d.N = shape
+    d.BT_pitch = d.BL_pitch = d.C_pitch = shape[4]
+    L = _lib.lib()
+    assert (L.m2d_scan_fwd_chain(ctypes.byref(d)), L.m2d_scan_bwd_chain(ctypes.byref(d))) == chains
 
 
 def test_boundary_rows_are_kept_where_a_later_sweep_needs_them():
