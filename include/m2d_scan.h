@@ -168,6 +168,11 @@ const char *m2d_strerror(int status);
  * Bytes of scratch m2d_scan_fwd / m2d_scan_bwd need for this problem on the current device (never
  * 0: the scratch starts with a status word).  Replaces the reference's Python-side allocations of
  * hs / dDAT / dDAL / omega (wavefront_cuda.py:152, :181-183).  Returns 0 for an invalid descriptor.
+ *
+ * What to expect, in bytes per element of x (a map's last band of eight rows, its columns and its channels rounded up):
+ *   many images   forward about 1; backward 64, with bf16 I/O 32, for the state record, + 16 states x 12 / E
+ *   few images    forward up to 8 (boundary rows of all bands: 537 MB for one 1024x1024x64 map, 2.1 GB for 2048x2048);
+ *                 backward 64 + 16, whatever the I/O type: this record is FP32 (725 MB for 2x200x336x64)
  */
 uint64_t m2d_scan_fwd_workspace(const m2d_scan_desc *desc);
 uint64_t m2d_scan_bwd_workspace(const m2d_scan_desc *desc);
@@ -218,10 +223,9 @@ int64_t m2d_wait_failure_mark(void);
 
 /*
  * The rule every launch applies when it picks, or has to shorten, the number of CTAs per image:
- * at most one CTA per band, and when CTAs own more than one band each (the chain closes into a
- * ring) fewer than one row of steps divided by the rows per band, so that the head of the ring
- * never waits on data that waits on the head.  Host-side arithmetic only; returns 0 for
- * non-positive arguments.  No counterpart in the reference.
+ * at most one CTA per band, and when CTAs own more than one band each fewer than one row of steps
+ * divided by the rows per band (a cautious limit: every wait ends without it).  Host-side
+ * arithmetic only; returns 0 for non-positive arguments.  No counterpart in the reference.
  */
 int m2d_scan_chain_bound(int want, int nbands, int steps_per_row, int rows_per_band);
 

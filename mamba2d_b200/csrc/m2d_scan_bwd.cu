@@ -51,8 +51,8 @@ inline BwdLayout bwd_layout(const m2d_scan_desc* d, const Plan& p) {
 }
 
 inline Plan plan_bwd(const m2d_scan_desc* d) {
-    // Batch or wave, as in plan_fwd.  Measured times per step of both sweeps together: 2.45 us in batch mode
-    // with two CTAs per SM, 1.95 us with one, 1.2 us in the wave kernel with two channels per lane (four
+    // Batch or wave, as in plan_fwd.  Measured times per step of both sweeps together, whatever the I/O type: 2.45 us in
+    // batch mode with two CTAs per SM, 1.95 us with one, 1.2 us in the wave kernel with two channels per lane (four
     // spill and are slower at every size measured).  56x56x64: wave up to batch 32, 581 against 738 us.
     Plan p{};
     double best = 1e30;

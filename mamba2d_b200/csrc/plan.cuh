@@ -189,10 +189,15 @@ inline size_t align256(size_t v) { return (v + 255) & ~(size_t)255; }
 constexpr size_t kStatusBytes = 256;
 
 // CTAs per image that a wave launch may use: at most one per band, and, when CTAs own more than one band
-// each (the chain closes into a ring), fewer than one row of steps divided by the rows of a band, so that a
-// CTA finds the band above its next one well ahead of it.  `want` is the chain the resident CTA slots allow;
+// each, fewer than one row of steps divided by the rows of a band.  `want` is the chain the resident CTA slots allow;
 // `steps_per_row` the steps a warp needs for one row.  Every place that picks or shortens a chain goes
 // through this rule.
+//
+// The second limit is cautious: the waits end without it.  A CTA finishes a band before it takes its next, bands are
+// taken in ascending order (descending in the adjoint sweep) and each waits only for the one before, so that
+// whatever the chain's length some CTA can always go on.  (Kernels whose CTAs walk their bands in lock-step need
+// it.)  On narrow maps it leaves SMs idle: 4x200x14x96 gets one CTA per image where six are free, 600 dependent
+// steps instead of 384; 3x45x31x192 135 instead of 115.
 inline int bound_chain(long long want, int nbands, int steps_per_row, int Rb) {
     if (want > nbands) want = nbands;
     if (want < nbands) {
@@ -226,9 +231,11 @@ inline size_t wave_edge_bytes(const m2d_scan_desc* d, const Plan& p, bool bwd) {
     return align256((size_t)p.grid_x * ((d->E + p.wave - 1) / p.wave) * wave_rows(p, bwd) * d->W * 16 * p.wave * sizeof(float));
 }
 
-// Steps a wave launch takes: bands walked one after the other by the busiest CTA, and the start-up of the
-// chain (a band can start when the one above it is about 15 columns in: the eight rows of its wave, the chunk
-// of columns being published, the trip through L2).
+// Steps a wave launch takes, as the plans compare them: bands walked one after the other by the busiest CTA, and the
+// start-up of the chain (a band can start when the one above it is about 15 columns in: the eight rows of its wave,
+// the chunk of columns being published, the trip through L2).  Too many where a CTA has several bands, because the
+// later rounds of the first CTAs run during the start-up: 173 against 128 by the dependences for 5x37x53x96, 951
+// against 786 for 2x200x336x64.  The measured times per step in plan_fwd and plan_bwd belong to this count.
 inline double wave_steps(const m2d_scan_desc* d, const Plan& p) {
     const long long slots = sm_count(), ctas = (long long)p.grid_x * p.groups * p.chain;
     const long long images = p.chain > 1 ? 1 : ((long long)d->B + p.grid_x - 1) / p.grid_x;
@@ -241,7 +248,7 @@ inline Plan plan_fwd(const m2d_scan_desc* d, bool allow_chain = true) {
     // wave kernels split an image over CTAs as well.  Measured times per step: 0.9 us (batch), 0.62 us (wave,
     // four channels per lane) and 0.42 us (two channels, twice the CTAs); they put the lines where the
     // measured times cross within 10 % (56x56x64: wave up to batch 64, 290 against 381 us there; 14x14x320:
-    // up to batch 8).  The batch kernel needs three columns.
+    // up to batch 8).  The batch kernel needs three columns.  (fp32 or bf16 I/O differ by less than that.)
     Plan p{};
     double best = 1e30;
     if (d->W >= 3) {

@@ -82,6 +82,20 @@ def test_workspace_queries(L):
     assert L.m2d_scan_fwd_workspace(ctypes.byref(_desc(H=1))) == 0    # invalid descriptor
 
 
+@pytest.mark.parametrize("B,H,W,E", [(2, 200, 336, 64), (6, 45, 31, 192), (1, 1024, 1024, 64), (4, 14, 14, 384), (1, 9, 2, 40), (400, 9, 2, 16)])
+@pytest.mark.parametrize("dtype", [_lib.M2D_F32, _lib.M2D_BF16])
+def test_scratch_of_few_images_is_bounded(L, B, H, W, E, dtype):
+    """Bytes per element as include/m2d_scan.h states them: rows in bands of eight, channels in groups of 16 or 32."""
+    d = ctypes.byref(_desc(B=B, H=H, W=W, E=E, dtype=dtype))
+    rows, bands, chans = (H + 7) // 8 * 8, (H + 7) // 8, (E + 31) // 32 * 32
+    boundary = B * bands * W * chans * 16 * 4                 # a row of 16 states per band
+    record = B * rows * (W + 7) * chans * 16 * 4              # every state of every step, fp32
+    sums = 0 if dtype == _lib.M2D_F32 else 4 * (3 * B * H * W * 16 + 2 * E * 16 + E)
+    slack = 8 * 256
+    assert L.m2d_scan_fwd_workspace(d) <= boundary + slack
+    assert L.m2d_scan_bwd_workspace(d) <= record + 2 * boundary + sums + slack
+
+
 def test_status_word_and_chain_queries(L):
     d = _desc(B=128, H=56, W=56)
     assert L.m2d_scan_fwd_status_offset(ctypes.byref(d)) == 0
@@ -90,8 +104,7 @@ def test_status_word_and_chain_queries(L):
     d = _desc(B=1, H=256, W=256)
     assert L.m2d_scan_fwd_chain(ctypes.byref(d)) > 1 and L.m2d_scan_bwd_chain(ctypes.byref(d)) > 1
     assert L.m2d_scan_fwd_status_offset(ctypes.byref(_desc(H=1))) == -1 and L.m2d_scan_fwd_chain(ctypes.byref(_desc(H=1))) == 0
-    # more bands than resident CTAs: the chain closes into a ring, which must stay shorter than one
-    # row of steps (W / Rb - 1 with eight row-warps)
+    # more bands than resident CTAs: the chain stays shorter than one row of steps (W / 8 - 1)
     d = _desc(B=1, H=2400, W=24, E=32)
     assert L.m2d_scan_fwd_chain(ctypes.byref(d)) == 24 // 8 - 1
     d = _desc(B=1, H=2400, W=200, E=32)
@@ -100,7 +113,7 @@ def test_status_word_and_chain_queries(L):
 
 def test_chain_bound_over_shrink_sequences(L):
     """A planned chain and every chain a launch may fall back to obey the same rule: never more CTAs
-    than bands, and a chain that closes into a ring stays below one row of steps per band height."""
+    than bands, and a chain shorter than that stays below one row of steps per band height."""
     for nbands in (1, 2, 7, 10, 128, 300):
         for steps in (2, 3, 12, 24, 56, 1024):
             for rb in (1, 2, 6, 8):
