@@ -1,7 +1,5 @@
 // Backward entry point of the wavefront scan: recompute sweep + adjoint sweep in one kernel,
 // followed by a small kernel that casts the fp32 accumulators of the reduced gradients.
-#include <cstdlib>
-
 #include "launch.cuh"
 #include "sweep_rows.cuh"
 #include "wave_bwd.cuh"
@@ -57,10 +55,7 @@ inline Plan plan_bwd(const m2d_scan_desc* d) {
     Plan p{};
     double best = 1e30;
     if (d->W >= 3) {
-        // tuning knob: M2D_BWD_WARPS=<1..max> overrides the row-warps per CTA of the batch kernel
-        int maxw = M2D_BWD_MAXW;
-        if (const char* e = getenv("M2D_BWD_WARPS")) { const int v = atoi(e); if (v >= 1 && v <= M2D_BWD_MAXW) maxw = v; }
-        p = plan_best(d, maxw, 2 * M2D_BWD_MAXW);
+        p = plan_best(d, M2D_BWD_MAXW, 2 * M2D_BWD_MAXW);
         p.smem = rows_bwd_smem_bytes(p.warps) + kParamF4 * sizeof(float4);
         best = ((long long)p.grid_x * p.groups > sm_count() ? 2.45 : 1.95) * batch_steps(d, p);
     }
@@ -257,7 +252,8 @@ static int launch_bwd(const m2d_scan_desc* d, const Plan& pl, bool vec, cudaStre
                                                : (vec ? m2d_bwd_kernel<io_t, true> : m2d_bwd_kernel<io_t, false>), a, p, st);
     if (rc != M2D_OK) return rc;
     if (d->dtype != M2D_F32) {
-        const int fin_blocks = (int)((npn + 255) / 256 < 148 * 8 ? (npn + 255) / 256 : 148 * 8);
+        const size_t fit = (size_t)sm_count() * 8;
+        const int fin_blocks = (int)((npn + 255) / 256 < fit ? (npn + 255) / 256 : fit);
         m2d_bwd_finalize<io_t><<<fin_blocks, 256, 0, st>>>(a.accBT, static_cast<io_t*>(d->d_BT), static_cast<io_t*>(d->d_BL),
                                                           static_cast<io_t*>(d->d_C), d->d_AT, d->d_AL, d->d_D,
                                                           (long long)npn, d->N, d->d_BC_pitch ? (int)d->d_BC_pitch : d->N, (long long)en, d->E, a.a_log, a.d_f32);

@@ -96,6 +96,15 @@ def test_scratch_of_few_images_is_bounded(L, B, H, W, E, dtype):
     assert L.m2d_scan_bwd_workspace(d) <= record + 2 * boundary + sums + slack
 
 
+def test_plans_do_not_depend_on_the_environment(L, monkeypatch):
+    """The workspace query and the launch plan separately; nothing a program can change in between may tell them apart."""
+    d = ctypes.byref(_desc(B=128, H=56, W=56))
+    before = L.m2d_scan_bwd_workspace(d), L.m2d_scan_fwd_workspace(d)
+    for v in "1235":
+        monkeypatch.setenv("M2D_BWD_WARPS", v)
+        assert (L.m2d_scan_bwd_workspace(d), L.m2d_scan_fwd_workspace(d)) == before
+
+
 def test_status_word_and_chain_queries(L):
     d = _desc(B=128, H=56, W=56)
     assert L.m2d_scan_fwd_status_offset(ctypes.byref(d)) == 0
