@@ -2,8 +2,9 @@
 // back through it, d_x += d_proj @ Wx.  Both have 10^2 ... 10^6 rows and at most a few hundred columns.
 //
 // The GEMM library runs fp32 at full precision on the CUDA cores, in tiles of 64 or 128 columns where these
-// products have 56 ... 156: 105 and 129 us at P = 401408, E = 64 (264 us at P = 1048576) for operands that
-// stream in 30 and 46 us (78 us), and 8 us for the 196 rows of one 14x14 image.
+// products have 56 ... 156: 102 and 132 us at P = 401408, E = 64 (262 us at P = 1048576) for operands that
+// stream in 30 and 46 us (78 us), and 7.7 us for the 196 rows of one 14x14 image; 53 and 106 (130), and 3.0 here.  (A
+// kernel's own times, in a graph; events around one call with the L2 flushed show 5 us more.)
 //
 // Here a float is split into three bf16 parts, exact to 24 bits, and a product of floats is the six products of
 // parts that reach above 2^-24 of it, on the tensor cores (mma.sync m16n8k16: fragments are split in registers, where
@@ -106,9 +107,9 @@ __device__ __forceinline__ void store2(const GemmArgs& a, long long row, int col
 
 // Many rows.  grid (CTAs, chunks of NT * 8 columns); a warp computes 16 rows at a time against the chunk, whose
 // fragments every CTA splits once into shared memory.  The rows come straight from global memory, two steps of 16
-// terms ahead, the first of the next tile among them.  Bound by the rate of mma.sync (four cycles of an SM each):
-// 60 us at P = 401408 (56 x 64), 139 us at P = 1048576.  Two 16-row tiles per warp, which halve the reads of the
-// fragments, need twice the registers: 62 us, and 166 against 115 us for the product that accumulates.
+// terms ahead, the first of the next tile among them.  Bound by the rate of mma.sync (four cycles of an SM each).  Two
+// 16-row tiles per warp, which halve the reads of the fragments, need twice the registers: 166 against 112 us for the
+// product that accumulates at P = 401408, E = 64, and nothing gained for the other (events, L2 flushed).
 template <int NT>
 __global__ void __launch_bounds__(256, 2) rows_gemm_kernel(const GemmArgs a) {
     extern __shared__ uint2 gemm_w[];              // [step][n-tile][part][lane]

@@ -601,8 +601,8 @@ static int launch_dt_bwd(const m2d_proj_desc* d, const ProjArgs& a, const ProjPl
 
 // Which kernels a call gets.  The tensor-core ones read and write rows of 16-byte pieces (E a multiple of 8,
 // aligned tensors), and the backward's sums fit its registers up to 39 ranks.  Measured, CUDA cores / tensor cores in
-// us (R = E / 16, cold L2):
-//   forward, bf16: 90 / 55 (P = 401408, E = 64), 68 / 37 (25088, 320), 12 / 10 (784, 384): tensor cores always.
+// us (R = E / 16; CUDA events around one call with the L2 flushed, which adds about 5 to a kernel's own time):
+//   forward, bf16: 92 / 56 (P = 401408, E = 64), 68 / 38 (25088, 320), 13 / 11 (784, 384): tensor cores always.
 //   forward, fp32 (a product is six), by elements P * E:
 //                E = 64      128       192       320       384       512       576
 //       2 M     14 / 16   16 / 16   18 / 23   25 / 26   25 / 33   40 / 29   35 / 43

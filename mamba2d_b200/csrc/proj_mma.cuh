@@ -2,8 +2,8 @@
 //
 // delta = softplus(r @ W^T + b) and its backward are contractions over a rank R of 4 ... 36 or over the
 // pixels, next to one transcendental per element.  On the CUDA cores they cost R multiply-adds per
-// element and were bound by issue slots (R = 20, E = 320: 59 us forward, 176 us backward for 16 M elements
-// of bf16 whose traffic takes 5 and 10 us).  The products are too small in K (forward) and N (backward)
+// element and were bound by issue slots (R = 20, E = 320: 60 us forward, 166 us backward for 16 M elements
+// of bf16 whose traffic takes 5 and 10 us; 33 and 56 here, all in a graph).  The products are too small in K (forward) and N (backward)
 // for tcgen05 to pay: a 128x256x16 tile would be nine tenths padding or wait on its own epilogue; mma.sync
 // fragments are consumed where they are produced.
 //

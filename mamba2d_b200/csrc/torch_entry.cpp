@@ -163,9 +163,17 @@ struct Projected {
 // the library calls transposed ones.
 void gemm(const Tensor& like, int64_t rows, int64_t n, int64_t k, const void* a, const void* w, bool transposed, bool accumulate, void* out) {
     // fp32: the library's tiles are 64 or 128 columns wide and its time for a few rows is several launches' worth.
-    // Against it, library / own: 110 / 60 us at 401408 x 64 -> 56, 52 / 45 at 100352 x 128 -> 64, 137 / 115 at
-    // 401408 x 56 -> 64, but 14 / 16 at 9805 x 60 -> 96 and 31 / 39 at 6272 x 512 -> 112; with few rows 14 / 8 at
-    // 196 x 320 -> 88 and 16 / 10 at 784 x 384 -> 96.
+    // Library / own, us, events around one call with the L2 flushed, by E (n = E or K = 56 ... 120 next to it):
+    //              x @ Wx^T (n = K)                                        d_x += d_proj @ Wx (n = E)
+    //     rows     64       192      320      384      512      576        64       192      320      384      512      576
+    //     196     9 / 6    12 / 8   15 / 8   16 / 9   19 / 10  21 / 10   10 / 8   10 / 8   10 / 8   10 / 8   12 / 8   12 / 9
+    //     784     9 / 7    12 / 8   15 / 10  16 / 10  20 / 10  22 / 12   10 / 8   10 / 8   11 / 11  12 / 12  12 / 14  12 / 14
+    //     2048    9 / 8    12 / 10  16 / 14  17 / 14  21 / 16  23 / 18   10 / 8   12 / 13  14 / 16  14 / 16  15 / 20  17 / 27
+    //     3136    9 / 8    12 / 12  16 / 18  18 / 21  23 / 21  25 / 25   10 / 10  12 / 14  14 / 19  15 / 23  18 / 27  22 / 29
+    //     9805   11 / 10   20 / 20  27 / 33  29 / 31  46 / 60  51 / 68   12 / 14  20 / 23  29 / 37  33 / 37  42 / 51  49 / 56
+    //     100352 38 / 22  104 / 70 156 / 132 180 / 158 269 / 286 299 / 322  39 / 39 121 / 98 209 / 174 254 / 196 360 / 288 413 / 347
+    // The line follows the first product.  For the second it lies up to 10 us too far between 800 and 2048 rows (the own
+    // kernel's error is a third of the library's, so it keeps them); beyond 25000 rows both would gain at more columns.
     if (like.scalar_type() == at::kFloat && (n <= 64 || rows <= 2048)) {
         const int rc = m2d_rows_gemm_f32(rows, (int)n, (int)k, static_cast<const float*>(a), static_cast<const float*>(w), transposed, accumulate,
                                          static_cast<float*>(out), stream_of(like));
