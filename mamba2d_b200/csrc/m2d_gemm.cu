@@ -3,7 +3,7 @@
 //
 // The GEMM library runs fp32 at full precision on the CUDA cores, in tiles of 64 or 128 columns where these
 // products have 56 ... 156: 102 and 132 us at P = 401408, E = 64 (262 us at P = 1048576) for operands that
-// stream in 30 and 46 us (78 us), and 7.7 us for the 196 rows of one 14x14 image; 53 and 106 (130), and 3.0 here.  (A
+// stream in 30 and 46 us (78 us), and 7.7 us for the 196 rows of one 14x14 image; 55 and 75 (137), and 3.0 here.  (A
 // kernel's own times, in a graph; events around one call with the L2 flushed show 5 us more.)
 //
 // Here a float is split into three bf16 parts, exact to 24 bits, and a product of floats is the six products of
@@ -94,15 +94,11 @@ __device__ __forceinline__ float4 load_w(const GemmArgs& a, int col, int k) {   
 __device__ __forceinline__ float4 load_a(const GemmArgs& a, long long row, int k) {
     return row < a.rows && k < a.k ? __ldg(reinterpret_cast<const float4*>(a.a + row * a.k + k)) : make_float4(0.f, 0.f, 0.f, 0.f);
 }
-__device__ __forceinline__ void store2(const GemmArgs& a, long long row, int col, float x, float y) {       // n is even
-    if (row >= a.rows || col >= a.n) return;
-    float2* o = reinterpret_cast<float2*>(a.out + row * a.n + col);
-    if (a.accumulate) {
-        const float2 old = *o;
-        x += old.x;
-        y += old.y;
-    }
-    *o = make_float2(x, y);
+__device__ __forceinline__ float2 load2(const GemmArgs& a, long long row, int col) {       // n is even
+    return row < a.rows && col < a.n ? *reinterpret_cast<const float2*>(a.out + row * a.n + col) : make_float2(0.f, 0.f);
+}
+__device__ __forceinline__ void put2(const GemmArgs& a, long long row, int col, const float2& v) {
+    if (row < a.rows && col < a.n) *reinterpret_cast<float2*>(a.out + row * a.n + col) = v;
 }
 
 // Many rows.  grid (CTAs, chunks of NT * 8 columns); a warp computes 16 rows at a time against the chunk, whose
@@ -171,12 +167,22 @@ __global__ void __launch_bounds__(256, 2) rows_gemm_kernel(const GemmArgs a) {
                 group(NT - NT % 4, b);
             }
         }
+        // What is there already: all of it on its way before the first sum is waited for and stored (one by one, each
+        // behind the store before it, was 16 trips to memory in a row).
+        float2 old[NT][2];
 #pragma unroll
-        for (int n = 0; n < NT; ++n) {
-            const int col = col0 + n * 8 + t * 2;
-            store2(a, row0 + g, col, acc[n][0], acc[n][1]);
-            store2(a, row0 + g + 8, col, acc[n][2], acc[n][3]);
-        }
+        for (int n = 0; n < NT; ++n)
+#pragma unroll
+            for (int h = 0; h < 2; ++h)
+                old[n][h] = a.accumulate ? load2(a, row0 + g + 8 * h, col0 + n * 8 + t * 2) : make_float2(0.f, 0.f);
+#pragma unroll
+        for (int n = 0; n < NT; ++n)
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                float2 v = make_float2(acc[n][2 * h], acc[n][2 * h + 1]);
+                if (a.accumulate) { v.x += old[n][h].x; v.y += old[n][h].y; }
+                put2(a, row0 + g + 8 * h, col0 + n * 8 + t * 2, v);
+            }
     }
 }
 
@@ -214,7 +220,14 @@ __global__ void __launch_bounds__(256) rows_gemm_small_kernel(const GemmArgs a) 
         x += sums[w][n][2 * h][lane];
         y += sums[w][n][2 * h + 1][lane];
     }
-    store2(a, row0 + h * 8 + g, col0 + n * 8 + t * 2, x, y);
+    const long long row = row0 + h * 8 + g;
+    const int col = col0 + n * 8 + t * 2;
+    if (a.accumulate) {
+        const float2 old = load2(a, row, col);
+        x += old.x;
+        y += old.y;
+    }
+    put2(a, row, col, make_float2(x, y));
 }
 
 template <int NT>

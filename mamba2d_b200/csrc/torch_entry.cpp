@@ -163,18 +163,18 @@ struct Projected {
 // the library calls transposed ones.
 void gemm(const Tensor& like, int64_t rows, int64_t n, int64_t k, const void* a, const void* w, bool transposed, bool accumulate, void* out) {
     // fp32: the library's tiles are 64 or 128 columns wide and its time for a few rows is several launches' worth.
-    // Library / own, us, events around one call with the L2 flushed, by E (n = E or K = 56 ... 120 next to it):
-    //              x @ Wx^T (n = K)                                        d_x += d_proj @ Wx (n = E)
-    //     rows     64       192      320      384      512      576        64       192      320      384      512      576
-    //     196     9 / 6    12 / 8   15 / 8   16 / 9   19 / 10  21 / 10   10 / 8   10 / 8   10 / 8   10 / 8   12 / 8   12 / 9
-    //     784     9 / 7    12 / 8   15 / 10  16 / 10  20 / 10  22 / 12   10 / 8   10 / 8   11 / 11  12 / 12  12 / 14  12 / 14
-    //     2048    9 / 8    12 / 10  16 / 14  17 / 14  21 / 16  23 / 18   10 / 8   12 / 13  14 / 16  14 / 16  15 / 20  17 / 27
-    //     3136    9 / 8    12 / 12  16 / 18  18 / 21  23 / 21  25 / 25   10 / 10  12 / 14  14 / 19  15 / 23  18 / 27  22 / 29
-    //     9805   11 / 10   20 / 20  27 / 33  29 / 31  46 / 60  51 / 68   12 / 14  20 / 23  29 / 37  33 / 37  42 / 51  49 / 56
-    //     100352 38 / 22  104 / 70 156 / 132 180 / 158 269 / 286 299 / 322  39 / 39 121 / 98 209 / 174 254 / 196 360 / 288 413 / 347
-    // The line follows the first product.  For the second it lies up to 10 us too far between 800 and 2048 rows (the own
-    // kernel's error is a third of the library's, so it keeps them); beyond 25000 rows both would gain at more columns.
-    if (like.scalar_type() == at::kFloat && (n <= 64 || rows <= 2048)) {
+    // Library / own, us, events around one call with the L2 flushed (which adds about 10), by E (n = K = 56 ... 120 or E):
+    //              x @ Wx^T (n = K)                                          d_x += d_proj @ Wx (n = E)
+    //     rows     64        128       192       320      384      512       64        128       192       320      384      512
+    //     784     26 / 16   17 / 17   20 / 14   24 / 18  25 / 16  29 / 17   23 / 19   16 / 15   17 / 15   17 / 17  18 / 18  19 / 20
+    //     2048    17 / 14   17 / 15   20 / 16   23 / 19  25 / 21  28 / 23   16 / 15   16 / 17   18 / 19   20 / 20  21 / 21  21 / 24
+    //     6272    19 / 15   20 / 19   23 / 23   28 / 29  30 / 31  38 / 46   18 / 17   19 / 18   21 / 23   29 / 28  29 / 29  38 / 39
+    //     12544   19 / 17   23 / 21   29 / 27   43 / 40  39 / 40  55 / 68   20 / 19   22 / 23   28 / 27   41 / 39  44 / 38  58 / 51
+    //     25088   23 / 20   29 / 26   41 / 37   55 / 59  61 / 57  92 / 91   22 / 24   31 / 29   46 / 35   63 / 56  70 / 57  97 / 81
+    //     100352  46 / 29   58 / 49  114 / 78                              46 / 38   69 / 56  127 / 81
+    // The first product follows its columns (E up to 192).  The second is the library's between 2048 and 12000 rows, where
+    // neither gains; below that the own kernel's error, a third of the library's, keeps what it has.
+    if (like.scalar_type() == at::kFloat && (n <= 72 || rows <= 2048 || (accumulate && rows >= 12000))) {
         const int rc = m2d_rows_gemm_f32(rows, (int)n, (int)k, static_cast<const float*>(a), static_cast<const float*>(w), transposed, accumulate,
                                          static_cast<float*>(out), stream_of(like));
         if (rc == M2D_OK) return;

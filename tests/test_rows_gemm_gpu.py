@@ -26,3 +26,9 @@ def test_rows_gemm(rows, n, k, transposed, accumulate):
     scale = (k + 1) ** 0.5                           # of one result
     assert float((out.double() - want).abs().max()) < 2e-6 * scale
     assert float((out.double() - want).norm() / want.norm()) < 3e-7
+
+
+@pytest.mark.parametrize("rows,n,k", [(12000, 96, 60), (12001, 128, 64), (12543, 192, 72), (13000, 320, 88), (12289, 512, 112), (12017, 576, 120)])
+def test_rows_gemm_adds_to_wide_rows(rows, n, k):
+    """d_x += d_proj @ Wx at the widths and row counts that no longer go to the GEMM library."""
+    test_rows_gemm(rows, n, k, 0, 1)
