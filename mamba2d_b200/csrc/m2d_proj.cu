@@ -9,6 +9,7 @@
 // a warp own consecutive channels of one pixel (coalesced rows), the per-pixel rank-R vectors sit
 // in shared memory, and the big reductions over pixels stay in registers until the end of the
 // kernel, when each CTA writes one partial result that a small second kernel sums.
+#include <type_traits>
 #include "m2d_proj.h"
 
 #include "common.cuh"
@@ -479,9 +480,11 @@ __global__ void __launch_bounds__(256) xproj_wgrad_kernel(const WgArgs a) {
 }
 
 // ------------------------------------------------------------------------------------------------
-// The parameters' gradients from the partial results, d_W[e][r] (r < R), d_b[e] (r == RB) and d_Wx: block (32, 8), 32
-// neighbouring results, the partial results dealt round-robin to the 8 rows of the block.  One launch for the
-// sums of both kernels (a launch costs a small call as much as the sums).
+// The parameters' gradients from the partial results, d_W[e][r] (r < R), d_b[e] (r == RB) and d_Wx: block (32, ROWS), 32
+// neighbouring results, the partial results dealt round-robin to the rows of the block.  One launch for the
+// sums of both kernels (a launch costs a small call as much as the sums).  Bound by the latency of its loads where the
+// results are few and the partial results many (571 of them at P = 401408, E = 64: eight rows make a thread add 70,
+// 19 us for 5 MB; 32 rows 6.4), by the number of its warps where the results are many.
 // ------------------------------------------------------------------------------------------------
 struct DtSums {
     const float* partials;             // [dir][cta][RB+1][EB]
@@ -497,9 +500,9 @@ struct WgSums {
     __host__ __device__ int blocks() const { return partials ? (int)((ke + 31) / 32) : 0; }
 };
 
-template <typename g_t>                // type of the parameters' gradients
-__global__ void proj_bwd_finalize(const DtSums dt, const WgSums wg) {
-    __shared__ float red[8][33];
+template <typename g_t, int ROWS>      // type of the parameters' gradients
+__global__ void __launch_bounds__(32 * ROWS) proj_bwd_finalize(const DtSums dt, const WgSums wg) {
+    __shared__ float red[ROWS][33];
     const bool is_dt = (int)blockIdx.x < dt.blocks();
     const long long idx = (long long)(is_dt ? blockIdx.x : blockIdx.x - dt.blocks()) * 32 + threadIdx.x;
     const long long step = is_dt ? (dt.RB + 1) * dt.EB : wg.ke, n = is_dt ? 2 * step : wg.ke;
@@ -508,15 +511,15 @@ __global__ void proj_bwd_finalize(const DtSums dt, const WgSums wg) {
     float s = 0.f;
     if (idx < n) {
         const float* src = (is_dt ? dt.partials + dir * count * step : wg.partials) + rem;
-#pragma unroll 4
-        for (int c = threadIdx.y; c < count; c += 8) s += src[c * step];
+#pragma unroll 8
+        for (int c = threadIdx.y; c < count; c += ROWS) s += src[c * step];
     }
     red[threadIdx.y][threadIdx.x] = s;
     __syncthreads();
     if (threadIdx.y != 0 || idx >= n) return;
     float t = 0.f;
 #pragma unroll
-    for (int y = 0; y < 8; ++y) t += red[y][threadIdx.x];
+    for (int y = 0; y < ROWS; ++y) t += red[y][threadIdx.x];
     if (!is_dt) {
         store1(static_cast<g_t*>(wg.d_Wx), idx, t);
         return;
@@ -572,8 +575,16 @@ static int launch_dt_fwd(const ProjArgs& a, const ProjPlan& p, cudaStream_t st) 
 template <typename io_t>
 static int launch_sums(const m2d_proj_desc* d, const DtSums& dt, const WgSums& wg, cudaStream_t st) {
     const int blocks = dt.blocks() + wg.blocks();
-    if (d->flags & M2D_PROJ_PARAMS_F32) proj_bwd_finalize<float><<<blocks, dim3(32, 8), 0, st>>>(dt, wg);
-    else proj_bwd_finalize<io_t><<<blocks, dim3(32, 8), 0, st>>>(dt, wg);
+    // 32 rows while a block per SM is not enough to keep its loads in flight.  8 / 32 rows, us: 132 blocks 19 / 6.4
+    // (P = 401408, E = 64), 328 blocks 9 / 6 (100352, 128); 1540 blocks 12 / 14 (25088, 320), 2848 blocks 8 / 19 (6272, 512).
+    const bool few = blocks < 4 * sm_count();
+    auto launch = [&](auto rows) {
+        constexpr int ROWS = decltype(rows)::value;
+        if (d->flags & M2D_PROJ_PARAMS_F32) proj_bwd_finalize<float, ROWS><<<blocks, dim3(32, ROWS), 0, st>>>(dt, wg);
+        else proj_bwd_finalize<io_t, ROWS><<<blocks, dim3(32, ROWS), 0, st>>>(dt, wg);
+    };
+    if (few) launch(std::integral_constant<int, 32>{});
+    else launch(std::integral_constant<int, 8>{});
     return cudaGetLastError() == cudaSuccess ? M2D_OK : M2D_ERR_LAUNCH;
 }
 static DtSums dt_sums(const m2d_proj_desc* d, const ProjPlan& p, int ctas) {
