@@ -479,6 +479,89 @@ __global__ void __launch_bounds__(256) xproj_wgrad_kernel(const WgArgs a) {
     }
 }
 
+// The same for fp32: a CTA of 128 threads, the even pixels of a stage for the first two warps, the odd ones for the
+// others, each thread an 8x8 block, the stages filled by asynchronous copies.  Bound by the loads from shared memory at a 4x4
+// block (two for 16 multiply-adds, that pipe 82 % busy, 93 us at P = 401408, E = 64); with four for 64, and no registers
+// for the next stage, 72 us (27 -> 22.6 at 6272 x 512).  (On the CUDA cores: TF32 would not hold the tolerance.)
+constexpr int kWgThreads = 128;
+
+__global__ void __launch_bounds__(kWgThreads, 4) xproj_wgrad_f32_kernel(const WgArgs a) {
+    __shared__ float4 tiles[2][2][32][16];         // [d_proj, x][buffer][pixel][quad]
+    const float* A = static_cast<const float*>(a.d_proj);
+    const float* B = static_cast<const float*>(a.x);
+    const int tid = threadIdx.x, half = tid >> 6, te = tid >> 2 & 7, tk = (tid & 3) + (tid >> 5 & 1) * 4;
+    const int e0 = blockIdx.y * 64, k0 = blockIdx.z * 64;
+    const int row0 = blockIdx.x * a.rows_per_slab, row_end = min(row0 + a.rows_per_slab, a.P);
+    const int chunks = (row_end - row0 + 31) / 32;
+
+    // each thread copies four quads of either per stage: rows lr, lr + 8, ..., column quad lc; zeros beyond the last row and column
+    const int lr = tid >> 4, lc = tid & 15, ka = k0 + lc * 4, eb = e0 + lc * 4;
+    const int a_bytes = 4 * max(0, min(4, a.K - ka)), b_bytes = eb < a.E ? 16 : 0;
+    const float* ap = A + (long long)(row0 + lr) * a.pitch + ka;
+    const float* bp = B + (long long)(row0 + lr) * a.E + eb;
+    const unsigned dst = smem_u32(&tiles[0][0][lr][lc]);
+    auto fetch = [&](int chunk) {
+#pragma unroll
+        for (int h = 0; h < 4; ++h) {
+            const bool on = row0 + chunk * 32 + lr + 8 * h < row_end;
+            const unsigned d = dst + (chunk & 1) * 8192 + h * 2048;
+            const float* const as = on && a_bytes ? ap + (long long)h * 8 * a.pitch : A;
+            const float* const bs = on && b_bytes ? bp + (long long)h * 8 * a.E : B;
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(as), "r"(on ? a_bytes : 0) : "memory");
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d + 16384), "l"(bs), "r"(on ? b_bytes : 0) : "memory");
+        }
+        ap += (long long)32 * a.pitch;
+        bp += (long long)32 * a.E;
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+
+    float acc[8][8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+#pragma unroll
+        for (int j = 0; j < 8; ++j) acc[i][j] = 0.f;
+    fetch(0);
+    for (int c = 0; c < chunks; ++c) {
+        cp_async_wait_all();
+        __syncthreads();                           // the stage is there, and the other buffer is free
+        if (c + 1 < chunks) fetch(c + 1);
+        const float4 (&As)[32][16] = tiles[0][c & 1];
+        const float4 (&Bs)[32][16] = tiles[1][c & 1];
+#pragma unroll 2
+        for (int p = half; p < 32; p += 2) {
+            const float4 a0 = As[p][tk], a1 = As[p][tk + 8], b0 = Bs[p][te], b1 = Bs[p][te + 8];
+            const float aa[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w}, bb[8] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
+#pragma unroll
+            for (int i = 0; i < 8; ++i)
+#pragma unroll
+                for (int j = 0; j < 8; ++j) acc[i][j] = fmaf(aa[i], bb[j], acc[i][j]);
+        }
+    }
+    // the odd pixels' share joins the even ones'
+    cp_async_wait_all();
+    __syncthreads();
+    float4* const meet = &tiles[0][0][0][0] + (tid & 63);
+    if (half) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+#pragma unroll
+            for (int j = 0; j < 2; ++j) meet[(i * 2 + j) * 64] = make_float4(acc[i][4 * j], acc[i][4 * j + 1], acc[i][4 * j + 2], acc[i][4 * j + 3]);
+    }
+    __syncthreads();
+    if (half) return;
+    float* part = a.partials + (size_t)blockIdx.x * a.K * a.E;
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+            const int k = k0 + tk * 4 + (i & 3) + (i >> 2) * 32, e = e0 + te * 4 + j * 32;
+            const float4 o = meet[(i * 2 + j) * 64];
+            if (k < a.K && e < a.E)
+                *reinterpret_cast<float4*>(part + (size_t)k * a.E + e) =
+                    make_float4(acc[i][4 * j] + o.x, acc[i][4 * j + 1] + o.y, acc[i][4 * j + 2] + o.z, acc[i][4 * j + 3] + o.w);
+        }
+}
+
 // ------------------------------------------------------------------------------------------------
 // The parameters' gradients from the partial results, d_W[e][r] (r < R), d_b[e] (r == RB) and d_Wx: block (32, ROWS), 32
 // neighbouring results, the partial results dealt round-robin to the rows of the block.  One launch for the
@@ -760,7 +843,8 @@ static int launch_wgrad(const m2d_proj_desc* d, const ProjPlan& p, float* partia
     a.P = (int)d->P; a.pitch = (int)d->proj_pitch; a.E = d->E; a.K = p.K; a.rows_per_slab = p.rows_per_slab;
     a.x = d->x; a.d_proj = d->d_proj;
     a.partials = partials;
-    xproj_wgrad_kernel<io_t><<<dim3(p.slabs, p.tilesE, p.tilesK), 256, 0, st>>>(a);
+    if (sizeof(io_t) == 4) xproj_wgrad_f32_kernel<<<dim3(p.slabs, p.tilesE, p.tilesK), kWgThreads, 0, st>>>(a);
+    else xproj_wgrad_kernel<io_t><<<dim3(p.slabs, p.tilesE, p.tilesK), 256, 0, st>>>(a);
     if (cudaGetLastError() != cudaSuccess) return M2D_ERR_LAUNCH;
     *sums = WgSums{partials, p.slabs, (long long)p.K * d->E, d->d_Wx};
     return M2D_OK;
