@@ -102,7 +102,7 @@ __global__ void __launch_bounds__(M2D_BWD_MAXW * 32, M2D_BWD_MINB) m2d_bwd_kerne
     __syncthreads();
 
     for (int b = (int)blockIdx.x; b < a.B; b += (int)gridDim.x) {
-        forward_rows<io_t, VEC, true>(a, smem, params, D_own, b, 0, 1);
+        forward_rows<io_t, VEC, true, false>(a, smem, params, D_own, b, 0, 1);
         reverse_rows<io_t, VEC>(a, smem, params, D_own, dAT, dAL, dD, b);
     }
 

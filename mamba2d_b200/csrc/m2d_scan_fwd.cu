@@ -13,7 +13,7 @@ __global__ void __launch_bounds__(256, 1) m2d_fwd_wave_kernel(const ScanArgs a) 
 }
 
 // Batch mode (one CTA per image and channel group): the sweep written as nested loops.
-template <typename io_t, bool VEC>
+template <typename io_t, bool VEC, bool ACT>
 __global__ void __launch_bounds__(256, 2) m2d_fwd_kernel(const ScanArgs a) {
     extern __shared__ float4 smem[];
     const int lane = threadIdx.x & 31;
@@ -32,7 +32,7 @@ __global__ void __launch_bounds__(256, 2) m2d_fwd_kernel(const ScanArgs a) {
     if (threadIdx.x < 32) stage_params<io_t>(params, a.AT, a.AL, a.N, ch0, chv, n0, nv, lane, a.a_log);
     __syncthreads();
     const int nb = (a.B - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x;
-    forward_rows<io_t, VEC, false>(a, smem, params, D_own, blockIdx.x, gridDim.x, nb);
+    forward_rows<io_t, VEC, false, ACT>(a, smem, params, D_own, blockIdx.x, gridDim.x, nb);
 }
 
 // The status word and, where CTAs of a wave launch read each other's, the boundary rows behind it.
@@ -49,7 +49,13 @@ static int launch_fwd(const m2d_scan_desc* d, const Plan& pl, bool vec, char* ws
     a.ring = reinterpret_cast<float4*>(ws + kStatusBytes);
     const size_t zero = pl.wave && pl.chain > 1 ? cleared_bytes(d, pl) : sizeof(int);
     if (!(d->flags & M2D_SCAN_WS_CLEARED) && cudaMemsetAsync(ws, 0, zero, st) != cudaSuccess) return M2D_ERR_LAUNCH;
-    if (!pl.wave) return launch_sweep_kernel(vec ? m2d_fwd_kernel<io_t, true> : m2d_fwd_kernel<io_t, false>, a, pl, st);
+    if (!pl.wave) {
+        auto pick = [&](auto act) {
+            constexpr bool ACT = decltype(act)::value;
+            return vec ? m2d_fwd_kernel<io_t, true, ACT> : m2d_fwd_kernel<io_t, false, ACT>;
+        };
+        return launch_sweep_kernel(a.act ? pick(std::true_type{}) : pick(std::false_type{}), a, pl, st);
+    }
     a.bnd = reinterpret_cast<float4*>(ws + kStatusBytes);
     a.bnd_rows = wave_rows(pl, false);
     Plan p = pl;
