@@ -6,10 +6,10 @@
 namespace m2d {
 
 // Few images: several CTAs per image.
-template <typename io_t, int C, bool VEC, bool ACT>
+template <typename io_t, int C, bool VEC, bool ACT, int COLS>
 __global__ void __launch_bounds__(256, 1) m2d_fwd_wave_kernel(const ScanArgs a) {
     extern __shared__ float4 smem[];
-    wave_forward<io_t, C, VEC, ACT ? kReadoutGelu : kReadout>(a, reinterpret_cast<char*>(smem));
+    wave_forward<io_t, C, VEC, ACT ? kReadoutGelu : kReadout, COLS>(a, reinterpret_cast<char*>(smem));
 }
 
 // Batch mode (one CTA per image and channel group): the sweep written as nested loops.
@@ -62,8 +62,10 @@ static int launch_fwd(const m2d_scan_desc* d, const Plan& pl, bool vec, char* ws
     p.smem = pl.wave == 4 ? WaveSmem<io_t, 4, false>::kBytes : WaveSmem<io_t, 2, false>::kBytes;
     auto pick = [&](auto act) {
         constexpr bool ACT = decltype(act)::value;
-        return pl.wave == 4 ? (vec ? m2d_fwd_wave_kernel<io_t, 4, true, ACT> : m2d_fwd_wave_kernel<io_t, 4, false, ACT>)
-                            : (vec ? m2d_fwd_wave_kernel<io_t, 2, true, ACT> : m2d_fwd_wave_kernel<io_t, 2, false, ACT>);
+        if (edge_pairs(d, pl))
+            return vec ? m2d_fwd_wave_kernel<io_t, 4, true, ACT, 2> : m2d_fwd_wave_kernel<io_t, 4, false, ACT, 2>;
+        return pl.wave == 4 ? (vec ? m2d_fwd_wave_kernel<io_t, 4, true, ACT, kChunk> : m2d_fwd_wave_kernel<io_t, 4, false, ACT, kChunk>)
+                            : (vec ? m2d_fwd_wave_kernel<io_t, 2, true, ACT, kChunk> : m2d_fwd_wave_kernel<io_t, 2, false, ACT, kChunk>);
     };
     return launch_sweep_kernel(a.act ? pick(std::true_type{}) : pick(std::false_type{}), a, p, st);
 }

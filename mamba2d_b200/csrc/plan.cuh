@@ -243,6 +243,15 @@ inline double wave_steps(const m2d_scan_desc* d, const Plan& p) {
     return (double)bands * ((d->W + 12) / 4 * 4) + (p.chain - 1) * 15.0;
 }
 
+// Whether a chained forward with four channels per lane hands its boundary rows over in pairs of columns instead of chunks
+// of four: a band then starts about 12 columns behind the one above instead of 15, and looks at the boundary twice per
+// chunk.  Worth it where the start-up of the chain is a quarter of the steps or more: 1024x1024x64 (35 %) 1734 us in
+// chunks, 1630 in pairs; below that they gain nothing or cost: 300x900x192 (16 %) 1122 / 1116, 512x512x192 (18 %) 1007 / 1056.
+// With two channels per lane, whose steps are shorter, pairs are slower (2x200x336x64 bf16 286 / 314).
+inline bool edge_pairs(const m2d_scan_desc* d, const Plan& p) {
+    return p.wave == 4 && p.chain > 1 && (p.chain - 1) * 15.0 * 4.0 >= wave_steps(d, p);
+}
+
 inline Plan plan_fwd(const m2d_scan_desc* d, bool allow_chain = true) {
     // The batch kernel runs one CTA per (image, 32 channels) and is at its best when those fill the GPU; the
     // wave kernels split an image over CTAs as well.  Measured times per step: 0.9 us (batch), 0.62 us (wave,

@@ -6,12 +6,13 @@
 
 namespace m2d {
 
-// The boundary row above a band, chunk by chunk: requested one chunk ahead, checked and parked in shared
-// memory when the chunk begins.
-template <int C>
+// The boundary row above a band, COLS columns at a time: requested one such piece ahead, checked and parked in shared
+// memory before the first step that needs it.
+template <int C, int COLS = kChunk>
 struct EdgeReader {
     static constexpr int EF = kEdgeFloats<C>;
-    static constexpr int kLoads = kChunk * EF / 4 / 32;
+    static constexpr int kLoads = COLS * EF / 4 / 32;
+    static_assert(COLS * EF % 128 == 0, "whole loads of a warp");
     uint4 v[kLoads];
     bool given_up = false;
     __device__ __forceinline__ bool mine(int k, int c0, int W, int lane) const { return c0 + (lane + 32 * k) / (EF / 4) < W; }
@@ -54,7 +55,10 @@ enum WaveKind { kReadout, kReadoutGelu, kRecord };
 // One band of image b (the `slot`-th image or list the launch has boundary rows for), top to bottom of the
 // image's dependences: lane row 0 leads, columns ascending.  kRecord writes
 // every state to `rec` ([t][m][lane], zeros for lanes outside the image) instead of the readout.
-template <typename io_t, int C, bool VEC, WaveKind KIND, bool BWD>
+//
+// COLS: boundary columns handed over at a time, a whole chunk of four or pairs: edge_pairs (plan.cuh).  Pairs are also taken
+// as late as they can be, before the step that reads the first of them.
+template <typename io_t, int C, bool VEC, WaveKind KIND, bool BWD, int COLS = kChunk>
 __device__ __forceinline__ void wave_forward_band(const ScanArgs& a, char* smem, const WaveLane<io_t, C, VEC, BWD>& ln, int b, int slot, int band, float4* rec) {
     typedef WaveSmem<io_t, C, BWD> S;
     typedef typename S::Stage L;
@@ -97,7 +101,7 @@ __device__ __forceinline__ void wave_forward_band(const ScanArgs& a, char* smem,
     const int ystep = a.dir * a.E;
     io_t* yp = static_cast<io_t*>(a.y) + (cpix * a.E + ln.ch0 + y_ch) - (r + 3) * ystep;    // stepped on before each use
     unsigned in_addr = zero_lane;
-    EdgeReader<C> reader;
+    EdgeReader<C, COLS> reader;
     typedef RecordBlock<C> Rec;
 
     auto stage_chunk = [&](int buf, int t0) {
@@ -131,10 +135,24 @@ __device__ __forceinline__ void wave_forward_band(const ScanArgs& a, char* smem,
         asm volatile("cp.async.commit_group;" ::: "memory");
         eb = eb == 2 ? 0 : eb + 1;
         const unsigned ebase = edge_lane + eb * kChunk * EB;
-        if (pull && t0 < W) {
-            reader.template settle<KIND == kRecord>(a, pull, t0, W, lane, smem_u32(edge) + eb * kChunk * EB);
-            if (t0 + kChunk < W) reader.request(pull, t0 + kChunk, W, lane);
-        }
+        auto take_edge = [&](const int s) {                              // columns t0 + s ... of the row above
+            if (s % COLS == 0 && pull && t0 + s < W) {
+                reader.template settle<KIND == kRecord>(a, pull, t0 + s, W, lane, smem_u32(edge) + (eb * kChunk + s) * EB);
+                if (t0 + s + COLS < W) reader.request(pull, t0 + s + COLS, W, lane);
+            }
+        };
+        auto give_edge = [&](const int s) {                              // lane row 7's columns of the steps up to s go out
+            if (s % COLS != COLS - 1 || !push) return;
+#pragma unroll
+            for (int k = 0; k < COLS * EF / 4 / 32; ++k) {
+                const int p = lane + 32 * k, from = s + 1 - COLS, col = t0 + from + p / (EF / 4) - kWaveRows;
+                if (col >= 0 && col < W)
+                    __stcg(reinterpret_cast<uint4*>(push + (size_t)col * EF) + p % (EF / 4),
+                           inverted(*reinterpret_cast<const uint4*>(edge + (3 * kChunk + from) * EB + p * 16)));
+            }
+            __syncwarp();
+        };
+        if (COLS == kChunk) take_edge(0);
         const unsigned out0 = r < kWaveRows - 1 ? slot_out : edge_lane + 3 * kChunk * EB;
         const int out_step = r < kWaveRows - 1 ? 0 : EB;
 
@@ -217,32 +235,27 @@ __device__ __forceinline__ void wave_forward_band(const ScanArgs& a, char* smem,
             first = firstN;
             in_addr = row0 ? zero_lane : (r > 0 ? slot_in : (band > 0 ? ebase + s * EB : zero_lane));
         };
-        if (t0 > kWaveRows && t0 + kChunk <= W) {
+        // (the boundary column of step s is read in step s + 1, where the recurrence of its cells is)
+        auto steps = [&](auto tag) {
 #pragma unroll
-            for (int s = 0; s < kChunk; ++s) step(std::false_type{}, s);
-        } else {
-#pragma unroll
-            for (int s = 0; s < kChunk; ++s) step(std::true_type{}, s);
-        }
-        if (push) {                                  // lane row 7's columns of this chunk go out
-#pragma unroll
-            for (int k = 0; k < kChunk * EF / 4 / 32; ++k) {
-                const int p = lane + 32 * k, col = t0 + p / (EF / 4) - kWaveRows;
-                if (col >= 0 && col < W)
-                    __stcg(reinterpret_cast<uint4*>(push + (size_t)col * EF) + p % (EF / 4), inverted(*reinterpret_cast<const uint4*>(edge + 3 * kChunk * EB + p * 16)));
+            for (int s = 0; s < kChunk; ++s) {
+                if (COLS < kChunk && s > 0) take_edge(s - 1);
+                step(tag, s);
+                give_edge(s);
             }
-            __syncwarp();
-        }
+        };
+        if (t0 > kWaveRows && t0 + kChunk <= W) steps(std::false_type{});
+        else steps(std::true_type{});
     }
 }
 
-template <typename io_t, int C, bool VEC, WaveKind KIND>
+template <typename io_t, int C, bool VEC, WaveKind KIND, int COLS = kChunk>
 __device__ __forceinline__ void wave_forward(const ScanArgs& a, char* smem) {
     WaveLane<io_t, C, VEC, false> ln;
     ln.init(a, smem);
     const int chains = (int)gridDim.x / a.chain, chain_id = (int)blockIdx.x / a.chain, cpos = (int)blockIdx.x % a.chain;
     for (int b = chain_id; b < a.B; b += chains)
-        for (int band = cpos; band < a.nbands; band += a.chain) wave_forward_band<io_t, C, VEC, KIND, false>(a, smem, ln, b, chain_id, band, nullptr);
+        for (int band = cpos; band < a.nbands; band += a.chain) wave_forward_band<io_t, C, VEC, KIND, false, COLS>(a, smem, ln, b, chain_id, band, nullptr);
 }
 
 }  // namespace m2d
