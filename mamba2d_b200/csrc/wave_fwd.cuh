@@ -103,6 +103,10 @@ __device__ __forceinline__ void wave_forward_band(const ScanArgs& a, char* smem,
     unsigned in_addr = zero_lane;
     EdgeReader<C, COLS> reader;
     typedef RecordBlock<C> Rec;
+    // Where the chunk's columns are sent from: from the steps, or, with bf16 I/O and four channels per lane, from one place
+    // behind them (512x512x192 bf16 1020 us from the steps, 1000 from behind; fp32 1004 and 1009; 512x512x64 fp32, two
+    // channels per lane, 608 and 638).
+    constexpr bool kGiveAfter = C == 4 && COLS == kChunk && sizeof(io_t) == 2;
 
     auto stage_chunk = [&](int buf, int t0) {
         const int off = buf * kChunk * L::kStepBytes + w * L::kCellBytes, col = t0 - w;
@@ -241,11 +245,12 @@ __device__ __forceinline__ void wave_forward_band(const ScanArgs& a, char* smem,
             for (int s = 0; s < kChunk; ++s) {
                 if (COLS < kChunk && s > 0) take_edge(s - 1);
                 step(tag, s);
-                give_edge(s);
+                if (!kGiveAfter) give_edge(s);
             }
         };
         if (t0 > kWaveRows && t0 + kChunk <= W) steps(std::false_type{});
         else steps(std::true_type{});
+        if (kGiveAfter) give_edge(kChunk - 1);
     }
 }
 
