@@ -62,7 +62,7 @@ static int launch_fwd(const m2d_scan_desc* d, const Plan& pl, bool vec, char* ws
     p.smem = pl.wave == 4 ? WaveSmem<io_t, 4, false>::kBytes : WaveSmem<io_t, 2, false>::kBytes;
     auto pick = [&](auto act) {
         constexpr bool ACT = decltype(act)::value;
-        if (edge_pairs(d, pl))
+        if (edge_pairs(d, pl, sizeof(io_t)))
             return vec ? m2d_fwd_wave_kernel<io_t, 4, true, ACT, 2> : m2d_fwd_wave_kernel<io_t, 4, false, ACT, 2>;
         return pl.wave == 4 ? (vec ? m2d_fwd_wave_kernel<io_t, 4, true, ACT, kChunk> : m2d_fwd_wave_kernel<io_t, 4, false, ACT, kChunk>)
                             : (vec ? m2d_fwd_wave_kernel<io_t, 2, true, ACT, kChunk> : m2d_fwd_wave_kernel<io_t, 2, false, ACT, kChunk>);

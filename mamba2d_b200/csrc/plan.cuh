@@ -245,11 +245,15 @@ inline double wave_steps(const m2d_scan_desc* d, const Plan& p) {
 
 // Whether a chained forward with four channels per lane hands its boundary rows over in pairs of columns instead of chunks
 // of four: a band then starts about 12 columns behind the one above instead of 15, and looks at the boundary twice per
-// chunk.  Worth it where the start-up of the chain is a quarter of the steps or more: 1024x1024x64 (35 %) 1734 us in
-// chunks, 1630 in pairs; below that they gain nothing or cost: 300x900x192 (16 %) 1122 / 1116, 512x512x192 (18 %) 1007 / 1056.
+// chunk.  Worth it where the start-up of the chain is a good part of the steps, with bf16 I/O, whose chunks are sent later
+// (kGiveAfter), a tenth, in fp32 three tenths.  Chunks / pairs, us, by the start-up's share of the steps:
+//   bf16  400x400x384 (7 %) 1143 / 1157, 3x85x96x384 (12 %) 205 / 204, 300x900x192 (16 %) 1125 / 1112, 512x512x192 (18 %) 1011 / 989,
+//         4x130x200x128 (22 %) 304 / 293, 300x500x192 (25 %) 680 / 668, 2x336x336x96 (33 %) 561 / 511
+//   fp32  512x512x192 (18 %) 1002 / 1051, 300x500x192 (25 %) 686 / 709, 3x200x300x96 (26 %) 420 / 435, 2x300x336x96 (33 %) 531 / 513,
+//         250x250x256 (33 %) 432 / 410, 1024x1024x64 (35 %) 1734 / 1626
 // With two channels per lane, whose steps are shorter, pairs are slower (2x200x336x64 bf16 286 / 314).
-inline bool edge_pairs(const m2d_scan_desc* d, const Plan& p) {
-    return p.wave == 4 && p.chain > 1 && (p.chain - 1) * 15.0 * 4.0 >= wave_steps(d, p);
+inline bool edge_pairs(const m2d_scan_desc* d, const Plan& p, size_t element) {
+    return p.wave == 4 && p.chain > 1 && (p.chain - 1) * 15.0 * 10.0 >= wave_steps(d, p) * (element == 2 ? 1 : 3);
 }
 
 inline Plan plan_fwd(const m2d_scan_desc* d, bool allow_chain = true) {

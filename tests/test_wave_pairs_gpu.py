@@ -1,6 +1,7 @@
 """Chained forwards that hand their boundary rows over in pairs of columns (few images, four channels per lane, a chain whose
-start-up is a quarter of the steps or more): maps that end inside a pair or a chunk, a last band of one row, a CTA that comes
-back for a later band, ragged channels.  The bounds are those of the other tests of these kernels."""
+start-up is three tenths of the steps or more, the line of fp32; bf16 has a lower one): maps that end inside a pair or a
+chunk, a last band of one row, a CTA that comes back for a later band, ragged channels.  The bounds are those of the other
+tests of these kernels."""
 import pytest
 import torch
 
