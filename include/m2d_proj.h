@@ -105,7 +105,8 @@ int m2d_xproj_wgrad_on_tensor_cores(const m2d_proj_desc *desc);
 /*
  * out (rows, n) = a (rows, k) @ w, or out += where `accumulate` is set; fp32, row-major and dense; `w` is (k, n), or
  * (n, k) where `transposed` is set.  The x projection of fp32 pixels, x @ Wx^T, and its contribution to d_x,
- * d_x += d_proj @ Wx, to the precision of fp32 products (split operands on the tensor cores).  n and k
+ * d_x += d_proj @ Wx, to the precision of fp32 products (split operands on the tensor cores; results that are not
+ * finite are those of fp32 sums).  n and k
  * multiples of 4 and 16-byte aligned pointers (M2D_ERR_PITCH otherwise), at most 4 * M2D_PROJ_MAX_E
  * columns or terms (M2D_ERR_TOO_LARGE).  No workspace.
  */

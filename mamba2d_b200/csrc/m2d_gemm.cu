@@ -11,6 +11,11 @@
 // tcgen05 would want the parts of every row staged in shared memory).  The six are summed
 // smallest first in a fresh accumulator per 16 terms and that sum is added to the running one by an ordinary
 // fp32 add: the tensor cores' own accumulation truncates, and over E / 16 steps that would show.
+//
+// Parts of an infinity, or of a float beyond 3.39e38 whose first part rounds to one, have differences of infinities in
+// them.  Whatever holds such a part sums to something that is not finite (inf * 0 is a NaN), so where the sums of a
+// lane are not all finite it computes its results again, from the floats.  (Below 2^-110 the last part of a float
+// falls under bf16's smallest number, 2^-133.)
 #include <algorithm>
 
 #include "m2d_proj.h"
@@ -101,13 +106,39 @@ __device__ __forceinline__ void put2(const GemmArgs& a, long long row, int col, 
     if (row < a.rows && col < a.n) *reinterpret_cast<float2*>(a.out + row * a.n + col) = v;
 }
 
+// Two neighbouring results as ordinary fp32 sums of products.  (A NaN stays one, whatever is added.)
+__device__ __forceinline__ float2 plain_sums(const GemmArgs& a, long long row, int col) {
+    float2 s = make_float2(0.f, 0.f);
+    if (row >= a.rows || col >= a.n) return s;
+    const float* x = a.a + row * a.k;
+    const float* w = a.w + (a.transposed ? (size_t)col * a.k : col);
+    const int next = a.transposed ? 1 : a.n, other = a.transposed ? a.k : 1;
+#pragma unroll 1
+    for (int k = 0; k < a.k && !(isnan(s.x) && isnan(s.y)); ++k, w += next) {
+        const float v = __ldg(x + k);
+        s.x = fmaf(v, __ldg(w), s.x);
+        s.y = fmaf(v, __ldg(w + other), s.y);
+    }
+    return s;
+}
+__device__ __forceinline__ void put_result(const GemmArgs& a, long long row, int col, float2 v) {
+    if (a.accumulate) {
+        const float2 old = load2(a, row, col);
+        v.x += old.x;
+        v.y += old.y;
+    }
+    put2(a, row, col, v);
+}
+
 // Many rows.  grid (CTAs, chunks of NT * 8 columns); a warp computes 16 rows at a time against the chunk, whose
 // fragments every CTA splits once into shared memory.  The rows come straight from global memory, two steps of 16
 // terms ahead, the first of the next tile among them.  Bound by the rate of mma.sync (four cycles of an SM each).  Two
 // 16-row tiles per warp, which halve the reads of the fragments, need twice the registers: 166 against 112 us for the
-// product that accumulates at P = 401408, E = 64, and nothing gained for the other (events, L2 flushed).
+// product that accumulates at P = 401408, E = 64, and nothing gained for the other (events, L2 flushed).  The look at
+// the sums costs nothing that shows (67.3 / 67.8 and 86.9 / 86.4 us there without / with); a branch for each pair of
+// results, between their stores, was 75 and 92.
 template <int NT>
-__global__ void __launch_bounds__(256, 2) rows_gemm_kernel(const GemmArgs a) {
+__global__ void __launch_bounds__(256, NT == 2 ? 3 : 2) rows_gemm_kernel(const GemmArgs a) {
     extern __shared__ uint2 gemm_w[];              // [step][n-tile][part][lane]
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
     const int col0 = blockIdx.y * NT * 8;
@@ -175,14 +206,28 @@ __global__ void __launch_bounds__(256, 2) rows_gemm_kernel(const GemmArgs a) {
 #pragma unroll
             for (int h = 0; h < 2; ++h)
                 old[n][h] = a.accumulate ? load2(a, row0 + g + 8 * h, col0 + n * 8 + t * 2) : make_float2(0.f, 0.f);
+        float size[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
         for (int n = 0; n < NT; ++n)
 #pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                float2 v = make_float2(acc[n][2 * h], acc[n][2 * h + 1]);
-                if (a.accumulate) { v.x += old[n][h].x; v.y += old[n][h].y; }
-                put2(a, row0 + g + 8 * h, col0 + n * 8 + t * 2, v);
+            for (int i = 0; i < 4; ++i) size[i] += fabsf(acc[n][i]);
+        if (size[0] + size[1] + (size[2] + size[3]) < INFINITY) {
+#pragma unroll
+            for (int n = 0; n < NT; ++n)
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    float2 v = make_float2(acc[n][2 * h], acc[n][2 * h + 1]);
+                    if (a.accumulate) { v.x += old[n][h].x; v.y += old[n][h].y; }
+                    put2(a, row0 + g + 8 * h, col0 + n * 8 + t * 2, v);
+                }
+        } else {
+#pragma unroll 1
+            for (int i = 0; i < 2 * NT; ++i) {
+                const long long row = row0 + g + i % 2 * 8;
+                const int col = col0 + i / 2 * 8 + t * 2;
+                put_result(a, row, col, plain_sums(a, row, col));
             }
+        }
     }
 }
 
@@ -222,12 +267,7 @@ __global__ void __launch_bounds__(256) rows_gemm_small_kernel(const GemmArgs a) 
     }
     const long long row = row0 + h * 8 + g;
     const int col = col0 + n * 8 + t * 2;
-    if (a.accumulate) {
-        const float2 old = load2(a, row, col);
-        x += old.x;
-        y += old.y;
-    }
-    put2(a, row, col, make_float2(x, y));
+    put_result(a, row, col, fabsf(x) + fabsf(y) < INFINITY ? make_float2(x, y) : plain_sums(a, row, col));
 }
 
 template <int NT>

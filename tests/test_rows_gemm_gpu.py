@@ -32,3 +32,39 @@ def test_rows_gemm(rows, n, k, transposed, accumulate):
 def test_rows_gemm_adds_to_wide_rows(rows, n, k):
     """d_x += d_proj @ Wx at the widths and row counts that no longer go to the GEMM library."""
     test_rows_gemm(rows, n, k, 0, 1)
+
+
+@pytest.mark.parametrize("transposed,accumulate", [(1, 0), (0, 1)])
+@pytest.mark.parametrize("rows,n,k", [(40, 60, 68), (5000, 12, 20), (20011, 64, 56), (12017, 112, 64)])
+def test_rows_gemm_of_values_that_bf16_parts_cannot_hold(rows, n, k, transposed, accumulate):
+    """Infinities, NaNs and floats that round to infinity in bf16, in either factor and in what is added to: each result is
+    the infinity, the NaN or the number that fp64 gives (rounded to fp32: a product beyond its range is infinite)."""
+    g = torch.Generator(device="cuda").manual_seed(rows + n)
+    inf, nan, most = float("inf"), float("nan"), 3.4e38
+    a = torch.randn(rows, k, generator=g, device="cuda")
+    w = torch.randn(n, k, generator=g, device="cuda")
+    w[:, k // 2:] = w[:, k // 2:].bfloat16().float()          # exact in one part: the others are zeros
+    w[1] = 0.0
+    w[3:9] *= 0.1                                             # no two large terms meet that only an fp32 sum would take
+    a[:, k - 1] *= 0.1                                        # out of range on its way, by the order of its terms
+    for i, v in enumerate((inf, -inf, nan, most, -most)):
+        a[7 * i, 3 * i] = v
+        a[rows - 1 - i, k - 1 - i] = v
+    w[5, 2], w[6, k - 7], w[8, k - 1] = inf, -inf, -most
+    out = torch.randn(rows, n, generator=g, device="cuda")
+    out[2, 3], out[rows - 3, 9], out[4, 4] = inf, -inf, nan
+    want = (a.double() @ w.double().t() + (out.double() if accumulate else 0.0)).float()
+    m = w if transposed else w.t().contiguous()
+    ptr = lambda t: ctypes.c_void_p(t.data_ptr())
+    rc = _lib.lib().m2d_rows_gemm_f32(ctypes.c_int64(rows), n, k, ptr(a), ptr(m), transposed, accumulate, ptr(out),
+                                      ctypes.c_void_p(torch.cuda.current_stream().cuda_stream))
+    assert rc == 0
+    assert torch.equal(out.isnan(), want.isnan())
+    assert torch.equal(out.isinf(), want.isinf()) and torch.equal(out[out.isinf()], want[want.isinf()])
+    ok = want.isfinite()
+    small = ok & (want.abs() < 1e30)
+    assert int(small.sum()) > 0.5 * rows * n
+    assert float((out.double() - want.double())[small].abs().max()) < 2e-6 * (k + 1) ** 0.5      # of one result, as above
+    large = ok & ~small                                       # at most three terms are large: a rounding of fp32 (6e-8) each
+    size = a.double().abs() @ w.double().abs().t()
+    assert int(large.sum()) > 0 and float(((out.double() - want.double()).abs() / size)[large].max()) < 1.8e-7
