@@ -174,7 +174,17 @@ void gemm(const Tensor& like, int64_t rows, int64_t n, int64_t k, const void* a,
     //     100352  46 / 29   58 / 49  114 / 78                              46 / 38   69 / 56  127 / 81
     // The first product follows its columns (E up to 192).  The second is the library's between 2048 and 12000 rows, where
     // neither gains; below that the own kernel's error, a third of the library's, keeps what it has.
-    if (like.scalar_type() == at::kFloat && (n <= 72 || rows <= 2048 || (accumulate && rows >= 12000))) {
+    //
+    // A caller that allows TF32 products gets them where the library's are faster then, by rows (TF32 / own, us, E = 64, 192, 512):
+    //              x @ Wx^T                          d_x += d_proj @ Wx
+    //     784      24 / 16   16 / 14   19 / 18       21 / 16   24 / 14   17 / 20
+    //     2100     15 / 15   16 / 17   20 / 23       14 / 14   15 / 19   20 / 32
+    //     12544    16 / 17   22 / 27   26 / 68       17 / 19   25 / 27   31 / 51
+    //     100352   31 / 30   37 / 79   64 / 294      42 / 37   55 / 80   91 / 233
+    //     401408   53 / 68                           94 / 89
+    const bool tf32 = at::globalContext().float32Precision(at::Float32Backend::CUDA, at::Float32Op::MATMUL) == at::Float32Precision::TF32;
+    const bool own = tf32 ? rows <= 1024 || (accumulate && n <= 64) : n <= 72 || rows <= 2048 || (accumulate && rows >= 12000);
+    if (like.scalar_type() == at::kFloat && own) {
         const int rc = m2d_rows_gemm_f32(rows, (int)n, (int)k, static_cast<const float*>(a), static_cast<const float*>(w), transposed, accumulate,
                                          static_cast<float*>(out), stream_of(like));
         if (rc == M2D_OK) return;

@@ -56,6 +56,31 @@ def test_scan_equals_the_op_by_op_path(dt, tol, monkeypatch):
         assert rel_err(a.float().cpu().numpy(), b.float().cpu().numpy()) < tol
 
 
+@pytest.mark.parametrize("E", [96, 128, 192])
+def test_a_caller_that_allows_tf32_products_gets_them(E, monkeypatch):
+    """Many rows: the x projection and what comes back through it, each by itself, show TF32's rounding (2^-11 of a factor) where it
+    is allowed and fp32's where it is not."""
+    w = inputs.make_module_params(E, 16, seed=5)
+    ws = [w[k].cuda() for k in NAMES]
+    g = torch.Generator().manual_seed(1)
+    x, gy = torch.randn(14, 30, 30, E, generator=g).cuda().requires_grad_(True), torch.randn(14, 30, 30, E, generator=g).cuda()
+
+    def both(fwd, bwd):
+        monkeypatch.setattr(torch.backends.cuda.matmul, "allow_tf32", fwd)
+        y = wc.wavefront_scan_cuda(x, *ws)
+        monkeypatch.setattr(torch.backends.cuda.matmul, "allow_tf32", bwd)
+        return y.detach(), torch.autograd.grad(y, x, gy)[0]
+
+    def far(a, b):
+        return float((a.double() - b.double()).norm() / b.double().norm())
+    y, dx = both(False, False)
+    y_f, _ = both(True, False)
+    y_b, dx_b = both(False, True)
+    assert torch.equal(y_b, y)
+    assert 5e-6 < far(y_f, y) < 5e-3
+    assert 5e-6 < far(dx_b, dx) < 5e-3
+
+
 def test_what_the_native_path_does_not_take_goes_op_by_op():
     w = inputs.make_module_params(36, 16, seed=5)                          # 36 channels: dt rank 20 is beyond the kernels' range
     w["dt_projT_w"], w["dt_projL_w"] = torch.randn(36, 20) * 0.2, torch.randn(36, 20) * 0.2
