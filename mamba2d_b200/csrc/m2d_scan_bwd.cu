@@ -1,5 +1,7 @@
 // Backward entry point of the wavefront scan: recompute sweep + adjoint sweep in one kernel,
 // followed by a small kernel that casts the fp32 accumulators of the reduced gradients.
+#include <algorithm>
+
 #include "launch.cuh"
 #include "sweep_rows.cuh"
 #include "wave_bwd.cuh"
@@ -269,8 +271,11 @@ static int launch_bwd(const m2d_scan_desc* d, const Plan& pl, bool vec, cudaStre
     if (d->dtype != M2D_F32) {
         const int pitch = d->d_BC_pitch ? (int)d->d_BC_pitch : d->N;
         const bool quads = d->N % 4 == 0 && pitch % 4 == 0 && aligned(d->d_BT, 8) && aligned(d->d_BL, 8) && aligned(d->d_C, 8);
-        const size_t fit = (size_t)sm_count() * 8, items = quads ? npn / 4 : npn;
-        const int fin_blocks = (int)((items + 255) / 256 < fit ? (items + 255) / 256 : fit);
+        // a thread per quad of B and C or per (channel, state), whichever are more: a 7x7 image of 512 channels has 196 of those
+        // and 8192 of these.  A grid for the quads alone / this one, us: 1x7x7x512 18.4 / 2.8, 1x5x5x576 19.8 / 2.4,
+        // 3x7x7x512 7.7 / 2.8, 4x14x14x384 3.5 / 2.8, 128x28x28x128 6.3 / 6.3
+        const size_t fit = (size_t)sm_count() * 8, items = std::max(quads ? npn / 4 : npn, en);
+        const int fin_blocks = (int)std::min((items + 255) / 256, fit);
         (quads ? m2d_bwd_finalize<io_t, true> : m2d_bwd_finalize<io_t, false>)<<<fin_blocks, 256, 0, st>>>(
             a.accBT, static_cast<io_t*>(d->d_BT), static_cast<io_t*>(d->d_BL), static_cast<io_t*>(d->d_C), d->d_AT, d->d_AL, d->d_D, (long long)npn,
             d->N, pitch, (long long)en, d->E, a.a_log, a.d_f32);
