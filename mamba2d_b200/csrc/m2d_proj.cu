@@ -397,15 +397,14 @@ __global__ void __launch_bounds__(MAXT) dtproj_bwd_kernel(const ProjArgs a) {
 // computes a 64x64 tile of the result over its slab of pixels, 32 pixels per shared-memory stage,
 // each thread a 4x4 block.
 // ------------------------------------------------------------------------------------------------
-__device__ __forceinline__ float4 load4g(const float* p) { return __ldg(reinterpret_cast<const float4*>(p)); }
 __device__ __forceinline__ float4 load4g(const __nv_bfloat16* p) {
     const uint2 u = __ldg(reinterpret_cast<const uint2*>(p));
     return make_float4(__uint_as_float(u.x << 16), __uint_as_float(u.x & 0xffff0000u),
                        __uint_as_float(u.y << 16), __uint_as_float(u.y & 0xffff0000u));
 }
 
-template <typename io_t>
-__global__ void __launch_bounds__(256) xproj_wgrad_kernel(const WgArgs a) {
+__global__ void __launch_bounds__(256) xproj_wgrad_kernel(const WgArgs a) {      // bf16
+    typedef __nv_bfloat16 io_t;
     __shared__ float4 As[2][32][16];
     __shared__ float4 Bs[2][32][16];
     const io_t* A = static_cast<const io_t*>(a.d_proj);
@@ -835,7 +834,7 @@ static int launch_wgrad_tc(const m2d_proj_desc* d, const ProjPlan& p, float* par
 
 template <typename io_t>
 static int launch_wgrad(const m2d_proj_desc* d, const ProjPlan& p, float* partials, WgSums* sums, cudaStream_t st) {
-    if (sizeof(io_t) == 2) {
+    if constexpr (sizeof(io_t) == 2) {
         const int rc = launch_wgrad_tc(d, p, partials, sums, st);
         if (rc >= 0) return rc;
     }
@@ -843,8 +842,8 @@ static int launch_wgrad(const m2d_proj_desc* d, const ProjPlan& p, float* partia
     a.P = (int)d->P; a.pitch = (int)d->proj_pitch; a.E = d->E; a.K = p.K; a.rows_per_slab = p.rows_per_slab;
     a.x = d->x; a.d_proj = d->d_proj;
     a.partials = partials;
-    if (sizeof(io_t) == 4) xproj_wgrad_f32_kernel<<<dim3(p.slabs, p.tilesE, p.tilesK), kWgThreads, 0, st>>>(a);
-    else xproj_wgrad_kernel<io_t><<<dim3(p.slabs, p.tilesE, p.tilesK), 256, 0, st>>>(a);
+    if constexpr (sizeof(io_t) == 4) xproj_wgrad_f32_kernel<<<dim3(p.slabs, p.tilesE, p.tilesK), kWgThreads, 0, st>>>(a);
+    else xproj_wgrad_kernel<<<dim3(p.slabs, p.tilesE, p.tilesK), 256, 0, st>>>(a);
     if (cudaGetLastError() != cudaSuccess) return M2D_ERR_LAUNCH;
     *sums = WgSums{partials, p.slabs, (long long)p.K * d->E, d->d_Wx};
     return M2D_OK;

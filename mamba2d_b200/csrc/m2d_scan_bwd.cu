@@ -161,9 +161,10 @@ __global__ void __launch_bounds__(M2D_BWD_MAXW * 32, M2D_BWD_MINB) m2d_bwd_kerne
 // they are gradients of the fp32 parameter A_log).  VEC: four states at a time (N and the pitch multiples of 4, tensors
 // on 8 bytes).  Bound by its traffic then; one state at a time, with a 64-bit division for its pixel, took 11.4 us at
 // 128 x 28 x 28 x 128 and 14.4 at 2 x 200 x 336 x 64, 6.6 and 7.2 now.
-template <typename io_t, bool VEC>
-__global__ void m2d_bwd_finalize(const float* __restrict__ acc, io_t* d_BT, io_t* d_BL, io_t* d_C, void* d_AT, void* d_AL,
+template <bool VEC>
+__global__ void m2d_bwd_finalize(const float* __restrict__ acc, __nv_bfloat16* d_BT, __nv_bfloat16* d_BL, __nv_bfloat16* d_C, void* d_AT, void* d_AL,
                                  void* d_D, long long npn, int N, int pitch, long long en, int E, int a_log, int d_f32) {
+    typedef __nv_bfloat16 io_t;
     const long long tid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     const long long nthreads = (long long)gridDim.x * blockDim.x;
     if (VEC) {
@@ -268,7 +269,7 @@ static int launch_bwd(const m2d_scan_desc* d, const Plan& pl, bool vec, cudaStre
     const int rc = launch_sweep_kernel(pl.wave ? (vec ? m2d_bwd_wave_kernel<io_t, true> : m2d_bwd_wave_kernel<io_t, false>)
                                                : (vec ? m2d_bwd_kernel<io_t, true> : m2d_bwd_kernel<io_t, false>), a, p, st);
     if (rc != M2D_OK) return rc;
-    if (d->dtype != M2D_F32) {
+    if constexpr (sizeof(io_t) == 2) {
         const int pitch = d->d_BC_pitch ? (int)d->d_BC_pitch : d->N;
         const bool quads = d->N % 4 == 0 && pitch % 4 == 0 && aligned(d->d_BT, 8) && aligned(d->d_BL, 8) && aligned(d->d_C, 8);
         // a thread per quad of B and C or per (channel, state), whichever are more: a 7x7 image of 512 channels has 196 of those
@@ -276,7 +277,7 @@ static int launch_bwd(const m2d_scan_desc* d, const Plan& pl, bool vec, cudaStre
         // 3x7x7x512 7.7 / 2.8, 4x14x14x384 3.5 / 2.8, 128x28x28x128 6.3 / 6.3
         const size_t fit = (size_t)sm_count() * 8, items = std::max(quads ? npn / 4 : npn, en);
         const int fin_blocks = (int)std::min((items + 255) / 256, fit);
-        (quads ? m2d_bwd_finalize<io_t, true> : m2d_bwd_finalize<io_t, false>)<<<fin_blocks, 256, 0, st>>>(
+        (quads ? m2d_bwd_finalize<true> : m2d_bwd_finalize<false>)<<<fin_blocks, 256, 0, st>>>(
             a.accBT, static_cast<io_t*>(d->d_BT), static_cast<io_t*>(d->d_BL), static_cast<io_t*>(d->d_C), d->d_AT, d->d_AL, d->d_D, (long long)npn,
             d->N, pitch, (long long)en, d->E, a.a_log, a.d_f32);
         if (cudaGetLastError() != cudaSuccess) return M2D_ERR_LAUNCH;
