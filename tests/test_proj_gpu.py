@@ -171,3 +171,19 @@ def test_xproj_weight_gradient_on_tensor_cores(P, E, R, monkeypatch):
     simt = wc._xproj_wgrad(d_proj, x, N, R)
     torch.cuda.synchronize()
     assert float((got.double() - simt.double()).abs().max()) <= 1e-2 * scale     # both round their fp32 sums to bf16
+
+
+@pytest.mark.parametrize("P,E,R,N,pitch", [(1000, 40, 5, 16, 60), (3001, 64, 4, 15, 56), (130, 132, 5, 15, 56), (77, 64, 5, 16, 64), (31, 576, 36, 11, 112)])
+@pytest.mark.parametrize("dt,tol", [(torch.float32, 2e-6), (torch.bfloat16, 8e-3)])
+def test_xproj_weight_gradient_of_rows_that_end_inside_a_quad(P, E, R, N, pitch, dt, tol):
+    """2R + 3N columns of a wider row, one to three of them in the last quad; what lies behind them is not read as numbers.
+    (Relative to the largest result: fp32 sums of P products, and the rounding of a result to bf16.)"""
+    from mamba2d_b200 import wavefront_cuda as wc
+    K = 2 * R + 3 * N
+    assert K % 4 and K < pitch
+    g = torch.Generator().manual_seed(P + E)
+    d_proj = torch.full((P, pitch), float("nan"))
+    d_proj[:, :K] = torch.randn(P, K, generator=g)
+    d_proj, x = d_proj.to(dt).cuda(), torch.randn(P, E, generator=g).to(dt).cuda()
+    want = d_proj[:, :K].double().T @ x.double()
+    assert rel_err(wc._xproj_wgrad(d_proj, x, N, R).double().cpu().numpy(), want.cpu().numpy()) < tol
