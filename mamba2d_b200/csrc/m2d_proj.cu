@@ -95,33 +95,6 @@ static ProjPlan plan_proj(const m2d_proj_desc* d) {
     return p;
 }
 
-// softplus with the reference's threshold of 20 (torch.nn.functional.softplus defaults)
-// log1p(t) for t in (0, 1] as 2*atanh(t / (2 + t)): the argument stays below 1/3, where seven terms of
-// the series are exact to fp32 rounding (next term 2 s^15 / 15 < 1e-8 of the result); half the
-// instructions of log1pf, which was a third of the forward kernel.
-__device__ __forceinline__ float log1p_unit(float t) {
-    const float s = __fdividef(t, 2.f + t), s2 = s * s;
-    float p = 1.f / 13.f;
-    p = fmaf(p, s2, 1.f / 11.f);
-    p = fmaf(p, s2, 1.f / 9.f);
-    p = fmaf(p, s2, 1.f / 7.f);
-    p = fmaf(p, s2, 1.f / 5.f);
-    p = fmaf(p, s2, 1.f / 3.f);
-    p = fmaf(p, s2, 1.f);
-    return 2.f * s * p;
-}
-// softplus(z) = max(z, 0) + log1p(exp(-|z|)); past the reference's threshold of 20 the second term is
-// below half an ulp of z, so the threshold of torch.nn.functional.softplus needs no branch
-__device__ __forceinline__ float softplus_f(float z) {
-    // exp(-|z|) = 2^(a + e): a is the rounded product with log2(e); e collects what that rounding and
-    // the rounding of the constant lost (without it the error grows with |z|: 3e-6 at |z| = 60)
-    const float m = -fabsf(z);
-    const float a = m * kLog2e;
-    const float e = fmaf(m, kLog2e, -a) + m * 1.92596299e-8f;
-    const float t = ex2(a) * fmaf(e, kLn2, 1.f);
-    return fmaxf(z, 0.f) + log1p_unit(t);
-}
-
 // ------------------------------------------------------------------------------------------------
 // delta = softplus(r @ W^T + b).  grid (ctas, 2 directions); block = EB channels x PS pixels.
 // ------------------------------------------------------------------------------------------------

@@ -61,10 +61,44 @@ __device__ __forceinline__ float rcp_approx(float v) {
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(v));
     return r;
 }
+// The larger of two, NaN if either is (fmaxf would drop it).
+__device__ __forceinline__ float max_nan(float a, float b) {
+    float m;
+    asm("max.NaN.f32 %0, %1, %2;" : "=f"(m) : "f"(a), "f"(b));
+    return m;
+}
+// softplus with the reference's threshold of 20 (torch.nn.functional.softplus defaults)
+// log1p(t) for t in (0, 1] as 2*atanh(t / (2 + t)): the argument stays below 1/3, where seven terms of
+// the series are exact to fp32 rounding (next term 2 s^15 / 15 < 1e-8 of the result); half the
+// instructions of log1pf, which was a third of the forward kernel.
+__device__ __forceinline__ float log1p_unit(float t) {
+    const float s = __fdividef(t, 2.f + t), s2 = s * s;
+    float p = 1.f / 13.f;
+    p = fmaf(p, s2, 1.f / 11.f);
+    p = fmaf(p, s2, 1.f / 9.f);
+    p = fmaf(p, s2, 1.f / 7.f);
+    p = fmaf(p, s2, 1.f / 5.f);
+    p = fmaf(p, s2, 1.f / 3.f);
+    p = fmaf(p, s2, 1.f);
+    return 2.f * s * p;
+}
+// softplus(z) = max(z, 0) + log1p(exp(-|z|)); past the reference's threshold of 20 the second term is
+// below half an ulp of z, so the threshold of torch.nn.functional.softplus needs no branch
+__device__ __forceinline__ float softplus_f(float z) {
+    // exp(-|z|) = 2^(a + e): a is the rounded product with log2(e); e collects what that rounding and
+    // the rounding of the constant lost (without it the error grows with |z|: 3e-6 at |z| = 60)
+    const float m = max_nan(-fabsf(z), -200.f);      // (exp is zero there; an infinity would leave no remainder)
+    const float a = m * kLog2e;
+    const float e = fmaf(m, kLog2e, -a) + m * 1.92596299e-8f;
+    const float t = ex2(a) * fmaf(e, kLn2, 1.f);
+    return fmaxf(z, 0.f) + log1p_unit(t);
+}
 // softplus of two values: max(z, 0) + log1p(exp(-|z|)), the arithmetic of softplus_f on packed pairs.  (The
 // divisor of the series' argument is 2 + t in (2, 3]: a plain reciprocal needs none of a division's scaling.)
+// Without ANY a |z| whose product with log2(e) overflows, from 2.3e38 on, gives NaN.
+template <bool ANY>
 __device__ __forceinline__ float2 softplus2(float2 z) {
-    const float2 m = make_float2(-fabsf(z.x), -fabsf(z.y));
+    const float2 m = ANY ? make_float2(max_nan(-fabsf(z.x), -200.f), max_nan(-fabsf(z.y), -200.f)) : make_float2(-fabsf(z.x), -fabsf(z.y));
     const float2 b = __fmul2_rn(m, dup2(-kLog2e));          // exp(-|z|) = 2^(-b + e), e what rounding b lost
     const float2 e = __ffma2_rn(m, dup2(1.92596299e-8f), __ffma2_rn(m, dup2(kLog2e), b));
     const float2 t = __fmul2_rn(make_float2(ex2(-b.x), ex2(-b.y)), __ffma2_rn(e, dup2(kLn2), dup2(1.f)));
@@ -95,7 +129,9 @@ __device__ __forceinline__ float2 softplus_grad2(float2 d) {
 // Forward.  grid (CTAs, 2 directions, channel chunks); a warp computes 16 pixels x the chunk's channels.  The
 // rank is extended to K' = R (bf16) or 6R (fp32, the six products side by side) and padded to 16.  Columns of
 // W are dealt to the fragments so that a lane's results over four n-tiles are 8 neighbouring channels:
-// 16-byte stores.
+// 16-byte stores.  What infinite and very large sums cost, us without / with: fp32 P = 401408, E = 64 80.5 / 81.1, 1048576, 64
+// 180.5 / 185.0, 25088, 320 57.9 / 58.5; bf16 401408, 64 60.5 / 62.4, 25088, 320 42.7 / 43.5 (events around one call, L2 flushed).
+// (The bounds are the CTAs an SM takes; left to itself the compiler spills fp32 into 48 registers for the sake of the call.)
 // ------------------------------------------------------------------------------------------------
 // Memory that a kernel zeroes before anything else, so that the stores drain while its weights and first rows
 // arrive: a memset of its own is a launch.  Worth it for small pieces; the 537 MB of boundary rows of a 1024x1024
@@ -116,6 +152,20 @@ struct MmaFwdArgs {
     void *dT, *dL;
 };
 
+// 16 pixels with ordinary multiply-adds, a lane owns a channel: for fp32 tiles that hold an infinity, a float that rounds
+// to one in bf16, or a sum beyond softplus2<false>'s range.  (The parts of the first two hold differences of infinities; all
+// three show as a NaN.)  Kept out of the kernel's registers and schedule: a branch inside its loop cost up to a tenth of it.
+template <typename io_t>
+__device__ __noinline__ void dtproj_fwd_plain(const io_t* proj, int pitch, int pixels, const void* W, int w0, int params_f32, int R, const float* bias, int ec,
+                                              io_t* out, int E) {
+    for (int ch = threadIdx.x & 31; ch < ec; ch += 32)
+        for (int i = 0; i < pixels; ++i) {
+            float z = bias[ch];
+            for (int r = 0; r < R; ++r) z = fmaf(load1(proj, (long long)i * pitch + r), load_param<io_t>(W, w0 + ch * R + r, params_f32), z);
+            store1(out, (long long)i * E + ch, softplus_f(z));
+        }
+}
+
 template <typename io_t> __host__ __device__ inline int mma_k(int R) { return ((sizeof(io_t) == 4 ? 6 * R : R) + 15) / 16; }
 __host__ __device__ inline size_t mma_fwd_smem(int chunk, int nk) {
     const int nt = chunk / 8;
@@ -123,7 +173,7 @@ __host__ __device__ inline size_t mma_fwd_smem(int chunk, int nk) {
 }
 
 template <typename io_t>
-__global__ void __launch_bounds__(256) dtproj_fwd_mma_kernel(const MmaFwdArgs a) {
+__global__ void __launch_bounds__(256, sizeof(io_t) == 4 ? 3 : 4) dtproj_fwd_mma_kernel(const MmaFwdArgs a) {
     extern __shared__ __align__(16) char smem_mma[];
     const int dir = blockIdx.y, e0 = blockIdx.z * a.chunk, ec = min(a.chunk, a.E - e0);
     const int nt = a.chunk / 8, nk = a.nk, ks = nk * 16, R = a.R;
@@ -181,6 +231,7 @@ __global__ void __launch_bounds__(256) dtproj_fwd_mma_kernel(const MmaFwdArgs a)
         __syncwarp();
         const bool ok0 = p0 + row < a.P, ok1 = p0 + row + 8 < a.P;
         io_t* const o0 = out + (long long)(p0 + row) * a.E, *const o1 = o0 + (long long)8 * a.E;
+        float2 sum = make_float2(0.f, 0.f);
         for (int g = 0; g < nt / 4; ++g) {
             float acc[4][4];
 #pragma unroll
@@ -202,8 +253,8 @@ __global__ void __launch_bounds__(256) dtproj_fwd_mma_kernel(const MmaFwdArgs a)
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
                     const float2 b = *reinterpret_cast<const float2*>(bias + ch + 2 * j);
-                    v0[j] = softplus2(__fadd2_rn(make_float2(acc[j][0], acc[j][1]), b));
-                    v1[j] = softplus2(__fadd2_rn(make_float2(acc[j][2], acc[j][3]), b));
+                    v0[j] = softplus2<!F32>(__fadd2_rn(make_float2(acc[j][0], acc[j][1]), b));
+                    v1[j] = softplus2<!F32>(__fadd2_rn(make_float2(acc[j][2], acc[j][3]), b));
                 }
                 if (F32) {
                     float* f0 = reinterpret_cast<float*>(o0 + ch), *f1 = reinterpret_cast<float*>(o1 + ch);
@@ -216,8 +267,14 @@ __global__ void __launch_bounds__(256) dtproj_fwd_mma_kernel(const MmaFwdArgs a)
                     if (ok0) *reinterpret_cast<uint4*>(o0 + ch) = make_uint4(pack_bf16x2(v0[0].x, v0[0].y), pack_bf16x2(v0[1].x, v0[1].y), pack_bf16x2(v0[2].x, v0[2].y), pack_bf16x2(v0[3].x, v0[3].y));
                     if (ok1) *reinterpret_cast<uint4*>(o1 + ch) = make_uint4(pack_bf16x2(v1[0].x, v1[0].y), pack_bf16x2(v1[1].x, v1[1].y), pack_bf16x2(v1[2].x, v1[2].y), pack_bf16x2(v1[3].x, v1[3].y));
                 }
+                if (F32) {                         // (no result is below zero: a NaN among them is one of the sum)
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) sum = __fadd2_rn(__fadd2_rn(v0[j], v1[j]), sum);
+                }
             }
         }
+        if (F32 && __any_sync(0xffffffffu, isnan(sum.x + sum.y)))
+            dtproj_fwd_plain<io_t>(proj + (long long)p0 * a.pitch, a.pitch, min(16, a.P - p0), W, e0 * R, a.params_f32, R, bias, ec, out + (long long)p0 * a.E, a.E);
     }
 }
 

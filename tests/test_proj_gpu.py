@@ -145,6 +145,27 @@ def test_fused_softplus_is_accurate_over_its_whole_range():
         assert float(rel) < 1e-6
 
 
+@pytest.mark.parametrize("dt", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("P,E,R", [(16, 64, 4), (40, 36, 4), (60000, 64, 4), (9500, 320, 20), (200, 328, 20)])      # either kernel
+def test_softplus_of_the_largest_arguments(P, E, R, dt):
+    """Sums of any size, infinite and undefined ones among them, and a channel whose bias is -inf: 0, the argument itself, or NaN,
+    like torch's softplus."""
+    from mamba2d_b200 import wavefront_cuda as wc
+    inf, nan, most = float("inf"), float("nan"), float(torch.finfo(dt).max)
+    z = [-inf, inf, nan, -most, most, -1e38, 1e38, -3e4, 3e4, -201.0, -199.0, 201.0, -88.0, 88.0, 0.0, 0.5]
+    proj = torch.zeros(1, 1, P, 2 * R + 48 + (-2 * R) % 4)
+    proj[0, 0, -16:, 0] = torch.tensor(z)
+    proj[0, 0, :16, R] = torch.tensor(z)
+    W, b = torch.zeros(E, R), torch.zeros(E)
+    W[:, 0] = 1.0
+    b[5] = -inf
+    proj = proj.to(dt)
+    got = wc._dtproj_fwd(proj.cuda(), *[t.to(dt).cuda() for t in (W, b, W, b)], 16)
+    for out, col in zip(got, (0, R)):
+        want = torch.nn.functional.softplus(proj[0, 0, :, col].double()[:, None] + b).to(dt)
+        assert torch.allclose(out[0, 0].cpu().float(), want.float(), rtol=1e-6 if dt == torch.float32 else 8e-3, atol=1e-37, equal_nan=True)
+
+
 @pytest.mark.parametrize("P,E,R", [(50176, 64, 4), (20000, 128, 8), (9999, 320, 20), (5000, 512, 32), (3000, 576, 36),
                                    (777, 40, 4), (64, 64, 4), (65, 192, 12)])
 def test_xproj_weight_gradient_on_tensor_cores(P, E, R, monkeypatch):
