@@ -252,6 +252,9 @@ inline double wave_steps(const m2d_scan_desc* d, const Plan& p) {
 //   fp32  512x512x192 (18 %) 1002 / 1051, 300x500x192 (25 %) 686 / 709, 3x200x300x96 (26 %) 420 / 435, 2x300x336x96 (33 %) 531 / 513,
 //         250x250x256 (33 %) 432 / 410, 1024x1024x64 (35 %) 1734 / 1626
 // With two channels per lane, whose steps are shorter, pairs are slower (2x200x336x64 bf16 286 / 314).
+// plan_fwd charges plans with pairs the 15 columns all the same: what it charges the two-channel plans is above their time
+// by more.  With 12 columns every 25th shape of the models' range goes from two channels to four and takes 1.14 times as long
+// (geometric mean of 90 of them; 2x306x183x96 fp32 346 / 410 us, 1x310x435x64 bf16 396 / 529, 2x502x452x64 fp32 829 / 777).
 inline bool edge_pairs(const m2d_scan_desc* d, const Plan& p, size_t element) {
     return p.wave == 4 && p.chain > 1 && (p.chain - 1) * 15.0 * 10.0 >= wave_steps(d, p) * (element == 2 ? 1 : 3);
 }
