@@ -204,6 +204,8 @@ int64_t m2d_scan_fwd_status_offset(const m2d_scan_desc *desc);
 int64_t m2d_scan_bwd_status_offset(const m2d_scan_desc *desc);   /* same, for m2d_scan_bwd's workspace */
 int m2d_scan_fwd_chain(const m2d_scan_desc *desc);
 int m2d_scan_bwd_chain(const m2d_scan_desc *desc);
+/* Columns of a boundary row that one CTA of m2d_scan_fwd hands to the next at a time (0: no CTA waits on another). */
+int m2d_scan_fwd_edge_columns(const m2d_scan_desc *desc);
 
 /*
  * 1 if a wait between CTAs has given up in any launch of this process since the last call of this

@@ -25,7 +25,7 @@ NOALLOC_SCRATCH_BYTES = 32 << 20     # M2D_NOALLOC_SCRATCH_BYTES in include/m2d_
 
 EXPORTS = ("m2d_abi_version", "m2d_strerror", "m2d_scan_fwd_workspace", "m2d_scan_bwd_workspace",
            "m2d_scan_fwd", "m2d_scan_bwd", "m2d_scan_fwd_noalloc", "m2d_scan_fwd_noalloc_need", "m2d_scan_fwd_status_offset",
-           "m2d_scan_bwd_status_offset", "m2d_scan_fwd_chain", "m2d_scan_bwd_chain", "m2d_scan_chain_bound", "m2d_take_wait_failure",
+           "m2d_scan_bwd_status_offset", "m2d_scan_fwd_chain", "m2d_scan_bwd_chain", "m2d_scan_fwd_edge_columns", "m2d_scan_chain_bound", "m2d_take_wait_failure",
            "m2d_wait_failure_mark",
            "m2d_proj_workspace", "m2d_dtproj_fwd", "m2d_dtproj_bwd", "m2d_xproj_wgrad",
            "m2d_xproj_wgrad_on_tensor_cores", "m2d_proj_bwd", "m2d_rows_gemm_f32",
@@ -81,7 +81,7 @@ def lib():
         L.m2d_abi_version.restype = ctypes.c_int
         L.m2d_strerror.restype = ctypes.c_char_p
         L.m2d_strerror.argtypes = [ctypes.c_int]
-        for name in ("m2d_scan_fwd_chain", "m2d_scan_bwd_chain"):
+        for name in ("m2d_scan_fwd_chain", "m2d_scan_bwd_chain", "m2d_scan_fwd_edge_columns"):
             getattr(L, name).restype = ctypes.c_int
             getattr(L, name).argtypes = [ctypes.POINTER(ScanDesc)]
         L.m2d_scan_chain_bound.restype = ctypes.c_int

@@ -97,6 +97,12 @@ extern "C" int m2d_scan_fwd_chain(const m2d_scan_desc* d) {
     return m2d::plan_fwd(d).chain;
 }
 
+extern "C" int m2d_scan_fwd_edge_columns(const m2d_scan_desc* d) {
+    if (m2d::check_desc(d, false, false) != M2D_OK) return 0;
+    const m2d::Plan p = m2d::plan_fwd(d);
+    return p.chain < 2 ? 0 : m2d::edge_pairs(d, p, d->dtype == M2D_F32 ? sizeof(float) : sizeof(__nv_bfloat16)) ? 2 : m2d::kChunk;
+}
+
 extern "C" int m2d_scan_chain_bound(int want, int nbands, int steps_per_row, int rows_per_band) {
     if (nbands < 1 || steps_per_row < 1 || rows_per_band < 1) return 0;
     return m2d::bound_chain(want, nbands, steps_per_row, rows_per_band);
