@@ -171,9 +171,11 @@ void gemm(const Tensor& like, int64_t rows, int64_t n, int64_t k, const void* a,
     //     6272    19 / 15   20 / 19   23 / 23   28 / 29  30 / 31  38 / 46   18 / 17   19 / 18   21 / 23   29 / 28  29 / 29  38 / 39
     //     12544   19 / 17   23 / 21   29 / 27   43 / 40  39 / 40  55 / 68   20 / 19   22 / 23   28 / 27   41 / 39  44 / 38  58 / 51
     //     25088   23 / 20   29 / 26   41 / 37   55 / 59  61 / 57  92 / 91   22 / 24   31 / 29   46 / 35   63 / 56  70 / 57  97 / 81
-    //     100352  46 / 29   58 / 49  114 / 78                              46 / 38   69 / 56  127 / 81
-    // The first product follows its columns (E up to 192).  The second is the library's between 2048 and 12000 rows, where
-    // neither gains; below that the own kernel's error, a third of the library's, keeps what it has.
+    //     37632                                 74 / 63  80 / 71  98 / 109
+    //     100352  46 / 29   58 / 49  114 / 78  165 / 137 187 / 160 278 / 294      46 / 38   69 / 56  127 / 81  215 / 144 262 / 160 367 / 233
+    // The first product follows its columns: up to 72 (E = 192) always, up to 96 (E = 384) where there are enough rows.  The
+    // second is the library's between 2048 and 12000 rows, where neither gains; below that the own kernel's error, a third of
+    // the library's, keeps what it has.
     //
     // A caller that allows TF32 products gets them where the library's are faster then, by rows (TF32 / own, us, E = 64, 192, 512):
     //              x @ Wx^T                          d_x += d_proj @ Wx
@@ -183,7 +185,7 @@ void gemm(const Tensor& like, int64_t rows, int64_t n, int64_t k, const void* a,
     //     100352   31 / 30   37 / 79   64 / 294      42 / 37   55 / 80   91 / 233
     //     401408   53 / 68                           94 / 89
     const bool tf32 = at::globalContext().float32Precision(at::Float32Backend::CUDA, at::Float32Op::MATMUL) == at::Float32Precision::TF32;
-    const bool own = tf32 ? rows <= 1024 || (accumulate && n <= 64) : n <= 72 || rows <= 2048 || (accumulate && rows >= 12000);
+    const bool own = tf32 ? rows <= 1024 || (accumulate && n <= 64) : n <= 72 || rows <= 2048 || (n <= 96 && rows >= 30000) || (accumulate && rows >= 12000);
     if (like.scalar_type() == at::kFloat && own) {
         const int rc = m2d_rows_gemm_f32(rows, (int)n, (int)k, static_cast<const float*>(a), static_cast<const float*>(w), transposed, accumulate,
                                          static_cast<float*>(out), stream_of(like));

@@ -34,6 +34,12 @@ def test_rows_gemm_adds_to_wide_rows(rows, n, k):
     test_rows_gemm(rows, n, k, 0, 1)
 
 
+@pytest.mark.parametrize("rows,n,k", [(30000, 76, 224), (30011, 88, 320), (40001, 96, 384)])
+def test_rows_gemm_of_many_rows_and_more_columns(rows, n, k):
+    """The x projection at the column and row counts around its line to the GEMM library."""
+    test_rows_gemm(rows, n, k, 1, 0)
+
+
 @pytest.mark.parametrize("transposed,accumulate", [(1, 0), (0, 1)])
 @pytest.mark.parametrize("rows,n,k", [(40, 60, 68), (5000, 12, 20), (20011, 64, 56), (12017, 112, 64)])
 def test_rows_gemm_of_values_that_bf16_parts_cannot_hold(rows, n, k, transposed, accumulate):
