@@ -184,9 +184,13 @@ void gemm(const Tensor& like, int64_t rows, int64_t n, int64_t k, const void* a,
     //     12544    16 / 17   22 / 27   26 / 68       17 / 19   25 / 27   31 / 51
     //     100352   31 / 30   37 / 79   64 / 294      42 / 37   55 / 80   91 / 233
     //     401408   53 / 68                           94 / 89
-    const bool tf32 = at::globalContext().float32Precision(at::Float32Backend::CUDA, at::Float32Op::MATMUL) == at::Float32Precision::TF32;
-    const bool own = tf32 ? rows <= 1024 || (accumulate && n <= 64) : n <= 72 || rows <= 2048 || (n <= 96 && rows >= 30000) || (accumulate && rows >= 12000);
-    if (like.scalar_type() == at::kFloat && own) {
+    auto own = [&] {
+        if (like.scalar_type() != at::kFloat) return false;
+        if (rows <= 1024) return true;
+        const bool tf32 = at::globalContext().float32Precision(at::Float32Backend::CUDA, at::Float32Op::MATMUL) == at::Float32Precision::TF32;
+        return tf32 ? accumulate && n <= 64 : n <= 72 || rows <= 2048 || (n <= 96 && rows >= 30000) || (accumulate && rows >= 12000);
+    };
+    if (own()) {
         const int rc = m2d_rows_gemm_f32(rows, (int)n, (int)k, static_cast<const float*>(a), static_cast<const float*>(w), transposed, accumulate,
                                          static_cast<float*>(out), stream_of(like));
         if (rc == M2D_OK) return;
