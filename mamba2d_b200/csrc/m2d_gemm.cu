@@ -3,7 +3,7 @@
 //
 // The GEMM library runs fp32 at full precision on the CUDA cores, in tiles of 64 or 128 columns where these
 // products have 56 ... 156: 102 and 132 us at P = 401408, E = 64 (262 us at P = 1048576) for operands that
-// stream in 30 and 46 us (78 us), and 7.7 us for the 196 rows of one 14x14 image; 55 and 75 (137), and 3.0 here.  (A
+// stream in 30 and 46 us (78 us), and 7.7 us for the 196 rows of one 14x14 image; 55 and 74 (132), and 3.3 here.  (A
 // kernel's own times, in a graph; events around one call with the L2 flushed show 5 us more.)
 //
 // Here a float is split into three bf16 parts, exact to 24 bits, and a product of floats is the six products of
@@ -199,7 +199,8 @@ __global__ void __launch_bounds__(256, NT == 2 ? 3 : 2) rows_gemm_kernel(const G
             }
         }
         // What is there already: all of it on its way before the first sum is waited for and stored (one by one, each
-        // behind the store before it, was 16 trips to memory in a row).
+        // behind the store before it, 103 us against 75 at P = 401408, E = 64, of 16 cycles per issue 9 waiting for
+        // global memory; 2 now).
         float2 old[NT][2];
 #pragma unroll
         for (int n = 0; n < NT; ++n)

@@ -453,7 +453,7 @@ __global__ void __launch_bounds__(256) xproj_wgrad_kernel(const WgArgs a) {     
 
 // The same for fp32: a CTA of 128 threads, the even pixels of a stage for the first two warps, the odd ones for the
 // others, each thread an 8x8 block, the stages filled by asynchronous copies.  Bound by the loads from shared memory at a 4x4
-// block (two for 16 multiply-adds, that pipe 82 % busy, 93 us at P = 401408, E = 64); with four for 64, and no registers
+// block (two for 16 multiply-adds, that pipe 83 % busy, 93 us at P = 401408, E = 64); with four for 64, and no registers
 // for the next stage, 72 us (27 -> 22.6 at 6272 x 512).  (On the CUDA cores: TF32 would not hold the tolerance.)
 constexpr int kWgThreads = 128;
 
