@@ -129,8 +129,9 @@ __device__ __forceinline__ float2 softplus_grad2(float2 d) {
 // Forward.  grid (CTAs, 2 directions, channel chunks); a warp computes 16 pixels x the chunk's channels.  The
 // rank is extended to K' = R (bf16) or 6R (fp32, the six products side by side) and padded to 16.  Columns of
 // W are dealt to the fragments so that a lane's results over four n-tiles are 8 neighbouring channels:
-// 16-byte stores.  What infinite and very large sums cost, us without / with: fp32 P = 401408, E = 64 80.5 / 81.1, 1048576, 64
-// 180.5 / 185.0, 25088, 320 57.9 / 58.5; bf16 401408, 64 60.5 / 62.4, 25088, 320 42.7 / 43.5 (events around one call, L2 flushed).
+// 16-byte stores.  What infinite and very large sums cost, us without / with: fp32 P = 401408, E = 64 80.5 / 80.7, 1048576, 64
+// 180.4 / 181.3, 25088, 320 57.1 / 58.0; bf16 401408, 64 60.2 / 61.7, 25088, 320 42.5 / 43.2 (events around one call, L2 flushed);
+// fp32 rows that are all NaN take up to three times as long.
 // (The bounds are the CTAs an SM takes; left to itself the compiler spills fp32 into 48 registers for the sake of the call.)
 // ------------------------------------------------------------------------------------------------
 // Memory that a kernel zeroes before anything else, so that the stores drain while its weights and first rows
@@ -156,12 +157,12 @@ struct MmaFwdArgs {
 // to one in bf16, or a sum beyond softplus2<false>'s range.  (The parts of the first two hold differences of infinities; all
 // three show as a NaN.)  Kept out of the kernel's registers and schedule: a branch inside its loop cost up to a tenth of it.
 template <typename io_t>
-__device__ __noinline__ void dtproj_fwd_plain(const io_t* proj, int pitch, int pixels, const void* W, int w0, int params_f32, int R, const float* bias, int ec,
+__device__ __noinline__ void dtproj_fwd_plain(const io_t* proj, int pitch, int pixels, const void* W, const void* bias, int e0, int params_f32, int R, int ec,
                                               io_t* out, int E) {
     for (int ch = threadIdx.x & 31; ch < ec; ch += 32)
         for (int i = 0; i < pixels; ++i) {
-            float z = bias[ch];
-            for (int r = 0; r < R; ++r) z = fmaf(load1(proj, (long long)i * pitch + r), load_param<io_t>(W, w0 + ch * R + r, params_f32), z);
+            float z = load_param<io_t>(bias, e0 + ch, params_f32);
+            for (int r = 0; r < R && !isnan(z); ++r) z = fmaf(load1(proj, (long long)i * pitch + r), load_param<io_t>(W, (e0 + ch) * R + r, params_f32), z);
             store1(out, (long long)i * E + ch, softplus_f(z));
         }
 }
@@ -207,7 +208,8 @@ __global__ void __launch_bounds__(256, sizeof(io_t) == 4 ? 3 : 4) dtproj_fwd_mma
             put(r, __float2bfloat16_rn(v));
         }
     }
-    for (int k = threadIdx.x; k < nt * 8; k += blockDim.x) bias[k] = e0 + k < a.E ? load_param<io_t>(bp, e0 + k, a.params_f32) : 0.f;
+    // (a bias of -inf is as good as -1e38: it must not send every tile the slow way)
+    for (int k = threadIdx.x; k < nt * 8; k += blockDim.x) bias[k] = e0 + k < a.E ? max_nan(load_param<io_t>(bp, e0 + k, a.params_f32), F32 ? -1e38f : -INFINITY) : 0.f;
     for (int k = lane; k < 16 * lda; k += 32) At[k] = __nv_bfloat16(0.f);
     __syncthreads();
 
@@ -274,7 +276,7 @@ __global__ void __launch_bounds__(256, sizeof(io_t) == 4 ? 3 : 4) dtproj_fwd_mma
             }
         }
         if (F32 && __any_sync(0xffffffffu, isnan(sum.x + sum.y)))
-            dtproj_fwd_plain<io_t>(proj + (long long)p0 * a.pitch, a.pitch, min(16, a.P - p0), W, e0 * R, a.params_f32, R, bias, ec, out + (long long)p0 * a.E, a.E);
+            dtproj_fwd_plain<io_t>(proj + (long long)p0 * a.pitch, a.pitch, min(16, a.P - p0), W, bp, e0, a.params_f32, R, ec, out + (long long)p0 * a.E, a.E);
     }
 }
 
