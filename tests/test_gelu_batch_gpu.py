@@ -21,3 +21,16 @@ def test_gelu_one_step_late(B, H, W, E, reverse):
     got = scan_fwd(*args, reverse=reverse, gelu_out=True).double()
     want = 0.5 * y * (1.0 + torch.erf(y * 0.5 ** 0.5))
     assert float(((got - want).abs() - 2e-7 * y.abs()).max()) < 4.5e-7
+
+
+@pytest.mark.parametrize("B,H,W,E", [(300, 2, 3, 32), (301, 9, 7, 40), (149, 23, 12, 64)])
+def test_gelu_one_step_late_bf16(B, H, W, E):
+    """The y to compare with is rounded to bf16, whose 8 bits leave 2^-8 of a value (times GELU's slope of 1.13 at most), and so is
+    the result, which is no larger than y."""
+    from mamba2d_b200 import scan_fwd
+    d = to_dev(inputs.make_inputs(B, H, W, E, 16, seed=B + W), torch.bfloat16)
+    args = [d[k] for k in ORDER]
+    y = scan_fwd(*args).double()
+    got = scan_fwd(*args, gelu_out=True).double()
+    want = 0.5 * y * (1.0 + torch.erf(y * 0.5 ** 0.5))
+    assert float(((got - want).abs() - 2.14 * 2.0 ** -8 * y.abs()).max()) < 4.5e-7
