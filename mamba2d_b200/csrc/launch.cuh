@@ -56,7 +56,7 @@ inline int launch_sweep_kernel(void (*kern)(const ScanArgs), ScanArgs& a, const 
             a.chain = bound_chain(a.chain > 2 ? a.chain - a.chain / 4 - 1 : 1, pl.nbands, a.W, pl.Rb);
         }
     }
-    dim3 grid(pl.grid_x, pl.groups);
+    const dim3 grid = pl.wave ? dim3(pl.grid_x, pl.groups) : dim3(pl.groups, pl.grid_x);
     kern<<<grid, block, pl.smem, st>>>(a);
     return cudaGetLastError() == cudaSuccess ? M2D_OK : M2D_ERR_LAUNCH;
 }

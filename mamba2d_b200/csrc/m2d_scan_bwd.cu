@@ -3,17 +3,8 @@
 #include <algorithm>
 
 #include "launch.cuh"
-#include "sweep_rows.cuh"
+#include "sweep_pairs.cuh"
 #include "wave_bwd.cuh"
-
-// Row-warps per CTA of the backward kernel (two CTAs per SM): the register budget per thread follows
-// from it (6 warps: 168 registers).
-#ifndef M2D_BWD_MAXW
-#define M2D_BWD_MAXW 6
-#endif
-#ifndef M2D_BWD_MINB
-#define M2D_BWD_MINB 2
-#endif
 
 namespace m2d {
 
@@ -22,15 +13,41 @@ namespace m2d {
 //   acc      bf16 I/O only: fp32 accumulators 3 x [B*H*W][N] | 2 x [E][N] | [E], zeroed before the
 //            main kernel (with the status word, in one memset) and cast by a second kernel.  With fp32 I/O
 //            the kernel accumulates straight into the caller's (zeroed) gradient tensors and this region is empty.
-//   edge     batch: per-CTA band-boundary ring, ctas*W*2 KiB (only if nbands > 1); wave: the boundary rows
+//   edge     batch: per-CTA band-boundary ring, ctas*W KiB (only if nbands > 1); wave: the boundary rows
 //            of the recompute sweep (h, downwards) and of the adjoint sweep (pT, upwards)
-//   hs       state record written by the recompute sweep: batch B*groups*H*W*2 KiB (1 KiB with bf16 I/O), wave
+//   hs       state record written by the recompute sweep: batch B*groups*H*W KiB (half with bf16 I/O), wave
 //            512*C bytes per (list, warp, band, step)
 struct BwdLayout {
     size_t edge, hs, acc, acc_bytes, total;
 };
 
-inline BwdLayout bwd_layout(const m2d_scan_desc* d, const Plan& p) {
+// The plans of a backward: `states` (batch mode) is the recompute sweep's, `wide` an fp32 state record.
+struct BwdPlan : Plan {
+    Plan states;
+    bool wide;
+};
+
+// With bf16 I/O the batch kernels keep the states of a large batch in bf16, which halves the traffic that the recompute sweep
+// waits for, and those of a few images in fp32, as the wave kernels do: the record is small then, and the gradients are
+// those of the unrounded states.  Few: where a wave launch takes less time than one CTA per image and 32 channels, with up to
+// six rows in flight each and twelve on an SM.
+inline bool few_images(const m2d_scan_desc* d) {
+    const int sms = sm_count(), g = (d->E - 1) / 32 + 1;
+    double best = -1.0, time = 0.0;
+    for (int w = 6; w >= 2; --w) {
+        int Rb = std::min(w, (int)d->H);
+        if (Rb < d->H && Rb > d->W - 2) Rb = std::max(1, (int)d->W - 2);
+        const int bands = (d->H - 1) / Rb + 1, lists = std::max(1, 12 / Rb * sms / g), per = (d->B - 1) / lists + 1;
+        const double ctas = (double)((d->B - 1) / per + 1) * g, score = std::min(ctas * Rb, 12.0 * sms) * d->H / ((double)bands * Rb);
+        if (score > best * 1.02) {
+            best = score;
+            time = (ctas > sms ? 2.45 : 1.95) * ((double)per * bands * d->W + Rb);
+        }
+    }
+    return 1.2 * wave_steps(d, plan_wave(d, 2)) + 10.0 < time;
+}
+
+inline BwdLayout bwd_layout(const m2d_scan_desc* d, const BwdPlan& p) {
     BwdLayout L;
     size_t off = kStatusBytes;
     L.acc = off;
@@ -42,27 +59,28 @@ inline BwdLayout bwd_layout(const m2d_scan_desc* d, const Plan& p) {
     off += L.acc_bytes;
     L.edge = off;
     if (p.wave) off += 2 * wave_edge_bytes(d, p, true);
-    else if (p.nbands > 1) off += align256((size_t)p.grid_x * p.groups * d->W * kSlotF4 * sizeof(float4));
+    else off += align256(std::max(pair_ring_bytes(d, p), pair_ring_bytes(d, p.states)));
     L.hs = off;
     if (p.wave) off += align256((size_t)p.grid_x * p.groups * p.warps * p.nbands * (d->W + 7) * p.wave * 512);
-    else off += align256((size_t)d->B * p.groups * d->H * d->W * (d->dtype == M2D_F32 ? 128 : 64) * sizeof(float4));
+    else off += align256((size_t)d->B * p.groups * d->H * d->W * (p.wide ? 64 : 32) * sizeof(float4));
     L.total = off;
     return L;
 }
 
-inline Plan plan_bwd(const m2d_scan_desc* d) {
-    // Batch or wave, as in plan_fwd.  Measured times per step of both sweeps together, whatever the I/O type: 2.45 us in
-    // batch mode with two CTAs per SM, 1.95 us with one, 1.2 us in the wave kernel with two channels per lane (four
-    // spill and are slower at every size measured).  56x56x64: wave up to batch 32, 581 against 738 us.
-    Plan p{};
+inline BwdPlan plan_bwd(const m2d_scan_desc* d) {
+    // Batch or wave, as in plan_fwd: 1.2 us per step of both sweeps in the wave kernel with two channels per lane (four
+    // spill and are slower at every size measured), whatever the I/O type.
+    BwdPlan p{};
     double best = 1e30;
     if (d->W >= 3) {
-        p = plan_best(d, M2D_BWD_MAXW, 2 * M2D_BWD_MAXW);
-        p.smem = rows_bwd_smem_bytes(p.warps) + kParamF4 * sizeof(float4);
-        best = ((long long)p.grid_x * p.groups > sm_count() ? 2.45 : 1.95) * batch_steps(d, p);
+        double states = 0.0;
+        static_cast<Plan&>(p) = plan_pairs(d, kPairAdjoint, &best);
+        p.states = plan_pairs(d, kPairStates, &states);
+        p.wide = d->dtype == M2D_F32 || few_images(d);
+        best = (best + states) * kWaveMargin;
     }
     const Plan w = plan_wave(d, 2);
-    if (1.2 * wave_steps(d, w) + 10.0 < best) p = w;
+    if (1.2 * wave_steps(d, w) + 10.0 < best) static_cast<Plan&>(p) = w;
     p.scratch = bwd_layout(d, p).total;
     return p;
 }
@@ -74,87 +92,64 @@ __global__ void __launch_bounds__(256, 1) m2d_bwd_wave_kernel(const ScanArgs a) 
     wave_backward<io_t, 2, VEC>(a, reinterpret_cast<char*>(smem));
 }
 
-// Batch mode (one CTA per image and channel group): both sweeps written as nested loops.
-template <typename io_t, bool VEC>
-__global__ void __launch_bounds__(M2D_BWD_MAXW * 32, M2D_BWD_MINB) m2d_bwd_kernel(const ScanArgs a) {
+// Batch mode (one CTA per image and channel group): the recompute sweep, which writes the state record and d_C, and the
+// adjoint sweep, each a kernel of its own: their registers, shared memory and bands need not be the same.
+template <typename io_t, typename rec_t, bool VEC>
+__global__ void __launch_bounds__(kPairWarps * 32, 2) m2d_bwd_states_kernel(const ScanArgs a) {
     extern __shared__ float4 smem[];
-    const int lane = threadIdx.x & 31, r = threadIdx.x >> 5;
-    const int nwarps = blockDim.x >> 5;
-    const int cq = lane >> 2, nq = lane & 3;
-    const int g = blockIdx.y;
-    const int ch0 = g * kGroup + cq * 4, n0 = nq * 4;
-    const int chv = min(4, max(0, a.E - ch0));
-    const int nv = min(4, max(0, a.N - n0));
+    const PairLane ln(a);
+    const unsigned params = begin_pairs<io_t>(a, smem, pairs_fwd_smem_bytes(ln.nwarps), ln);
+    forward_pairs<io_t, rec_t, VEC, true, false>(a, smem_u32(smem), params, 0.f, blockIdx.y, gridDim.y, images_of_cta(a));
+}
 
-    const int total = (int)(rows_bwd_smem_bytes(nwarps) / sizeof(float4));
-    for (int k = threadIdx.x; k < total; k += blockDim.x) smem[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+template <typename io_t, typename rec_t, bool VEC>
+__global__ void __launch_bounds__(kPairWarps * 32, 2) m2d_bwd_kernel(const ScanArgs a) {
+    extern __shared__ float4 smem[];
+    const PairLane ln(a);
+    const unsigned params = begin_pairs<io_t>(a, smem, pairs_bwd_smem_bytes(ln.nwarps), ln);
+    const int o_ch = ln.ch0 + (ln.nq & 1);
+    const float D_lane = o_ch < a.E ? load_D<io_t>(a, o_ch) : 0.f;
+    Quad dAT[2], dAL[2];
+    clear(dAT);
+    clear(dAL);
+    float dD = 0.f;
+    reverse_pairs<io_t, rec_t, VEC>(a, smem_u32(smem), params, D_lane, dAT, dAL, dD, blockIdx.y, gridDim.y, images_of_cta(a));
 
-    const int ch_own = g * kGroup + lane;
-    const float D_own = ch_own < a.E ? load_D<io_t>(a, ch_own) : 0.f;
-    float dAT[4][4], dAL[4][4], dD[4];
+    // ---- per-(channel, state) sums: fold the CTA's warps through shared memory, then one atomic per value from warp 0
+    constexpr int kSums = 17;
+    float s[kSums];
 #pragma unroll
-    for (int c = 0; c < 4; ++c) {
-        dD[c] = 0.f;
+    for (int c = 0; c < 2; ++c)
 #pragma unroll
-        for (int n = 0; n < 4; ++n) dAT[c][n] = dAL[c][n] = 0.f;
-    }
+        for (int k = 0; k < 2; ++k) {
+            s[c * 4 + k * 2] = dAT[c][k].x; s[c * 4 + k * 2 + 1] = dAT[c][k].y;
+            s[8 + c * 4 + k * 2] = dAL[c][k].x; s[8 + c * 4 + k * 2 + 1] = dAL[c][k].y;
+        }
+    s[16] = dD;
+    float* const red = reinterpret_cast<float*>(smem);     // (2.2 KB per warp, of 12 that it has)
     __syncthreads();
-    float4* const params = reinterpret_cast<float4*>(reinterpret_cast<char*>(smem) + rows_bwd_smem_bytes(nwarps));
-    if (threadIdx.x < 32) stage_params<io_t>(params, a.AT, a.AL, a.N, ch0, chv, n0, nv, lane, a.a_log);
+#pragma unroll
+    for (int k = 0; k < kSums; ++k) red[threadIdx.x * kSums + k] = s[k];
     __syncthreads();
-
-    for (int b = (int)blockIdx.x; b < a.B; b += (int)gridDim.x) {
-        forward_rows<io_t, VEC, true, false>(a, smem, params, D_own, b, 0, 1);
-        reverse_rows<io_t, VEC>(a, smem, params, D_own, dAT, dAL, dD, b);
-    }
-
-    // ---- per-(channel,state) sums: fold the CTA's row-warps through shared memory, then one
-    //      atomic per value from warp 0 ----------------------------------------------------------
-    float* red = reinterpret_cast<float*>(smem);        // reuse: needs 36 floats per thread
-    const int slot = (int)rows_handoff_f4(nwarps) * 4;   // floats available
-    const bool fits = (int)blockDim.x * 36 <= slot;
-    if (fits && nwarps > 1) {
-        float* mine = red + (size_t)threadIdx.x * 36;
+    if (ln.r != 0) return;
+    for (int w = 1; w < ln.nwarps; ++w)
 #pragma unroll
-        for (int c = 0; c < 4; ++c) {
+        for (int k = 0; k < kSums; ++k) s[k] += red[(w * 32 + ln.lane) * kSums + k];
 #pragma unroll
-            for (int n = 0; n < 4; ++n) { mine[c * 4 + n] = dAT[c][n]; mine[16 + c * 4 + n] = dAL[c][n]; }
-            mine[32 + c] = dD[c];
-        }
-        __syncthreads();
-        if (r == 0) {
-            for (int w = 1; w < nwarps; ++w) {
-                const float* o = red + (size_t)(w * 32 + lane) * 36;
+    for (int c = 0; c < 2; ++c)
 #pragma unroll
-                for (int c = 0; c < 4; ++c) {
-#pragma unroll
-                    for (int n = 0; n < 4; ++n) { dAT[c][n] += o[c * 4 + n]; dAL[c][n] += o[16 + c * 4 + n]; }
-                    dD[c] += o[32 + c];
-                }
+        for (int n = 0; n < 4; ++n)
+            if (c < ln.chv && n < ln.nv) {
+                const long long idx = (long long)(ln.ch0 + c) * a.N + ln.n0 + n;
+                // with A given as A_log the gradient asked for is d_A_log = d_A * A (A = -exp(A_log),
+                // models/kernels/wavefront_cuda.py:72-73); the product is linear, so every CTA
+                // scales its own partial sum
+                const float sT = a.a_log ? load_A<io_t>(a.AT, idx, 1, true) : 1.f;
+                const float sL = a.a_log ? load_A<io_t>(a.AL, idx, 1, true) : 1.f;
+                atomicAdd(a.accAT + idx, s[c * 4 + n] * sT);
+                atomicAdd(a.accAL + idx, s[8 + c * 4 + n] * sL);
             }
-        }
-    }
-    if (r == 0 || !(fits && nwarps > 1)) {
-#pragma unroll
-        for (int c = 0; c < 4; ++c) {
-            if (c < chv) {
-#pragma unroll
-                for (int n = 0; n < 4; ++n) {
-                    if (n < nv) {
-                        const long long idx = (long long)(ch0 + c) * a.N + n0 + n;
-                        // with A given as A_log the gradient asked for is d_A_log = d_A * A (A = -exp(A_log),
-                        // models/kernels/wavefront_cuda.py:72-73); the product is linear, so every CTA
-                        // scales its own partial sum
-                        const float sT = a.a_log ? load_A<io_t>(a.AT, idx, 1, true) : 1.f;
-                        const float sL = a.a_log ? load_A<io_t>(a.AL, idx, 1, true) : 1.f;
-                        atomicAdd(a.accAT + idx, dAT[c][n] * sT);
-                        atomicAdd(a.accAL + idx, dAL[c][n] * sL);
-                    }
-                }
-                if (nq == 0) atomicAdd(a.accD + ch0 + c, dD[c]);
-            }
-        }
-    }
+    if (o_ch < a.E) atomicAdd(a.accD + o_ch, s[16]);      // (two lanes each: one for each row)
 }
 
 // bf16 I/O: cast the fp32 accumulators into the caller's gradient tensors (d_AT / d_AL stay fp32 when
@@ -212,8 +207,15 @@ static bool zero_columns(const ScanArgs& a, const m2d_scan_desc* d, cudaStream_t
            cudaMemset2DAsync(a.accC, pitch, 0, width, rows, st) == cudaSuccess;
 }
 
+typedef void (*SweepKernel)(const ScanArgs);
+
 template <typename io_t>
-static int launch_bwd(const m2d_scan_desc* d, const Plan& pl, bool vec, cudaStream_t st) {
+static int launch_bwd(const m2d_scan_desc* d, const BwdPlan& pl, bool vec, cudaStream_t st) {
+    // (a kernel by the type of its record and its kind of loads)
+    auto pick = [](bool vec, bool wide, auto kernel) -> SweepKernel {
+        if (wide || sizeof(io_t) == 4) return vec ? kernel(float{}, std::true_type{}) : kernel(float{}, std::false_type{});
+        return vec ? kernel(io_t{}, std::true_type{}) : kernel(io_t{}, std::false_type{});
+    };
     const BwdLayout L = bwd_layout(d, pl);
     char* ws = static_cast<char*>(d->workspace);
     ScanArgs a;
@@ -266,8 +268,18 @@ static int launch_bwd(const m2d_scan_desc* d, const Plan& pl, bool vec, cudaStre
         a.acc_vec = d->N % 4 == 0 && a.acc_pitch % 4 == 0 && aligned(a.accBT, 16) && aligned(a.accBL, 16) && aligned(a.accC, 16);
         p.smem = WaveSmem<io_t, 2, true>::kBytes;
     }
+    if (!pl.wave) {
+        a.Rb = pl.states.Rb;
+        a.nbands = pl.states.nbands;
+        const int rc = launch_sweep_kernel(pick(vec, pl.wide, [](auto rec, auto v) { return m2d_bwd_states_kernel<io_t, decltype(rec), decltype(v)::value>; }),
+                                           a, pl.states, st);
+        if (rc != M2D_OK) return rc;
+        a.Rb = pl.Rb;
+        a.nbands = pl.nbands;
+    }
     const int rc = launch_sweep_kernel(pl.wave ? (vec ? m2d_bwd_wave_kernel<io_t, true> : m2d_bwd_wave_kernel<io_t, false>)
-                                               : (vec ? m2d_bwd_kernel<io_t, true> : m2d_bwd_kernel<io_t, false>), a, p, st);
+                                               : pick(vec, pl.wide, [](auto rec, auto v) { return m2d_bwd_kernel<io_t, decltype(rec), decltype(v)::value>; }),
+                                       a, p, st);
     if (rc != M2D_OK) return rc;
     if constexpr (sizeof(io_t) == 2) {
         const int pitch = d->d_BC_pitch ? (int)d->d_BC_pitch : d->N;
@@ -305,7 +317,7 @@ extern "C" int m2d_scan_bwd_chain(const m2d_scan_desc* d) {
 extern "C" int m2d_scan_bwd(const m2d_scan_desc* d, void* stream) {
     int rc = m2d::check_desc(d, true, true);
     if (rc != M2D_OK) return rc;
-    const m2d::Plan pl = m2d::plan_bwd(d);
+    const m2d::BwdPlan pl = m2d::plan_bwd(d);
     if (!d->workspace || d->workspace_bytes < pl.scratch || (reinterpret_cast<uintptr_t>(d->workspace) & 255))
         return M2D_ERR_WORKSPACE;
     const bool vec = m2d::vector_ok(d, true);

@@ -1,6 +1,6 @@
 // Forward entry point of the wavefront scan: one fused kernel, y written directly.
 #include "launch.cuh"
-#include "sweep_rows.cuh"
+#include "sweep_pairs.cuh"
 #include "wave_fwd.cuh"
 
 namespace m2d {
@@ -14,25 +14,12 @@ __global__ void __launch_bounds__(256, 1) m2d_fwd_wave_kernel(const ScanArgs a) 
 
 // Batch mode (one CTA per image and channel group): the sweep written as nested loops.
 template <typename io_t, bool VEC, bool ACT>
-__global__ void __launch_bounds__(256, 2) m2d_fwd_kernel(const ScanArgs a) {
+__global__ void __launch_bounds__(kPairWarps * 32, 2) m2d_fwd_kernel(const ScanArgs a) {
     extern __shared__ float4 smem[];
-    const int lane = threadIdx.x & 31;
-    const int nwarps = blockDim.x >> 5;
-    const int cq = lane >> 2, nq = lane & 3;
-    const int g = blockIdx.y;
-    const int ch0 = g * kGroup + cq * 4, n0 = nq * 4;
-    const int chv = min(4, max(0, a.E - ch0));
-    const int nv = min(4, max(0, a.N - n0));
-    const int total = (int)(rows_fwd_smem_bytes(nwarps) / sizeof(float4));
-    for (int k = threadIdx.x; k < total; k += blockDim.x) smem[k] = make_float4(0.f, 0.f, 0.f, 0.f);
-    const int ch_own = g * kGroup + lane;
-    const float D_own = ch_own < a.E ? load_D<io_t>(a, ch_own) : 0.f;
-    __syncthreads();
-    float4* const params = reinterpret_cast<float4*>(reinterpret_cast<char*>(smem) + rows_fwd_smem_bytes(nwarps));
-    if (threadIdx.x < 32) stage_params<io_t>(params, a.AT, a.AL, a.N, ch0, chv, n0, nv, lane, a.a_log);
-    __syncthreads();
-    const int nb = (a.B - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x;
-    forward_rows<io_t, VEC, false, ACT>(a, smem, params, D_own, blockIdx.x, gridDim.x, nb);
+    const PairLane ln(a);
+    const unsigned params = begin_pairs<io_t>(a, smem, pairs_fwd_smem_bytes(ln.nwarps), ln);
+    const int y_ch = ln.ch0 + (ln.nq & 1);
+    forward_pairs<io_t, float, VEC, false, ACT>(a, smem_u32(smem), params, y_ch < a.E ? load_D<io_t>(a, y_ch) : 0.f, blockIdx.y, gridDim.y, images_of_cta(a));
 }
 
 // The status word and, where CTAs of a wave launch read each other's, the boundary rows behind it.

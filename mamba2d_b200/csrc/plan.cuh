@@ -119,68 +119,57 @@ inline bool vector_ok(const m2d_scan_desc* d, bool bwd) {
     return ok;
 }
 
-// Row-warps per CTA: as many as allowed, traded against rows lost to padding in the last band
-// (score = warps x fraction of useful rows; ties go to the better fraction).
-inline int pick_warps(int H, int max_warps) {
-    if (H <= max_warps) return H;
-    int best = max_warps;
-    double best_score = -1.0, best_eff = 0.0;
-    for (int w = max_warps; w >= 2; --w) {
-        const int bands = (H + w - 1) / w;
-        const double eff = (double)H / ((double)bands * w);
-        const double score = w * eff;
-        if (score > best_score + 1e-9 || (score > best_score - 1e-9 && eff > best_eff)) {
-            best_score = score; best_eff = eff; best = w;
-        }
-    }
-    return best;
-}
+// Batch mode: one CTA per (image, 16 channels), images chained per CTA; a warp owns two rows of a band.
+constexpr int kPairWarps = 8;            // warps per CTA, at most (128 registers: 16 per SM)
+enum PairKernel { kPairForward, kPairStates, kPairAdjoint };
 
-// Batch mode: one CTA per (image, 32-channel group), images chained per CTA.
-inline Plan plan_common(const m2d_scan_desc* d, int max_warps, int warps_per_sm) {
-    Plan p{};
-    p.groups = (d->E + kGroup - 1) / kGroup;
-    p.warps = pick_warps(d->H, max_warps);
-    p.Rb = p.warps;
-    p.nbands = (d->H + p.Rb - 1) / p.Rb;
-    if (p.nbands > 1 && p.Rb > d->W - 2) {
+// Time of a batch launch, us, as the plans compare it: the steps of the busiest CTA, times a time per step that grows with
+// the warps of the busiest SM that have a row and with the share of the steps in which some warp of a CTA starts a row (and,
+// where the record is written, with the CTAs), and something per band.  Least squares over 34 shapes of the models' range
+// (1 ... 128 images, 5 ... 2400 rows) x 1 ... 8 warps: 5 % mean error; the number of warps taken by it costs 0.6 % (2 % where the
+// record is written) on the best one, geometric mean, and 7 ... 15 % at worst.
+inline double pair_time(const m2d_scan_desc* d, const Plan& p, PairKernel k, int per_sm, int sms) {
+    const int per = (d->B - 1) / p.grid_x + 1;
+    const long long ctas = (long long)p.grid_x * p.groups;
+    const int fill = (int)((ctas + sms - 1) / sms);
+    const double bands = (double)per * p.nbands, steps = bands * d->W + 2 * p.warps + 1, on_sm = fill < per_sm ? fill : per_sm;
+    const double w = on_sm * d->H / (2.0 * p.nbands), wrap = 2 * p.warps < d->W ? 2.0 * p.warps / d->W : 1.0;
+    const double t = k == kPairForward ? 1.2 + 1.37 * bands + (0.312 + 0.0340 * w + 0.089 * wrap) * steps
+                     : k == kPairStates ? 1.5 + 1.38 * bands + (0.338 + 0.0435 * w + 0.024 * wrap + 0.0070 * on_sm) * steps
+                                        : 0.5 + 1.86 * bands + (0.601 + 0.0768 * w + 0.075 * wrap) * steps;
+    return fill > per_sm ? t * fill / per_sm : t;
+}
+// The wave kernels' times below are upper bounds, by about this much where they are compared with the batch kernels'.
+constexpr double kWaveMargin = 1.08;
+
+// Every number of warps is tried; the plan with the least time is kept (in *time, us).
+inline Plan plan_pairs(const m2d_scan_desc* d, PairKernel k, double* time) {
+    Plan best{};
+    const int sms = sm_count();
+    for (int nw = kPairWarps; nw >= 1; --nw) {
+        Plan p{};
+        p.groups = (d->E + kGroup - 1) / kGroup;
+        p.Rb = d->H < 2 * nw ? d->H : 2 * nw;
         // a band boundary must be written two steps before the band below reads it
-        p.Rb = d->W - 2 > 1 ? d->W - 2 : 1;
-        p.warps = p.Rb;
+        if (p.Rb < d->H && p.Rb > d->W - 2) p.Rb = d->W - 2 > 1 ? (d->W - 2) & ~1 : 1;
+        p.warps = (p.Rb + 1) / 2;
         p.nbands = (d->H + p.Rb - 1) / p.Rb;
-    }
-    const int ctas_per_sm = warps_per_sm / p.warps > 0 ? warps_per_sm / p.warps : 1;
-    const long long slots = (long long)ctas_per_sm * sm_count();
-    // all CTAs resident at once: CTAs per channel group = floor(slots / groups), images per CTA to match
-    long long per_group = slots / p.groups;
-    if (per_group < 1) per_group = 1;
-    const long long per = (d->B + per_group - 1) / per_group;    // images per CTA
-    p.grid_x = (int)((d->B + per - 1) / per);
-    p.chain = 1;
-    return p;
-}
-
-// Try every cap on the row-warps per CTA and keep the plan that keeps the most warps resident,
-// discounted by the rows lost to padding; ties go to the larger CTA.
-inline Plan plan_best(const m2d_scan_desc* d, int max_warps, int warps_per_sm) {
-    Plan best = plan_common(d, max_warps, warps_per_sm);
-    double best_score = -1.0;
-    const double cap = (double)warps_per_sm * sm_count();
-    for (int w = max_warps; w >= 2; --w) {
-        const Plan p = plan_common(d, w, warps_per_sm);
-        double resident = (double)p.grid_x * p.groups * p.warps;
-        if (resident > cap) resident = cap;
-        const double eff = (double)d->H / ((double)p.nbands * p.Rb);
-        const double score = resident * eff;
-        if (score > best_score * 1.02) { best_score = score; best = p; }
+        p.smem = (k == kPairAdjoint ? pairs_bwd_smem_bytes(p.warps) : pairs_fwd_smem_bytes(p.warps)) + kParamF4 * sizeof(float4);
+        const int fit = (int)((kMaxSmem + 1024) / (p.smem + 1024)), per_sm = fit < 16 / p.warps ? fit : 16 / p.warps;
+        // all CTAs resident at once: CTAs per channel group = floor(slots / groups), images per CTA to match
+        int per_group = per_sm * sms / p.groups;
+        if (per_group < 1) per_group = 1;
+        const int per = (d->B - 1) / per_group + 1;                  // images per CTA
+        p.grid_x = (d->B - 1) / per + 1;
+        p.chain = 1;
+        const double t = pair_time(d, p, k, per_sm, sms);
+        if (best.warps == 0 || t < *time) { best = p; *time = t; }
     }
     return best;
 }
-
-// Steps the busiest CTA of a batch launch takes.
-inline double batch_steps(const m2d_scan_desc* d, const Plan& p) {
-    const long long per = ((long long)d->B + p.grid_x - 1) / p.grid_x;
-    return (double)per * p.nbands * d->W + p.Rb;
+// Bytes of the rings that carry a band's last row to the next band.
+inline size_t pair_ring_bytes(const m2d_scan_desc* d, const Plan& p) {
+    return p.nbands > 1 ? (size_t)p.grid_x * p.groups * d->W * kSlotF4 * sizeof(float4) : 0;
 }
 
 inline size_t align256(size_t v) { return (v + 255) & ~(size_t)255; }
@@ -260,19 +249,15 @@ inline bool edge_pairs(const m2d_scan_desc* d, const Plan& p, size_t element) {
 }
 
 inline Plan plan_fwd(const m2d_scan_desc* d, bool allow_chain = true) {
-    // The batch kernel runs one CTA per (image, 32 channels) and is at its best when those fill the GPU; the
-    // wave kernels split an image over CTAs as well.  Measured times per step: 0.9 us (batch), 0.62 us (wave,
-    // four channels per lane) and 0.42 us (two channels, twice the CTAs); they put the lines where the
-    // measured times cross within 10 % (56x56x64: wave up to batch 64, 290 against 381 us there; 14x14x320:
-    // up to batch 8).  The batch kernel needs three columns.  (fp32 or bf16 I/O differ by less than that.)
+    // The batch kernel runs one CTA per (image, 16 channels) and is at its best when those fill the GPU; the wave kernels
+    // split an image over CTAs as well.  Measured times per step of those: 0.62 us with four channels per lane, 0.42 us
+    // with two and twice the CTAs.  The batch kernel needs three columns.
     Plan p{};
     double best = 1e30;
     if (d->W >= 3) {
-        p = plan_best(d, 8, 16);
-        p.smem = rows_fwd_smem_bytes(p.warps) + kParamF4 * sizeof(float4);
-        p.scratch = kStatusBytes;
-        if (p.nbands > 1) p.scratch += align256((size_t)p.grid_x * p.groups * d->W * kSlotF4 * sizeof(float4));
-        best = 0.9 * batch_steps(d, p);
+        p = plan_pairs(d, kPairForward, &best);
+        best *= kWaveMargin;
+        p.scratch = kStatusBytes + align256(pair_ring_bytes(d, p));
     }
     for (const int C : {4, 2}) {
         if (!allow_chain && d->W >= 3) break;

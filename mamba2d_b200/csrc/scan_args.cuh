@@ -53,8 +53,7 @@ struct ScanArgs {
     int d_f32;                // D and d_D are fp32 whatever the I/O type
     // ---- backward only ----
     const void* gy;
-    float4* hs;               // full state record: [b][group][H*W] blocks; a block is [4][32] float4 (fp32 I/O)
-                              // or [2][32] uint4 holding 16 bf16 states per lane (bf16 I/O)
+    float4* hs;               // state record; batch kernels: [group][pixel] blocks of two (fp32) or one (bf16) float4 per lane
     // fp32 accumulators of the reduced gradients, zeroed before the kernel.  For fp32 I/O they are
     // the caller's gradient tensors themselves; for bf16 I/O they live in the workspace.
     float *accBT, *accBL, *accC;   // [B*H*W] rows of N values at a pitch of acc_pitch
@@ -73,7 +72,7 @@ __device__ __forceinline__ int scan_pixel(const ScanArgs& a, int b, int i, int j
 }
 
 // float4 units of one (cell, warp) block of the state record
-template <typename io_t> struct HsBlock { static constexpr int f4 = sizeof(io_t) == 2 ? 64 : 128; };
+template <typename rec_t> struct HsBlock { static constexpr int f4 = sizeof(rec_t) == 2 ? 32 : 64; };
 
 // Element (e, n) of AT / AL as a float.  With `a_log` the tensors hold the fp32 parameter A_log and
 // A = -exp(A_log), rounded to the I/O type the way the reference's cast does
@@ -99,7 +98,7 @@ template <typename io_t>
 __device__ __forceinline__ void stage_params(float4* dst, const void* AT, const void* AL, int N, int ch0, int chv, int n0, int nv, int lane,
                                              int a_log) {
 #pragma unroll
-    for (int c = 0; c < 4; ++c) {
+    for (int c = 0; c < 2; ++c) {
         float t[4], l[4];
 #pragma unroll
         for (int n = 0; n < 4; ++n) {
@@ -108,7 +107,7 @@ __device__ __forceinline__ void stage_params(float4* dst, const void* AT, const 
             l[n] = ok ? load_A<io_t>(AL, (long long)(ch0 + c) * N + n0 + n, a_log) * kLog2e : 0.f;
         }
         dst[c * 32 + lane] = make_float4(t[0], t[1], t[2], t[3]);
-        dst[128 + c * 32 + lane] = make_float4(l[0], l[1], l[2], l[3]);
+        dst[64 + c * 32 + lane] = make_float4(l[0], l[1], l[2], l[3]);
     }
 }
 

@@ -1,0 +1,48 @@
+"""The batch kernels (a warp owns two rows of 16 channels) at the edges of their tiles: an odd last row, bands cut short by
+narrow maps, one row per band, ragged channels and states, lists of several images per CTA, both types of the state record."""
+import ctypes
+
+import pytest
+import torch
+
+from mamba2d_b200 import _lib, scan_bwd, scan_fwd
+from oracle import cpu, inputs
+from helpers import rel_err
+
+pytestmark = pytest.mark.gpu
+ORDER = ("x", "dT", "dL", "AT", "AL", "BT", "BL", "C", "D")
+SHAPES = [
+    (200, 2, 3, 16, 16),      # one pair of rows, the narrowest map
+    (150, 7, 3, 20, 16),      # bands of one row: no second row anywhere; ragged second group
+    (130, 9, 4, 32, 16),      # bands of two rows, an odd last one
+    (600, 3, 6, 48, 12),      # an odd last row in a single band, lists of images
+    (140, 33, 5, 34, 16),     # 17 bands, the last of one row
+    (700, 7, 7, 40, 16),      # the last stage of a model, lists of images, ragged group
+    (90, 17, 19, 66, 5),      # scalar loads, ragged states
+    (70, 31, 12, 96, 16),
+    (12, 20, 20, 128, 16),    # bf16: few images, the record stays fp32
+]
+
+
+@pytest.mark.parametrize("shape", SHAPES)
+@pytest.mark.parametrize("dt,tol", [(torch.float32, 1e-4), (torch.bfloat16, 2e-2)])
+@pytest.mark.parametrize("reverse", [False, True])
+def test_batch_kernels_against_the_oracle(shape, dt, tol, reverse):
+    d = _lib.ScanDesc()
+    d.struct_bytes = ctypes.sizeof(d)
+    d.B, d.H, d.W, d.E, d.N = shape
+    d.BT_pitch = d.BL_pitch = d.C_pitch = shape[4]
+    assert (_lib.lib().m2d_scan_fwd_chain(ctypes.byref(d)), _lib.lib().m2d_scan_bwd_chain(ctypes.byref(d))) == (1, 1)
+    inp = inputs.make_inputs(*shape, seed=sum(shape), strided_bc=True)
+    inp = {k: v.to(dt).float() for k, v in inp.items()}
+    dev = {k: v.cuda().to(dt) for k, v in inp.items()}
+    ref = {k: (v.flip(1, 2).contiguous() if v.dim() == 4 else v) for k, v in inp.items()} if reverse else inp
+
+    def back(a):
+        return a[:, ::-1, ::-1] if reverse and a.ndim == 4 else a
+    y = scan_fwd(*[dev[k] for k in ORDER], reverse=reverse)
+    assert rel_err(y.float().cpu().numpy(), back(cpu.forward(ref, "f64"))) < tol
+    grads = scan_bwd(*[dev[k] for k in ORDER], dev["gy"], reverse=reverse)
+    want = cpu.backward(ref, mode="f64")
+    for name, t in zip(cpu.GRAD_NAMES, grads):
+        assert rel_err(t.float().cpu().numpy(), back(want[name])) < tol, name
