@@ -47,7 +47,7 @@ inline int launch_sweep_kernel(void (*kern)(const ScanArgs), ScanArgs& a, const 
         const long long fit = (long long)per_sm * sm_count() / ((long long)pl.grid_x * pl.groups);
         if (fit < a.chain) a.chain = bound_chain(fit, pl.nbands, a.W, pl.Rb);
         for (;;) {
-            dim3 grid(pl.grid_x * a.chain, pl.groups);
+            const dim3 grid = pl.wave ? dim3(pl.grid_x * a.chain, pl.groups) : dim3(pl.groups, pl.grid_x * a.chain);
             void* args[] = {&a};
             const cudaError_t e = cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(kern), grid, block, args, pl.smem, st);
             if (e == cudaSuccess) return M2D_OK;

@@ -59,6 +59,7 @@ inline BwdLayout bwd_layout(const m2d_scan_desc* d, const BwdPlan& p) {
     off += L.acc_bytes;
     L.edge = off;
     if (p.wave) off += 2 * wave_edge_bytes(d, p, true);
+    else if (p.chain > 1) off += pair_edge_bytes(d, p.states) + pair_edge_bytes(d, p);
     else off += align256(std::max(pair_ring_bytes(d, p), pair_ring_bytes(d, p.states)));
     L.hs = off;
     if (p.wave) off += align256((size_t)p.grid_x * p.groups * p.warps * p.nbands * (d->W + 7) * p.wave * 512);
@@ -67,7 +68,7 @@ inline BwdLayout bwd_layout(const m2d_scan_desc* d, const BwdPlan& p) {
     return L;
 }
 
-inline BwdPlan plan_bwd(const m2d_scan_desc* d) {
+inline BwdPlan make_plan_bwd(const m2d_scan_desc* d) {
     // Batch or wave, as in plan_fwd: 1.2 us per step of both sweeps in the wave kernel with two channels per lane (four
     // spill and are slower at every size measured), whatever the I/O type.
     BwdPlan p{};
@@ -80,9 +81,23 @@ inline BwdPlan plan_bwd(const m2d_scan_desc* d) {
         best = (best + states) * kWaveMargin;
     }
     const Plan w = plan_wave(d, 2);
-    if (1.2 * wave_steps(d, w) + 10.0 < best) static_cast<Plan&>(p) = w;
+    const double wave = 1.2 * wave_steps(d, w) + 10.0;
+    if (wave < best) static_cast<Plan&>(p) = w;
+    double adjoint = 0.0, states = 0.0;
+    const Plan pa = plan_pair_chain(d, kPairAdjoint, &adjoint), ps = plan_pair_chain(d, kPairStates, &states);
+    const double chained = adjoint + states + (pa.warps && ps.warps ? (pair_edge_bytes(d, pa) + pair_edge_bytes(d, ps)) / 5e6 : 1e30);    // (and clearing)
+    if (chained < kChainShare * wave && chained < 0.9 * best) {
+        static_cast<Plan&>(p) = pa;
+        p.states = ps;
+        p.wide = true;
+    }
     p.scratch = bwd_layout(d, p).total;
     return p;
+}
+
+inline BwdPlan plan_bwd(const m2d_scan_desc* d) {
+    static thread_local LastPlan<BwdPlan> last;
+    return last.get(d, [&] { return make_plan_bwd(d); });
 }
 
 // Few images: several CTAs per image.
@@ -92,17 +107,17 @@ __global__ void __launch_bounds__(256, 1) m2d_bwd_wave_kernel(const ScanArgs a) 
     wave_backward<io_t, 2, VEC>(a, reinterpret_cast<char*>(smem));
 }
 
-// Batch mode (one CTA per image and channel group): the recompute sweep, which writes the state record and d_C, and the
+// Batch mode (one CTA per image and channel group, or a chain of them): the recompute sweep, which writes the state record and d_C, and the
 // adjoint sweep, each a kernel of its own: their registers, shared memory and bands need not be the same.
-template <typename io_t, typename rec_t, bool VEC>
+template <typename io_t, typename rec_t, bool VEC, bool CHAIN>
 __global__ void __launch_bounds__(kPairWarps * 32, 2) m2d_bwd_states_kernel(const ScanArgs a) {
     extern __shared__ float4 smem[];
     const PairLane ln(a);
     const unsigned params = begin_pairs<io_t>(a, smem, pairs_fwd_smem_bytes(ln.nwarps), ln);
-    forward_pairs<io_t, rec_t, VEC, true, false>(a, smem_u32(smem), params, 0.f, blockIdx.y, gridDim.y, images_of_cta(a));
+    forward_pairs<io_t, rec_t, VEC, true, false, CHAIN>(a, smem_u32(smem), params, 0.f);
 }
 
-template <typename io_t, typename rec_t, bool VEC>
+template <typename io_t, typename rec_t, bool VEC, bool CHAIN>
 __global__ void __launch_bounds__(kPairWarps * 32, 2) m2d_bwd_kernel(const ScanArgs a) {
     extern __shared__ float4 smem[];
     const PairLane ln(a);
@@ -113,7 +128,7 @@ __global__ void __launch_bounds__(kPairWarps * 32, 2) m2d_bwd_kernel(const ScanA
     clear(dAT);
     clear(dAL);
     float dD = 0.f;
-    reverse_pairs<io_t, rec_t, VEC>(a, smem_u32(smem), params, D_lane, dAT, dAL, dD, blockIdx.y, gridDim.y, images_of_cta(a));
+    reverse_pairs<io_t, rec_t, VEC, CHAIN>(a, smem_u32(smem), params, D_lane, dAT, dAL, dD);
 
     // ---- per-(channel, state) sums: fold the CTA's warps through shared memory, then one atomic per value from warp 0
     constexpr int kSums = 17;
@@ -211,10 +226,11 @@ typedef void (*SweepKernel)(const ScanArgs);
 
 template <typename io_t>
 static int launch_bwd(const m2d_scan_desc* d, const BwdPlan& pl, bool vec, cudaStream_t st) {
-    // (a kernel by the type of its record and its kind of loads)
-    auto pick = [](bool vec, bool wide, auto kernel) -> SweepKernel {
-        if (wide || sizeof(io_t) == 4) return vec ? kernel(float{}, std::true_type{}) : kernel(float{}, std::false_type{});
-        return vec ? kernel(io_t{}, std::true_type{}) : kernel(io_t{}, std::false_type{});
+    // (a kernel by the type of its record, its kind of loads and whether its CTAs are chained)
+    auto pick = [&](auto kernel) -> SweepKernel {
+        auto loads = [&](auto rec, auto chain) { return vec ? kernel(rec, std::true_type{}, chain) : kernel(rec, std::false_type{}, chain); };
+        if (pl.chain > 1) return loads(float{}, std::true_type{});           // (a chain has few images: few_images)
+        return pl.wide || sizeof(io_t) == 4 ? loads(float{}, std::false_type{}) : loads(io_t{}, std::false_type{});
     };
     const BwdLayout L = bwd_layout(d, pl);
     char* ws = static_cast<char*>(d->workspace);
@@ -229,6 +245,11 @@ static int launch_bwd(const m2d_scan_desc* d, const BwdPlan& pl, bool vec, cudaS
         a.bnd_up = reinterpret_cast<float4*>(ws + L.edge + edge);
         a.bnd_rows = wave_rows(pl, true);
         if (pl.chain > 1) zero_bytes = L.edge + 2 * edge;
+    } else if (pl.chain > 1) {
+        const size_t states = pair_edge_bytes(d, pl.states);
+        a.bnd = reinterpret_cast<float4*>(ws + L.edge);
+        a.bnd_up = reinterpret_cast<float4*>(ws + L.edge + states);
+        zero_bytes = L.edge + states + pair_edge_bytes(d, pl);
     }
     if (cudaMemsetAsync(ws, 0, zero_bytes, st) != cudaSuccess) return M2D_ERR_LAUNCH;
     a.gy = d->gy;
@@ -271,14 +292,16 @@ static int launch_bwd(const m2d_scan_desc* d, const BwdPlan& pl, bool vec, cudaS
     if (!pl.wave) {
         a.Rb = pl.states.Rb;
         a.nbands = pl.states.nbands;
-        const int rc = launch_sweep_kernel(pick(vec, pl.wide, [](auto rec, auto v) { return m2d_bwd_states_kernel<io_t, decltype(rec), decltype(v)::value>; }),
+        a.chain = pl.states.chain;
+        const int rc = launch_sweep_kernel(pick([](auto rec, auto v, auto ch) { return m2d_bwd_states_kernel<io_t, decltype(rec), decltype(v)::value, decltype(ch)::value>; }),
                                            a, pl.states, st);
         if (rc != M2D_OK) return rc;
         a.Rb = pl.Rb;
         a.nbands = pl.nbands;
+        a.chain = pl.chain;
     }
     const int rc = launch_sweep_kernel(pl.wave ? (vec ? m2d_bwd_wave_kernel<io_t, true> : m2d_bwd_wave_kernel<io_t, false>)
-                                               : pick(vec, pl.wide, [](auto rec, auto v) { return m2d_bwd_kernel<io_t, decltype(rec), decltype(v)::value>; }),
+                                               : pick([](auto rec, auto v, auto ch) { return m2d_bwd_kernel<io_t, decltype(rec), decltype(v)::value, decltype(ch)::value>; }),
                                        a, p, st);
     if (rc != M2D_OK) return rc;
     if constexpr (sizeof(io_t) == 2) {

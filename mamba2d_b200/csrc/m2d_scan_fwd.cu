@@ -19,7 +19,7 @@ __global__ void __launch_bounds__(kPairWarps * 32, 2) m2d_fwd_kernel(const ScanA
     const PairLane ln(a);
     const unsigned params = begin_pairs<io_t>(a, smem, pairs_fwd_smem_bytes(ln.nwarps), ln);
     const int y_ch = ln.ch0 + (ln.nq & 1);
-    forward_pairs<io_t, float, VEC, false, ACT>(a, smem_u32(smem), params, y_ch < a.E ? load_D<io_t>(a, y_ch) : 0.f, blockIdx.y, gridDim.y, images_of_cta(a));
+    forward_pairs<io_t, float, VEC, false, ACT, false>(a, smem_u32(smem), params, y_ch < a.E ? load_D<io_t>(a, y_ch) : 0.f);
 }
 
 // The status word and, where CTAs of a wave launch read each other's, the boundary rows behind it.

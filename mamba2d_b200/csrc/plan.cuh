@@ -119,6 +119,28 @@ inline bool vector_ok(const m2d_scan_desc* d, bool bwd) {
     return ok;
 }
 
+inline size_t align256(size_t v) { return (v + 255) & ~(size_t)255; }
+
+// CTAs per image that a chained launch may use: at most one per band, and, when CTAs own more than one band
+// each, fewer than one row of steps divided by the rows of a band.  `want` is the chain the resident CTA slots allow;
+// `steps_per_row` the steps a warp needs for one row.  Every place that picks or shortens a chain goes
+// through this rule.
+//
+// The batch kernels need the second limit: their warps walk a CTA's bands in lock step, so that a first warp that waits for
+// its next band holds up the last columns of this one, and with them the bands below it that it waits for.  For the wave
+// kernels it is cautious: a CTA finishes a band before it takes its next, bands are taken in ascending order (descending in
+// the adjoint sweep) and each waits only for the one before, so that whatever the chain's length some CTA can always go on.
+// On narrow maps it leaves SMs idle: 4x200x14x96 gets one CTA per image where six are free, 600 dependent
+// steps instead of 384; 3x45x31x192 135 instead of 115.
+inline int bound_chain(long long want, int nbands, int steps_per_row, int Rb) {
+    if (want > nbands) want = nbands;
+    if (want < nbands) {
+        const long long lim = steps_per_row / Rb - 1;
+        if (want > lim) want = lim;
+    }
+    return want < 1 ? 1 : (int)want;
+}
+
 // Batch mode: one CTA per (image, 16 channels), images chained per CTA; a warp owns two rows of a band.
 constexpr int kPairWarps = 8;            // warps per CTA, at most (128 registers: 16 per SM)
 enum PairKernel { kPairForward, kPairStates, kPairAdjoint };
@@ -141,6 +163,22 @@ inline double pair_time(const m2d_scan_desc* d, const Plan& p, PairKernel k, int
 }
 // The wave kernels' times below are upper bounds, by about this much where they are compared with the batch kernels'.
 constexpr double kWaveMargin = 1.08;
+
+// The same for the sweeps of a backward with the bands of an image in `chain` CTAs.  A band starts kPairLag columns behind
+// the last row of the one above, and a CTA takes its next one when it has finished one.  8 % mean error over 13 shapes, above for short ones.
+constexpr int kPairLag = 5;
+inline double pair_chain_time(const m2d_scan_desc* d, const Plan& p, PairKernel k, int sms) {
+    const double lag = p.Rb + kPairLag;
+    const double start = p.chain * lag >= d->W ? (p.nbands - 1) * lag : (p.nbands - 1) / p.chain * (double)d->W + (p.nbands - 1) % p.chain * lag;
+    const double steps = start + d->W + 2 * p.warps + 1, w = (double)(((long long)d->B * p.groups * p.chain + sms - 1) / sms) * p.warps;
+    return k == kPairStates ? (0.54 + 0.025 * w) * steps : (0.84 + 0.043 * w) * steps;
+}
+// Chained sweeps are taken where they come to less than this share of a wave launch, whose time is an upper bound: where the
+// bands are more than the CTAs the wave kernels can have resident.  Backward, us, wave / chained: 16x100x112x64 fp32 1064 /
+// 769 (of a share of 0.63), 1x400x400x384 fp32 4683 / 3382 (0.66); but 5x37x53x96 154 / 188 (0.86), 3x80x80x96 290 / 339 (0.95),
+// 2x200x336x64 bf16 982 / 1079 (0.97): a step of these kernels takes longer where it is the chain that bounds.  (In the
+// forward 16x100x112x64 gains 270 / 219; not taken.)
+constexpr double kChainShare = 0.80;
 
 // Every number of warps is tried; the plan with the least time is kept (in *time, us).
 inline Plan plan_pairs(const m2d_scan_desc* d, PairKernel k, double* time) {
@@ -167,34 +205,37 @@ inline Plan plan_pairs(const m2d_scan_desc* d, PairKernel k, double* time) {
     }
     return best;
 }
+// The plan for few images: bands of at least eight rows (the scratch of a band's boundary row), all CTAs resident.
+inline Plan plan_pair_chain(const m2d_scan_desc* d, PairKernel k, double* time) {
+    Plan best{};
+    const int sms = sm_count();
+    for (int nw = kPairWarps; nw >= 4; --nw) {
+        Plan p{};
+        p.groups = (d->E + kGroup - 1) / kGroup;
+        p.Rb = 2 * nw;
+        if (p.Rb >= d->H || p.Rb > d->W - 2) continue;
+        p.warps = nw;
+        p.nbands = (d->H + p.Rb - 1) / p.Rb;
+        p.smem = (k == kPairAdjoint ? pairs_bwd_smem_bytes(nw) : pairs_fwd_smem_bytes(nw)) + kParamF4 * sizeof(float4);
+        const int fit = (int)((kMaxSmem + 1024) / (p.smem + 1024)), per_sm = fit < 16 / nw ? fit : 16 / nw;
+        p.chain = bound_chain((long long)per_sm * sms / ((long long)d->B * p.groups), p.nbands, d->W, p.Rb);
+        if (p.chain < 2) continue;
+        p.grid_x = d->B;
+        const double t = pair_chain_time(d, p, k, sms);
+        if (best.warps == 0 || t < *time) { best = p; *time = t; }
+    }
+    return best;
+}
+inline size_t pair_edge_bytes(const m2d_scan_desc* d, const Plan& p) {
+    return align256((size_t)d->B * p.groups * p.nbands * d->W * kSlotF4 * sizeof(float4));
+}
 // Bytes of the rings that carry a band's last row to the next band.
 inline size_t pair_ring_bytes(const m2d_scan_desc* d, const Plan& p) {
     return p.nbands > 1 ? (size_t)p.grid_x * p.groups * d->W * kSlotF4 * sizeof(float4) : 0;
 }
 
-inline size_t align256(size_t v) { return (v + 255) & ~(size_t)255; }
-
 // Scratch layout shared by every entry point: [status word, 256 bytes][the rest].
 constexpr size_t kStatusBytes = 256;
-
-// CTAs per image that a wave launch may use: at most one per band, and, when CTAs own more than one band
-// each, fewer than one row of steps divided by the rows of a band.  `want` is the chain the resident CTA slots allow;
-// `steps_per_row` the steps a warp needs for one row.  Every place that picks or shortens a chain goes
-// through this rule.
-//
-// The second limit is cautious: the waits end without it.  A CTA finishes a band before it takes its next, bands are
-// taken in ascending order (descending in the adjoint sweep) and each waits only for the one before, so that
-// whatever the chain's length some CTA can always go on.  (Kernels whose CTAs walk their bands in lock-step need
-// it.)  On narrow maps it leaves SMs idle: 4x200x14x96 gets one CTA per image where six are free, 600 dependent
-// steps instead of 384; 3x45x31x192 135 instead of 115.
-inline int bound_chain(long long want, int nbands, int steps_per_row, int Rb) {
-    if (want > nbands) want = nbands;
-    if (want < nbands) {
-        const long long lim = steps_per_row / Rb - 1;
-        if (want > lim) want = lim;
-    }
-    return want < 1 ? 1 : (int)want;
-}
 
 // Wave kernels (wave.cuh): bands of eight rows, 8 * C channels per CTA, one CTA per SM.  Where images and
 // channel groups alone do not fill the GPU every image gets a chain of CTAs; otherwise a CTA walks a list of
@@ -248,7 +289,24 @@ inline bool edge_pairs(const m2d_scan_desc* d, const Plan& p, size_t element) {
     return p.wave == 4 && p.chain > 1 && (p.chain - 1) * 15.0 * 10.0 >= wave_steps(d, p) * (element == 2 ? 1 : 3);
 }
 
-inline Plan plan_fwd(const m2d_scan_desc* d, bool allow_chain = true) {
+// A thread's last plan of a kind.  A call asks for its plan several times (workspace, chain, launch), at 1 ... 2 us each; the
+// plan depends on what is compared here and on nothing else.
+template <typename P>
+struct LastPlan {
+    int device = -2, B, H, W, E, N, dtype;
+    P plan;
+    template <typename F>
+    const P& get(const m2d_scan_desc* d, F make) {
+        const int dev = device_index();
+        if (dev != device || d->B != B || d->H != H || d->W != W || d->E != E || d->N != N || (int)d->dtype != dtype) {
+            plan = make();
+            device = dev; B = d->B; H = d->H; W = d->W; E = d->E; N = d->N; dtype = (int)d->dtype;
+        }
+        return plan;
+    }
+};
+
+inline Plan make_plan_fwd(const m2d_scan_desc* d, bool allow_chain) {
     // The batch kernel runs one CTA per (image, 16 channels) and is at its best when those fill the GPU; the wave kernels
     // split an image over CTAs as well.  Measured times per step of those: 0.62 us with four channels per lane, 0.42 us
     // with two and twice the CTAs.  The batch kernel needs three columns.
@@ -267,6 +325,11 @@ inline Plan plan_fwd(const m2d_scan_desc* d, bool allow_chain = true) {
         if (t < best) { best = t; p = w; p.scratch = kStatusBytes + wave_edge_bytes(d, w, false); }
     }
     return p;
+}
+
+inline Plan plan_fwd(const m2d_scan_desc* d, bool allow_chain = true) {
+    static thread_local LastPlan<Plan> last;
+    return allow_chain ? last.get(d, [&] { return make_plan_fwd(d, true); }) : make_plan_fwd(d, false);
 }
 
 }  // namespace m2d

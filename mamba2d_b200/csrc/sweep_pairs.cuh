@@ -210,6 +210,77 @@ __device__ __forceinline__ void read_cell(CellIn& v, unsigned px, unsigned pn) {
     lds_in4<io_t>(v.bL, pn + 64);
     if (READ_C) lds_in4<io_t>(v.c, pn + 128);
 }
+// ---- bands in several CTAs (CHAIN) ---------------------------------------------------------------------------------
+// Where there are few images the bands of one go to `chain` CTAs, CTA c taking the bands c, c + chain, ...; a boundary row in
+// global memory then takes the place of the ring.  As in the wave kernels it is zeroed before the launch and holds states
+// with their bits inverted, so that a block that is not there yet shows: no arithmetic returns the NaN that would read as
+// zero.  A block is requested two steps ahead like everything else; where it was not there, the warp that needs it polls,
+// and the CTA falls behind the one above until its requests find what they ask for.
+__device__ __forceinline__ uint4 invert_bits(const float4& v) {
+    return make_uint4(~__float_as_uint(v.x), ~__float_as_uint(v.y), ~__float_as_uint(v.z), ~__float_as_uint(v.w));
+}
+__device__ __forceinline__ bool arrived(const float4& v) {
+    return __float_as_uint(v.x) != 0 && __float_as_uint(v.y) != 0 && __float_as_uint(v.z) != 0 && __float_as_uint(v.w) != 0;
+}
+// Makes sure that the block in S buffer `smem` is the one at `src`.  Every poll is bounded; a warp that has given up once
+// waits no more (what it reads then are NaNs).  (Waiting for a block two, four or six columns on as well, so that later
+// requests come back in time, costs half a microsecond per band and column and gains nothing: 716, 744 and 786 us against
+// 697 in the adjoint sweep at 2x200x336x64.)
+__device__ __forceinline__ void wait_for_block(const ScanArgs& a, unsigned smem, const float4* src, bool& given_up) {
+    if (__all_sync(0xffffffffu, arrived(lds4(smem)) && arrived(lds4(smem + 512)))) return;
+#pragma unroll 1
+    for (int polls = 0;; ++polls) {
+        float4 v[2];
+#pragma unroll
+        for (int c = 0; c < 2; ++c)
+            asm volatile("ld.volatile.global.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v[c].x), "=f"(v[c].y), "=f"(v[c].z), "=f"(v[c].w) : "l"(src + c * 32) : "memory");
+        if (polls > a.wait_limit || *reinterpret_cast<volatile int*>(a.status) != 0) {
+            if (!given_up) {
+                atomicExch(a.status, 1);
+                if (a.host_flag) *reinterpret_cast<volatile int*>(a.host_flag) = 1;
+            }
+            given_up = true;
+        }
+        given_up = __any_sync(0xffffffffu, given_up);
+        if (__all_sync(0xffffffffu, arrived(v[0]) && arrived(v[1])) || given_up) {
+            sts4(smem, v[0]);
+            sts4(smem + 512, v[1]);
+            return;
+        }
+    }
+}
+__device__ __forceinline__ float2 flip_bits(float2 v, unsigned mask) {
+    return make_float2(__uint_as_float(__float_as_uint(v.x) ^ mask), __uint_as_float(__float_as_uint(v.y) ^ mask));
+}
+template <bool CHAIN> __device__ __forceinline__ void push_block(float4* dst, const Quad& s0, const Quad& s1) {
+    if (CHAIN) {
+        __stcg(reinterpret_cast<uint4*>(dst), invert_bits(quad_f4(s0)));
+        __stcg(reinterpret_cast<uint4*>(dst + 32), invert_bits(quad_f4(s1)));
+    } else {
+        __stcg(dst, quad_f4(s0));
+        __stcg(dst + 32, quad_f4(s1));
+    }
+}
+
+// What a CTA walks: the images blockIdx.y, blockIdx.y + gridDim.y, ... of channel group blockIdx.x with all their bands, or
+// (CHAIN) every chain-th band of one image.  (The groups of an image have neighbouring blocks, run at the same time and find
+// each other's lines of B, C and their gradients in L2.)
+template <bool CHAIN>
+struct PairWork {
+    int img0, img_stride, nb, q0, dq, items;
+    __device__ __forceinline__ PairWork(const ScanArgs& a) {
+        if (CHAIN) {
+            img0 = blockIdx.y / a.chain; img_stride = 0; nb = 1;
+            q0 = blockIdx.y % a.chain; dq = a.chain;
+            items = (a.nbands - q0 + dq - 1) / dq;
+        } else {
+            img0 = blockIdx.y; img_stride = gridDim.y; nb = (a.B - (int)blockIdx.y + (int)gridDim.y - 1) / (int)gridDim.y;
+            q0 = 0; dq = 1;
+            items = nb * a.nbands;
+        }
+    }
+};
+
 // The rotation of the three buffers, as byte offsets.
 struct Rotation {
     unsigned rd = kRot, wr = 0, ho = 2 * kRot;
@@ -234,10 +305,6 @@ __device__ __forceinline__ unsigned begin_pairs(const ScanArgs& a, float4* smem,
     return smem_u32(params + ln.lane);
 }
 
-// A CTA walks the images blockIdx.y, blockIdx.y + gridDim.y, ... of channel group blockIdx.x.  (The groups of an image
-// have neighbouring blocks, run at the same time and find each other's lines of B, C and their gradients in L2.)
-__device__ __forceinline__ int images_of_cta(const ScanArgs& a) { return (a.B - (int)blockIdx.y + (int)gridDim.y - 1) / (int)gridDim.y; }
-
 // How a step is compiled.  kInside: both cells exist and lie inside the map, where the weights are constants.  kTop: the
 // same with A in row 0, which has no direction T.  kBorder: both exist, one of them in column 0; weights and zeros for
 // missing neighbours are chosen without a branch, so that the two cells overlap as they do inside.  kPartial: one cell is
@@ -256,14 +323,16 @@ __device__ __forceinline__ float2 lane_D(const ScanArgs& a, const PairLane& ln) 
 //
 // ACT: gelu(y) goes out instead of y.  It is worked out and stored in the warp's next step: behind the sum over states, at
 // the end of its own, its chain of fifteen dependent instructions lies open in every step.
-template <typename io_t, typename rec_t, bool VEC, bool RECORD, bool ACT>
-__device__ __forceinline__ void forward_pairs(const ScanArgs& a, unsigned smem, unsigned params, float D_lane,
-                                              int img0, int img_stride, int nb) {
+template <typename io_t, typename rec_t, bool VEC, bool RECORD, bool ACT, bool CHAIN>
+__device__ __forceinline__ void forward_pairs(const ScanArgs& a, unsigned smem, unsigned params, float D_lane) {
     constexpr int HB = HsBlock<rec_t>::f4;
     const PairLane ln(a);
     const int lane = ln.lane, r = ln.r, cq = ln.cq, nq = ln.nq, g = ln.g;
     const int W = a.W, H = a.H, E = a.E, Rb = a.Rb, nbands = a.nbands;
-    float4* const ring = a.ring + ((size_t)(blockIdx.y * gridDim.x + blockIdx.x) * W) * kSlotF4 + lane;
+    const PairWork<CHAIN> work(a);
+    // the ring, or the boundary rows of this image and group
+    float4* const ring = CHAIN ? a.bnd + ((size_t)(work.img0 * gridDim.x + g) * nbands * W) * kSlotF4 + lane
+                               : a.ring + ((size_t)(blockIdx.y * gridDim.x + blockIdx.x) * W) * kSlotF4 + lane;
     const unsigned blk = smem + r * kFwdBlock + lane * 16;                // S of the row above; + kFwdBlock: of the row below
     const unsigned stage = smem + r * kFwdBlock + 3 * kRot;
     const unsigned stage_x = stage + cell_x<io_t>(cq), stage_n = stage + cell_n(nq), stage_o = stage + cell_out<io_t>(cq, nq), stage_w = stage + PairCopy<io_t, VEC>::slot(lane);
@@ -289,25 +358,27 @@ __device__ __forceinline__ void forward_pairs(const ScanArgs& a, unsigned smem, 
     clear(hB);
     Rotation rot;
 
-    struct Rows { bool hasA, hasB, row0, pull, pushA, pushB; int pix; };   // pix: memory pixel of column 0 of row A
+    struct Rows { bool hasA, hasB, row0, pull, pushA, pushB; int pix, edge; };   // pix: memory pixel of column 0 of row A; edge: CHAIN, block 0 of this band's boundary row
     auto make_rows = [&](int bi, int q) {
         Rows w;
         const int i = q * Rb + 2 * r;
-        w.hasA = bi < nb && 2 * r < Rb && i < H;
+        w.hasA = bi < work.nb && 2 * r < Rb && i < H;
         w.hasB = w.hasA && 2 * r + 1 < Rb && i + 1 < H;
         w.row0 = (i == 0);
         w.pull = w.hasA && (r == 0) && (q > 0);
-        w.pushA = w.hasA && (2 * r == Rb - 1) && (q < nbands - 1);
-        w.pushB = w.hasB && (2 * r + 1 == Rb - 1) && (q < nbands - 1);
-        w.pix = scan_pixel(a, img0 + bi * img_stride, i, 0);
+        const bool push = q < nbands - 1 && !(CHAIN && a.withhold && work.img0 == 0 && q == 0);
+        w.pushA = w.hasA && (2 * r == Rb - 1) && push;
+        w.pushB = w.hasB && (2 * r + 1 == Rb - 1) && push;
+        w.pix = scan_pixel(a, work.img0 + bi * work.img_stride, i, 0);
+        w.edge = CHAIN ? q * W : 0;
         return w;
     };
     // What is requested next: cell (A, s_col) by the lower half of the warp, cell (B, s_col - 1) by the upper one, each at its s_pix.
     bool s_on = false, s_pull = false;
-    int s_pix = 0, s_col = 0;
+    int s_pix = 0, s_col = 0, s_edge = 0;         // s_edge: the row above's boundary blocks
     auto request = [&](bool on) {
         copy.issue(stage_w + rot.wr, on, s_pix, E);
-        if (s_pull) cp_async_block(blk + rot.wr, ring + s_col * kSlotF4);
+        if (s_pull) cp_async_block(blk + rot.wr, ring + (s_edge + s_col) * kSlotF4);
         s_pix += dir;
         ++s_col;
     };
@@ -315,6 +386,7 @@ __device__ __forceinline__ void forward_pairs(const ScanArgs& a, unsigned smem, 
         if (!upper) { s_on = w.hasA; s_pix = w.pix; }
         s_pull = w.pull;
         s_col = 0;
+        s_edge = CHAIN ? w.edge - W : 0;
     };
     auto next_B = [&](const Rows& w) {
         if (upper) { s_on = w.hasB; s_pix = w.pix + dir * W; }
@@ -328,12 +400,15 @@ __device__ __forceinline__ void forward_pairs(const ScanArgs& a, unsigned smem, 
     };
 
     // one step: cell (A, colA) and cell (B, colB)
-    bool hasA = false, hasB = false, row0 = false, pushA = false, pushB = false;
-    int pixA = 0, pixB = 0;
+    bool hasA = false, hasB = false, row0 = false, pushA = false, pushB = false, given_up = false;
+    int pixA = 0, pixB = 0, edgeA = 0, edgeB = 0;
     auto step = [&](auto tag, const int colA, const int colB) {
         constexpr int KIND = decltype(tag)::value;
         constexpr bool FAST = KIND <= kTop, ALL = KIND != kPartial;
         if (ACT) store_held();
+        const bool pulled = CHAIN && r == 0 && KIND != kTop && hasA && !row0;
+        if (CHAIN && pulled) wait_for_block(a, blk + rot.rd, ring + (edgeA - W + colA) * kSlotF4, given_up);
+        const unsigned flip = pulled ? 0xffffffffu : 0u;
         Quad dC[2];
         float2 yv[2];
         Quad topB[2];
@@ -371,6 +446,7 @@ __device__ __forceinline__ void forward_pairs(const ScanArgs& a, unsigned smem, 
                 if (w) { top[0] = topB[c][0]; top[1] = topB[c][1]; }
                 else if (!NO_T) {
                     lds_in4<float>(top, blk + rot.rd + c * 512);
+                    if (CHAIN) { top[0] = flip_bits(top[0], flip); top[1] = flip_bits(top[1], flip); }
                     if (!FAST) { top[0] = keep(!row0, top[0]); top[1] = keep(!row0, top[1]); }
                 }
                 float2 acc = make_float2(0.f, 0.f);
@@ -393,14 +469,8 @@ __device__ __forceinline__ void forward_pairs(const ScanArgs& a, unsigned smem, 
         }
         sts4(blk + kFwdBlock + rot.ho, quad_f4(hB[0]));
         sts4(blk + kFwdBlock + rot.ho + 512, quad_f4(hB[1]));
-        if (pushB) {
-            __stcg(ring + colB * kSlotF4, quad_f4(hB[0]));
-            __stcg(ring + colB * kSlotF4 + 32, quad_f4(hB[1]));
-        }
-        if (!ALL && pushA) {
-            __stcg(ring + colA * kSlotF4, quad_f4(hA[0]));
-            __stcg(ring + colA * kSlotF4 + 32, quad_f4(hA[1]));
-        }
+        if (pushB) push_block<CHAIN>(ring + (edgeB + colB) * kSlotF4, hB[0], hB[1]);
+        if (!ALL && pushA) push_block<CHAIN>(ring + (edgeA + colA) * kSlotF4, hA[0], hA[1]);
         if (RECORD) {
             if (ALL || hasA) write_record<rec_t>(hs_img + (ptrdiff_t)pixA * HB, hA);
             if (ALL || hasB) write_record<rec_t>(hs_img + (ptrdiff_t)pixB * HB, hB);
@@ -425,21 +495,22 @@ __device__ __forceinline__ void forward_pairs(const ScanArgs& a, unsigned smem, 
     // 2r idle steps, two steps that only request, W steps per (image, band) item, one for the last cell of row B, and
     // idle steps until the last warp is done
     for (int k = 0; k < 2 * r; ++k) rot.end_step();
-    Rows cur = make_rows(0, 0);
-    int bi = 0, q = 0;
+    int bi = 0, q = work.q0;
+    Rows cur = make_rows(bi, q);
     next_A(cur);
     request(s_on);
     rot.end_step();
     next_B(cur);
     request(s_on);
     rot.end_step();
-    const int items = nb * nbands;
+    const int items = work.items;
     for (int m = 0; m <= items; ++m) {
         hasA = cur.hasA;
         row0 = cur.row0;
         pushA = cur.pushA;
         pixA = cur.pix;
-        if (++q == nbands) { q = 0; ++bi; }
+        if (CHAIN) edgeA = cur.edge;
+        if ((q += work.dq) >= nbands) { q = work.q0; ++bi; }
         Rows nxt = cur;
         const bool fast = cur.hasA && cur.hasB;
         const int cols = m < items ? W : 1;
@@ -459,6 +530,7 @@ __device__ __forceinline__ void forward_pairs(const ScanArgs& a, unsigned smem, 
             if (col == 1) {
                 hasB = cur.hasB;
                 pushB = cur.pushB;
+                if (CHAIN) edgeB = cur.edge;
                 pixB = cur.pix + dir * W;
             }
             if (hasA && hasB) step(StepTag<kBorder>{}, col, col == 0 ? W - 1 : col - 1);
@@ -486,16 +558,18 @@ __device__ __forceinline__ void forward_pairs(const ScanArgs& a, unsigned smem, 
 // Adjoint sweep of one CTA over its images.  Bands are visited last to first, the bottom row of a band leads, columns run
 // right to left: in step j a warp computes cell (B, j) and cell (A, j+1); at j = W-1 that is column 0 of A in the band
 // before.  Warp r runs two steps behind warp r+1.
-template <typename io_t, typename rec_t, bool VEC>
+template <typename io_t, typename rec_t, bool VEC, bool CHAIN>
 __device__ __forceinline__ void reverse_pairs(const ScanArgs& a, unsigned smem, unsigned params, float D_lane,
-                                              Quad (&dAT)[2], Quad (&dAL)[2], float& dD, int img0, int img_stride, int nb) {
+                                              Quad (&dAT)[2], Quad (&dAL)[2], float& dD) {
     constexpr int HB = HsBlock<rec_t>::f4;     // float4 units per state-record block
     const PairLane ln(a);
     const int lane = ln.lane, r = ln.r, cq = ln.cq, nq = ln.nq, g = ln.g, nwarps = ln.nwarps;
     const int W = a.W, H = a.H, E = a.E, Rb = a.Rb, nbands = a.nbands;
     const int rr = nwarps - 1 - r;             // rank in the reverse sweep
     const int dir = a.dir;
-    float4* const ring = a.ring + ((size_t)(blockIdx.y * gridDim.x + blockIdx.x) * W) * kSlotF4 + lane;
+    const PairWork<CHAIN> work(a);
+    float4* const ring = CHAIN ? a.bnd_up + ((size_t)(work.img0 * gridDim.x + g) * nbands * W) * kSlotF4 + lane
+                               : a.ring + ((size_t)(blockIdx.y * gridDim.x + blockIdx.x) * W) * kSlotF4 + lane;
     const unsigned blk = smem + 3 * kRot + r * kBwdBlock + lane * 16;     // S: pT of row A; + kBwdBlock: of the row below B
     const unsigned stage = smem + 6 * kRot + r * kBwdBlock;
     const unsigned stage_x = stage + cell_x<io_t>(cq), stage_n = stage + cell_n(nq), stage_o = stage + cell_out<io_t>(cq, nq), stage_w = stage + PairCopy<io_t, VEC>::slot(lane);
@@ -520,19 +594,20 @@ __device__ __forceinline__ void reverse_pairs(const ScanArgs& a, unsigned smem, 
     clear(carry);
     Rotation rot;
 
-    struct Rows { bool hasA, hasB, row0, pullA, pullB, push, top, bottom; int pix; };   // pix: memory pixel of column W-1 of row A
+    struct Rows { bool hasA, hasB, row0, pullA, pullB, push, top, bottom; int pix, edge; };   // pix: memory pixel of column W-1 of row A; edge: CHAIN, block 0 of the boundary row below
     auto make_rows = [&](int bi, int q) {
         Rows w;
         const int i = q * Rb + 2 * r;
-        w.hasA = bi < nb && 2 * r < Rb && i < H;
+        w.hasA = bi < work.nb && 2 * r < Rb && i < H;
         w.hasB = w.hasA && 2 * r + 1 < Rb && i + 1 < H;
         w.row0 = (i == 0);
         w.pullA = w.hasA && (2 * r == Rb - 1) && i + 1 < H;       // pT of the row below comes through the ring
         w.pullB = w.hasB && (2 * r + 1 == Rb - 1) && i + 2 < H;
-        w.push = w.hasA && (r == 0) && (q > 0);       // pT of row A goes to the band above through the ring
+        w.push = w.hasA && (r == 0) && (q > 0) && !(CHAIN && q == a.mute_up);       // pT of row A goes to the band above through the ring
         w.top = w.hasA && (r == 0) && (i > 0);        // h of the row above is not requested by a warp of this band
         w.bottom = i + 2 >= H;                        // nothing below row B
-        w.pix = scan_pixel(a, img0 + bi * img_stride, i, W - 1);
+        w.pix = scan_pixel(a, work.img0 + bi * work.img_stride, i, W - 1);
+        w.edge = CHAIN ? q * W : 0;
         return w;
     };
     const int down = dir * W;                         // from a pixel to the one below it
@@ -543,7 +618,7 @@ __device__ __forceinline__ void reverse_pairs(const ScanArgs& a, unsigned smem, 
     // What is requested next: cell (B, s_j), below pixel s_pixL of row A, by the upper half of the warp, cell (A, s_j + 1), at
     // s_pixA, by the lower one, each at its s_pix.
     bool s_on = false, s_hasA, s_hasB, s_pullB, t_pullA = false, t_top = false;
-    int s_pix = 0, s_pixL, s_pixA = 0, s_j = W - 1;
+    int s_pix = 0, s_pixL, s_pixA = 0, s_j = W - 1, s_edge = 0, t_edge = 0;
     auto request = [&](auto tag) {
         constexpr bool FAST = decltype(tag)::value;       // both rows exist, and s_j > 0
         copy.issue(stage_w + rot.wr, FAST || s_on, s_pix, E);
@@ -551,8 +626,8 @@ __device__ __forceinline__ void reverse_pairs(const ScanArgs& a, unsigned smem, 
         if (FAST || s_hasA) request_record<rec_t>(blk + kHA + rot.wr, ph);
         if (FAST || (s_hasB && s_j > 0)) request_record<rec_t>(blk + kHB + rot.wr, ph + (ptrdiff_t)(down - dir) * HB);
         if (t_top) request_record<rec_t>(blk + kUp + rot.wr, hs_img + (ptrdiff_t)(s_pixA - down) * HB);
-        if (s_pullB) cp_async_block(blk + kBwdBlock + rot.wr, ring + s_j * kSlotF4);
-        if (!FAST && t_pullA) cp_async_block(blk + kBwdBlock + rot.wr, ring + (s_j == W - 1 ? 0 : s_j + 1) * kSlotF4);
+        if (s_pullB) cp_async_block(blk + kBwdBlock + rot.wr, ring + (s_edge + s_j) * kSlotF4);
+        if (!FAST && t_pullA) cp_async_block(blk + kBwdBlock + rot.wr, ring + (t_edge + (s_j == W - 1 ? 0 : s_j + 1)) * kSlotF4);
         s_pix -= dir;
         s_pixL -= dir;
         s_pixA -= dir;
@@ -560,18 +635,23 @@ __device__ __forceinline__ void reverse_pairs(const ScanArgs& a, unsigned smem, 
     };
     auto lead = [&](const Rows& w) {
         s_hasA = w.hasA; s_hasB = w.hasB; s_pullB = w.pullB; s_pixL = w.pix; s_j = W - 1;
+        if (CHAIN) s_edge = w.edge;
         if (upper) { s_on = w.hasB; s_pix = w.pix + down; }
     };
     auto trail = [&](const Rows& w) {
         t_pullA = w.pullA; t_top = w.top; s_pixA = w.pix;
+        if (CHAIN) t_edge = w.edge;
         if (!upper) { s_on = w.hasA; s_pix = w.pix; }
     };
 
-    bool hasA = false, hasB = false, row0 = false, pullA = false, push = false;
-    int pixA = 0, pixB = 0;
+    bool hasA = false, hasB = false, row0 = false, pullA = false, pullB = false, push = false, given_up = false;
+    int pixA = 0, pixB = 0, edgeA = 0, edgeB = 0;
     auto step = [&](auto tag, const int j, const int jA) {
         constexpr int KIND = decltype(tag)::value;
         constexpr bool FAST = KIND <= kTop, ALL = KIND != kPartial;
+        if (CHAIN && (pullB || (!ALL && pullA)))
+            wait_for_block(a, blk + kBwdBlock + rot.rd, ring + (pullB ? edgeB + j : edgeA + jA) * kSlotF4, given_up);
+        const unsigned flip = CHAIN && pullB ? 0xffffffffu : 0u;
         float2 o_dT[2], o_dL[2], o_dx[2];
 #pragma unroll
         for (int w = 0; w < 2; ++w) {
@@ -615,9 +695,14 @@ __device__ __forceinline__ void reverse_pairs(const ScanArgs& a, unsigned smem, 
                 lds_in4<float>(aL, params + 1024 + c * 512);
                 if (!NO_T) lds_record<rec_t>(ht, blk + rot.rd + (w ? kHA : kUp), c);
                 lds_record<rec_t>(hl, blk + rot.rd + (w ? kHB : kHA), c);
-                if (w) lds_in4<float>(pd, blk + kBwdBlock + rot.rd + c * 512);
-                else { pd[0] = carry[c][0]; pd[1] = carry[c][1]; }
-                if (!ALL && w == 0 && pullA) lds_in4<float>(pd, blk + kBwdBlock + rot.rd + c * 512);
+                if (w) {
+                    lds_in4<float>(pd, blk + kBwdBlock + rot.rd + c * 512);
+                    if (CHAIN) { pd[0] = flip_bits(pd[0], flip); pd[1] = flip_bits(pd[1], flip); }
+                } else { pd[0] = carry[c][0]; pd[1] = carry[c][1]; }
+                if (!ALL && w == 0 && pullA) {
+                    lds_in4<float>(pd, blk + kBwdBlock + rot.rd + c * 512);
+                    if (CHAIN) { pd[0] = flip_bits(pd[0], 0xffffffffu); pd[1] = flip_bits(pd[1], 0xffffffffu); }
+                }
                 if (!FAST) {
 #pragma unroll
                     for (int k = 0; k < 2; ++k) {
@@ -650,7 +735,11 @@ __device__ __forceinline__ void reverse_pairs(const ScanArgs& a, unsigned smem, 
                 else if (!NO_T) {
                     // pT of row A goes to the row above: through its slot, and the ring when that row is in another band
                     sts4(blk + rot.ho + c * 512, quad_f4(pd));
-                    if (push) __stcg(ring + jA * kSlotF4 + c * 32, quad_f4(pd));
+                    if (push) {
+                        float4* const up = ring + (edgeA - (CHAIN ? W : 0) + jA) * kSlotF4 + c * 32;
+                        if (CHAIN) __stcg(reinterpret_cast<uint4*>(up), invert_bits(quad_f4(pd)));
+                        else __stcg(up, quad_f4(pd));
+                    }
                 }
                 sTs[c] = sT.x + sT.y; sLs[c] = sL.x + sL.y;
                 qTs[c] = qT.x + qT.y; qLs[c] = qL.x + qL.y;
@@ -678,9 +767,9 @@ __device__ __forceinline__ void reverse_pairs(const ScanArgs& a, unsigned smem, 
     // ---- the warp's sequence ---------------------------------------------------------------------
     // 2rr idle steps (in the last of them the right-most state block of row B is requested for the warp below), two steps
     // that only request, W steps per band, one for the last cell of row A, and idle steps until the last warp is done
-    Rows cur = make_rows(0, nbands - 1);
-    int bi = 0, q = nbands - 1;
-    const int items = nb * nbands;
+    const int items = work.items, q_last = CHAIN ? work.q0 + (items - 1) * work.dq : nbands - 1;
+    int bi = 0, q = q_last;
+    Rows cur = make_rows(bi, q);
     for (int k = 0; k < 2 * rr; ++k) {
         if (k == 2 * rr - 1) request_row_end(cur);
         rot.end_step();
@@ -692,8 +781,10 @@ __device__ __forceinline__ void reverse_pairs(const ScanArgs& a, unsigned smem, 
     request(std::false_type{});
     rot.end_step();
     for (int m = 0; m <= items; ++m) {
-        if (--q < 0) { q = nbands - 1; ++bi; }                // (bi, q): the next item; nothing exists past the last one
+        if ((q -= work.dq) < 0) { q = q_last; ++bi; }         // (bi, q): the next item; nothing exists past the last one
         hasB = cur.hasB;
+        pullB = cur.pullB;
+        if (CHAIN) edgeB = cur.edge;
         if (cur.bottom && cur.hasB)                           // nothing arrives from below: B's cells read zeros from S
 #pragma unroll
             for (int k = 0; k < 6; ++k) sts4(blk + kBwdBlock + k * 512, make_float4(0.f, 0.f, 0.f, 0.f));
@@ -736,6 +827,7 @@ __device__ __forceinline__ void reverse_pairs(const ScanArgs& a, unsigned smem, 
                 hasA = cur.hasA;
                 row0 = cur.row0;
                 pullA = cur.pullA;
+                if (CHAIN) edgeA = cur.edge;
                 push = cur.push;
                 pixA = cur.pix;
                 clear(pLA);

@@ -6,6 +6,7 @@ import pytest
 import torch
 
 from mamba2d_b200 import _lib, scan_bwd, scan_fwd
+from mamba2d_b200 import wavefront_cuda as wc
 from oracle import cpu, inputs
 from helpers import rel_err
 
@@ -28,11 +29,20 @@ SHAPES = [
 @pytest.mark.parametrize("dt,tol", [(torch.float32, 1e-4), (torch.bfloat16, 2e-2)])
 @pytest.mark.parametrize("reverse", [False, True])
 def test_batch_kernels_against_the_oracle(shape, dt, tol, reverse):
+    assert _chains(shape) == (1, 1)
+    _check(shape, 1, dt, tol, reverse)
+
+
+def _chains(shape):
     d = _lib.ScanDesc()
     d.struct_bytes = ctypes.sizeof(d)
     d.B, d.H, d.W, d.E, d.N = shape
     d.BT_pitch = d.BL_pitch = d.C_pitch = shape[4]
-    assert (_lib.lib().m2d_scan_fwd_chain(ctypes.byref(d)), _lib.lib().m2d_scan_bwd_chain(ctypes.byref(d))) == (1, 1)
+    return _lib.lib().m2d_scan_fwd_chain(ctypes.byref(d)), _lib.lib().m2d_scan_bwd_chain(ctypes.byref(d))
+
+
+def _check(shape, chain, dt, tol, reverse):
+    assert _chains(shape)[1] == chain
     inp = inputs.make_inputs(*shape, seed=sum(shape), strided_bc=True)
     inp = {k: v.to(dt).float() for k, v in inp.items()}
     dev = {k: v.cuda().to(dt) for k, v in inp.items()}
@@ -46,3 +56,39 @@ def test_batch_kernels_against_the_oracle(shape, dt, tol, reverse):
     want = cpu.backward(ref, mode="f64")
     for name, t in zip(cpu.GRAD_NAMES, grads):
         assert rel_err(t.float().cpu().numpy(), back(want[name])) < tol, name
+
+
+# the same sweeps with the bands of an image in several CTAs, backward only: an image's bands in one round and in two, an odd
+# last band, ragged channels
+CHAINED = [((40, 56, 56, 64, 16), 3), ((4, 64, 48, 320, 16), 3), ((2, 75, 80, 500, 12), 4), ((9, 61, 60, 130, 5), 3)]
+
+
+@pytest.mark.parametrize("shape,chain", CHAINED)
+@pytest.mark.parametrize("dt,tol", [(torch.float32, 1e-4), (torch.bfloat16, 2e-2)])
+@pytest.mark.parametrize("reverse", [False, True])
+def test_chained_sweeps_against_the_oracle(shape, chain, dt, tol, reverse):
+    _check(shape, chain, dt, tol, reverse)
+
+
+@pytest.mark.parametrize("hook", [_lib.M2D_SCAN_TEST_WITHHOLD, _lib.M2D_SCAN_TEST_WITHHOLD_UP])
+def test_waits_of_chained_sweeps_give_up(hook, monkeypatch):
+    """A band that hands nothing on: the launch ends, says so, and the next one is right."""
+    monkeypatch.setenv("M2D_TEST_HOOKS", "1")
+    shape = (4, 64, 48, 320, 16)
+    dev = {k: v.cuda() for k, v in inputs.make_inputs(*shape, seed=3).items()}
+    want = scan_bwd(*[dev[k] for k in ORDER], dev["gy"])
+    d, keep = wc._make_desc(*[dev[k] for k in ORDER])
+    d.flags = hook
+    L = _lib.lib()
+    d.gy = dev["gy"].data_ptr()
+    outs = [torch.zeros_like(t) for t in want]
+    for name, t in zip(("d_x", "d_dT", "d_dL", "d_AT", "d_AL", "d_BT", "d_BL", "d_C", "d_D"), outs):
+        setattr(d, name, t.data_ptr())
+    wc._workspace(d, L.m2d_scan_bwd_workspace(ctypes.byref(d)), dev["x"].device, keep)
+    assert L.m2d_scan_bwd(ctypes.byref(d), ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)) == 0
+    torch.cuda.synchronize()
+    assert wc._status_word(keep[-1], L.m2d_scan_bwd_status_offset(ctypes.byref(d))) != 0
+    assert torch.isnan(outs[1]).any()                        # (d_deltaT: a row that never came reads as NaN)
+    again = scan_bwd(*[dev[k] for k in ORDER], dev["gy"])
+    for a, b in zip(again, want):
+        assert float((a - b).abs().max()) <= 1e-5 * float(b.abs().max())
