@@ -86,7 +86,7 @@ inline BwdPlan make_plan_bwd(const m2d_scan_desc* d) {
     double adjoint = 0.0, states = 0.0;
     const Plan pa = plan_pair_chain(d, kPairAdjoint, &adjoint), ps = plan_pair_chain(d, kPairStates, &states);
     const double chained = adjoint + states + (pa.warps && ps.warps ? (pair_edge_bytes(d, pa) + pair_edge_bytes(d, ps)) / 5e6 : 1e30);    // (and clearing)
-    if (chained < kChainShare * wave && chained < 0.9 * best) {
+    if (chained < kChainShare * wave && chained < kChainShareOfBatch * best) {
         static_cast<Plan&>(p) = pa;
         p.states = ps;
         p.wide = true;

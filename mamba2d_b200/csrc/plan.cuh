@@ -179,6 +179,10 @@ inline double pair_chain_time(const m2d_scan_desc* d, const Plan& p, PairKernel 
 // 2x200x336x64 bf16 982 / 1079 (0.97): a step of these kernels takes longer where it is the chain that bounds.  (In the
 // forward 16x100x112x64 gains 270 / 219; not taken.)
 constexpr double kChainShare = 0.80;
+// ... and to less than this share of one CTA per image, whose estimate is high by about as much as this one is low.  Backward, us,
+// one CTA per image / chained, without clearing: 20x45x31x192 bf16 294 / 332 (0.87), 32x56x56x64 fp32 424 / 414 (0.73),
+// 48x64x80x64 bf16 947 / 809 (0.65), 40x100x120x64 fp32 2258 / 1797 (0.63).
+constexpr double kChainShareOfBatch = 0.70;
 
 // Every number of warps is tried; the plan with the least time is kept (in *time, us).
 inline Plan plan_pairs(const m2d_scan_desc* d, PairKernel k, double* time) {

@@ -60,7 +60,7 @@ def _check(shape, chain, dt, tol, reverse):
 
 # the same sweeps with the bands of an image in several CTAs, backward only: an image's bands in one round and in two, an odd
 # last band, ragged channels
-CHAINED = [((40, 56, 56, 64, 16), 3), ((4, 64, 48, 320, 16), 3), ((2, 75, 80, 500, 12), 4), ((9, 61, 60, 130, 5), 3)]
+CHAINED = [((40, 56, 56, 64, 16), 3), ((4, 70, 64, 320, 16), 3), ((2, 75, 80, 500, 12), 4), ((9, 61, 60, 130, 5), 3)]
 
 
 @pytest.mark.parametrize("shape,chain", CHAINED)
@@ -74,7 +74,7 @@ def test_chained_sweeps_against_the_oracle(shape, chain, dt, tol, reverse):
 def test_waits_of_chained_sweeps_give_up(hook, monkeypatch):
     """A band that hands nothing on: the launch ends, says so, and the next one is right."""
     monkeypatch.setenv("M2D_TEST_HOOKS", "1")
-    shape = (4, 64, 48, 320, 16)
+    shape = (4, 70, 64, 320, 16)
     dev = {k: v.cuda() for k, v in inputs.make_inputs(*shape, seed=3).items()}
     want = scan_bwd(*[dev[k] for k in ORDER], dev["gy"])
     d, keep = wc._make_desc(*[dev[k] for k in ORDER])
