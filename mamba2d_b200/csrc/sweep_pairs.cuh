@@ -22,13 +22,14 @@
 // A band boundary must be written at least two steps before the band below reads it: the plan keeps Rb <= W - 2.
 //
 // Against one row of 32 channels per warp, a lane 4 x 4 of it (us, kernel times, before / now): 128x56x56x64 fp32 forward
-// 364 / 321, backward 1400 / 507 + 682 (its two sweeps are kernels of their own now); 128x28x28x128 bf16 190 / 172 and
-// 656 / 186 + 403; 128x14x14x320 bf16 129 / 123 and 403 / 142 + 253; 128x7x7x512 fp32 64 / 55 and 199 / 64 + 117.  Instructions
+// 364 / 312, backward 1400 / 507 + 684 (its two sweeps are kernels of their own now); 128x28x28x128 bf16 190 / 171 and
+// 656 / 183 + 402; 128x14x14x320 bf16 129 / 121 and 403 / 137 + 252; 128x7x7x512 fp32 64 / 52 and 199 / 63 + 116.  Instructions
 // per 512 states (56x56x64 fp32): forward 224 -> 202, both sweeps of the backward 803 -> 232 + 500; wavefronts of the
 // shared-memory pipe, which was half busy, 250 -> 56 + 152.  What bounds them now: the forward and the adjoint the latency of
 // a warp's instructions at 16 warps per SM (128 registers; an instruction every 2.0 and 1.7 cycles of a scheduler), and
 // that 512 CTAs put four on some SMs and three on others; the recompute sweep in fp32 the writing of the record (2.5 GB
-// through DRAM in 507 us; with a bf16 record, 373).  Blocks of one anti-diagonal side by side in the record, and inputs
+// through DRAM in 507 us; with a bf16 record, 369).  Blocks of one anti-diagonal side by side in the record, blocks copied out
+// of shared memory in bulk (505 / 509, 231 / 245 at 28x28x128), and inputs
 // requested into L2 four columns ahead, did not change the last.
 #pragma once
 
@@ -411,13 +412,10 @@ __device__ __forceinline__ void forward_pairs(const ScanArgs& a, unsigned smem, 
         const unsigned flip = pulled ? 0xffffffffu : 0u;
         Quad dC[2];
         float2 yv[2];
-        Quad topB[2];
+        // B first: what is above it is A's state of the last step, still in place (A first, with a copy of it, 320 us against 312 at
+        // 128x56x56x64 fp32, 55 against 52 at 7x7x512; both cells read before either is computed, 315 and 54)
 #pragma unroll
-        for (int c = 0; c < 2; ++c)
-#pragma unroll
-            for (int k = 0; k < 2; ++k) topB[c][k] = hA[c][k];
-#pragma unroll
-        for (int w = 0; w < 2; ++w) {
+        for (int w = 1; w >= 0; --w) {
             Quad (&h)[2] = w ? hB : hA;
             const bool NO_T = KIND == kTop && w == 0;         // (a constant: the loop is unrolled)
             yv[w] = dC[w][0] = dC[w][1] = make_float2(0.f, 0.f);
@@ -443,7 +441,7 @@ __device__ __forceinline__ void forward_pairs(const ScanArgs& a, unsigned smem, 
 #pragma unroll
             for (int c = 0; c < 2; ++c) {
                 Quad top;
-                if (w) { top[0] = topB[c][0]; top[1] = topB[c][1]; }
+                if (w) { top[0] = hA[c][0]; top[1] = hA[c][1]; }
                 else if (!NO_T) {
                     lds_in4<float>(top, blk + rot.rd + c * 512);
                     if (CHAIN) { top[0] = flip_bits(top[0], flip); top[1] = flip_bits(top[1], flip); }
