@@ -48,10 +48,10 @@ METRIC = "2D-scan fwd+bwd elements/s"
 UNIT = "elements/s"
 BYTES = {"f32": 4, "bf16": 2}
 
-# DRAM bytes (read + write) of ONE launch of the dominant kernel, from an ncu capture of this same
+# DRAM bytes (read + write) of the backward's two kernels, once each, from an ncu capture of this same
 # workload; see profiles/ for the capture summaries.  None = not captured for that dtype.
-NCU_TRAFFIC = {"f32": 6.064e9, "bf16": 3.696e9}
-NCU_TRAFFIC_FROM = "538d212"  # the commit whose kernels were captured
+NCU_TRAFFIC = {"f32": 5.54e9, "bf16": None}
+NCU_TRAFFIC_FROM = "c65fd61"  # the commit whose kernels were captured
 
 
 def fwd_bytes(D, HW, s, B=BATCH, N=NSTATE):
@@ -264,9 +264,9 @@ def summarise(dtype, r, world, steps):
                 "d2h_bytes_per_step": e["d2h"], "steps": e["steps"], "gpu_launches": e["launches"],
                 "note": "HostScanPipeline: pinned host inputs -> device, fwd+bwd, y and all nine gradients -> pinned host, "
                         "every step; copy-in / kernels / copy-out of consecutive calls overlap on three streams"},
-        # per shape: forward kernel, backward kernel (+ cast kernel for bf16)
-        "gpu_launches": steps * len(STAGES) * (2 if dtype == "f32" else 3),
-        "roofline": {"bound": "hbm", "kernel": "m2d_bwd_kernel @ D=64,H=W=56,B=128", "achieved": dom_bytes / dom["bwd_ms"] / 1e6,
+        # per shape: forward kernel, the backward's two (+ cast kernel for bf16)
+        "gpu_launches": steps * len(STAGES) * (3 if dtype == "f32" else 4),
+        "roofline": {"bound": "hbm", "kernel": "m2d_bwd_states_kernel + m2d_bwd_kernel @ D=64,H=W=56,B=128", "achieved": dom_bytes / dom["bwd_ms"] / 1e6,
                      "peak": peak, "unit": "GB/s", "frac": dom_bytes / dom["bwd_ms"] / 1e6 / peak,
                      "peak_kind": peak_kind, "algorithmic_bytes": dom_bytes, "ms": dom["bwd_ms"],
                      "traffic": NCU_TRAFFIC[dtype], "traffic_from_commit": NCU_TRAFFIC_FROM if NCU_TRAFFIC[dtype] else None},

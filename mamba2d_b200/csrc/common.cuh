@@ -122,9 +122,9 @@ __host__ __device__ inline size_t pairs_bwd_smem_bytes(int warps) { return (size
 
 // Host-side launch plan shared by the workspace queries and the launches.
 struct Plan {
-    int groups;        // ceil(E / 32)
-    int warps;         // row-warps per CTA
-    int Rb;            // rows per band (<= warps)
+    int groups;        // ceil(E / channels of a CTA)
+    int warps;         // warps per CTA
+    int Rb;            // rows per band
     int nbands;        // ceil(H / Rb)
     int grid_x;        // image chains per channel group; chain k walks images k, k + grid_x, ...
     int chain;         // CTAs per chain (> 1 when there are far fewer images than SMs)
