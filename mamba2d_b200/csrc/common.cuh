@@ -70,23 +70,10 @@ __device__ __forceinline__ unsigned pack_bf16x2(float lo, float hi) {
     asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(hi), "f"(lo));
     return r;
 }
-// ---- input staging in shared memory ------------------------------------------------------------
-// Per warp and parity: 44 slots of 16 bytes: x[8] dT[8] dL[8] gy[8] (one slot per 4-channel block)
-// then BT[4] BL[4] C[4] (one slot per 4-state block).  A slot holds four elements of the I/O type
-// (fp32: 16 bytes, bf16: the first 8 bytes).
+// ---- input staging in shared memory (batch kernels) ------------------------------------------------
+// A cell: 28 slots of 16 bytes, x[4] dT[4] dL[4] gy[4] (one slot per four channels), BT[4] BL[4] C[4] (one slot per four
+// states).  A slot holds four elements of the I/O type (fp32: 16 bytes, bf16: the first 8 bytes).
 constexpr int kCellSlots = 28;
-constexpr int kStageBytes = 2 * kCellSlots * 16;
-
-// Read a staged slot back as four floats.
-template <typename io_t> __device__ __forceinline__ float4 unstage4(const char* slot);
-template <> __device__ __forceinline__ float4 unstage4<float>(const char* slot) {
-    return *reinterpret_cast<const float4*>(slot);
-}
-template <> __device__ __forceinline__ float4 unstage4<__nv_bfloat16>(const char* slot) {
-    const uint2 u = *reinterpret_cast<const uint2*>(slot);
-    return make_float4(__uint_as_float(u.x << 16), __uint_as_float(u.x & 0xffff0000u),
-                       __uint_as_float(u.y << 16), __uint_as_float(u.y & 0xffff0000u));
-}
 
 // ---- scalar element loads / stores --------------------------------------------------------------
 __device__ __forceinline__ float bf16_bits_to_float(unsigned short b) { return __uint_as_float(static_cast<unsigned>(b) << 16); }
