@@ -253,8 +253,8 @@ int m2d_scan_bwd(const m2d_scan_desc *desc, void *stream);
  *   - The array is M2D_NOALLOC_SCRATCH_BYTES (32 MiB) and every GPU that loads the library keeps
  *     it until the process exits.
  *   - A problem needing more scratch than that returns M2D_ERR_TOO_LARGE before any device work.
- *     m2d_scan_fwd_noalloc_need() reports the need.  A problem that m2d_scan_fwd would split over
- *     several CTAs per image runs with one where only that fits the array.
+ *     m2d_scan_fwd_noalloc_need() reports the need.  A problem whose m2d_scan_fwd needs more
+ *     runs as the fastest launch that fits the array: fewer CTAs, longer bands, one CTA per image.
  *   - All calls on a device share the array.  The call clears the one word that must start at
  *     zero itself, but calls that overlap in time on one GPU race on the array: keep them on one
  *     stream or order them with events.

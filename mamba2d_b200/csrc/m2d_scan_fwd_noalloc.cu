@@ -52,11 +52,11 @@ static int ring_address(float4** out) {
     return M2D_OK;
 }
 
-// The plan of the regular entry where its scratch fits the array, else one CTA per (image, channel group),
-// which needs the per-CTA rings only.
+// The plan of the regular entry where its scratch fits the array, else the fastest that does: fewer CTAs with more warps and
+// longer bands, or no chains of CTAs.
 static Plan plan_noalloc(const m2d_scan_desc* d) {
     const Plan p = plan_fwd(d);
-    return p.scratch <= M2D_NOALLOC_SCRATCH_BYTES ? p : plan_fwd(d, false);
+    return p.scratch <= M2D_NOALLOC_SCRATCH_BYTES ? p : make_plan_fwd(d, M2D_NOALLOC_SCRATCH_BYTES);
 }
 
 }  // namespace m2d

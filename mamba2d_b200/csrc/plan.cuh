@@ -184,9 +184,17 @@ constexpr double kChainShare = 0.80;
 // 48x64x80x64 bf16 947 / 809 (0.65), 40x100x120x64 fp32 2258 / 1797 (0.63).
 constexpr double kChainShareOfBatch = 0.70;
 
-// Every number of warps is tried; the plan with the least time is kept (in *time, us).
-inline Plan plan_pairs(const m2d_scan_desc* d, PairKernel k, double* time) {
+// Bytes of the rings that carry a band's last row to the next band.
+inline size_t pair_ring_bytes(const m2d_scan_desc* d, const Plan& p) {
+    return p.nbands > 1 ? (size_t)p.grid_x * p.groups * d->W * kSlotF4 * sizeof(float4) : 0;
+}
+
+// Every number of warps is tried; of the plans whose rings take at most `ring_limit` bytes the one with the least time is kept
+// (in *time, us).  Fewer warps are more bands, more CTAs and more rings: 18x6x593x892 needs 612 MB of them with one warp per
+// CTA and none with three.  Where no plan has room, the one with the smallest rings.
+inline Plan plan_pairs(const m2d_scan_desc* d, PairKernel k, double* time, size_t ring_limit = SIZE_MAX) {
     Plan best{};
+    size_t best_over = 0;
     const int sms = sm_count();
     for (int nw = kPairWarps; nw >= 1; --nw) {
         Plan p{};
@@ -205,7 +213,8 @@ inline Plan plan_pairs(const m2d_scan_desc* d, PairKernel k, double* time) {
         p.grid_x = (d->B - 1) / per + 1;
         p.chain = 1;
         const double t = pair_time(d, p, k, per_sm, sms);
-        if (best.warps == 0 || t < *time) { best = p; *time = t; }
+        const size_t ring = pair_ring_bytes(d, p), over = ring > ring_limit ? ring : 0;
+        if (best.warps == 0 || over < best_over || (over == best_over && t < *time)) { best = p; best_over = over; *time = t; }
     }
     return best;
 }
@@ -232,10 +241,6 @@ inline Plan plan_pair_chain(const m2d_scan_desc* d, PairKernel k, double* time) 
 }
 inline size_t pair_edge_bytes(const m2d_scan_desc* d, const Plan& p) {
     return align256((size_t)d->B * p.groups * p.nbands * d->W * kSlotF4 * sizeof(float4));
-}
-// Bytes of the rings that carry a band's last row to the next band.
-inline size_t pair_ring_bytes(const m2d_scan_desc* d, const Plan& p) {
-    return p.nbands > 1 ? (size_t)p.grid_x * p.groups * d->W * kSlotF4 * sizeof(float4) : 0;
 }
 
 // Scratch layout shared by every entry point: [status word, 256 bytes][the rest].
@@ -310,30 +315,37 @@ struct LastPlan {
     }
 };
 
-inline Plan make_plan_fwd(const m2d_scan_desc* d, bool allow_chain) {
+// The fastest plan, or with a `scratch_limit` the fastest that fits it; where none does, one that says how much it needs.
+inline Plan make_plan_fwd(const m2d_scan_desc* d, size_t scratch_limit = SIZE_MAX) {
     // The batch kernel runs one CTA per (image, 16 channels) and is at its best when those fill the GPU; the wave kernels
     // split an image over CTAs as well.  Measured times per step of those: 0.62 us with four channels per lane, 0.42 us
     // with two and twice the CTAs.  The batch kernel needs three columns.
     Plan p{};
     double best = 1e30;
     if (d->W >= 3) {
-        p = plan_pairs(d, kPairForward, &best);
+        p = plan_pairs(d, kPairForward, &best, scratch_limit - kStatusBytes);
         best *= kWaveMargin;
         p.scratch = kStatusBytes + align256(pair_ring_bytes(d, p));
     }
+    auto consider = [&](Plan w, double step) {
+        const double t = step * wave_steps(d, w);
+        w.scratch = kStatusBytes + wave_edge_bytes(d, w, false);
+        const bool room = w.scratch <= scratch_limit, had = best < 1e30 && p.scratch <= scratch_limit;
+        if (best == 1e30 || (room && (!had || t < best))) { best = t; p = w; }
+    };
     for (const int C : {4, 2}) {
-        if (!allow_chain && d->W >= 3) break;
         Plan w = plan_wave(d, C);
-        if (!allow_chain) w.chain = 1;
-        const double t = (C == 4 ? 0.62 : 0.42) * wave_steps(d, w);
-        if (t < best) { best = t; p = w; p.scratch = kStatusBytes + wave_edge_bytes(d, w, false); }
+        consider(w, C == 4 ? 0.62 : 0.42);
+        if (scratch_limit == SIZE_MAX || w.chain == 1) continue;
+        w.chain = 1;                     // (two boundary rows in turn, instead of one per band)
+        consider(w, C == 4 ? 0.62 : 0.42);
     }
     return p;
 }
 
-inline Plan plan_fwd(const m2d_scan_desc* d, bool allow_chain = true) {
+inline Plan plan_fwd(const m2d_scan_desc* d) {
     static thread_local LastPlan<Plan> last;
-    return allow_chain ? last.get(d, [&] { return make_plan_fwd(d, true); }) : make_plan_fwd(d, false);
+    return last.get(d, [&] { return make_plan_fwd(d); });
 }
 
 }  // namespace m2d

@@ -64,3 +64,31 @@ def test_noalloc_rejects_problems_beyond_its_capacity():
         setattr(d, name, fake)
     assert L.m2d_scan_fwd_noalloc(ctypes.byref(d), None) == -9
     assert "capacity" in _lib.strerror(-9)
+
+
+# Shapes whose fastest plan needs more scratch than the array holds, and some other plan does not: fewer CTAs of more warps
+# where bands are short and images many, no chain of CTAs, and the wave kernels' boundary rows where channels are few.
+TIGHT = [(105, 16, 16, 320, 16), (90, 20, 31, 320, 16), (18, 6, 593, 892, 5), (12, 1505, 62, 1216, 5), (200, 20, 170, 1, 4), (346, 127, 347, 2, 5),
+         (128, 32, 50, 128, 16), (570, 48, 24, 441, 5)]
+
+
+@pytest.mark.parametrize("shape", TIGHT)
+@pytest.mark.parametrize("dtype", [_lib.M2D_F32, _lib.M2D_BF16])
+def test_noalloc_takes_a_plan_that_fits(shape, dtype):
+    L = _lib.lib()
+    d = _lib.ScanDesc()
+    d.struct_bytes = ctypes.sizeof(_lib.ScanDesc)
+    d.dtype = dtype
+    d.B, d.H, d.W, d.E, d.N = shape
+    d.BT_pitch = d.BL_pitch = d.C_pitch = d.N
+    assert 256 <= L.m2d_scan_fwd_noalloc_need(ctypes.byref(d)) <= _lib.NOALLOC_SCRATCH_BYTES
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("shape", [TIGHT[0], TIGHT[4]])
+@pytest.mark.parametrize("kind,tol", [(torch.float32, 1e-4), (torch.bfloat16, 2e-2)])
+def test_noalloc_with_a_plan_of_its_own(shape, kind, tol):
+    dev = {k: v.to("cuda", kind) for k, v in inputs.make_inputs(*shape, seed=15).items()}
+    want = wc.scan_fwd(*[dev[k] for k in ORDER])
+    got = _call_noalloc(dev)
+    assert float((got.float() - want.float()).abs().max()) <= tol * float(want.float().abs().max())
