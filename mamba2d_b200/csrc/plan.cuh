@@ -1,6 +1,7 @@
 // Host-side descriptor validation and launch planning (header-only, used by both entry points).
 #pragma once
 
+#include <algorithm>
 #include <array>
 #include <atomic>
 #include <cstdlib>
@@ -189,10 +190,14 @@ inline size_t pair_ring_bytes(const m2d_scan_desc* d, const Plan& p) {
     return p.nbands > 1 ? (size_t)p.grid_x * p.groups * d->W * kSlotF4 * sizeof(float4) : 0;
 }
 
+// Rings beyond this (three quarters of the L2) also cost the trip to DRAM that pair_time leaves out: such a plan is taken only where every
+// other has as large ones.
+constexpr size_t kRingBytes = 96u << 20;
+
 // Every number of warps is tried; of the plans whose rings take at most `ring_limit` bytes the one with the least time is kept
 // (in *time, us).  Fewer warps are more bands, more CTAs and more rings: 18x6x593x892 needs 612 MB of them with one warp per
 // CTA and none with three.  Where no plan has room, the one with the smallest rings.
-inline Plan plan_pairs(const m2d_scan_desc* d, PairKernel k, double* time, size_t ring_limit = SIZE_MAX) {
+inline Plan plan_pairs(const m2d_scan_desc* d, PairKernel k, double* time, size_t ring_limit = kRingBytes) {
     Plan best{};
     size_t best_over = 0;
     const int sms = sm_count();
@@ -323,7 +328,7 @@ inline Plan make_plan_fwd(const m2d_scan_desc* d, size_t scratch_limit = SIZE_MA
     Plan p{};
     double best = 1e30;
     if (d->W >= 3) {
-        p = plan_pairs(d, kPairForward, &best, scratch_limit - kStatusBytes);
+        p = plan_pairs(d, kPairForward, &best, std::min(kRingBytes, scratch_limit - kStatusBytes));
         best *= kWaveMargin;
         p.scratch = kStatusBytes + align256(pair_ring_bytes(d, p));
     }

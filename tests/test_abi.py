@@ -96,6 +96,15 @@ def test_scratch_of_few_images_is_bounded(L, B, H, W, E, dtype):
     assert L.m2d_scan_bwd_workspace(d) <= record + 2 * boundary + sums + slack
 
 
+@pytest.mark.parametrize("B,H,W,E,N", [(564, 3, 2984, 392, 16), (427, 8, 1611, 74, 16), (43, 3, 2615, 879, 5), (18, 6, 593, 892, 5), (72, 33, 327, 351, 16)])
+def test_rings_stay_small_where_some_plan_has_small_ones(L, B, H, W, E, N):
+    """A launch of many short bands is not bought with gigabytes of boundary rows; the backward's are beside the record."""
+    d = _desc(B=B, H=H, W=W, E=E, N=N, BT_pitch=N, BL_pitch=N, C_pitch=N)
+    rings = 96 << 20
+    assert L.m2d_scan_fwd_workspace(ctypes.byref(d)) <= 256 + rings
+    assert L.m2d_scan_bwd_workspace(ctypes.byref(d)) <= 256 + rings + B * H * W * ((E + 15) // 16) * 1024
+
+
 def test_plans_do_not_depend_on_the_environment(L, monkeypatch):
     """The workspace query and the launch plan separately; nothing a program can change in between may tell them apart."""
     d = ctypes.byref(_desc(B=128, H=56, W=56))
