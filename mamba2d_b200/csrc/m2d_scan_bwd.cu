@@ -72,6 +72,8 @@ inline BwdLayout bwd_layout(const m2d_scan_desc* d, const BwdPlan& p) {
     return L;
 }
 
+constexpr size_t kLargeScratch = (size_t)4 << 30;
+
 inline BwdPlan make_plan_bwd(const m2d_scan_desc* d) {
     // Batch or wave, as in plan_fwd: 1.2 us per step of both sweeps in the wave kernel with two channels per lane (four
     // spill and are slower at every size measured), whatever the I/O type.
@@ -95,6 +97,15 @@ inline BwdPlan make_plan_bwd(const m2d_scan_desc* d) {
         p.states = ps;
     }
     p.scratch = bwd_layout(d, p).total;
+    // The batch kernels' record holds every image of the call, the wave kernels' those that are under way.  Beyond a few GB a call
+    // that the wave kernels are for (few_images) keeps to theirs where it is less than half: 316x7x9400x71 needs 12 GB there and 106
+    // here, most of the device.
+    if (!p.wave && p.scratch > kLargeScratch && few_images(d)) {
+        BwdPlan q = p;
+        static_cast<Plan&>(q) = w;
+        q.scratch = bwd_layout(d, q).total;
+        if (q.scratch < p.scratch / 2) return q;
+    }
     return p;
 }
 

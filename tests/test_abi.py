@@ -119,6 +119,13 @@ def test_type_of_the_state_record(L, B, H, W, E, chained, few):
         assert bytes_ + sums <= L.m2d_scan_bwd_workspace(ctypes.byref(d)) <= bytes_ + sums + rows + 512
 
 
+@pytest.mark.parametrize("B,H,W,E,dtype,limit", [(316, 7, 9400, 71, _lib.M2D_F32, 12e9), (226, 7, 5000, 100, _lib.M2D_BF16, 8e9)])
+def test_large_calls_keep_to_the_record_of_the_images_under_way(L, B, H, W, E, dtype, limit):
+    """A record of all images would take 106 and 58 GB; the wave kernels' lists of images need one each."""
+    d = ctypes.byref(_desc(B=B, H=H, W=W, E=E, dtype=dtype))
+    assert L.m2d_scan_bwd_workspace(d) <= limit and L.m2d_scan_bwd_chain(d) == 1
+
+
 def test_plans_do_not_depend_on_the_environment(L, monkeypatch):
     """The workspace query and the launch plan separately; nothing a program can change in between may tell them apart."""
     d = ctypes.byref(_desc(B=128, H=56, W=56))
