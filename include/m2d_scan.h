@@ -119,10 +119,13 @@ typedef enum m2d_status {
  * M2D_SCAN_TEST_WITHHOLD_UP (m2d_scan_bwd only): the same in the adjoint sweep, where the last band of every image
  * hands nothing up.
  * M2D_SCAN_TEST_REPORT: with one of the two, the failure also counts for m2d_take_wait_failure().
+ * M2D_SCAN_TEST_SHORT: test hook, under the same variable.  A launch of several CTAs per image is made with half as many, as
+ * where fewer are resident than were planned; its results are those of any other launch.
  */
 #define M2D_SCAN_TEST_WITHHOLD 0x100u
 #define M2D_SCAN_TEST_WITHHOLD_UP 0x200u
 #define M2D_SCAN_TEST_REPORT 0x400u
+#define M2D_SCAN_TEST_SHORT 0x800u
 
 /*
  * Problem descriptor.  Tensor layouts are the ones the reference op receives:

@@ -19,6 +19,7 @@ M2D_SCAN_BC_ZEROED = 0x20
 M2D_SCAN_TEST_WITHHOLD = 0x100
 M2D_SCAN_TEST_WITHHOLD_UP = 0x200
 M2D_SCAN_TEST_REPORT = 0x400
+M2D_SCAN_TEST_SHORT = 0x800
 M2D_PROJ_PARAMS_F32 = 1
 ABI_VERSION = 4
 NOALLOC_SCRATCH_BYTES = 32 << 20     # M2D_NOALLOC_SCRATCH_BYTES in include/m2d_scan.h

@@ -28,6 +28,7 @@ inline void fill_common_args(ScanArgs& a, const m2d_scan_desc* d, const Plan& pl
     a.d_f32 = (d->flags & M2D_SCAN_D_F32) || d->dtype == M2D_F32 ? 1 : 0;
     const bool hook = (d->flags & (M2D_SCAN_TEST_WITHHOLD | M2D_SCAN_TEST_WITHHOLD_UP)) != 0;
     a.withhold = (d->flags & M2D_SCAN_TEST_WITHHOLD) ? 1 : 0;
+    a.shorten = (d->flags & M2D_SCAN_TEST_SHORT) ? 1 : 0;
     a.mute_up = (d->flags & M2D_SCAN_TEST_WITHHOLD_UP) ? pl.nbands - 1 : 0;
     a.wait_limit = hook ? (1 << 9) : kWaitPolls;
     a.host_flag = pl.chain > 1 && (!hook || (d->flags & M2D_SCAN_TEST_REPORT)) ? wait_failure_flag() : nullptr;
@@ -44,7 +45,8 @@ inline int launch_sweep_kernel(void (*kern)(const ScanArgs), ScanArgs& a, const 
     if (a.chain > 1) {
         const int per_sm = resident_ctas(reinterpret_cast<const void*>(kern), (int)block.x, pl.smem);
         if (per_sm < 1) return M2D_ERR_LAUNCH;
-        const long long fit = (long long)per_sm * sm_count() / ((long long)pl.grid_x * pl.groups);
+        long long fit = (long long)per_sm * sm_count() / ((long long)pl.grid_x * pl.groups);
+        if (a.shorten) fit = std::min(fit, (long long)a.chain / 2);
         if (fit < a.chain) a.chain = bound_chain(fit, pl.nbands, a.W, pl.Rb);
         for (;;) {
             const dim3 grid = pl.wave ? dim3(pl.grid_x * a.chain, pl.groups) : dim3(pl.groups, pl.grid_x * a.chain);

@@ -83,7 +83,7 @@ inline int check_desc(const m2d_scan_desc* d, bool bwd, bool need_ptrs) {
     {
         unsigned known = M2D_SCAN_REVERSE | M2D_SCAN_A_LOG | M2D_SCAN_D_F32;
         known |= bwd ? M2D_SCAN_BC_ZEROED : M2D_SCAN_GELU_OUT | M2D_SCAN_WS_CLEARED;      // an output activation exists in the forward only, gradients in the backward
-        const unsigned hooks = M2D_SCAN_TEST_WITHHOLD | M2D_SCAN_TEST_REPORT | (bwd ? M2D_SCAN_TEST_WITHHOLD_UP : 0u);
+        const unsigned hooks = M2D_SCAN_TEST_WITHHOLD | M2D_SCAN_TEST_REPORT | M2D_SCAN_TEST_SHORT | (bwd ? M2D_SCAN_TEST_WITHHOLD_UP : 0u);
         if ((d->flags & hooks) && test_hooks_enabled()) known |= hooks;
         if (d->flags & ~known) return M2D_ERR_FLAGS;
     }

@@ -48,6 +48,7 @@ struct ScanArgs {
     int wait_limit;           // polls before such a wait gives up
     int withhold;             // test hook: the first band of image 0 never hands over its last row
     int mute_up;              // test hook: this band (0: none) hands nothing up in the adjoint sweep
+    int shorten;              // test hook: half as many CTAs per image as planned (host side only)
     int act;                  // forward only: 1 = apply GELU (erf form) to y before it is stored
     int a_log;                // AT / AL hold the fp32 parameter A_log (A = -exp(A_log)); d_AT / d_AL are then fp32 d_A_log
     int d_f32;                // D and d_D are fp32 whatever the I/O type

@@ -99,3 +99,35 @@ def test_waits_of_chained_sweeps_give_up(hook, monkeypatch):
     again = scan_bwd(*[dev[k] for k in ORDER], dev["gy"])
     for a, b in zip(again, want):
         assert float((a - b).abs().max()) <= 1e-5 * float(b.abs().max())
+
+
+@pytest.mark.parametrize("shape,chain", [((4, 70, 64, 320, 16), 3), ((2, 75, 80, 500, 12), 4),      # chained batch sweeps backward
+                                         ((2, 41, 64, 96, 16), 6), ((1, 200, 9, 64, 16), 25)])      # wave kernels, which all take forward
+@pytest.mark.parametrize("dt,tol", [(torch.float32, 1e-4), (torch.bfloat16, 2e-2)])
+def test_launches_with_fewer_ctas_than_planned(shape, chain, dt, tol, monkeypatch):
+    """What a launch does where fewer CTAs are resident than its plan says: half the chain, down to one CTA per image."""
+    monkeypatch.setenv("M2D_TEST_HOOKS", "1")
+    assert _chains(shape)[0] > 1 and _chains(shape)[1] == chain
+    inp = {k: v.to(dt).float() for k, v in inputs.make_inputs(*shape, seed=4).items()}
+    dev = {k: v.cuda().to(dt) for k, v in inp.items()}
+    L = _lib.lib()
+    stream = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    d, keep = wc._make_desc(*[dev[k] for k in ORDER])
+    d.flags = _lib.M2D_SCAN_TEST_SHORT
+    y = torch.full_like(dev["x"], float("nan"))
+    d.y = y.data_ptr()
+    wc._workspace(d, L.m2d_scan_fwd_workspace(ctypes.byref(d)), y.device, keep)
+    assert L.m2d_scan_fwd(ctypes.byref(d), stream) == 0
+    assert rel_err(y.float().cpu().numpy(), cpu.forward(inp, "f64")) < tol
+    want = cpu.backward(inp, mode="f64")
+    outs = [torch.full_like(dev[k], float("nan")) for k in ("x", "dT", "dL", "AT", "AL", "BT", "BL", "C", "D")]
+    for name, t in zip(("d_x", "d_dT", "d_dL", "d_AT", "d_AL", "d_BT", "d_BL", "d_C", "d_D"), outs):
+        setattr(d, name, t.data_ptr())
+    d.gy = dev["gy"].data_ptr()
+    wc._workspace(d, L.m2d_scan_bwd_workspace(ctypes.byref(d)), y.device, keep)
+    assert L.m2d_scan_bwd(ctypes.byref(d), stream) == 0
+    torch.cuda.synchronize()
+    assert wc._status_word(keep[-1], L.m2d_scan_bwd_status_offset(ctypes.byref(d))) == 0
+    got = dict(zip(("d_x", "d_dT", "d_dL", "d_AT", "d_AL", "d_BT", "d_BL", "d_C", "d_D"), outs))
+    for name in cpu.GRAD_NAMES:
+        assert rel_err(got[name].float().cpu().numpy(), want[name]) < tol, name
