@@ -135,6 +135,47 @@ def test_plans_do_not_depend_on_the_environment(L, monkeypatch):
         assert (L.m2d_scan_bwd_workspace(d), L.m2d_scan_fwd_workspace(d)) == before
 
 
+def test_a_kept_plan_is_used_for_its_own_sizes_only(L, monkeypatch):
+    """A thread keeps its last plan of each kind.  Descriptors that differ in one size, asked for in turn, from two threads and under
+    other environments, get what a thread that has kept nothing gets."""
+    import threading
+    base = dict(B=24, H=57, W=50, E=64, N=16, dtype=_lib.M2D_BF16)
+    others = [dict(base, **c) for c in ({}, {"B": 25}, {"H": 58}, {"W": 51}, {"E": 80}, {"N": 12}, {"dtype": _lib.M2D_F32})]
+
+    def ask(c):
+        d = ctypes.byref(_desc(**c))
+        return (L.m2d_scan_fwd_workspace(d), L.m2d_scan_bwd_workspace(d), L.m2d_scan_fwd_chain(d), L.m2d_scan_bwd_chain(d),
+                L.m2d_scan_fwd_cleared(d), L.m2d_scan_fwd_noalloc_need(d))
+
+    def in_a_thread(f):
+        out = []
+        t = threading.Thread(target=lambda: out.append(f()))
+        t.start()
+        t.join()
+        return out[0]
+    want = [in_a_thread(lambda c=c: ask(c)) for c in others]
+    assert len(set(want)) == len(others)
+    for v in "1235":
+        monkeypatch.setenv("M2D_BWD_WARPS", v)
+        for i in range(len(others)):
+            for k in (0, i, 0, i, i):
+                assert ask(others[k]) == want[k]
+    # two threads in step, each with sizes of its own
+    gate, got = threading.Barrier(2), {}
+
+    def turns(k):
+        got[k] = []
+        for _ in range(20):
+            gate.wait(20)
+            got[k].append(ask(others[k]))
+    both = [threading.Thread(target=turns, args=(k,)) for k in (1, 2)]
+    for t in both:
+        t.start()
+    for t in both:
+        t.join()
+    assert got == {k: [want[k]] * 20 for k in (1, 2)}
+
+
 def test_status_word_and_chain_queries(L):
     d = _desc(B=128, H=56, W=56)
     assert L.m2d_scan_fwd_status_offset(ctypes.byref(d)) == 0
