@@ -234,3 +234,61 @@ def test_a_waiting_call_lets_other_threads_run():
     stop.set()
     t.join()
     assert sum(any(a + 0.2 * (b - a) < m < b - 0.2 * (b - a) for m in marks) for a, b in spans) >= 3
+
+
+def _mid_sized():
+    """A batch whose backward runs the batch sweeps with the bands of an image in several CTAs."""
+    shape = (24, 57, 50, 64, 16)
+    inp = inputs.make_inputs(*shape, seed=6)
+    dev = {k: v.cuda() for k, v in inp.items()}
+    d, _ = wc._make_desc(*[dev[k] for k in ORDER])
+    L = _lib.lib()
+    assert L.m2d_scan_bwd_chain(ctypes.byref(d)) == 3
+    record, rows = 24 * 57 * 50 * 4 * 1024, 24 * 8 * 50 * 4 * 1024
+    assert L.m2d_scan_bwd_workspace(ctypes.byref(d)) < record + 2 * rows + 4096      # (the wave kernels' record is wider: 64 rows of 57 columns)
+    return dev
+
+
+@pytest.mark.parametrize("call", [_scan, _block])
+@pytest.mark.parametrize("hook", [DOWN, UP])
+def test_a_chained_batch_backward_raises_before_its_gradients_are_used(call, hook, monkeypatch):
+    monkeypatch.setenv("M2D_TEST_HOOKS", "1")
+    dev = _mid_sized()
+    y, leaves = call(dev, True)
+    want = _grads(y, leaves, dev["gy"])
+    y, leaves = call(dev, True, bwd=hook | REPORT)
+    with pytest.raises(RuntimeError, match="m2d_scan_bwd: a wait between CTAs timed out"):
+        _grads(y, leaves, dev["gy"])
+    y, leaves = call(dev, True)
+    for a, b in zip(_grads(y, leaves, dev["gy"]), want):
+        assert float((a - b).abs().max()) <= 1e-5 * float(b.abs().max())
+    assert _lib.lib().m2d_take_wait_failure() == 0
+
+
+@pytest.mark.parametrize("call", [_scan, _block])
+def test_a_chained_batch_backward_in_a_graph(call):
+    dev = _mid_sized()
+    y, leaves = call(dev, True)
+    want = [y.detach().clone(), *(_grads(y, leaves, dev["gy"]))]
+
+    def run():
+        entry, own = _lib.entry(), [t.detach().requires_grad_() for t in leaves]         # (leaves that no other stream has used)
+        y = entry.scan(*own, False, False, True, 0, 0) if call is _scan else entry.block(*own, False, False, False, True, 0, 0)
+        return [y.detach(), *_grads(y, own, dev["gy"])]
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        for _ in range(2):
+            run()
+    torch.cuda.current_stream().wait_stream(side)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        got = run()
+    for _ in range(2):
+        for t in got:
+            t.fill_(float("nan"))
+        graph.replay()
+        torch.cuda.synchronize()
+        for a, b in zip(got, want):
+            assert float((a - b).abs().max()) <= 1e-5 * float(b.abs().max())
+    assert _lib.lib().m2d_take_wait_failure() == 0
