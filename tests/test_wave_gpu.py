@@ -68,3 +68,36 @@ def test_boundary_rows_are_kept_where_a_later_sweep_needs_them():
     few = L.m2d_scan_fwd_workspace(ctypes.byref(d))
     d.H = 160
     assert L.m2d_scan_fwd_workspace(ctypes.byref(d)) == few
+
+
+def _is_wave_backward(shape, dt):
+    """Whether the backward is planned for the wave kernels, by the size of its workspace (mamba2d_b200/csrc/m2d_scan_bwd.cu)."""
+    B, H, W, E, N = shape
+    d = _lib.ScanDesc()
+    d.struct_bytes = ctypes.sizeof(d)
+    d.dtype = _lib.M2D_F32 if dt == torch.float32 else _lib.M2D_BF16
+    d.B, d.H, d.W, d.E, d.N = shape
+    d.BT_pitch = d.BL_pitch = d.C_pitch = N
+
+    def up(v):
+        return (v + 255) // 256 * 256
+    sums = 0 if dt == torch.float32 else up(4 * (3 * B * H * W * N + 2 * E * N + E))
+    bands, groups = (H + 7) // 8, (E + 15) // 16
+    edge = up(B * ((E + 1) // 2) * (bands if bands > 1 else 0) * W * 32 * 4)
+    return _lib.lib().m2d_scan_bwd_workspace(ctypes.byref(d)) == 256 + sums + 2 * edge + up(B * groups * 8 * bands * (W + 7) * 1024)
+
+
+@pytest.mark.parametrize("shape", [(2, 41, 64, 96, 16), (1, 21, 18, 96, 16), (3, 24, 13, 18, 5)])
+@pytest.mark.parametrize("columns", ["neighbours", "apart", "flag"])
+@pytest.mark.parametrize("kind", ["f32", "bf16"])
+def test_wave_gradients_of_b_and_c_as_columns_of_a_wider_buffer(shape, columns, kind):
+    import test_scan_gpu
+    assert _is_wave_backward(shape, torch.float32 if kind == "f32" else torch.bfloat16)
+    test_scan_gpu.test_gradients_of_b_and_c_as_columns_of_a_wider_buffer(shape, columns, kind)
+
+
+@pytest.mark.parametrize("shape", [(1, 700, 6, 32, 16), (1, 33, 4, 34, 16)])     # 88 bands that one CTA walks; a band each for five
+@pytest.mark.parametrize("dt,tol", [(torch.float32, 1e-4), (torch.bfloat16, 2e-2)])
+def test_wave_backward_of_narrow_maps(shape, dt, tol):
+    assert _is_wave_backward(shape, dt)
+    test_wave_kernels_against_the_oracle(shape, dt, tol, False)
