@@ -313,12 +313,6 @@ __device__ __forceinline__ unsigned begin_pairs(const ScanArgs& a, float4* smem,
 enum StepKind { kInside, kTop, kBorder, kPartial };
 template <int K> struct StepTag { static constexpr int value = K; };
 
-// D of this lane's two channels, in lane nq == 0 only: gy*D and x*D enter the sums over states once.
-template <typename io_t>
-__device__ __forceinline__ float2 lane_D(const ScanArgs& a, const PairLane& ln) {
-    return make_float2(ln.nq == 0 && ln.chv > 0 ? load_D<io_t>(a, ln.ch0) : 0.f, ln.nq == 0 && ln.chv > 1 ? load_D<io_t>(a, ln.ch0 + 1) : 0.f);
-}
-
 // RECORD (the backward's recompute sweep): every fresh state block goes to the state record a.hs, of type rec_t, and d_C is
 // accumulated, and nothing is written to y.  D_lane: D of the channel whose y this lane stores.
 //
