@@ -70,13 +70,6 @@ def test_chained_sweeps_against_the_oracle(shape, chain, dt, tol, reverse):
     _check(shape, chain, dt, tol, reverse)
 
 
-@pytest.mark.parametrize("shape,chain", [((53, 19, 59, 34, 5), 2), ((50, 24, 57, 34, 5), 3), ((22, 20, 52, 100, 8), 2)])
-@pytest.mark.parametrize("reverse", [False, True])
-def test_chained_sweeps_with_a_bf16_record_against_the_oracle(shape, chain, reverse):
-    """Odd and cut last bands, ragged channels and states (scalar loads); vector loads with a ragged last group."""
-    _check(shape, chain, torch.bfloat16, 2e-2, reverse)
-
-
 @pytest.mark.parametrize("hook", [_lib.M2D_SCAN_TEST_WITHHOLD, _lib.M2D_SCAN_TEST_WITHHOLD_UP])
 def test_waits_of_chained_sweeps_give_up(hook, monkeypatch):
     """A band that hands nothing on: the launch ends, says so, and the next one is right."""
