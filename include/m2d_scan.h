@@ -174,6 +174,9 @@ const char *m2d_strerror(int status);
  *
  * What to expect, in bytes per element of x (a map's last band of eight rows, its columns and its channels rounded up):
  *   many images   forward about 1; backward 64, with bf16 I/O 32, for the state record, + 16 states x 12 / E
+ *   mid-sized     (m2d_scan_bwd_chain > 1 for more than a few images) backward 64 whatever the I/O type, for a record of all
+ *                 images, + 16 for boundary rows: 1.73 GB for 8x82x84x384, 1.98 GB for 40x79x122x64; beyond 16 GB in all
+ *                 the plan for one of the other two lines, where that asks for less
  *   few images    forward up to 8 (boundary rows of all bands: 537 MB for one 1024x1024x64 map, 2.1 GB for 2048x2048);
  *                 backward 64 + 16, whatever the I/O type: this record is FP32 (725 MB for 2x200x336x64)
  */

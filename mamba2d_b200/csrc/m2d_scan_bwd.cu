@@ -1,5 +1,6 @@
-// Backward entry point of the wavefront scan: recompute sweep + adjoint sweep in one kernel,
-// followed by a small kernel that casts the fp32 accumulators of the reduced gradients.
+// Backward entry point of the wavefront scan: recompute sweep and adjoint sweep, two kernels in batch mode (one CTA per
+// image and channel group, or a chain of them) and one of the wave kernels, followed with bf16 I/O by a small kernel that casts
+// the fp32 accumulators of the reduced gradients.
 #include <algorithm>
 
 #include "launch.cuh"
@@ -68,7 +69,14 @@ inline BwdLayout bwd_layout(const m2d_scan_desc* d, const BwdPlan& p) {
     return L;
 }
 
-constexpr size_t kLargeScratch = (size_t)4 << 30;
+// Scratch beyond which a call's memory comes before its time, a tenth of the device's.  Three choices that are faster ask for more:
+//   - chained sweeps keep an fp32 record, also where one CTA per image keeps a bf16 one, and boundary rows: 40x56x56x64 bf16 666 MB
+//     for 290, 8x82x84x384 1.73 GB for 0.70.  (With a bf16 record 409 MB and 1.05 GB, and whole training calls of 850 for 872 us and
+//     1863 for 1937; but the weights' gradients differ by 1e-3 then.)
+//   - the batch kernels' record, chained or not, holds every image of the call, the wave kernels' those that are under way:
+//     316x7x9400x71 fp32 106 GB for 11, 40x900x900x64 bf16 172 for 90.
+//   - the wave kernels' record is fp32, with seven columns more than the map has: 5x3470x5x589 bf16 5.2 GB for 1.7.
+constexpr size_t kLargeScratch = (size_t)16 << 30;
 
 inline BwdPlan make_plan_bwd(const m2d_scan_desc* d) {
     // Batch or wave, as in plan_fwd: 1.2 us per step of both sweeps in the wave kernel with two channels per lane (four
@@ -82,7 +90,9 @@ inline BwdPlan make_plan_bwd(const m2d_scan_desc* d) {
         p.wide = d->dtype == M2D_F32 || few_images(d);
         best = (best + states) * kWaveMargin;
     }
+    BwdPlan small = p;                   // few images: the wave kernels, else one CTA per image
     const Plan w = plan_wave(d, 2);
+    if (d->W < 3 || few_images(d)) static_cast<Plan&>(small) = w;
     const double wave = 1.2 * wave_steps(d, w) + 10.0;
     if (wave < best) static_cast<Plan&>(p) = w;
     double adjoint = 0.0, states = 0.0;
@@ -94,14 +104,9 @@ inline BwdPlan make_plan_bwd(const m2d_scan_desc* d) {
         p.wide = true;
     }
     p.scratch = bwd_layout(d, p).total;
-    // The batch kernels' record holds every image of the call, the wave kernels' those that are under way.  Beyond a few GB a call
-    // that the wave kernels are for (few_images) keeps to theirs where it is less than half: 316x7x9400x71 needs 12 GB there and 106
-    // here, most of the device.
-    if (!p.wave && p.scratch > kLargeScratch && few_images(d)) {
-        BwdPlan q = p;
-        static_cast<Plan&>(q) = w;
-        q.scratch = bwd_layout(d, q).total;
-        if (q.scratch < p.scratch / 2) return q;
+    if (p.scratch > kLargeScratch) {
+        small.scratch = bwd_layout(d, small).total;
+        if (small.scratch < p.scratch - p.scratch / 8) return small;
     }
     return p;
 }

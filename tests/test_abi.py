@@ -105,11 +105,26 @@ def test_rings_stay_small_where_some_plan_has_small_ones(L, B, H, W, E, N):
     assert L.m2d_scan_bwd_workspace(ctypes.byref(d)) <= 256 + rings + B * H * W * ((E + 15) // 16) * 1024
 
 
-@pytest.mark.parametrize("B,H,W,E,dtype,limit", [(316, 7, 9400, 71, _lib.M2D_F32, 12e9), (226, 7, 5000, 100, _lib.M2D_BF16, 8e9)])
-def test_large_calls_keep_to_the_record_of_the_images_under_way(L, B, H, W, E, dtype, limit):
-    """A record of all images would take 106 and 58 GB; the wave kernels' lists of images need one each."""
+@pytest.mark.parametrize("B,H,W,E,dtype,limit", [(316, 7, 9400, 71, _lib.M2D_F32, 12e9), (226, 7, 5000, 100, _lib.M2D_BF16, 8e9),
+                                                 (40, 900, 900, 64, _lib.M2D_BF16, 91e9), (40, 700, 700, 64, _lib.M2D_F32, 51e9)])
+def test_large_calls_take_the_plan_of_less_scratch(L, B, H, W, E, dtype, limit):
+    """The wave kernels' lists of images need a record each; one of all images would take 106, 58, 172 and 100 GB."""
     d = ctypes.byref(_desc(B=B, H=H, W=W, E=E, dtype=dtype))
     assert L.m2d_scan_bwd_workspace(d) <= limit and L.m2d_scan_bwd_chain(d) == 1
+
+
+@pytest.mark.parametrize("B,H,W,E,chained,wide", [
+    (128, 28, 28, 128, False, False), (40, 56, 56, 64, True, True), (8, 69, 49, 320, True, True), (8, 82, 84, 384, True, True),
+    (12, 20, 20, 128, False, True), (4, 70, 64, 320, True, True), (10, 62, 63, 128, True, True)])
+def test_type_of_the_state_record(L, B, H, W, E, chained, wide):
+    """bf16 I/O: a large batch keeps its states in bf16 (32 bytes per element), few images and the calls with several CTAs per image in
+    fp32 (64), as fp32 I/O always does.  Beside it at most a boundary row per band of eight for each sweep."""
+    record = B * H * W * ((E + 15) // 16) * 16 * 16 * 4
+    rows = 2 * B * ((H + 7) // 8) * W * ((E + 15) // 16) * 16 * 16 * 4 + 2 * 256
+    for dtype, sums, size in ((_lib.M2D_F32, 0, record), (_lib.M2D_BF16, 4 * (3 * B * H * W * 16 + 2 * E * 16 + E) + 256, record if wide else record // 2)):
+        d = _desc(B=B, H=H, W=W, E=E, dtype=dtype)
+        assert (L.m2d_scan_bwd_chain(ctypes.byref(d)) > 1) == chained
+        assert size + sums - 256 <= L.m2d_scan_bwd_workspace(ctypes.byref(d)) <= size + sums + rows + 512
 
 
 def test_plans_do_not_depend_on_the_environment(L, monkeypatch):
