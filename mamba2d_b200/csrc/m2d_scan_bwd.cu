@@ -14,10 +14,10 @@ namespace m2d {
 //   acc      bf16 I/O only: fp32 accumulators 3 x [B*H*W][N] | 2 x [E][N] | [E], zeroed before the
 //            main kernel (with the status word, in one memset) and cast by a second kernel.  With fp32 I/O
 //            the kernel accumulates straight into the caller's (zeroed) gradient tensors and this region is empty.
-//   edge     batch: per-CTA band-boundary ring, ctas*W KiB (only if nbands > 1); wave: the boundary rows
-//            of the recompute sweep (h, downwards) and of the adjoint sweep (pT, upwards)
-//   hs       state record written by the recompute sweep: batch B*groups*H*W KiB (half with bf16 I/O), wave
-//            512*C bytes per (list, warp, band, step)
+//   edge     batch: per-CTA band-boundary ring, ctas*W KiB (only if nbands > 1); wave and chained batch sweeps: the
+//            boundary rows of the recompute sweep (h, downwards) and of the adjoint sweep (pT, upwards)
+//   hs       state record written by the recompute sweep: batch, chained or not, B*groups*H*W KiB (half where it is
+//            bf16: BwdPlan::wide), wave 512*C bytes per (list, warp, band, step)
 struct BwdLayout {
     size_t edge, hs, acc, acc_bytes, total;
 };
@@ -28,10 +28,13 @@ struct BwdPlan : Plan {
     bool wide;
 };
 
-// With bf16 I/O the batch kernels keep the states of a large batch in bf16, which halves the traffic that the recompute sweep
-// waits for, and those of a few images in fp32, as the wave kernels do: the record is small then, and the gradients are
-// those of the unrounded states.  Few: where a wave launch takes less time than one CTA per image and 32 channels, with up to
-// six rows in flight each and twelve on an SM.
+// With bf16 I/O the batch kernels with one CTA per image keep the states of a large batch in bf16, which halves the traffic that
+// the recompute sweep waits for, and those of a few images in fp32, as the wave kernels and the chained sweeps do: the gradients
+// are then those of the unrounded states.
+//
+// This line decides what a call's gradients are, so it stays where it was, whatever today's kernels take: "few" is where a wave
+// launch comes to less time than one CTA per image and 32 channels with up to six rows in flight each and twelve on an SM.  The
+// times per step are those of that division of the work.
 inline bool few_images(const m2d_scan_desc* d) {
     const int sms = sm_count(), g = (d->E - 1) / 32 + 1;
     double best = -1.0, time = 0.0;
@@ -245,7 +248,7 @@ static int launch_bwd(const m2d_scan_desc* d, const BwdPlan& pl, bool vec, cudaS
     // (a kernel by the type of its record, its kind of loads and whether its CTAs are chained)
     auto pick = [&](auto kernel) -> SweepKernel {
         auto loads = [&](auto rec, auto chain) { return vec ? kernel(rec, std::true_type{}, chain) : kernel(rec, std::false_type{}, chain); };
-        if (pl.chain > 1) return loads(float{}, std::true_type{});           // (a chain has few images: few_images)
+        if (pl.chain > 1) return loads(float{}, std::true_type{});           // (fp32, whatever few_images says: kLargeScratch)
         return pl.wide || sizeof(io_t) == 4 ? loads(float{}, std::false_type{}) : loads(io_t{}, std::false_type{});
     };
     const BwdLayout L = bwd_layout(d, pl);

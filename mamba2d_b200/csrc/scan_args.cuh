@@ -36,13 +36,13 @@ struct ScanArgs {
     long long pBT, pBL, pC;   // pixel pitch (elements) of BT, BL, C
     void* y;
     int dir;                  // +1: scan from the top-left corner; -1: from the bottom-right one (same memory, walked backwards)
-    float4* ring;             // batch kernels: per-CTA band-boundary ring, [cta][W][4][32] float4
+    float4* ring;             // batch kernels: per-CTA band-boundary ring, [cta][W][2][32] float4
     int Rb, nbands;
-    // ---- wave kernels: CTA c of a chain of `chain` CTAs owns the bands q = c, c + chain, ... of its
-    // images; the last row of band q reaches band q+1 through `bnd`
+    // ---- wave kernels and chained batch sweeps: CTA c of a chain of `chain` CTAs owns the bands q = c, c + chain, ... of
+    // its images; the last row of band q reaches band q+1 through `bnd`
     int chain;                // 1 = one CTA per image
-    float4* bnd;              // boundary rows, see wave_fwd.cuh
-    int bnd_rows;             // rows kept per (chain, channel group): one per band, or two in turn
+    float4* bnd;              // boundary rows, see wave_fwd.cuh; chained batch sweeps: [image][group][band][W][2][32] float4
+    int bnd_rows;             // wave kernels: rows kept per (chain, channel group), one per band or two in turn
     int* status;              // nonzero if a wait for a boundary row gave up (results are then invalid); never null
     int* host_flag;           // the same news in host memory, where the next call sees it without synchronising; may be null
     int wait_limit;           // polls before such a wait gives up
@@ -60,7 +60,7 @@ struct ScanArgs {
     float *accBT, *accBL, *accC;   // [B*H*W] rows of N values at a pitch of acc_pitch
     int acc_pitch;
     int acc_vec;                   // wave kernel: rows of accBT, accBL, accC take 16-byte accesses
-    float4* bnd_up;                // wave kernel: boundary rows of the adjoint sweep
+    float4* bnd_up;                // as bnd, for the adjoint sweep
     float *accAT, *accAL;          // [E][N]
     float* accD;                   // [E]
     void *d_x, *d_dT, *d_dL;

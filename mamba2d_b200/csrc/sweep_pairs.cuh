@@ -24,7 +24,7 @@
 // Against one row of 32 channels per warp, a lane 4 x 4 of it (us, kernel times, before / now): 128x56x56x64 fp32 forward
 // 364 / 312, backward 1400 / 507 + 684 (its two sweeps are kernels of their own now); 128x28x28x128 bf16 190 / 171 and
 // 656 / 183 + 402; 128x14x14x320 bf16 129 / 121 and 403 / 137 + 252; 128x7x7x512 fp32 64 / 52 and 199 / 63 + 116.  Instructions
-// per 512 states (56x56x64 fp32): forward 224 -> 202, both sweeps of the backward 803 -> 232 + 500; wavefronts of the
+// per 512 states (56x56x64 fp32): forward 224 -> 189, both sweeps of the backward 803 -> 217 + 521; wavefronts of the
 // shared-memory pipe, which was half busy, 250 -> 56 + 152.  What bounds them now: the forward and the adjoint the latency of
 // a warp's instructions at 16 warps per SM (128 registers; an instruction every 2.0 and 1.7 cycles of a scheduler), and
 // that 512 CTAs put four on some SMs and three on others; the recompute sweep in fp32 the writing of the record (2.5 GB
