@@ -50,8 +50,8 @@ BYTES = {"f32": 4, "bf16": 2}
 
 # DRAM bytes (read + write) of the backward's two kernels, once each, from an ncu capture of this same
 # workload; see profiles/ for the capture summaries.  None = not captured for that dtype.
-NCU_TRAFFIC = {"f32": 5.54e9, "bf16": None}
-NCU_TRAFFIC_FROM = "c65fd61"  # the commit whose kernels were captured
+NCU_TRAFFIC = {"f32": 5.57e9, "bf16": 3.04e9}
+NCU_TRAFFIC_FROM = {"f32": "9a1a1ed", "bf16": "fe09dc1"}  # the commit whose kernels were captured
 
 
 def fwd_bytes(D, HW, s, B=BATCH, N=NSTATE):
@@ -269,7 +269,7 @@ def summarise(dtype, r, world, steps):
         "roofline": {"bound": "hbm", "kernel": "m2d_bwd_states_kernel + m2d_bwd_kernel @ D=64,H=W=56,B=128", "achieved": dom_bytes / dom["bwd_ms"] / 1e6,
                      "peak": peak, "unit": "GB/s", "frac": dom_bytes / dom["bwd_ms"] / 1e6 / peak,
                      "peak_kind": peak_kind, "algorithmic_bytes": dom_bytes, "ms": dom["bwd_ms"],
-                     "traffic": NCU_TRAFFIC[dtype], "traffic_from_commit": NCU_TRAFFIC_FROM if NCU_TRAFFIC[dtype] else None},
+                     "traffic": NCU_TRAFFIC[dtype], "traffic_from_commit": NCU_TRAFFIC_FROM[dtype] if NCU_TRAFFIC[dtype] else None},
         "roofline_step": {"bound": "hbm", "achieved": step_bytes / step_kernel_ms / 1e6, "peak": peak, "unit": "GB/s",
                           "frac": step_bytes / step_kernel_ms / 1e6 / peak, "algorithmic_bytes": step_bytes},
         "per_shape": per,
