@@ -195,7 +195,7 @@ uint64_t m2d_scan_fwd_cleared(const m2d_scan_desc *desc);
 int m2d_scan_fwd(const m2d_scan_desc *desc, void *stream);
 
 /*
- * With few images on a large map several CTAs share an image and wait on one another through
+ * With few images on a large map, in the backward with mid-sized batches too, several CTAs share an image and wait on one another through
  * global memory (inside a CTA the row-warps meet at block barriers with uniform trip counts).  Every
  * wait between CTAs is bounded.  If one ever gives up (it cannot when the kernel has the GPU
  * to itself), all later waits return at once, the kernel terminates normally and leaves a nonzero

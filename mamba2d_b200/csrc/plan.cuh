@@ -182,7 +182,10 @@ inline double pair_chain_time(const m2d_scan_desc* d, const Plan& p, PairKernel 
 constexpr double kChainShare = 0.80;
 // ... and to less than this share of one CTA per image, whose estimate is high by about as much as this one is low.  Backward, us,
 // one CTA per image / chained, without clearing: 20x45x31x192 bf16 294 / 332 (0.87), 32x56x56x64 fp32 424 / 414 (0.73),
-// 48x64x80x64 bf16 947 / 809 (0.65), 40x100x120x64 fp32 2258 / 1797 (0.63).
+// 48x64x80x64 bf16 947 / 809 (0.65), 40x100x120x64 fp32 2258 / 1797 (0.63).  What the two lines leave out is that a call waits for a
+// chained scan before it returns: 20 ... 40 us of the host's lead.  Whole training calls at the line, back to back, not chained / chained: 8x39x34x320 fp32 573 / 544,
+// 47x40x35x64 517 / 508, 4x36x53x320 535 / 487, 15x40x63x96 bf16 588 / 547, 14x39x42x192 bf16 573 / 563, 55x49x30x64 bf16 535 / 555, 23x58x32x128
+// bf16 592 / 615; well below it 8x69x49x320 bf16 1061 / 906, 28x89x102x96 bf16 2639 / 2357.  (The two that lose would keep their states in bf16.)
 constexpr double kChainShareOfBatch = 0.70;
 
 // Bytes of the rings that carry a band's last row to the next band.
